@@ -111,16 +111,20 @@ IDL_API int idl_context_synchronize(idl_context* ctx);
 /* Bytes of device workspace currently held by the context. */
 IDL_API int idl_context_workspace_bytes(idl_context* ctx, int64_t* bytes_out);
 
-/* Propagation schedule from scratch (reference semantics): the first
+/* Propagation schedule from scratch (reference semantics).
+ * IDL_SCHEDULE_DIRECT (the default): the passes are not run; the fixed point
+ * they reach is read off the exact diagram, and run only where that is not
+ * decided (resolve.cu).  Any other value runs the passes: the first
  * `dense_rounds` tile rounds (one HBM round trip per round of several passes,
  * over every tile that can change; see idl_context_set_tile), the rest in the persistent
  * sparse kernel; 0 = sparse kernel only, < 0 = tile rounds to convergence.
  * A continued propagation (an incremental object's insert using this context)
- * runs in the sparse kernel, or with dense_rounds < 0 as tile rounds starting
- * from the tiles around the new seeds.  Results do not depend on it, only the
- * time does.  Default 3 (the fastest at 4096 x 4096 with 200 000 uniform seeds;
- * integer_delauney_b200.autotune picks per input class).  No counterpart in
+ * runs in the sparse kernel, or with dense_rounds < 0 (IDL_SCHEDULE_DIRECT
+ * excepted) as tile rounds starting from the tiles around the new seeds.
+ * Results do not depend on it, only the time does
+ * (integer_delauney_b200.autotune picks per input class).  No counterpart in
  * the reference (its schedule is one full pass per launch). */
+#define IDL_SCHEDULE_DIRECT (-1073741824)
 IDL_API int idl_context_set_schedule(idl_context* ctx, int dense_rounds);
 
 /* Tile shape of a from-scratch propagation's tile rounds (reference

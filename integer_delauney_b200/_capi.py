@@ -29,6 +29,9 @@ MODE_NUMPY = 1
 MODE_EXACT = 2
 MODES = {"reference": MODE_REFERENCE, "numpy": MODE_NUMPY, "exact": MODE_EXACT}
 
+# propagation schedule (idl_context_set_schedule): the default, no passes run
+SCHEDULE_DIRECT = -1073741824
+
 AUTO_BORDER_PADDING = -1
 DEFAULT_BORDER_PADDING = 16
 

@@ -1,13 +1,14 @@
 """Autotuning of the propagation schedule and tile shape.
 
-From scratch, the reference-semantics propagation runs its first passes as
-tile rounds (several passes per HBM round trip over every tile that can still
-change) and hands the tail to the persistent sparse kernel.  Two knobs decide
-its speed, never its result:
+From scratch, the reference-semantics propagation by default reads its fixed
+point off the exact diagram (SCHEDULE_DIRECT); the other schedules run its
+passes: the first ones as tile rounds (several passes per HBM round trip over
+every tile that can still change), the tail in the persistent sparse kernel.
+Two knobs decide its speed, never its result:
 
-* the schedule (idl_context_set_schedule): how many tile rounds run before the
-  sparse kernel takes over (0 = sparse kernel only, -1 = tile rounds to
-  convergence);
+* the schedule (idl_context_set_schedule): SCHEDULE_DIRECT, or how many tile
+  rounds run before the sparse kernel takes over (0 = sparse kernel only, -1 =
+  tile rounds to convergence);
 * the tile shape (idl_context_set_tile), one of twelve:
   0-3 are register tile rounds (inner tile / passes per round trip:
   48 x 48 / 8, 48 x 112 / 8, 56 x 56 / 4, 40 x 104 / 12), one launch per
@@ -34,7 +35,7 @@ import numpy as np
 
 from . import _capi
 
-SCHEDULES = (0, 1, 2, 3, 4, 6, -1)
+SCHEDULES = (_capi.SCHEDULE_DIRECT, 0, 1, 2, 3, 4, 6, -1)
 _cache: dict[tuple, tuple[int, int]] = {}
 # the timings of the last tuning run: {(schedule, shape): best ms of the repeats}
 last_report: dict[tuple[int, int], float] = {}
@@ -61,11 +62,11 @@ def input_class(width: int, height: int, n_seeds: int, occ: float = 1.0) -> tupl
 
 
 def candidates(n_shapes: int, schedules: Iterable[int] = SCHEDULES) -> list[tuple[int, int]]:
-    """Every (schedule, shape) pair; the sparse-only schedule has no tile rounds,
-    so it is tried once."""
+    """Every (schedule, shape) pair; the schedules with no tile rounds are tried
+    once."""
     out = []
     for sched in schedules:
-        for shape in ([0] if sched == 0 else range(n_shapes)):
+        for shape in ([0] if sched in (0, _capi.SCHEDULE_DIRECT) else range(n_shapes)):
             out.append((int(sched), int(shape)))
     return out
 

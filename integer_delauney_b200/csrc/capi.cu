@@ -230,10 +230,48 @@ struct StageTimer {
     }
 };
 
+// Stage (a) by running the passes, from the sorted seeds of C.pos.
+int64_t run_passes(Context& C, int mode, const Canvas& cv, int64_t n)
+{
+    init_labels(C, cv, C.pos.as<uint32_t>(), n);
+    return propagate(C, mode, cv, C.pos.as<uint32_t>(), n);
+}
+
+// Stage (a) from scratch into C.lab[0].  Returns true if the labels come from
+// resolve_exact: the caller has to look at finish_resolved once the scalars
+// have been read back.  Otherwise *passes (may be nullptr) takes the pass count.
+bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, bool want_passes, int64_t* passes = nullptr)
+{
+    if (mode == IDL_MODE_REFERENCE && C.direct()) {
+        C.prof.pass_ns.clear();
+        C.prof.pass_tiles.clear();
+        propagate_exact(C, cv, C.pos.as<uint32_t>(), n);
+        resolve_exact(C, cv, C.pos.as<uint32_t>(), n, want_passes);
+        return true;
+    }
+    int64_t p = 0;
+    if (mode == IDL_MODE_EXACT) propagate_exact(C, cv, C.pos.as<uint32_t>(), n);
+    else p = run_passes(C, mode, cv, n);
+    if (passes) *passes = p;
+    return false;
+}
+
+// After a read-back of the scalars: whether resolve_exact's labels stand (and
+// its pass count, where wanted, is known).
+bool finish_resolved(Context& C, bool want_passes, int64_t* passes = nullptr)
+{
+    if (C.host_sc->resolve_fail) return false;
+    if (!want_passes) return true;
+    const int64_t p = resolved_passes(*C.host_sc);
+    C.prof.passes = p;
+    if (passes) *passes = p;
+    return p >= 0;
+}
+
 // Run stages (a) (b) (d) with seeds already in C.seeds_in.  Leaves labels in
 // C.lab[0], triangles in C.tris, pixel ids in C.tgrid; returns triangle count.
 int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgrid_host_or_dev, bool vgrid_on_host,
-                        int P, int mode, float* timings, int64_t* passes_out, Canvas& cv_out)
+                        int P, int mode, float* timings, Canvas& cv_out)
 {
     const Canvas cv = make_canvas(W + 2 * P, H + 2 * P);
     cv_out = cv;
@@ -246,14 +284,9 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     C.mark(PM_SEEDS);
 
     StageTimer T(C, timings != nullptr);
-    int64_t passes = 0;
+    bool resolved = false;
     if (P > 0 || !vgrid_host_or_dev) {
-        if (mode == IDL_MODE_EXACT) {
-            propagate_exact(C, cv, C.pos.as<uint32_t>(), n);
-        } else {
-            init_labels(C, cv, C.pos.as<uint32_t>(), n);
-            passes = propagate(C, mode, cv, C.pos.as<uint32_t>(), n);
-        }
+        resolved = start_labels(C, mode, cv, n, C.prof.enabled);
     } else {
         const size_t gbytes = (size_t)W * H * 2 * sizeof(int32_t);
         C.vgrid.ensure(gbytes);
@@ -268,7 +301,6 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         C.fetch_scalars();
         if (C.host_sc->err_label) invalid("voronoi_grid seed ids must lie in [-1, number of seeds)");
     }
-    if (passes_out) *passes_out = passes;
     C.mark(PM_PROPAGATE);
 
     T.mark(0);
@@ -276,6 +308,14 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     // enumeration and canonical ranking (the reference's thrust sort/unique)
     detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, P,
                      T.on ? C.timing.ev[1] : nullptr);
+    if (resolved && !finish_resolved(C, C.prof.enabled)) {
+        // the exact diagram did not decide the fixed point: run the passes
+        run_passes(C, mode, cv, n);
+        C.mark(PM_PROPAGATE);
+        T.mark(0);
+        detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, P,
+                         T.on ? C.timing.ev[1] : nullptr);
+    }
     T.mark(2);
     C.mark(PM_DEDUP);
     // the triangle count came back with detection's own read-back (ranking
@@ -519,20 +559,23 @@ int idl_voronoi(idl_context* ctx, int width, int height, const int32_t* seeds_xy
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
     sort_seeds_device(C, width, height, n_seeds, 0);
     int64_t passes = 0;
-    if (mode == IDL_MODE_EXACT) {
-        propagate_exact(C, cv, C.pos.as<uint32_t>(), n_seeds);
-    } else {
-        init_labels(C, cv, C.pos.as<uint32_t>(), n_seeds);
-        passes = propagate(C, mode, cv, C.pos.as<uint32_t>(), n_seeds);
-    }
+    const bool resolved = start_labels(C, mode, cv, n_seeds, passes_out != nullptr, &passes);
     const size_t bytes = (size_t)width * height * 2 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
-    dim3 gr(ceil_div(width, 256), height);
-    k_compose2<<<gr, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, width, height, C.pos.as<uint32_t>(),
-                                         C.outgrid.as<int32_t>());
-    IDL_LAUNCH();
-    IDL_CUDA(cudaMemcpyAsync(grid_out, C.outgrid.ptr, bytes, cudaMemcpyDeviceToHost, C.stream));
-    IDL_CUDA(cudaStreamSynchronize(C.stream));
+    auto deliver = [&] {
+        dim3 gr(ceil_div(width, 256), height);
+        k_compose2<<<gr, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, width, height, C.pos.as<uint32_t>(),
+                                             C.outgrid.as<int32_t>());
+        IDL_LAUNCH();
+        IDL_CUDA(cudaMemcpyAsync(grid_out, C.outgrid.ptr, bytes, cudaMemcpyDeviceToHost, C.stream));
+        if (resolved) C.fetch_scalars();
+        else IDL_CUDA(cudaStreamSynchronize(C.stream));
+    };
+    deliver();
+    if (resolved && !finish_resolved(C, passes_out != nullptr, &passes)) {
+        passes = run_passes(C, mode, cv, n_seeds);
+        deliver();
+    }
     if (passes_out) *passes_out = passes;
     IDL_API_END
 }
@@ -554,8 +597,7 @@ int idl_triangulate(idl_context* ctx, int width, int height, const int32_t* seed
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
     Canvas cv;
     const bool from_grid = (P == 0 && voronoi_grid != nullptr);
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, voronoi_grid, true, P, mode, timings_out,
-                                       nullptr, cv);
+    const int64_t nt = run_triangulate(C, width, height, n_seeds, voronoi_grid, true, P, mode, timings_out, cv);
     const size_t bytes = (size_t)width * height * 3 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
     compose_triangulation(C, cv, width, height, P, from_grid, C.outgrid.as<int32_t>());
@@ -623,7 +665,7 @@ int idl_triangulate_device(idl_context* ctx, int width, int height, const int32_
     const int P = resolve_padding(border_padding);
     upload_seeds(C, d_seeds_xy, n_seeds, cudaMemcpyDeviceToDevice);
     Canvas cv;
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, false, P, mode, nullptr, nullptr, cv);
+    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, false, P, mode, nullptr, cv);
     compose_triangulation(C, cv, width, height, P, false, d_grid_out);
     if (n_triangles_out) {
         IDL_CUDA(cudaStreamSynchronize(C.stream));

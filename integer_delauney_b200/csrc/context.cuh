@@ -101,7 +101,15 @@ struct Scalars {
     int32_t n_big;            // tall triangles the raster hands to its block-per-triangle pass
     int32_t n_handoff;        // micro-tiles the last tile round hands to the persistent kernel
     int32_t tile_remaining;   // tiles listed for the tile round after the last one launched
+    // resolve.cu, cleared together (RESOLVE_SCALARS values from n_roots on)
+    int32_t n_roots, n_more;  // suspects: the roots, and those that hang on them
+    int32_t n_open;           // suspects left to the window kernel
+    int32_t resolve_fail;     // the fixed point was not decided: iterate instead
+    int32_t arrive_max;       // latest last change known exactly (passes done by then)
+    int32_t late_max;         // latest upper bound of a decided suspect's last change
+    int32_t sus_far;          // longest owner distance among the n_more suspects
 };
+constexpr int RESOLVE_SCALARS = 7;
 
 struct Timing {
     cudaEvent_t ev[8] = {};
@@ -156,8 +164,12 @@ struct Context {
     DevBuf cellbits;      // cell-list tile rounds: three last-pass change bitmaps, in rotation
     DevBuf exact_dy;      // exact mode: row distance to each cell's column-nearest seed
     DevBuf exact_rmin;    // exact mode: per row, smallest squared row distance of each 32-column block
+    DevBuf sus_bits, sus_list;  // resolve.cu: suspect bits, suspect list with results and open indices
     int32_t stamp_epoch = 0;
-    int dense_rounds = 3;  // propagation schedule from scratch (propagate.cu; idl_context_set_schedule)
+    // propagation schedule from scratch (resolve.cu, propagate.cu; idl_context_set_schedule)
+    int dense_rounds = IDL_SCHEDULE_DIRECT;
+    bool direct() const { return dense_rounds == IDL_SCHEDULE_DIRECT; }
+    int rounds_schedule() const { return direct() ? 3 : dense_rounds; }   // when the passes are run after all
     int key_tile = 9;      // tile shape of the owner-key tile round (propagate.cu; idl_context_set_tile)
     // The persistent kernel advances several passes per grid barrier once its
     // work list holds at most this many micro-tiles (sparse_jacobi.cu; 0:
@@ -216,7 +228,8 @@ struct Context {
     void each_buf(F&& f)
     {
         DevBuf* all[] = {&seeds_in, &xs, &ys, &pos, &bitmap, &scan_a, &scan_b, &scan_c, &lab[0], &lab[1],
-                         &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &exact_dy, &exact_rmin, &hkeys,
+                         &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
+                         &exact_dy, &exact_rmin, &sus_bits, &sus_list, &hkeys,
                          &ukeys, &uvals, &cnt, &off, &fill, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
                          &batch_img, &batch_seed_img, &batch_rows, &batch_sid, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
@@ -334,6 +347,22 @@ void grid_barrier_selftest(Context& C, int missing_arrivals, unsigned spin_limit
 // for the n (x, y)-sorted seeds `pos` of the canvas; labels into C.lab[0]
 // (C.lab[1] is scratch).
 void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n);
+
+// Turns the exact labels propagate_exact left in C.lab[0] (and the column
+// plane in C.lab[1]) into the reference semantics' fixed point from scratch
+// (resolve.cu).  Reads nothing back: C.sc()->resolve_fail, with the scalars'
+// next read-back, tells whether the passes have to be run instead.  `passes`:
+// also what resolved_passes needs.  Batch atlas: `bounds` is each image's
+// padded canvas (x0, y0, x1, y1), `seed_img` the image of each seed.
+void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes,
+                   const int4* bounds = nullptr, const int32_t* seed_img = nullptr);
+// The iteration's pass count from the scalars read back after resolve_exact
+// with `passes`, or -1 if they do not determine it.
+inline int64_t resolved_passes(const Scalars& s)
+{
+    const bool sure = !s.resolve_fail && s.late_max <= s.arrive_max && (s.n_more == 0 || s.sus_far < s.arrive_max);
+    return sure ? (int64_t)s.arrive_max + 1 : -1;
+}
 
 // Reserve a range of per-item stamp values for `steps` steps (propagate.cu).
 int32_t claim_stamps(Context& C, int n_items, int64_t steps);

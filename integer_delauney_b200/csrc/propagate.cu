@@ -1205,20 +1205,21 @@ int64_t propagate_rounds(Context& C, int mode, const Canvas& cv, const uint32_t*
                          int64_t n_new, bool keys, const uint32_t* start_pos, int64_t n_start)
 {
     // Reference semantics.  A continued propagation (seed_pos) is local from
-    // its first pass: the sparse kernel alone, or with C.dense_rounds < 0 tile
+    // its first pass: the sparse kernel alone, or with a schedule < 0 tile
     // rounds starting from the tiles around the new seeds (plain launches, no
     // device-wide persistent grid, so streams of other work overlap them).
     // From scratch, the first passes change most of the canvas, which the
     // tile rounds (several passes per HBM round trip, no per-pass bookkeeping)
     // do best; once the changes thin out, the sparse kernel takes over the
-    // tail, whose single passes touch few cells.  C.dense_rounds sets the
+    // tail, whose single passes touch few cells.  The schedule sets the
     // switch (0: sparse only, < 0: tile rounds to convergence).
-    const bool seeded_rounds = mode == IDL_MODE_REFERENCE && seed_pos && C.dense_rounds < 0;
-    const bool hybrid = mode == IDL_MODE_REFERENCE && !seed_pos && C.dense_rounds != 0;
+    const int schedule = C.rounds_schedule();
+    const bool seeded_rounds = mode == IDL_MODE_REFERENCE && seed_pos && schedule < 0;
+    const bool hybrid = mode == IDL_MODE_REFERENCE && !seed_pos && schedule != 0;
     if (mode == IDL_MODE_REFERENCE && !hybrid && !seeded_rounds)
         return propagate_sparse(C, cv, pos, seed_pos, n_new, keys);
     if (seed_pos && n_new == 0) return 0;
-    const int64_t round_limit = hybrid && C.dense_rounds > 0 ? C.dense_rounds : -1;
+    const int64_t round_limit = hybrid && schedule > 0 ? schedule : -1;
     const int tile = std::min(std::max(C.key_tile, 0), key_tile_shapes() - 1);
     const bool cells = keys && tile >= 2 * N_KEY_SHAPES;
     const int base_shape = cells ? 0 : tile % N_KEY_SHAPES;
