@@ -414,11 +414,13 @@ struct BatchPlan {
 };
 
 // Exact-semantics labels of every image into C.lab[0] (the atlas's walls
-// stay); C.lab[1] and C.exact_dy are scratch.
-void exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
+// stay), the column pass's into C.lab[1]; C.exact_dy is scratch.  Returns the
+// images' padded canvases (x0, y0, x1, y1) on the device.
+const int4* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
 {
     const int n_images = (int)pl.imgs.size();
     std::vector<XImg> xi(n_images);
+    std::vector<int4> bounds(n_images);
     std::vector<int32_t> colimg, rowimg;
     int max_wp = 0, max_hp = 0;
     for (int i = 0; i < n_images; ++i) {
@@ -432,24 +434,27 @@ void exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
         m.row_off = (int)rowimg.size();
         m.s0 = b.seed_off;
         m.s1 = i + 1 < n_images ? pl.imgs[i + 1].seed_off : pl.n_seeds;
+        bounds[i] = make_int4(m.ox, m.oy, m.ox + m.Wp, m.oy + m.Hp);
         colimg.insert(colimg.end(), (size_t)m.Wp + 1, i);
         rowimg.insert(rowimg.end(), (size_t)m.Hp, i);
         max_wp = std::max(max_wp, m.Wp);
         max_hp = std::max(max_hp, m.Hp);
     }
     const int64_t n_cols = (int64_t)colimg.size(), n_rows = (int64_t)rowimg.size();
-    C.batch_ximg.ensure(xi.size() * sizeof(XImg));
+    C.batch_ximg.ensure(xi.size() * (sizeof(int4) + sizeof(XImg)));
+    int4* d_bounds = C.batch_ximg.as<int4>();
+    XImg* d_xi = reinterpret_cast<XImg*>(d_bounds + n_images);
+    IDL_CUDA(cudaMemcpyAsync(d_bounds, bounds.data(), bounds.size() * sizeof(int4), cudaMemcpyHostToDevice, C.stream));
     C.batch_colimg.ensure((size_t)n_cols * 4);
     C.batch_rowimg.ensure((size_t)n_rows * 4);
     C.counts.ensure((size_t)n_cols * 4);
     C.exact_dy.ensure((size_t)cv.pitch * cv.Hd * 4);
-    IDL_CUDA(cudaMemcpyAsync(C.batch_ximg.ptr, xi.data(), xi.size() * sizeof(XImg), cudaMemcpyHostToDevice,
+    IDL_CUDA(cudaMemcpyAsync(d_xi, xi.data(), xi.size() * sizeof(XImg), cudaMemcpyHostToDevice,
                              C.stream));
     IDL_CUDA(cudaMemcpyAsync(C.batch_colimg.ptr, colimg.data(), (size_t)n_cols * 4, cudaMemcpyHostToDevice,
                              C.stream));
     IDL_CUDA(cudaMemcpyAsync(C.batch_rowimg.ptr, rowimg.data(), (size_t)n_rows * 4, cudaMemcpyHostToDevice,
                              C.stream));
-    const XImg* d_xi = C.batch_ximg.as<XImg>();
     const int32_t* d_colimg = C.batch_colimg.as<int32_t>();
     int32_t* cs = C.counts.as<int32_t>();
     const uint32_t* pos = C.pos.as<uint32_t>();
@@ -475,6 +480,7 @@ void exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
             C.lab[0].as<int32_t>());
     }
     IDL_LAUNCH();
+    return d_bounds;
 }
 
 void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, int64_t* tri_counts,
@@ -540,24 +546,33 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
                                            C.ys.as<int32_t>(), C.pos.as<uint32_t>(), C.batch_sid.as<int32_t>());
     IDL_LAUNCH();
 
-    // atlas planes: walls everywhere, each image's padded canvas open, seeds in
     const Canvas cv{pl.AW, pl.AH, (pl.AW + 31) / 32 * 32};
     const size_t plane = (size_t)cv.pitch * cv.Hd * 4;
     C.lab[0].ensure(plane);
     C.lab[1].ensure(plane);
-    IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
-    IDL_CUDA(cudaMemsetAsync(C.lab[1].ptr, 0xFE, plane, C.stream));
-    k_b_open<<<dim3(64, n_images), 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), C.lab[1].as<int32_t>(), cv.pitch,
-                                                       d_imgs, P);
-    IDL_LAUNCH();
     mark(1);
-    if (mode == IDL_MODE_EXACT) {
-        exact_atlas(C, pl, P, cv);
-    } else {
+    auto run_passes = [&] {
+        // atlas planes: walls everywhere, each image's padded canvas open, seeds in
+        IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
+        IDL_CUDA(cudaMemsetAsync(C.lab[1].ptr, 0xFE, plane, C.stream));
+        k_b_open<<<dim3(64, n_images), 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), C.lab[1].as<int32_t>(), cv.pitch,
+                                                           d_imgs, P);
+        IDL_LAUNCH();
         k_b_seeds<<<nblk(n), 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), C.lab[1].as<int32_t>(), cv.pitch,
                                                 C.pos.as<uint32_t>(), n);
         IDL_LAUNCH();
         propagate(C, IDL_MODE_REFERENCE, cv, C.pos.as<uint32_t>(), n);
+    };
+    const bool direct = mode == IDL_MODE_REFERENCE && C.direct();
+    if (mode == IDL_MODE_EXACT || direct) {
+        // the exact passes write every cell of every image; the walls between
+        // them are read by the block rule (and by resolve_exact) in plane 0 only
+        IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
+        const int4* bounds = exact_atlas(C, pl, P, cv);
+        if (direct)
+            resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, bounds, C.batch_sid.as<int32_t>());
+    } else {
+        run_passes();
     }
     mark(2);
     auto bp = std::make_shared<BatchPlan>();
@@ -567,8 +582,20 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     bp->n_seeds = n;
     bp->exact = mode == IDL_MODE_EXACT;
     C.batch_plan = bp;
-    if (labels_only) return;
+    if (labels_only) {
+        if (direct) {
+            C.fetch_scalars();
+            if (C.host_sc->resolve_fail) run_passes();
+        }
+        return;
+    }
     detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, 0, timings ? ev[3] : nullptr);
+    if (direct && C.host_sc->resolve_fail) {
+        // the exact diagram did not decide some image's fixed point: run the passes
+        run_passes();
+        mark(2);
+        detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, 0, timings ? ev[3] : nullptr);
+    }
 
     // per-image counts, offsets and windows; raster; compose
     int32_t* cnt = C.batch_stats.as<int32_t>();

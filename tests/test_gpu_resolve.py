@@ -77,3 +77,30 @@ def test_fixed_point_and_passes(ctx, kind, W, H):
         got, passes = _voronoi(ctx, W, H, seeds)
         np.testing.assert_array_equal(got, want, err_msg=f"{kind} {W}x{H} seed {seed}")
         assert passes == want_passes, f"{kind} {W}x{H} seed {seed}"
+
+
+def test_batch_labels_equal_single_images(ctx):
+    """The atlas form: images of mixed layouts beside each other, image sides
+    off every tile boundary, each equal to its own single-image diagram; then
+    the same batch through the passes."""
+    images = []
+    for i, (kind, W, H) in enumerate([("circle", 131, 97), ("uniform", 64, 200), ("lattice", 97, 61),
+                                      ("clustered", 180, 141), ("disc", 90, 120), ("sparse", 211, 57),
+                                      ("line", 65, 129), ("uniform", 1, 1), ("dense", 33, 47)]):
+        images.append((W, H, _layout(kind, W, H, 1 + i % 3) if W > 1 else np.zeros((1, 2), np.int32)))
+    dims = np.array([(w, h) for w, h, _ in images], np.int32)
+    counts = np.array([len(s) for _, _, s in images], np.int64)
+    seeds = np.ascontiguousarray(np.concatenate([s for _, _, s in images]).astype(np.int32))
+    lib = _capi.load()
+    for schedule in (None, 3):
+        if schedule is not None:
+            ctx.set_schedule(schedule)
+        grids = np.empty((int((dims[:, 0].astype(int) * dims[:, 1]).sum()), 3), np.int32)
+        _capi.check(lib.idl_triangulate_batch(ctx.handle, len(images), dims.ctypes.data, counts.ctypes.data,
+                                              seeds.ctypes.data, 8, _capi.MODE_REFERENCE, grids.ctypes.data, None,
+                                              None))
+        at = 0
+        for w, h, s in images:
+            _, want, _ = oracle.triangulate(w, h, oracle.sort_seeds(s, w, h), 8, "reference")
+            np.testing.assert_array_equal(grids[at:at + w * h].reshape(h, w, 3), want, err_msg=f"{w}x{h} {schedule}")
+            at += w * h
