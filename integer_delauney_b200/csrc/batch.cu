@@ -23,7 +23,7 @@
 // The number of launches and host synchronisations is independent of the
 // number of images.
 #include "raster.cuh"
-#include "row_hull.cuh"
+#include "exact_pass.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -111,132 +111,6 @@ __global__ void k_b_seeds(int32_t* __restrict__ a, int32_t* __restrict__ b, int 
     const size_t o = (size_t)pos_y(p) * pitch + pos_x(p);
     a[o] = (int32_t)i;
     b[o] = (int32_t)i;
-}
-
-// ---- exact semantics over the atlas -------------------------------------
-// The separable nearest-seed search of the single-image exact mode (exact.cu),
-// run for every image of the atlas at once and kept inside each image: a
-// column walk uses only its image's seeds, a row scan only its image's
-// columns, so no label crosses a wall.  Labels are global seed ids, as the
-// Jacobi path leaves them.
-struct XImg {
-    int ox, oy, Wp, Hp;    // padded canvas origin and size in the atlas
-    int col_off, row_off;  // first entry of this image in the column / row tables
-    long long s0, s1;      // its seeds: global ids [s0, s1), (x, y)-sorted
-};
-constexpr int XCHUNK = 64;
-
-// cs[col_off + c] = first seed of the image with atlas x >= ox + c, c in [0, Wp].
-__global__ void k_bx_col_start(const uint32_t* __restrict__ pos, const XImg* __restrict__ xi,
-                               const int32_t* __restrict__ colimg, int64_t n_cols, int32_t* __restrict__ cs)
-{
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n_cols) return;
-    const XImg m = xi[colimg[g]];
-    const int c = m.ox + (int)(g - m.col_off);
-    long long lo = m.s0, hi = m.s1;
-    while (lo < hi) {
-        const long long mid = (lo + hi) >> 1;
-        if ((int)pos_x(__ldg(&pos[mid])) < c) lo = mid + 1;
-        else hi = mid;
-    }
-    cs[g] = (int32_t)lo;
-}
-
-// Nearest seed of each cell within its image column (a tie between the seed
-// above and the one below goes to the lower one, the higher id), and its row
-// distance; one thread walks one column through a band of XCHUNK rows.
-__global__ void k_bx_col_nearest(const uint32_t* __restrict__ pos, const XImg* __restrict__ xi,
-                                 const int32_t* __restrict__ colimg, const int32_t* __restrict__ cs, int64_t n_cols,
-                                 int pitch, int32_t* __restrict__ col, int32_t* __restrict__ coldy)
-{
-    const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n_cols) return;
-    const XImg m = xi[colimg[g]];
-    const int c = (int)(g - m.col_off);
-    const int y0 = blockIdx.y * XCHUNK;
-    if (c >= m.Wp || y0 >= m.Hp) return;   // the image's extra start entry, or past its rows
-    const int y1 = min(m.Hp, y0 + XCHUNK);
-    const int x = m.ox + c;
-    const int32_t lo = cs[g], hi = cs[g + 1];
-    if (lo == hi) {
-        for (int y = y0; y < y1; ++y) {
-            col[(size_t)(m.oy + y) * pitch + x] = UNDEF;
-            coldy[(size_t)(m.oy + y) * pitch + x] = 0;
-        }
-        return;
-    }
-    int32_t a = lo, b = hi;   // first seed of the column at or below the band
-    while (a < b) {
-        const int32_t mid = (a + b) >> 1;
-        if ((int)pos_y(__ldg(&pos[mid])) < m.oy + y0) a = mid + 1;
-        else b = mid;
-    }
-    int next_y = a < hi ? (int)pos_y(__ldg(&pos[a])) : 0x7FFFFFFF;
-    int prev_y = a > lo ? (int)pos_y(__ldg(&pos[a - 1])) : -0x3FFFFFFF;
-    for (int y = y0; y < y1; ++y) {
-        const int ya = m.oy + y;
-        while (next_y < ya) {
-            prev_y = next_y;
-            ++a;
-            next_y = a < hi ? (int)pos_y(__ldg(&pos[a])) : 0x7FFFFFFF;
-        }
-        const int below = next_y - ya, above = ya - prev_y;
-        const bool take_below = a < hi && (a == lo || below <= above);
-        col[(size_t)ya * pitch + x] = take_below ? a : a - 1;
-        coldy[(size_t)ya * pitch + x] = take_below ? below : above;
-    }
-}
-
-// Best column candidate of each cell of an image row, scanning outward until
-// no column further away can beat or tie it.
-__global__ void k_bx_row_nearest(const int32_t* __restrict__ col, const int32_t* __restrict__ coldy,
-                                 const XImg* __restrict__ xi, const int32_t* __restrict__ rowimg, int pitch,
-                                 int32_t* __restrict__ lab)
-{
-    const int64_t r = blockIdx.x;
-    const XImg m = xi[rowimg[r]];
-    const int x = blockIdx.y * blockDim.x + threadIdx.x;
-    if (x >= m.Wp) return;
-    const int y = m.oy + (int)(r - m.row_off);
-    const int32_t* row = col + (size_t)y * pitch + m.ox;
-    const int32_t* rdy = coldy + (size_t)y * pitch + m.ox;
-    int32_t bl = row[x];
-    long long bd = 0x7FFFFFFFFFFFFFFFll;
-    if (bl >= 0) {
-        const long long dy = rdy[x];
-        bd = dy * dy;
-    }
-    for (int k = 1;; ++k) {
-        const long long kk = (long long)k * k;
-        if (kk > bd || (x - k < 0 && x + k >= m.Wp)) break;
-#pragma unroll
-        for (int side = 0; side < 2; ++side) {
-            const int xx = side ? x + k : x - k;
-            if (xx < 0 || xx >= m.Wp) continue;
-            const int32_t l = row[xx];
-            if (l < 0) continue;
-            const long long dy = rdy[xx];
-            const long long d = kk + dy * dy;
-            if (d < bd || (d == bd && l > bl)) {
-                bd = d;
-                bl = l;
-            }
-        }
-    }
-    lab[(size_t)y * pitch + m.ox + x] = bl;
-}
-
-// The lower-hull row pass (row_hull.cuh) on one image row of the atlas per
-// block: O(Wp) whatever the image's seed layout.
-__global__ void __launch_bounds__(HULL_THREADS)
-k_bx_row_hull(const int32_t* __restrict__ col, const int32_t* __restrict__ coldy, const XImg* __restrict__ xi,
-              const int32_t* __restrict__ rowimg, int pitch, int32_t* __restrict__ lab)
-{
-    const int64_t r = blockIdx.x;
-    const XImg m = xi[rowimg[r]];
-    const size_t o = (size_t)(m.oy + (int)(r - m.row_off)) * pitch + m.ox;
-    row_hull(col + o, coldy + o, m.Wp, lab + o);
 }
 
 __device__ __forceinline__ int tri_image(const int32_t* row, const int32_t* __restrict__ sid_img)
@@ -414,15 +288,18 @@ struct BatchPlan {
 };
 
 // Exact-semantics labels of every image into C.lab[0] (the atlas's walls
-// stay), the column pass's into C.lab[1]; C.exact_dy is scratch.  Returns the
-// images' padded canvases (x0, y0, x1, y1) on the device.
-const int4* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
+// stay) by the passes of exact.cu, each image kept within its own canvas: a
+// column walk uses only its image's seeds, a row only its image's columns, so
+// no label crosses a wall.  Labels are global seed ids, as the Jacobi path
+// leaves them; the column pass's plane is in C.lab[1].  Returns the image
+// table on the device.
+const XImg* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
 {
     const int n_images = (int)pl.imgs.size();
     std::vector<XImg> xi(n_images);
-    std::vector<int4> bounds(n_images);
-    std::vector<int32_t> colimg, rowimg;
+    std::vector<int32_t> pair_img, row_img;
     int max_wp = 0, max_hp = 0;
+    int64_t band_entries = 0;
     for (int i = 0; i < n_images; ++i) {
         const BImg& b = pl.imgs[i];
         XImg& m = xi[i];
@@ -430,57 +307,30 @@ const int4* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
         m.oy = b.oy;
         m.Wp = b.W + 2 * P;
         m.Hp = b.H + 2 * P;
-        m.col_off = (int)colimg.size();
-        m.row_off = (int)rowimg.size();
-        m.s0 = b.seed_off;
-        m.s1 = i + 1 < n_images ? pl.imgs[i + 1].seed_off : pl.n_seeds;
-        bounds[i] = make_int4(m.ox, m.oy, m.ox + m.Wp, m.oy + m.Hp);
-        colimg.insert(colimg.end(), (size_t)m.Wp + 1, i);
-        rowimg.insert(rowimg.end(), (size_t)m.Hp, i);
+        m.pair_off = (int)pair_img.size();
+        m.row_off = (int)row_img.size();
+        m.band_off = (int)band_entries;
+        m.s0 = (int)b.seed_off;
+        m.s1 = (int)(i + 1 < n_images ? pl.imgs[i + 1].seed_off : pl.n_seeds);
+        pair_img.insert(pair_img.end(), (size_t)(m.Wp + 1) / 2, i);
+        row_img.insert(row_img.end(), (size_t)m.Hp, i);
+        band_entries += (int64_t)x_bands(m) * m.Wp;
         max_wp = std::max(max_wp, m.Wp);
         max_hp = std::max(max_hp, m.Hp);
     }
-    const int64_t n_cols = (int64_t)colimg.size(), n_rows = (int64_t)rowimg.size();
-    C.batch_ximg.ensure(xi.size() * (sizeof(int4) + sizeof(XImg)));
-    int4* d_bounds = C.batch_ximg.as<int4>();
-    XImg* d_xi = reinterpret_cast<XImg*>(d_bounds + n_images);
-    IDL_CUDA(cudaMemcpyAsync(d_bounds, bounds.data(), bounds.size() * sizeof(int4), cudaMemcpyHostToDevice, C.stream));
-    C.batch_colimg.ensure((size_t)n_cols * 4);
-    C.batch_rowimg.ensure((size_t)n_rows * 4);
-    C.counts.ensure((size_t)n_cols * 4);
-    C.exact_dy.ensure((size_t)cv.pitch * cv.Hd * 4);
-    IDL_CUDA(cudaMemcpyAsync(d_xi, xi.data(), xi.size() * sizeof(XImg), cudaMemcpyHostToDevice,
+    C.batch_ximg.ensure(xi.size() * sizeof(XImg));
+    C.batch_colimg.ensure(pair_img.size() * 4);
+    C.batch_rowimg.ensure(row_img.size() * 4);
+    IDL_CUDA(cudaMemcpyAsync(C.batch_ximg.ptr, xi.data(), xi.size() * sizeof(XImg), cudaMemcpyHostToDevice,
                              C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_colimg.ptr, colimg.data(), (size_t)n_cols * 4, cudaMemcpyHostToDevice,
+    IDL_CUDA(cudaMemcpyAsync(C.batch_colimg.ptr, pair_img.data(), pair_img.size() * 4, cudaMemcpyHostToDevice,
                              C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_rowimg.ptr, rowimg.data(), (size_t)n_rows * 4, cudaMemcpyHostToDevice,
+    IDL_CUDA(cudaMemcpyAsync(C.batch_rowimg.ptr, row_img.data(), row_img.size() * 4, cudaMemcpyHostToDevice,
                              C.stream));
-    const int32_t* d_colimg = C.batch_colimg.as<int32_t>();
-    int32_t* cs = C.counts.as<int32_t>();
-    const uint32_t* pos = C.pos.as<uint32_t>();
-    k_bx_col_start<<<nblk(n_cols), 256, 0, C.stream>>>(pos, d_xi, d_colimg, n_cols, cs);
-    IDL_LAUNCH();
-    k_bx_col_nearest<<<dim3(nblk(n_cols, 128), (unsigned)((max_hp + XCHUNK - 1) / XCHUNK)), 128, 0, C.stream>>>(
-        pos, d_xi, d_colimg, cs, n_cols, cv.pitch, C.lab[1].as<int32_t>(), C.exact_dy.as<int32_t>());
-    IDL_LAUNCH();
-    if (max_wp <= HULL_MAX_W) {
-        static std::atomic<uint64_t> opted{0};   // the shared-memory opt-in is per device
-        const uint64_t bit = 1ull << (C.device & 63);
-        if (!(opted.load(std::memory_order_acquire) & bit)) {
-            IDL_CUDA(cudaFuncSetAttribute((const void*)k_bx_row_hull, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)row_hull_smem(HULL_MAX_W)));
-            opted.fetch_or(bit, std::memory_order_acq_rel);
-        }
-        k_bx_row_hull<<<(unsigned)n_rows, HULL_THREADS, row_hull_smem(max_wp), C.stream>>>(
-            C.lab[1].as<int32_t>(), C.exact_dy.as<int32_t>(), d_xi, C.batch_rowimg.as<int32_t>(), cv.pitch,
-            C.lab[0].as<int32_t>());
-    } else {
-        k_bx_row_nearest<<<dim3((unsigned)n_rows, (unsigned)((max_wp + 255) / 256)), 256, 0, C.stream>>>(
-            C.lab[1].as<int32_t>(), C.exact_dy.as<int32_t>(), d_xi, C.batch_rowimg.as<int32_t>(), cv.pitch,
-            C.lab[0].as<int32_t>());
-    }
-    IDL_LAUNCH();
-    return d_bounds;
+    const XImg* d_xi = C.batch_ximg.as<XImg>();
+    exact_images(C, cv.pitch, C.pos.as<uint32_t>(), d_xi, C.batch_colimg.as<int32_t>(), (int)pair_img.size(),
+                 C.batch_rowimg.as<int32_t>(), (int)row_img.size(), max_wp, max_hp, band_entries);
+    return d_xi;
 }
 
 void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, int64_t* tri_counts,
@@ -568,9 +418,8 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
         // the exact passes write every cell of every image; the walls between
         // them are read by the block rule (and by resolve_exact) in plane 0 only
         IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
-        const int4* bounds = exact_atlas(C, pl, P, cv);
-        if (direct)
-            resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, bounds, C.batch_sid.as<int32_t>());
+        const XImg* xi = exact_atlas(C, pl, P, cv);
+        if (direct) resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, xi, C.batch_sid.as<int32_t>());
     } else {
         run_passes();
     }

@@ -162,8 +162,7 @@ struct Context {
     DevBuf bits;          // work-list dedup bitmaps of the persistent propagation kernel
     DevBuf big_tiles;     // tile rounds' last work list, handed to the persistent kernel
     DevBuf cellbits;      // cell-list tile rounds: three last-pass change bitmaps, in rotation
-    DevBuf exact_dy;      // exact mode: row distance to each cell's column-nearest seed
-    DevBuf exact_rmin;    // exact mode: per row, smallest squared row distance of each 32-column block
+    DevBuf exact_bands;   // exact mode: per band of rows and column, its first seed (exact_pass.cuh)
     DevBuf sus_bits, sus_list;  // resolve.cu: suspect bits, suspect list with results and open indices
     int32_t stamp_epoch = 0;
     // propagation schedule from scratch (resolve.cu, propagate.cu; idl_context_set_schedule)
@@ -229,7 +228,7 @@ struct Context {
     {
         DevBuf* all[] = {&seeds_in, &xs, &ys, &pos, &bitmap, &scan_a, &scan_b, &scan_c, &lab[0], &lab[1],
                          &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
-                         &exact_dy, &exact_rmin, &sus_bits, &sus_list, &hkeys,
+                         &exact_bands, &sus_bits, &sus_list, &hkeys,
                          &ukeys, &uvals, &cnt, &off, &fill, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
                          &batch_img, &batch_seed_img, &batch_rows, &batch_sid, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
@@ -345,17 +344,25 @@ void grid_barrier_selftest(Context& C, int missing_arrivals, unsigned spin_limit
 
 // Stage (a), exact semantics (exact.cu): nearest seed, ties to the higher id,
 // for the n (x, y)-sorted seeds `pos` of the canvas; labels into C.lab[0]
-// (C.lab[1] is scratch).
+// (C.lab[1] holds the column pass's offsets, C.exact_bands its table).
+struct XImg;
 void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n);
+// The same for the images of a batch atlas (exact.cu): device tables of the
+// images, of each column pair's and each row's image; C.lab[0] and C.lab[1]
+// hold planes of the atlas.
+void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, const int32_t* pair_img, int n_pairs,
+                  const int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries);
+// The one image of a single canvas with n seeds.
+XImg whole_canvas(const Canvas& cv, int64_t n);
 
 // Turns the exact labels propagate_exact left in C.lab[0] (and the column
 // plane in C.lab[1]) into the reference semantics' fixed point from scratch
 // (resolve.cu).  Reads nothing back: C.sc()->resolve_fail, with the scalars'
 // next read-back, tells whether the passes have to be run instead.  `passes`:
-// also what resolved_passes needs.  Batch atlas: `bounds` is each image's
-// padded canvas (x0, y0, x1, y1), `seed_img` the image of each seed.
+// also what resolved_passes needs.  Batch atlas: `images` is the table
+// exact_images used, `seed_img` the image of each seed.
 void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes,
-                   const int4* bounds = nullptr, const int32_t* seed_img = nullptr);
+                   const XImg* images = nullptr, const int32_t* seed_img = nullptr);
 // The iteration's pass count from the scalars read back after resolve_exact
 // with `passes`, or -1 if they do not determine it.
 inline int64_t resolved_passes(const Scalars& s)

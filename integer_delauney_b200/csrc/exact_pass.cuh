@@ -1,0 +1,387 @@
+// Device side of the exact diagram (exact.cu), shared by the single-image and
+// the batched pipelines (an image is one padded canvas of the atlas; a single
+// image is the whole plane).
+//
+// Column pass: each cell's signed row offset to the nearest seed of its own
+// column (ties to the lower one, the higher id), two bytes per cell, and a
+// small table that turns (column, row of a seed) into the seed's id.
+// Row pass: each cell's winner among its row's column candidates, and its id.
+#pragma once
+
+#include "common.cuh"
+
+namespace idl {
+
+struct XImg {
+    int ox, oy, Wp, Hp;    // padded canvas origin and size on the plane
+    int pair_off;          // first entry of this image in the column-pair table
+    int row_off;           // first entry in the row table
+    int band_off;          // first entry in the band table
+    int s0, s1;            // its seeds: ids [s0, s1), (x, y)-sorted
+};
+
+constexpr int BAND = 64;                       // rows a thread of the column pass walks
+constexpr int16_t NO_SEED = (int16_t)-32768;   // a column without seeds
+
+__host__ __device__ inline int x_bands(const XImg& m) { return (m.Hp + BAND - 1) / BAND; }
+
+// First of the image's seeds at or after (x, y) in (x, y) order.
+__device__ __forceinline__ int x_lower_bound(const uint32_t* __restrict__ pos, const XImg& m, int x, int y)
+{
+    int lo = m.s0, hi = m.s1;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        const uint32_t p = __ldg(&pos[mid]);
+        const int px = pos_x(p);
+        if (px < x || (px == x && (int)pos_y(p) < y)) lo = mid + 1;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// Id of the seed at (x, y) of the plane, which must exist: bands holds, per
+// band of rows and column, the first seed at or below the band's first row.
+__device__ __forceinline__ int32_t x_seed_at(const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
+                                             const XImg& m, int x, int y)
+{
+    int32_t a = __ldg(&bands[m.band_off + (y - m.oy) / BAND * m.Wp + (x - m.ox)]);
+    while (a < m.s1 - 1 && (int)pos_y(__ldg(&pos[a])) < y) ++a;
+    return a;
+}
+
+// One thread walks two adjacent columns (the pair starting at image column c)
+// through the rows of one band, so that a warp writes 128 bytes of a row at
+// once; its place in each column's seeds comes from one search of the sorted
+// seeds.  Two bytes per cell is all that is written (the planes of 4-byte ids
+// and distances this replaces took four times the traffic).
+__device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, const XImg& m, int c, int band,
+                                              int pitch, int16_t* __restrict__ off, int32_t* __restrict__ bands)
+{
+    const int y0 = band * BAND, y1 = min(m.Hp, y0 + BAND);
+    int a[2], next_y[2], prev_y[2];
+    bool any[2];
+    constexpr int FAR_BELOW = 0x3FFFFFFF, FAR_ABOVE = -0x3FFFFFFF;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+        next_y[k] = FAR_BELOW;
+        prev_y[k] = FAR_ABOVE;
+        any[k] = false;
+        a[k] = 0;
+        if (c + k < m.Wp) {
+            const int x = m.ox + c + k;
+            a[k] = x_lower_bound(pos, m, x, m.oy + y0);
+            bands[m.band_off + band * m.Wp + c + k] = a[k];
+            if (a[k] < m.s1) {
+                const uint32_t p = __ldg(&pos[a[k]]);
+                if ((int)pos_x(p) == x) next_y[k] = (int)pos_y(p) - m.oy;
+            }
+            if (a[k] > m.s0) {
+                const uint32_t p = __ldg(&pos[a[k] - 1]);
+                if ((int)pos_x(p) == x) prev_y[k] = (int)pos_y(p) - m.oy;
+            }
+            any[k] = next_y[k] != FAR_BELOW || prev_y[k] != FAR_ABOVE;
+        }
+    }
+    int16_t* dst = off + (size_t)(m.oy + y0) * pitch + m.ox + c;
+    const bool paired = c + 1 < m.Wp && ((m.ox | pitch) & 1) == 0;   // c is even
+    for (int y = y0; y < y1; ++y, dst += pitch) {
+        int v[2];
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            while (next_y[k] < y) {   // the seed below was passed: it becomes the one above
+                prev_y[k] = next_y[k];
+                next_y[k] = FAR_BELOW;
+                if (++a[k] < m.s1) {
+                    const uint32_t p = __ldg(&pos[a[k]]);
+                    if ((int)pos_x(p) == m.ox + c + k) next_y[k] = (int)pos_y(p) - m.oy;
+                }
+            }
+            const int below = next_y[k] - y, above = y - prev_y[k];   // tie: the larger y, the higher id
+            v[k] = any[k] ? (below <= above ? below : -above) : NO_SEED;
+        }
+        if (paired) {
+            *reinterpret_cast<short2*>(dst) = make_short2((short)v[0], (short)v[1]);
+        } else {
+            if (c < m.Wp) dst[0] = (int16_t)v[0];
+            if (c + 1 < m.Wp) dst[1] = (int16_t)v[1];
+        }
+    }
+}
+
+// ---- row pass -----------------------------------------------------------
+//
+// With F_x = dy_x^2 + x^2 for each column x that has a candidate, the cell at
+// column t takes the column minimising F_x - 2 t x (its squared distance minus
+// t^2), ties to the larger x, the higher id.  All of it fits 32 bits: F_x <
+// 2^31, 2 t x < 2^31 and F_x - 2 t x >= -t^2.
+//  1. A column on or above the line between two others, one on each side, wins
+//     no cell (only the vertices of the lower convex hull of the points
+//     (x, F_x) do; on an edge the right end ties too).  Each warp thins out its
+//     share of the columns: a parallel test of every column against its two
+//     neighbours in the list, the survivors moved together, again and again
+//     (the first pass tests three pairs).  4 096 columns go to 1 610, 962 and
+//     665 in three passes at 200 000 uniform seeds (the hull has 559).
+//     Whatever is left over costs time only.
+//  2. A cell's winner never moves left as t grows, so the winners of the cells
+//     1024 apart, then 256 apart, then 32 apart bound those in between: the
+//     first two by a warp over the list range, the last by a lane each.
+//  3. A warp takes 32 cells and tests the list between its two bounds, a
+//     broadcast load and four instructions per column.
+// The work is O(W) per row whatever the seed layout (the ranges of one step
+// add up to the list and one column per cell looked at).  It is bound by
+// instruction issue; a monotone chain per thread in step 1 (its pops diverge)
+// took twice the instructions, merging such hulls pairwise left most lanes
+// idle.
+// Shared memory is 8 bytes per column, so that enough rows share an SM: the
+// offsets, the columns' list, and room for W / 2 list entries with their F; a
+// longer list (seed sets denser than one in ten cells) holds columns only and
+// works F out again each time.
+constexpr int ROW_STEP = 32, ROW_MID = 256, ROW_TOP = 1024;
+constexpr int ROW_THIN = 5;    // thinning passes at most
+constexpr int ROW_BYTES = 8;   // shared memory per column
+constexpr int ROW_SHARE = 528;
+// stands for a missing column's square: with any other it outweighs twice any
+// real square, and two of them still fit
+constexpr uint32_t NO_SQUARE = 0x7FFFFF00u;
+
+inline size_t row_pass_smem(int W)
+{
+    const size_t w = (size_t)(W + 7) / 4 * 4;
+    return w * ROW_BYTES + (size_t)(W / ROW_STEP + 3) * 2 + 16;
+}
+// Threads per row: warps of at most ROW_SHARE columns, up to 8.
+inline int row_pass_threads(int W)
+{
+    return W <= ROW_SHARE ? 32 : W <= 2 * ROW_SHARE ? 64 : W <= 4 * ROW_SHARE ? 128 : 256;
+}
+
+// Steps 2 and 3 of the row pass over a list of n columns; cost(k, t) is
+// F - 2 t x of its entry k.
+template <int T, class Cost>
+__device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* listx, uint16_t* buf, uint16_t* hx,
+                                           uint16_t* win, const int16_t* off, int n, int W, int y, const XImg& m,
+                                           const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
+                                           int32_t* __restrict__ out, Cost cost, bool packed)
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = T / 32;
+    auto sync = [] {
+        if (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+    auto best_in = [&](int t, int lo, int hi) {
+        int arg = lo;
+        int32_t best = cost(lo, t);
+        for (int k = lo + 1; k <= hi; ++k) {
+            const int32_t c = cost(k, t);
+            if (c <= best) {
+                best = c;
+                arg = k;
+            }
+        }
+        return arg;
+    };
+    auto by_warp = [&](int t, int lo, int hi) {
+        int32_t best = 0x7FFFFFFF;
+        int arg = lo;
+        for (int k = lo + lane; k <= hi; k += 32) {
+            const int32_t c = cost(k, t);
+            if (c <= best) {
+                best = c;
+                arg = k;
+            }
+        }
+        const int32_t low = __reduce_min_sync(0xFFFFFFFFu, best);
+        return (int)__reduce_max_sync(0xFFFFFFFFu, best == low ? arg : -1);
+    };
+
+    // 2. winners of the cells ROW_TOP, ROW_MID and ROW_STEP apart
+    const int steps = (W + ROW_STEP - 1) / ROW_STEP;
+    constexpr int TOP = ROW_TOP / ROW_STEP, MID = ROW_MID / ROW_STEP;
+    for (int i = warp * TOP; i < steps; i += NW * TOP) {
+        const int a = by_warp(i * ROW_STEP, 0, n - 1);
+        if (lane == 0) win[i] = (uint16_t)a;
+    }
+    if (tid == 0) win[steps] = (uint16_t)(n - 1);
+    sync();
+    for (int i = warp * MID; i < steps; i += NW * MID) {
+        if (i % TOP == 0) continue;
+        const int up = i / TOP * TOP;
+        const int a = by_warp(i * ROW_STEP, win[up], win[min(up + TOP, steps)]);
+        if (lane == 0) win[i] = (uint16_t)a;
+    }
+    sync();
+    for (int i = tid; i < steps; i += T) {
+        if (i % MID == 0) continue;
+        const int up = i / MID * MID;
+        win[i] = (uint16_t)best_in(i * ROW_STEP, win[up], win[min(up + MID, steps)]);
+    }
+    if (packed) {
+        // ids of the listed columns' seeds: the offsets move aside first, then
+        // buf and hx take the ids' halves (each list entry is one thread's)
+        for (int k = tid; k < n; k += T) hx[k] = (uint16_t)off[list2[k].y / -2];
+        sync();
+        for (int k = tid; k < n; k += T) {
+            const int32_t id = x_seed_at(pos, bands, m, m.ox + list2[k].y / -2, y + (int16_t)hx[k]);
+            buf[k] = (uint16_t)(id & 0xFFFF);
+            hx[k] = (uint16_t)(id >> 16);
+        }
+    }
+    sync();
+
+    // 3. every cell, from the list between its interval's bounds
+    for (int i = warp; i < steps; i += NW) {
+        const int t = i * ROW_STEP + lane;
+        const int arg = best_in(t, win[i], win[i + 1]);
+        if (t >= W) continue;
+        if (packed) {
+            out[t] = (int32_t)buf[arg] | (int32_t)hx[arg] << 16;
+        } else {
+            const int x = listx[arg];
+            out[t] = x_seed_at(pos, bands, m, m.ox + x, y + off[x]);
+        }
+    }
+}
+
+// row: the row's offsets; y: its row on the plane; out: its labels.
+template <int T>
+__device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, const XImg& m,
+                                      const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
+                                      int32_t* __restrict__ out)
+{
+    extern __shared__ __align__(16) unsigned char row_smem[];
+    __shared__ int s_sum[T / 32 + 1];
+    const int W = m.Wp;
+    const int w = (W + 7) / 4 * 4;
+    constexpr int LIST_BYTES = ROW_BYTES - 4;
+    const int cap = w * LIST_BYTES / 8;                            // (F, -2 x) entries that fit
+    int2* list2 = reinterpret_cast<int2*>(row_smem);
+    uint16_t* listx = reinterpret_cast<uint16_t*>(row_smem);       // the longer list
+    uint16_t* buf = reinterpret_cast<uint16_t*>(row_smem + (size_t)w * LIST_BYTES);   // offsets, then id low halves
+    uint16_t* hx = buf + w;                                        // columns kept, then id high halves
+    uint16_t* win = hx + w;                                        // winner at each 32nd cell
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    constexpr int NW = T / 32;
+    auto sync = [] {
+        if (T == 32) __syncwarp();
+        else __syncthreads();
+    };
+
+    // the row's offsets, by aligned words (an odd start brings one cell of its
+    // left neighbour along)
+    const int skew = (int)((reinterpret_cast<uintptr_t>(row) >> 1) & 1);
+    {
+        const uint32_t* src = reinterpret_cast<const uint32_t*>(row - skew);
+        uint32_t* dst = reinterpret_cast<uint32_t*>(buf);
+        for (int i = tid; i < (W + skew + 1) / 2; i += T) dst[i] = __ldg(&src[i]);
+    }
+    const int16_t* off = reinterpret_cast<const int16_t*>(buf) + skew;
+    sync();
+    auto value = [&](int x) {
+        const int d = off[x];
+        return d * d + x * x;
+    };
+
+    // 1. each warp thins its share of the columns [s0, s1) into hx[s0, s0 + kept)
+    const int share = ((W + NW - 1) / NW + 31) / 32 * 32;
+    const int s0 = min(W, warp * share), s1 = min(W, s0 + share);
+    const unsigned below = (1u << lane) - 1u;
+    int kept = 0;
+    // the first test, two columns a lane, against the columns 1, 2 and 4 to
+    // either side (at equal distances k it is d_l^2 + d_r^2 + 2 k^2 <= 2 d_x^2)
+    for (int base = s0; base < s1; base += 64) {
+        const int x = base + 2 * lane;
+        uint32_t q[10];   // squares of columns x - 4 .. x + 5; beyond the warp's 64: not there
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int d = x + c < W ? off[x + c] : NO_SEED;
+            q[4 + c] = d == NO_SEED ? NO_SQUARE : (uint32_t)(d * d);
+        }
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+#pragma unroll
+            for (int j = 1; j <= 2; ++j) {
+                const uint32_t l = __shfl_up_sync(0xFFFFFFFFu, q[4 + c], j);
+                const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, q[4 + c], j);
+                q[4 + c - 2 * j] = lane >= j ? l : NO_SQUARE;
+                q[4 + c + 2 * j] = lane + j < 32 ? r : NO_SQUARE;
+            }
+        }
+        bool keep[2];
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t d = q[4 + c], dd = 2u * d;
+            keep[c] = x + c < s1 && d != NO_SQUARE && q[3 + c] + q[5 + c] + 2u > dd &&
+                      q[2 + c] + q[6 + c] + 8u > dd && q[c] + q[8 + c] + 32u > dd;
+        }
+        const unsigned k0 = __ballot_sync(0xFFFFFFFFu, keep[0]), k1 = __ballot_sync(0xFFFFFFFFu, keep[1]);
+        const int at0 = s0 + kept + __popc(k0 & below) + __popc(k1 & below);
+        if (keep[0]) hx[at0] = (uint16_t)x;
+        if (keep[1]) hx[at0 + (keep[0] ? 1 : 0)] = (uint16_t)(x + 1);
+        kept += __popc(k0) + __popc(k1);
+    }
+    __syncwarp();
+    for (int pass = 1; pass < ROW_THIN && kept > 2; ++pass) {
+        // in place: a group's writes stay at or before its own reads, and
+        // reach a later group's left neighbour only where nothing was dropped
+        int now = 0;
+        for (int base = 0; base < kept; base += 32) {
+            const int i = base + lane;
+            bool keep = i < kept;
+            int x = 0;
+            if (keep) {
+                x = hx[s0 + i];
+                if (i > 0 && i + 1 < kept) {
+                    const int xl = hx[s0 + i - 1], xr = hx[s0 + i + 1];
+                    const int32_t f = value(x), fl = value(xl), fr = value(xr);
+                    keep = (long long)(x - xl) * (fr - f) > (long long)(f - fl) * (xr - x);
+                }
+            }
+            const unsigned k = __ballot_sync(0xFFFFFFFFu, keep);
+            __syncwarp();
+            if (keep) hx[s0 + now + __popc(k & below)] = (uint16_t)x;
+            now += __popc(k);
+            __syncwarp();
+        }
+        const bool settled = kept - now < kept / 8;
+        kept = now;
+        if (settled) break;
+    }
+    // one list of all of them
+    int at = 0, n = kept;
+    if (T > 32) {
+        if (lane == 0) s_sum[warp] = kept;
+        __syncthreads();
+        n = 0;
+#pragma unroll
+        for (int k = 0; k < NW; ++k) {
+            const int v = s_sum[k];
+            at += k < warp ? v : 0;
+            n += v;
+        }
+    }
+    const bool packed = n <= cap;
+    for (int j = lane; j < kept; j += 32) {
+        const int x = hx[s0 + j];
+        if (packed) list2[at + j] = make_int2(value(x), -2 * x);
+        else listx[at + j] = (uint16_t)x;
+    }
+    sync();
+    if (n == 0) {
+        for (int t = tid; t < W; t += T) out[t] = UNDEF;
+        return;
+    }
+    if (packed) {
+        x_row_fill<T>(list2, listx, buf, hx, win, off, n, W, y, m, pos, bands, out, [&](int k, int t) {
+            const int2 c = list2[k];
+            return c.x + t * c.y;
+        }, true);
+    } else {
+        x_row_fill<T>(list2, listx, buf, hx, win, off, n, W, y, m, pos, bands, out, [&](int k, int t) {
+            const int x = listx[k];
+            return value(x) - 2 * t * x;
+        }, false);
+    }
+}
+
+}  // namespace idl

@@ -58,6 +58,7 @@
 // Cost at 4096 x 4096, 200 000 uniform seeds: one read of the label plane for
 // the roots; the rest touches a few thousand cells.
 #include "context.cuh"
+#include "exact_pass.cuh"
 #include "stencil.cuh"
 
 #include <atomic>
@@ -67,13 +68,14 @@ namespace {
 
 struct View {
     const int32_t* lab;      // exact labels
-    const int32_t* col;      // column pass: nearest seed of each cell within its column
+    const int16_t* off;      // column pass: row offset to the nearest seed of the cell's column
+    const int32_t* bands;    // and its table
     const uint32_t* pos;
     const uint32_t* sus;     // suspect bits, rows of `words` words
-    const int4* bounds;      // batch: padded canvas (x0, y0, x1, y1) of each image, else null
+    const XImg* images;      // batch: image table, else null
     const int32_t* seed_img; // batch: image of each seed
     int pitch, Wd, Hd, words;
-    int32_t n;               // seeds
+    XImg whole;              // not a batch: the one image
 };
 
 __device__ __forceinline__ int sgn(int v) { return (v > 0) - (v < 0); }
@@ -242,26 +244,26 @@ struct WarpScratch {
     int n, n_rival, budget;
 };
 
-// Offers every seed m of image columns x0..x1 that beats (d, s) at (x, y) to
-// f(m); a lane takes every 32nd column.  The column pass's plane gives each
-// column's nearest seed at row y; its neighbours in id order are the column's
-// other seeds.  f returns false to stop the lane.
+// Offers every seed m of the image that beats (d, s) at (x, y) to f(m); a lane
+// takes every 32nd column.  The column pass's plane gives each column's
+// nearest seed at row y; its neighbours in id order are the column's other
+// seeds.  f returns false to stop the lane.
 template <class F>
-__device__ __forceinline__ void for_better(const View& V, int x, int y, int32_t d, int32_t s, const int4& b, int lane,
+__device__ __forceinline__ void for_better(const View& V, int x, int y, int32_t d, int32_t s, const XImg& b, int lane,
                                            F&& f)
 {
     const int R = isqrt(d);
-    const int lo = max(b.x, x - R), hi = min(b.z - 1, x + R);
+    const int lo = max(b.ox, x - R), hi = min(b.ox + b.Wp - 1, x + R);
     for (int xx = lo + lane; xx <= hi; xx += 32) {
-        const int32_t c = __ldg(&V.col[(size_t)y * V.pitch + xx]);
-        if (c < 0) continue;
+        const int o = __ldg(&V.off[(size_t)y * V.pitch + xx]);
+        if (o == NO_SEED || (long long)o * o + (long long)(xx - x) * (xx - x) > d) continue;
+        const int32_t c = x_seed_at(V.pos, V.bands, b, xx, y + o);
         for (int step = 1; step >= -1; step -= 2) {
-            for (int32_t m = step > 0 ? c : c - 1; m >= 0 && m < V.n; m += step) {
-                // past the column's (or the image's) run: another column, or d beyond reach
+            for (int32_t m = step > 0 ? c : c - 1; m >= b.s0 && m < b.s1; m += step) {
                 const uint32_t p = __ldg(&V.pos[m]);
-                if ((int)pos_x(p) != xx) break;
+                if ((int)pos_x(p) != xx) break;   // past the column's run
                 const int32_t dm = dist2(x, y, p);
-                if (dm > d || (int)pos_y(p) < b.y || (int)pos_y(p) >= b.w) break;
+                if (dm > d) break;
                 if (m != s && beats(dm, m, d, s) && !f(m, p)) return;
             }
         }
@@ -284,16 +286,16 @@ __device__ __forceinline__ bool may_display(const View& V, int x, int y, int32_t
     return true;
 }
 
-__device__ __forceinline__ int4 image_bounds(const View& V, int32_t seed)
+__device__ __forceinline__ XImg image_of(const View& V, int32_t seed)
 {
-    return V.bounds ? __ldg(&V.bounds[V.seed_img[seed]]) : make_int4(0, 0, V.Wd, V.Hd);
+    return V.images ? V.images[V.seed_img[seed]] : V.whole;
 }
 
 // S.rival[LEVEL]: the seeds that beat k at (x, y) and can be there by the time
 // k can (|q - m| <= |q - k|); their number, above MAX_CAND if they do not fit or the
 // budget is spent.
 template <int LEVEL>
-__device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int y, int32_t k, const int4& b, int lane)
+__device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int y, int32_t k, const XImg& b, int lane)
 {
     const int t = l1_to(V, x, y, k);
     const int32_t d = d2_to(V, x, y, k);
@@ -315,12 +317,12 @@ __device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int 
 }
 
 template <int LEVEL>
-__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const int4& b, int lane);
+__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane);
 
 // Rule "yes": k certainly arrives at (px, py), at its L1 distance.  LEVEL 1: a
 // rival that never arrives at a cell does not count there.  Warp-wide.
 template <int LEVEL>
-__device__ bool arrives(const View& V, WarpScratch& S, int px, int py, int32_t k, const int4& b, int lane)
+__device__ bool arrives(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane)
 {
     const uint32_t kp = __ldg(&V.pos[k]);
     const int gx = sgn((int)pos_x(kp) - px), gy = sgn((int)pos_y(kp) - py);
@@ -357,7 +359,7 @@ __device__ bool arrives(const View& V, WarpScratch& S, int px, int py, int32_t k
 // Rule "no": k certainly never arrives at (px, py).  LEVEL 1: a cell where a
 // rival of k certainly arrives no later than k can is closed to k.  Warp-wide.
 template <int LEVEL>
-__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const int4& b, int lane)
+__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane)
 {
     uint32_t* seen = S.seen[LEVEL];
     int ns = 1, head = 0;
@@ -415,7 +417,7 @@ k_resolve(View V, const int32_t* __restrict__ list, int cap, int32_t* __restrict
     for (int i = blockIdx.x * RES_WARPS + (threadIdx.x >> 5); i < n; i += gridDim.x * RES_WARPS) {
         const uint32_t pk = (uint32_t)list[i];
         const int px = pos_x(pk), py = pos_y(pk);
-        const int4 b = image_bounds(V, label_at(V, px, py));
+        const XImg b = image_of(V, label_at(V, px, py));
         // f: the best owner of the settled neighbours
         int32_t f = -1, fd = FAR;
         int f_at = 0;   // when the settled neighbour holding f displays it, plus one
@@ -646,7 +648,7 @@ __global__ void k_resolve_apply(int32_t* __restrict__ lab, int pitch, const int3
 
 }  // namespace
 
-void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes, const int4* bounds,
+void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes, const XImg* images,
                    const int32_t* seed_img)
 {
     const int words = ceil_div(cv.Wd, 32);
@@ -662,8 +664,8 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     uint32_t* sus = C.sus_bits.as<uint32_t>();
     IDL_CUDA(cudaMemsetAsync(sus, 0, bits, C.stream));
     IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
-    const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int32_t>(), pos, sus, bounds, seed_img, cv.pitch, cv.Wd, cv.Hd,
-                 words, (int32_t)n};
+    const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), C.exact_bands.as<int32_t>(), pos, sus, images,
+                 seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n)};
     const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 8 * ROOT_ROWS));
     if (passes)
         k_roots<true><<<g, 256, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());

@@ -104,3 +104,13 @@ def test_batch_labels_equal_single_images(ctx):
             _, want, _ = oracle.triangulate(w, h, oracle.sort_seeds(s, w, h), 8, "reference")
             np.testing.assert_array_equal(grids[at:at + w * h].reshape(h, w, 3), want, err_msg=f"{w}x{h} {schedule}")
             at += w * h
+
+
+@pytest.mark.parametrize("W,H,n", [(31, 3, 5), (32, 65, 40), (33, 64, 33), (257, 5, 700), (528, 2, 3), (529, 4, 1500),
+                                   (1025, 3, 9), (2113, 2, 2000), (4230, 3, 6000), (17001, 2, 40), (32767, 1, 9000)])
+def test_exact_rows(W, H, n):
+    """The row pass at its interval (32, 256, 1024), warp share and list-length
+    edges: few seeds, and more than half of the columns in the list."""
+    seeds = random_seeds(W, H, n, 5)
+    want, _ = oracle.voronoi("exact", W, H, oracle.sort_seeds(seeds, W, H))
+    np.testing.assert_array_equal(cu.Voronoi().compute(W, H, seeds, voronoi_mode="exact"), want)
