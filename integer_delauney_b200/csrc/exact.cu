@@ -49,22 +49,22 @@ k_bx_column_off(const uint32_t* __restrict__ pos, const XImg* __restrict__ xi, c
 template <int T>
 __global__ void __launch_bounds__(T)
 k_row_win(const int16_t* __restrict__ off, XImg m, int pitch, const uint32_t* __restrict__ pos,
-          const int32_t* __restrict__ bands, int32_t* __restrict__ lab)
+          const int32_t* __restrict__ bands, int32_t* __restrict__ lab, int list_bytes)
 {
     const int y = blockIdx.x;
-    x_row<T>(off + (size_t)y * pitch, y, m, pos, bands, lab + (size_t)y * pitch);
+    x_row<T>(off + (size_t)y * pitch, y, m, pos, bands, lab + (size_t)y * pitch, list_bytes);
 }
 
 template <int T>
 __global__ void __launch_bounds__(T)
 k_bx_row_win(const int16_t* __restrict__ off, const XImg* __restrict__ xi, const int32_t* __restrict__ row_img,
              int pitch, const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-             int32_t* __restrict__ lab)
+             int32_t* __restrict__ lab, int list_bytes)
 {
     const XImg m = xi[row_img[blockIdx.x]];
     const int y = m.oy + (int)blockIdx.x - m.row_off;
     const size_t o = (size_t)y * pitch + m.ox;
-    x_row<T>(off + o, y, m, pos, bands, lab + o);
+    x_row<T>(off + o, y, m, pos, bands, lab + o, list_bytes);
 }
 
 template <class K, class... A>
@@ -88,8 +88,8 @@ void rows_for_width(Context& C, int width, unsigned rows, A... args)
     const int threads = row_pass_threads(width);
     const size_t smem = row_pass_smem(width);
     auto go = [&](auto single, auto batch, int slot) {
-        if constexpr (BATCH) launch_rows(C, batch, opted[slot], rows, threads, smem, args...);
-        else launch_rows(C, single, opted[slot], rows, threads, smem, args...);
+        if constexpr (BATCH) launch_rows(C, batch, opted[slot], rows, threads, smem, args..., row_list_bytes(width));
+        else launch_rows(C, single, opted[slot], rows, threads, smem, args..., row_list_bytes(width));
     };
     if (threads == 32) go(k_row_win<32>, k_bx_row_win<32>, 0);
     else if (threads == 64) go(k_row_win<64>, k_bx_row_win<64>, 1);

@@ -135,19 +135,21 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
 // Shared memory is 8 bytes per column, so that enough rows share an SM: the
 // offsets, the columns' list, and room for W / 2 list entries with their F; a
 // longer list (seed sets denser than one in ten cells) holds columns only and
-// works F out again each time.
+// works F out again each time.  Rows of more than ROW_WIDE columns get 6 bytes
+// per column, room for W / 4 entries.
 constexpr int ROW_STEP = 32, ROW_MID = 256, ROW_TOP = 1024;
 constexpr int ROW_THIN = 5;    // thinning passes at most
-constexpr int ROW_BYTES = 8;   // shared memory per column
+constexpr int ROW_WIDE = 27000;
 constexpr int ROW_SHARE = 528;
 // stands for a missing column's square: with any other it outweighs twice any
 // real square, and two of them still fit
 constexpr uint32_t NO_SQUARE = 0x7FFFFF00u;
 
+inline int row_list_bytes(int W) { return W > ROW_WIDE ? 2 : 4; }   // per column, for the widest row of a launch
 inline size_t row_pass_smem(int W)
 {
     const size_t w = (size_t)(W + 7) / 4 * 4;
-    return w * ROW_BYTES + (size_t)(W / ROW_STEP + 3) * 2 + 16;
+    return w * (4 + row_list_bytes(W)) + (size_t)(W / ROW_STEP + 3) * 2 + 16;
 }
 // Threads per row: warps of at most ROW_SHARE columns, up to 8.
 inline int row_pass_threads(int W)
@@ -243,21 +245,21 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
     }
 }
 
-// row: the row's offsets; y: its row on the plane; out: its labels.
+// row: the row's offsets; y: its row on the plane; out: its labels;
+// list_bytes: row_list_bytes of the launch.
 template <int T>
 __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, const XImg& m,
                                       const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-                                      int32_t* __restrict__ out)
+                                      int32_t* __restrict__ out, int list_bytes)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
     __shared__ int s_sum[T / 32 + 1];
     const int W = m.Wp;
     const int w = (W + 7) / 4 * 4;
-    constexpr int LIST_BYTES = ROW_BYTES - 4;
-    const int cap = w * LIST_BYTES / 8;                            // (F, -2 x) entries that fit
+    const int cap = w * list_bytes / 8;                            // (F, -2 x) entries that fit
     int2* list2 = reinterpret_cast<int2*>(row_smem);
     uint16_t* listx = reinterpret_cast<uint16_t*>(row_smem);       // the longer list
-    uint16_t* buf = reinterpret_cast<uint16_t*>(row_smem + (size_t)w * LIST_BYTES);   // offsets, then id low halves
+    uint16_t* buf = reinterpret_cast<uint16_t*>(row_smem + (size_t)w * list_bytes);   // offsets, then id low halves
     uint16_t* hx = buf + w;                                        // columns kept, then id high halves
     uint16_t* win = hx + w;                                        // winner at each 32nd cell
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

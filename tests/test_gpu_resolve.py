@@ -107,7 +107,8 @@ def test_batch_labels_equal_single_images(ctx):
 
 
 @pytest.mark.parametrize("W,H,n", [(31, 3, 5), (32, 65, 40), (33, 64, 33), (257, 5, 700), (528, 2, 3), (529, 4, 1500),
-                                   (1025, 3, 9), (2113, 2, 2000), (4230, 3, 6000), (17001, 2, 40), (32767, 1, 9000)])
+                                   (1025, 3, 9), (2113, 2, 2000), (4230, 3, 6000), (27001, 1, 20000),
+                                   (32767, 1, 9000)])
 def test_exact_rows(W, H, n):
     """The row pass at its interval (32, 256, 1024), warp share and list-length
     edges: few seeds, and more than half of the columns in the list."""
