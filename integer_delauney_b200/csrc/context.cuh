@@ -90,13 +90,13 @@ struct DevBuf {
 // Device-side counters and flags of one pipeline run.  Lives in device memory;
 // a pinned host mirror receives it when the host needs a count.
 struct Scalars {
-    int64_t n_triangles;      // unique triangles after dedup
-    int64_t n_inserted;       // keys inserted into the hash table
+    int64_t n_triangles;      // unique triangles after dedup (the first 16 bytes are cleared together)
+    int32_t n_blocks;         // 2 x 2 blocks detection leaves to its second pass
+    int32_t overflow;         // hash table over its load limit or probe bound
     int64_t last_change;      // last propagation step (0-based) that changed a cell
     int32_t err_oob;          // a seed lay outside the canvas
     int32_t err_dup;          // two seeds share a pixel
     int32_t err_label;        // a caller-supplied label was outside [-1, n)
-    int32_t overflow;         // hash table over its load limit or probe bound
     int32_t max_side;         // longest triangle side, float-truncated (triangulation.cu:355-368)
     int32_t n_big;            // tall triangles the raster hands to its block-per-triangle pass
     int32_t n_handoff;        // micro-tiles the last tile round hands to the persistent kernel

@@ -44,92 +44,82 @@ __device__ __forceinline__ unsigned long long mix64(unsigned long long k)
 // (the zero vector included, atan2(+0, +0) = +0), y > 0 gives (0, pi) and
 // (x < 0, y == 0) gives pi.  Within the two open half planes the order is
 // the sign of the cross product.
-__device__ __forceinline__ int angle_class(long long x, long long y)
+__device__ __forceinline__ int angle_class(int x, int y)
 {
     if (y < 0) return 0;
     if (y == 0) return x >= 0 ? 1 : 3;
     return 2;
 }
 
-__device__ __forceinline__ bool angle_less(long long ax, long long ay, long long bx, long long by)
+__device__ __forceinline__ bool angle_less(int ax, int ay, int bx, int by)
 {
     const int ca = angle_class(ax, ay), cb = angle_class(bx, by);
     if (ca != cb) return ca < cb;
     if (ca == 1 || ca == 3) return false;
-    return ax * by - ay * bx > 0;
+    return (long long)ax * by - (long long)ay * bx > 0;
 }
 
 struct Emit {
-    int32_t o[2][3];
+    int32_t o0[3], o1[3];
     int n;
 };
 
+template <class V>
+__device__ __forceinline__ V pick(int i, V a, V b, V c, V d)
+{
+    return i == 0 ? a : i == 1 ? b : i == 2 ? c : d;
+}
+
 // The block rule of triangle_detect.cuh:75-166 on labels (a, b, c, d) =
-// (top-left, top-right, bottom-left, bottom-right).
+// (top-left, top-right, bottom-left, bottom-right).  Written without indexed
+// arrays, so that everything stays in registers.
 __device__ __forceinline__ void block_rule(int32_t a, int32_t b, int32_t c, int32_t d,
                                            const uint32_t* __restrict__ pos, Emit& e)
 {
     e.n = 0;
-    const int32_t q[4] = {a, b, c, d};
-    int32_t s[4];
-    int n = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        if (q[i] < 0) return;
-        bool dup = false;
-        for (int j = 0; j < n; ++j) dup |= (s[j] == q[i]);
-        if (!dup) s[n++] = q[i];
-    }
-    if (n == 3) {
-        e.o[0][0] = s[0]; e.o[0][1] = s[1]; e.o[0][2] = s[2];
+    if ((a | b | c | d) < 0) return;
+    const int same = (a == b) + (a == c) + (a == d) + (b == c) + (b == d) + (c == d);
+    if (same > 1) return;
+    if (same == 1) {   // three labels, in first-seen order
+        const bool bb = b == a, cc = c == a || c == b;
+        e.o0[0] = a;
+        e.o0[1] = bb ? c : b;
+        e.o0[2] = bb || cc ? d : c;
         e.n = 1;
         return;
     }
-    if (n != 4) return;
-
-    long long px[4], py[4];
-    long long sxs = 0, sys = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t p = __ldg(&pos[q[i]]);
-        px[i] = pos_x(p);
-        py[i] = pos_y(p);
-        sxs += px[i];
-        sys += py[i];
-    }
+    const uint32_t p0 = __ldg(&pos[a]), p1 = __ldg(&pos[b]), p2 = __ldg(&pos[c]), p3 = __ldg(&pos[d]);
+    const int x0 = pos_x(p0), x1 = pos_x(p1), x2 = pos_x(p2), x3 = pos_x(p3);
+    const int y0 = pos_y(p0), y1 = pos_y(p1), y2 = pos_y(p2), y3 = pos_y(p3);
+    const int sx = x0 + x1 + x2 + x3, sy = y0 + y1 + y2 + y3;
     // 4 * (p - centroid), exact in integers
-    long long vx[4], vy[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) { vx[i] = 4 * px[i] - sxs; vy[i] = 4 * py[i] - sys; }
-    int ord[4] = {0, 1, 2, 3};
-    for (int i = 1; i < 4; ++i) {   // stable insertion sort by angle
-        const int k = ord[i];
-        int j = i - 1;
-        while (j >= 0 && angle_less(vx[k], vy[k], vx[ord[j]], vy[ord[j]])) { ord[j + 1] = ord[j]; --j; }
-        ord[j + 1] = k;
-    }
+    const int vx0 = 4 * x0 - sx, vx1 = 4 * x1 - sx, vx2 = 4 * x2 - sx, vx3 = 4 * x3 - sx;
+    const int vy0 = 4 * y0 - sy, vy1 = 4 * y1 - sy, vy2 = 4 * y2 - sy, vy3 = 4 * y3 - sy;
+    // places in the stable order by angle: a later one goes first only if strictly less
+    const bool l10 = angle_less(vx1, vy1, vx0, vy0), l20 = angle_less(vx2, vy2, vx0, vy0),
+               l30 = angle_less(vx3, vy3, vx0, vy0), l21 = angle_less(vx2, vy2, vx1, vy1),
+               l31 = angle_less(vx3, vy3, vx1, vy1), l32 = angle_less(vx3, vy3, vx2, vy2);
+    const int r0 = l10 + l20 + l30, r1 = !l10 + l21 + l31, r2 = !l20 + !l21 + l32, r3 = !l30 + !l31 + !l32;
+    auto at_rank = [&](int r) { return r0 == r ? 0 : r1 == r ? 1 : r2 == r ? 2 : r3 == r ? 3 : 3; };
+    const int o0 = at_rank(0), o1 = at_rank(1), o2 = at_rank(2), o3 = at_rank(3);
     auto len2 = [&](int i, int j) {
-        const long long dx = px[i] - px[j], dy = py[i] - py[j];
-        return dx * dx + dy * dy;
+        const int dx = pick(i, x0, x1, x2, x3) - pick(j, x0, x1, x2, x3);
+        const int dy = pick(i, y0, y1, y2, y3) - pick(j, y0, y1, y2, y3);
+        return (uint32_t)(dx * dx) + (uint32_t)(dy * dy);
     };
-    const int d0a = ord[0], d0b = ord[2], d1a = ord[1], d1b = ord[3];
-    const long long l0 = len2(d0a, d0b), l1 = len2(d1a, d1b);
-    int pa, pb;
-    if (l0 < l1) { pa = d0a; pb = d0b; }
-    else if (l1 < l0) { pa = d1a; pb = d1b; }
-    else {
-        int lowest = 0;
-        for (int i = 1; i < 4; ++i) if (q[i] < q[lowest]) lowest = i;
-        if (lowest == d0a || lowest == d0b) { pa = d1a; pb = d1b; }
-        else { pa = d0a; pb = d0b; }
+    const uint32_t l0 = len2(o0, o2), l1 = len2(o1, o3);
+    bool first = l0 < l1;   // the diagonal o0 - o2
+    if (l0 == l1) {
+        const int lowest = a < b && a < c && a < d ? 0 : b < c && b < d ? 1 : c < d ? 2 : 3;
+        first = !(lowest == o0 || lowest == o2);
     }
-    int ra = -1, rb = -1;
-    for (int i = 0; i < 4; ++i) {
-        if (i == pa || i == pb) continue;
-        if (ra < 0) ra = i; else rb = i;
-    }
-    e.o[0][0] = q[pa]; e.o[0][1] = q[pb]; e.o[0][2] = q[ra];
-    e.o[1][0] = q[pa]; e.o[1][1] = q[pb]; e.o[1][2] = q[rb];
+    const int pa = first ? o0 : o1, pb = first ? o2 : o3;
+    const int u = first ? o1 : o0, v = first ? o3 : o2;
+    const int ra = min(u, v), rb = max(u, v);
+    e.o0[0] = e.o1[0] = pick(pa, a, b, c, d);
+    e.o0[1] = e.o1[1] = pick(pb, a, b, c, d);
+    e.o0[2] = pick(ra, a, b, c, d);
+    e.o1[2] = pick(rb, a, b, c, d);
     e.n = 2;
 }
 
@@ -169,37 +159,130 @@ __device__ __forceinline__ void hash_insert(unsigned long long key, unsigned lon
     atomicOr(&sc->overflow, 1);
 }
 
-// One thread per 2 x 2 block; a warp covers 32 adjacent blocks of a row.  A
-// key the block one column left (the previous lane) emitted as well is not
-// inserted again: that block's row-major index is smaller, so its atomicMin
-// already keeps a smaller witness than this one would.
-__global__ void __launch_bounds__(256)
-k_detect(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
-         const int32_t* __restrict__ rank, unsigned long long* __restrict__ table, unsigned long long mask,
-         Scalars* __restrict__ sc)
+__device__ __forceinline__ void detect_block(const int32_t* __restrict__ lab, int pitch, int Wd,
+                                             const uint32_t* __restrict__ pos, const int32_t* __restrict__ rank,
+                                             int x, int y, unsigned long long* __restrict__ table,
+                                             unsigned long long mask, Scalars* __restrict__ sc)
 {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (y >= Hd - 1) return;   // uniform over the warp (blockDim.x = 32)
-    unsigned long long k0 = EMPTY_KEY, k1 = EMPTY_KEY;
-    unsigned code0 = 0, code1 = 0;
-    if (x < Wd - 1) {
-        const int32_t a = lab[(size_t)y * pitch + x], b = lab[(size_t)y * pitch + x + 1];
-        const int32_t c = lab[(size_t)(y + 1) * pitch + x], d = lab[(size_t)(y + 1) * pitch + x + 1];
-        if (!(a == b && a == c && a == d) && !((a == b && c == d) || (a == c && b == d))) {
-            Emit e;
-            block_rule(a, b, c, d, pos, e);
-            if (e.n > 0) make_key(e.o[0], rank, k0, code0);
-            if (e.n > 1) make_key(e.o[1], rank, k1, code1);
-        }
-    }
-    const unsigned long long l0 = __shfl_up_sync(0xffffffffu, k0, 1), l1 = __shfl_up_sync(0xffffffffu, k1, 1);
-    const bool first = threadIdx.x == 0;
+    const int32_t* p = lab + (size_t)y * pitch + x;
+    Emit e;
+    block_rule(p[0], p[1], p[pitch], p[pitch + 1], pos, e);
     const unsigned long long blk = (unsigned long long)y * Wd + x;
-    if (k0 != EMPTY_KEY && (first || (k0 != l0 && k0 != l1))) hash_insert(k0, (blk << 4) | code0, table, mask, sc);
-    if (k1 != EMPTY_KEY && (first || (k1 != l0 && k1 != l1))) hash_insert(k1, (blk << 4) | code1, table, mask, sc);
+    unsigned long long key;
+    unsigned code;
+    if (e.n > 0) {
+        make_key(e.o0, rank, key, code);
+        hash_insert(key, (blk << 4) | code, table, mask, sc);
+    }
+    if (e.n > 1) {
+        make_key(e.o1, rank, key, code);
+        hash_insert(key, (blk << 4) | code, table, mask, sc);
+    }
 }
 
+// A warp covers a strip of DET_COLS x DET_ROWS blocks (2 x 2 cells each, by
+// their top-left cell): four columns per lane, the label rows streaming
+// through registers, so that the plane is read once and a block costs a few
+// comparisons.  The blocks with three or four labels (one in forty at 200 000
+// seeds in 4096 x 4096) go into a queue in shared memory first and are worked
+// off 32 at a time: run in place, the rule and the table's round trips occupy
+// a whole warp for the one or two lanes that have a vertex.  A strip with more
+// than DET_OWN of them (a dense blob) leaves the others to k_detect_rest, which
+// spreads them over the device.
+// Canvases too small to fill the device with such strips use shorter ones.
+constexpr int DET_COLS = 128, DET_ROWS = 16, DET_ROWS_SMALL = 4, DET_WARPS = 4, DET_OWN = 96;
+static_assert(DET_ROWS * 4 == 64, "a lane's blocks are the bits of one 64-bit mask");
+
+template <int ROWS>
+__global__ void __launch_bounds__(DET_WARPS * 32)
+k_detect(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
+         const int32_t* __restrict__ rank, unsigned long long* __restrict__ table, unsigned long long mask,
+         Scalars* __restrict__ sc, uint32_t* __restrict__ rest, int rest_cap)
+{
+    __shared__ uint16_t queue[DET_WARPS][DET_COLS * ROWS];
+    uint16_t* q = queue[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int xs = blockIdx.x * DET_COLS, ys = (blockIdx.y * DET_WARPS + (threadIdx.x >> 5)) * ROWS;
+    if (ys >= Hd - 1) return;
+    const int x0 = xs + lane * 4;
+    // one row's five labels: the lane's four columns and the next (rows are
+    // padded to a multiple of 32 columns; blocks beyond Wd - 1 are masked out;
+    // a row past the canvas has none).  Four rows are loaded at a time.
+    auto load = [&](int y, int4& v, int32_t& edge) {
+        const int32_t* p = lab + (size_t)y * pitch + x0;
+        const bool in = y < Hd && x0 < Wd;
+        v = in ? __ldg(reinterpret_cast<const int4*>(p)) : make_int4(-1, -1, -1, -1);
+        edge = in && lane == 31 && x0 + 4 < Wd ? __ldg(p + 4) : -1;
+    };
+    int4 up;
+    int32_t up_edge;
+    load(ys, up, up_edge);
+    int32_t up_next = __shfl_down_sync(0xffffffffu, up.x, 1);
+    if (lane == 31) up_next = up_edge;
+    unsigned long long hit = 0;
+#pragma unroll
+    for (int r0 = 0; r0 < ROWS; r0 += 4) {
+        int4 v[4];
+        int32_t edge[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) load(ys + r0 + j + 1, v[j], edge[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int4 dn = v[j];
+            int32_t dn_next = __shfl_down_sync(0xffffffffu, dn.x, 1);
+            if (lane == 31) dn_next = edge[j];
+            const int32_t u[5] = {up.x, up.y, up.z, up.w, up_next}, d[5] = {dn.x, dn.y, dn.z, dn.w, dn_next};
+            unsigned here = 0;
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int32_t A = u[c], B = u[c + 1], C = d[c], D = d[c + 1];
+                // three or four different labels: at most one of the six pairs is equal
+                const int same = (A == B) + (C == D) + (A == C) + (B == D) + (A == D) + (B == C);
+                if (same <= 1 && (A | B | C | D) >= 0) here |= 1u << c;
+            }
+            hit |= (unsigned long long)here << (4 * (r0 + j));
+            up = dn;
+            up_next = dn_next;
+        }
+    }
+    // columns whose block has no right cell
+    const int valid = min(max(Wd - 1 - x0, 0), 4);
+    if (valid < 4) hit &= 0x1111111111111111ull * ((1u << valid) - 1u);
+    const int mine = __popcll(hit);
+    int incl = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+    }
+    const int total = __shfl_sync(0xffffffffu, incl, 31);
+    for (int at = incl - mine; hit; ++at) {
+        const int b = __ffsll((long long)hit) - 1;
+        hit &= hit - 1;
+        q[at] = (uint16_t)((b >> 2) * DET_COLS + lane * 4 + (b & 3));
+    }
+    __syncwarp();
+    for (int i = lane; i < min(total, DET_OWN); i += 32)
+        detect_block(lab, pitch, Wd, pos, rank, xs + q[i] % DET_COLS, ys + q[i] / DET_COLS, table, mask, sc);
+    if (total <= DET_OWN) return;
+    int at = lane == 0 ? atomicAdd(&sc->n_blocks, total - DET_OWN) : 0;
+    at = __shfl_sync(0xffffffffu, at, 0);
+    for (int i = DET_OWN + lane; i < total; i += 32) {
+        const int x = xs + q[i] % DET_COLS, y = ys + q[i] / DET_COLS, k = at + i - DET_OWN;
+        if (k < rest_cap) rest[k] = pack_pos(x, y);
+        else detect_block(lab, pitch, Wd, pos, rank, x, y, table, mask, sc);
+    }
+}
+
+__global__ void __launch_bounds__(128)
+k_detect_rest(const int32_t* __restrict__ lab, int pitch, int Wd, const uint32_t* __restrict__ pos,
+              const int32_t* __restrict__ rank, unsigned long long* __restrict__ table, unsigned long long mask,
+              Scalars* __restrict__ sc, const uint32_t* __restrict__ rest, int rest_cap)
+{
+    const int n = min(sc->n_blocks, rest_cap);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+        detect_block(lab, pitch, Wd, pos, rank, pos_x(rest[i]), pos_y(rest[i]), table, mask, sc);
+}
 
 // Compaction of the occupied slots with one atomic per block on the row
 // counter (one per warp, 65 k of them on a 2 M-slot table, serialised on that
@@ -301,7 +384,8 @@ void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const
                       int shift, cudaEvent_t mid, const int32_t* rank)
 {
     // Unique triangles of a planar triangulation number under 2n; the table
-    // starts at four times that, and on the rare probe overflow it grows and
+    // starts at four times that (a table half that size probes longer: 70 us
+    // against 53 us of detection at 200 000 seeds), and on the rare probe overflow it grows and
     // the detection is redone.  The occupied slots are counted while they are
     // compacted (one atomic per block), not while they are inserted, where a
     // single counter would serialise every new key.
@@ -319,14 +403,23 @@ void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const
         C.grp.ensure((size_t)cap * 4);
         C.tris.ensure((size_t)cap * 5 * 4);
         IDL_CUDA(cudaMemsetAsync(C.hkeys.ptr, 0xFF, (size_t)cap * 16, C.stream));
-        IDL_CUDA(cudaMemsetAsync(&C.sc()->overflow, 0, sizeof(int32_t), C.stream));
-        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, sizeof(int64_t), C.stream));
+        // the blocks left to k_detect_rest wait in the grouping buffer, free until then
+        uint32_t* rest = C.grp.as<uint32_t>();
+        static_assert(offsetof(Scalars, overflow) == 12 && offsetof(Scalars, n_blocks) == 8, "cleared together");
+        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
         IDL_CUDA(cudaMemsetAsync(C.cnt.ptr, 0, (size_t)(n + 1) * 4, C.stream));
 
-        dim3 blk(32, 8);
-        dim3 grd(ceil_div(std::max(cv.Wd - 1, 1), 32), ceil_div(std::max(cv.Hd - 1, 1), 8));
-        k_detect<<<grd, blk, 0, C.stream>>>(labels, cv.pitch, cv.Wd, cv.Hd, pos, rank, C.hkeys.as<unsigned long long>(),
-                                            (unsigned long long)(cap - 1), C.sc());
+        const int strips = ceil_div(std::max(cv.Wd - 1, 1), DET_COLS);
+        const bool small = strips * ceil_div(cv.Hd, DET_ROWS) < C.num_sms * 16;
+        const dim3 grd(strips, ceil_div(std::max(cv.Hd - 1, 1), (small ? DET_ROWS_SMALL : DET_ROWS) * DET_WARPS));
+        auto* detect = small ? k_detect<DET_ROWS_SMALL> : k_detect<DET_ROWS>;
+        detect<<<grd, DET_WARPS * 32, 0, C.stream>>>(labels, cv.pitch, cv.Wd, cv.Hd, pos, rank,
+                                                     C.hkeys.as<unsigned long long>(), (unsigned long long)(cap - 1),
+                                                     C.sc(), rest, (int)cap);
+        IDL_LAUNCH();
+        k_detect_rest<<<C.num_sms * 4, 128, 0, C.stream>>>(labels, cv.pitch, cv.Wd, pos, rank,
+                                                          C.hkeys.as<unsigned long long>(),
+                                                          (unsigned long long)(cap - 1), C.sc(), rest, (int)cap);
         IDL_LAUNCH();
         if (mid) IDL_CUDA(cudaEventRecord(mid, C.stream));
         C.mark(PM_DETECT);
