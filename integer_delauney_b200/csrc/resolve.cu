@@ -117,47 +117,48 @@ __device__ __forceinline__ int isqrt(int32_t v)   // floor, v >= 0
 
 // ---- (1) roots and suspects -------------------------------------------
 
-// A warp walks 128 columns (four per lane) down ROOT_ROWS rows with the rows
-// above, at and below in registers, so the label plane is read once (plus two
-// rows per strip); cells whose four neighbours share their owner are skipped
-// without a seed-table load.  PASSES: also the largest A of a linked cell
-// (sc->arrive_max) for the pass count.
-constexpr int ROOT_ROWS = 16;
+// A warp takes 128 columns (four per lane) by ROOT_ROWS rows, loaded at once
+// with the rows above and below; cells whose four neighbours share their owner
+// are skipped without a seed-table load.  PASSES: also the largest A of a
+// linked cell (sc->arrive_max) for the pass count.
+constexpr int ROOT_ROWS = 8;
 
 template <bool PASSES>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(128)
 k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
         uint32_t* __restrict__ sus, int words, int32_t* __restrict__ list, int cap, Scalars* __restrict__ sc)
 {
     const int lane = threadIdx.x & 31;
     const int x0 = (blockIdx.x * 32 + lane) * 4;
-    const int y0 = (blockIdx.y * 8 + (threadIdx.x >> 5)) * ROOT_ROWS;
+    const int y0 = (blockIdx.y * 4 + (threadIdx.x >> 5)) * ROOT_ROWS;
     if (y0 >= Hd) return;
-    const int y1 = min(Hd, y0 + ROOT_ROWS);
-    auto load = [&](int y, int32_t (&r)[4]) {
-        const bool row_in = y >= 0 && y < Hd;
-        if (row_in && x0 < Wd) {   // rows are padded to a multiple of 32 columns
-            const int4 v = *reinterpret_cast<const int4*>(lab + (size_t)y * pitch + x0);
-            r[0] = v.x; r[1] = v.y; r[2] = v.z; r[3] = v.w;
-        } else {
-            r[0] = r[1] = r[2] = r[3] = OUTSIDE;
-        }
-    };
-    int32_t up[4], cur[4], dn[4];
-    load(y0 - 1, up);
-    load(y0, cur);
+    int4 v[ROOT_ROWS + 2];
+    int32_t edge[ROOT_ROWS];   // lane 0: the cell left of the warp's columns, lane 31: right of them
+#pragma unroll
+    for (int j = 0; j < ROOT_ROWS + 2; ++j) {
+        const int y = y0 + j - 1;
+        const bool in = y >= 0 && y < Hd && x0 < Wd;   // rows are padded to a multiple of 32 columns
+        const int32_t* p = lab + (size_t)y * pitch + x0;
+        v[j] = in ? __ldg(reinterpret_cast<const int4*>(p)) : make_int4(OUTSIDE, OUTSIDE, OUTSIDE, OUTSIDE);
+        if (j >= 1 && j <= ROOT_ROWS)
+            edge[j - 1] = in && lane == 0 && x0 > 0 ? __ldg(p - 1)
+                          : in && lane == 31 && x0 + 4 < Wd ? __ldg(p + 4) : OUTSIDE;
+    }
     int far = 0;
-    for (int y = y0; y < y1; ++y) {
-        load(y + 1, dn);
-        int32_t lf = __shfl_up_sync(FULL, cur[3], 1), rt = __shfl_down_sync(FULL, cur[0], 1);
-        if (lane == 0 && x0 > 0 && x0 < Wd) lf = lab[(size_t)y * pitch + x0 - 1];
-        if (lane == 31 && x0 + 4 < Wd) rt = lab[(size_t)y * pitch + x0 + 4];
+#pragma unroll
+    for (int j = 1; j <= ROOT_ROWS; ++j) {
+        const int y = y0 + j - 1;
+        const int4 up = v[j - 1], cur = v[j], dn = v[j + 1];
+        int32_t lf = __shfl_up_sync(FULL, cur.w, 1), rt = __shfl_down_sync(FULL, cur.x, 1);
+        if (lane == 0) lf = edge[j - 1];
+        if (lane == 31) rt = edge[j - 1];
+        const int32_t row[6] = {lf, cur.x, cur.y, cur.z, cur.w, rt};
+        const int32_t above[4] = {up.x, up.y, up.z, up.w}, below[4] = {dn.x, dn.y, dn.z, dn.w};
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
             const int x = x0 + c;
-            const int32_t s = cur[c];
+            const int32_t s = row[c + 1], L = row[c], R = row[c + 2], U = above[c], D = below[c];
             if (x >= Wd || s < 0) continue;
-            const int32_t L = c > 0 ? cur[c - 1] : lf, R = c < 3 ? cur[c + 1] : rt, U = up[c], D = dn[c];
             if (!PASSES && L == s && R == s && U == s && D == s) continue;
             const uint32_t p = __ldg(&pos[s]);
             const int dx = pos_x(p) - x, dy = pos_y(p) - y;
@@ -171,11 +172,6 @@ k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32
             } else if (PASSES) {
                 far = max(far, abs(dx) + abs(dy));
             }
-        }
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            up[c] = cur[c];
-            cur[c] = dn[c];
         }
     }
     if (PASSES) {
@@ -666,11 +662,11 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
     const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), C.exact_bands.as<int32_t>(), pos, sus, images,
                  seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n)};
-    const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 8 * ROOT_ROWS));
+    const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 4 * ROOT_ROWS));
     if (passes)
-        k_roots<true><<<g, 256, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
+        k_roots<true><<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
     else
-        k_roots<false><<<g, 256, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
+        k_roots<false><<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
     IDL_LAUNCH();
     const int gs = std::max(1, std::min(ceil_div(cap, 128), C.num_sms));
     k_suspects<<<gs, 128, 0, C.stream>>>(V, sus, list, cap, C.sc());
