@@ -43,7 +43,8 @@ struct BImg {
     int ox, oy;        // atlas origin of the padded canvas
     long long seed_off;  // first global seed id
     long long px_off;    // first output pixel (prefix of W*H); also the bitmap base
-    long long row_off;   // first output row (prefix of H)
+    int tile_off;        // first raster tile
+    int tiles_x;         // raster tiles per row
 };
 
 __global__ void k_b_mark(const int32_t* __restrict__ xy, int64_t n, const int32_t* __restrict__ seed_img,
@@ -118,64 +119,107 @@ __device__ __forceinline__ int tri_image(const int32_t* row, const int32_t* __re
     return sid_img[min(row[2], min(row[3], row[4]))];
 }
 
-// Per-image triangle count and per-image longest side.
-__global__ void k_b_tri_stats(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc,
-                              const int32_t* __restrict__ sid_img, const int32_t* __restrict__ xs,
-                              const int32_t* __restrict__ ys, int32_t* __restrict__ count, int32_t* __restrict__ side)
+// off[i] = first triangle of image i (off[n_images]: all of them).  Triangles
+// are numbered by their smallest vertex and seeds image after image, so an
+// image's triangles are contiguous: each boundary is written once, with no
+// count per triangle (those atomics on a few hundred counters took 460 us for
+// 1.2 M triangles of 512 images).
+__global__ void k_b_tri_off(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc,
+                            const int32_t* __restrict__ sid_img, int n_images, int32_t* __restrict__ off)
 {
     const long long nt = sc->n_triangles;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nt;
+    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t <= nt;
          t += (long long)gridDim.x * blockDim.x) {
-        const int32_t* row = tris + t * 5;
-        const int im = tri_image(row, sid_img);
-        atomicAdd(&count[im], 1);
-        const int s = tri_max_side(row + 2, xs, ys);
-        if (s > 0) atomicMax(&side[im], s);
+        const int im = t < nt ? tri_image(tris + t * 5, sid_img) : n_images;
+        const int before = t > 0 ? tri_image(tris + (t - 1) * 5, sid_img) : -1;
+        for (int i = before + 1; i <= im; ++i) off[i] = (int32_t)t;
     }
 }
 
-// One warp per triangle, into its own image's grid, with its image's window.
+// The raster passes of raster.cu over the tiles of all images; the longest
+// side is kept per image.
 __global__ void __launch_bounds__(256)
-k_b_raster(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, const int32_t* __restrict__ sid_img,
-           const BImg* __restrict__ imgs, const int32_t* __restrict__ xs, const int32_t* __restrict__ ys,
-           const int32_t* __restrict__ side, const int32_t* __restrict__ tri_off, int32_t* __restrict__ tgrid)
+k_b_raster_count(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc,
+                 const int32_t* __restrict__ sid_img, const BImg* __restrict__ imgs, const int32_t* __restrict__ xs,
+                 const int32_t* __restrict__ ys, int32_t* __restrict__ side, RasterWork w)
 {
-    const long long nt = sc->n_triangles;
-    const int lane = threadIdx.x & 31;
-    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += warps) {
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    const bool on = t < sc->n_triangles;
+    Tri u{};
+    int im = -1, side_here = 0, W = 0, H = 0, tile_off = 0, tiles_x = 0;
+    if (on) {
         const int32_t* row = tris + t * 5;
-        const int im = tri_image(row, sid_img);
-        const BImg m = imgs[im];
-        raster_one(row + 2, (int32_t)(t - tri_off[im]), xs, ys, m.W, m.H, max(20, side[im] + 3),
-                   tgrid + m.px_off, lane);
+        im = tri_image(row, sid_img);
+        u = load_tri(row + 2, xs, ys);
+        side_here = longest_side(u);
+        W = imgs[im].W;
+        H = imgs[im].H;
+        tile_off = imgs[im].tile_off;
+        tiles_x = imgs[im].tiles_x;
     }
+    // a warp's triangles are mostly one image's: one atomic for all of them
+    const int im0 = __shfl_sync(0xFFFFFFFFu, im, 0);
+    if (__all_sync(0xFFFFFFFFu, im == im0 || im < 0)) {
+        const int s = __reduce_max_sync(0xFFFFFFFFu, side_here);
+        if ((threadIdx.x & 31) == 0 && im0 >= 0) atomicMax(&side[im0], s);
+    } else if (on) {
+        atomicMax(&side[im], side_here);
+    }
+    raster_count<TileLarge>(w, on, (int32_t)t, u, W, H, tile_off, tiles_x);
+    raster_offsets<256>(w);
 }
 
-// Block per output row: (local seed id, squared distance, triangle id).
-__global__ void k_b_compose(const int32_t* __restrict__ lab, int pitch, int P, const BImg* __restrict__ imgs,
-                            const int32_t* __restrict__ row_img, const int32_t* __restrict__ xs,
-                            const int32_t* __restrict__ ys, const int32_t* __restrict__ tgrid,
-                            int32_t* __restrict__ out)
+__global__ void __launch_bounds__(256)
+k_b_raster_fill(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc,
+                const int32_t* __restrict__ sid_img, const BImg* __restrict__ imgs, RasterWork w)
 {
-    const long long r = blockIdx.x;
-    const int im = row_img[r];
-    const BImg m = imgs[im];
-    const int y = (int)(r - m.row_off);
-    const int32_t* src = lab + (size_t)(m.oy + P + y) * pitch + m.ox + P;
-    const size_t base = (size_t)m.px_off + (size_t)y * m.W;
-    for (int x = threadIdx.x; x < m.W; x += blockDim.x) {
-        const int32_t l = src[x];
-        int32_t d = -1, id = l;
-        if (l >= 0) {
-            const int32_t dx = x - __ldg(&xs[l]), dy = y - __ldg(&ys[l]);
-            d = dx * dx + dy * dy;
-            id = (int32_t)(l - m.seed_off);
-        }
-        int32_t* o = out + (base + x) * 3;
-        o[0] = id;
-        o[1] = d;
-        o[2] = tgrid[base + x];
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (w.head->overflow) return;
+    const bool on = t < sc->n_triangles;
+    const BImg& m = imgs[on ? tri_image(tris + t * 5, sid_img) : 0];
+    raster_fill<TileLarge>(w, on, (int32_t)t, m.W, m.H, m.tile_off, m.tiles_x);
+}
+
+// A tile of its image drawn and composed: (local seed id, squared distance,
+// triangle id) per pixel.
+__global__ void __launch_bounds__(TILE_THREADS)
+k_b_raster_compose(RasterWork w, const BImg* __restrict__ imgs, int n_images, const int32_t* __restrict__ tri_off,
+                   const int32_t* __restrict__ lab, int pitch, int P, const int32_t* __restrict__ xs,
+                   const int32_t* __restrict__ ys, int32_t* __restrict__ out)
+{
+    __shared__ int32_t pix[TileLarge::H * TileLarge::PITCH];
+    int lo = 0, hi = n_images - 1;   // the last image whose first tile is at or before this one
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(&imgs[mid].tile_off) <= (int)blockIdx.x) lo = mid;
+        else hi = mid - 1;
+    }
+    const BImg m = imgs[lo];
+    const int k = (int)blockIdx.x - m.tile_off, tx = k % m.tiles_x, ty = k / m.tiles_x;
+    raster_tile<TileLarge>(w, pix, blockIdx.x, tx, ty, m.W, m.H, tri_off[lo]);
+    compose_tile<TileLarge>(pix, tx, ty, m.W, m.H, lab + (size_t)(m.oy + P) * pitch + m.ox + P, pitch, xs, ys,
+                 (int32_t)m.seed_off, out + m.px_off * 3);
+}
+
+__global__ void __launch_bounds__(128)
+k_b_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc,
+                const int32_t* __restrict__ sid_img, const BImg* __restrict__ imgs, const int32_t* __restrict__ xs,
+                const int32_t* __restrict__ ys, const int32_t* __restrict__ side,
+                const int32_t* __restrict__ tri_off, int32_t* __restrict__ out, RasterWork w)
+{
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    const bool all = w.head->overflow != 0;
+    const long long n = all ? sc->n_triangles : w.head->n_lines;
+    for (long long i = warp; i < n; i += warps) {
+        const int32_t t = all ? (int32_t)i : w.lines[i];
+        const int32_t* row = tris + (size_t)t * 5;
+        const int im = tri_image(row, sid_img);
+        const BImg& m = imgs[im];
+        const Tri u = load_tri(row + 2, xs, ys);
+        int32_t* ids = out + m.px_off * 3 + 2;
+        const int32_t id = t - tri_off[im];
+        if (!u.line) raster_direct(u, ids, 3, m.W, m.H, id);
+        else if ((threadIdx.x & 31) == 0) raster_line(u, ids, 3, m.W, m.H, id, max(20, side[im] + 3));
     }
 }
 
@@ -201,9 +245,9 @@ inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::max<int64_t
 
 struct Plan {
     std::vector<BImg> imgs;
-    std::vector<int32_t> seed_img, row_img;
+    std::vector<int32_t> seed_img;
     int AW = 0, AH = 0;
-    int64_t n_seeds = 0, n_px = 0, n_rows = 0;
+    int64_t n_seeds = 0, n_px = 0, n_tiles = 0;
 };
 
 // Shelf packing of the padded canvases, tallest first, one wall cell apart.
@@ -231,10 +275,11 @@ Plan make_plan(int n_images, const int32_t* dims, const int64_t* counts, int P)
         m.H = H;
         m.seed_off = pl.n_seeds;
         m.px_off = pl.n_px;
-        m.row_off = pl.n_rows;
         pl.n_seeds += n;
         pl.n_px += (int64_t)W * H;
-        pl.n_rows += H;
+        m.tile_off = (int)pl.n_tiles;
+        m.tiles_x = ceil_div(W, TileLarge::W);
+        pl.n_tiles += (int64_t)m.tiles_x * ceil_div(H, TileLarge::H);
         area += (double)(W + 2 * P + 1) * (H + 2 * P + 1);
         max_wp = std::max(max_wp, W + 2 * P + 1);
     }
@@ -264,10 +309,8 @@ Plan make_plan(int n_images, const int32_t* dims, const int64_t* counts, int P)
     pl.AW = AW;
     pl.AH = (int)AH;
     pl.seed_img.resize(pl.n_seeds);
-    pl.row_img.resize(pl.n_rows);
     for (int i = 0; i < n_images; ++i) {
         std::fill(pl.seed_img.begin() + pl.imgs[i].seed_off, pl.seed_img.begin() + pl.imgs[i].seed_off + counts[i], i);
-        std::fill(pl.row_img.begin() + pl.imgs[i].row_off, pl.row_img.begin() + pl.imgs[i].row_off + pl.imgs[i].H, i);
     }
     return pl;
 }
@@ -340,15 +383,12 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     const int64_t n = pl.n_seeds;
     C.batch_img.ensure(pl.imgs.size() * sizeof(BImg));
     C.batch_seed_img.ensure((size_t)n * 4);
-    C.batch_rows.ensure((size_t)pl.n_rows * 4);
     C.batch_sid.ensure((size_t)n * 4);
-    C.batch_stats.ensure(((size_t)n_images * 3 + 1) * 4);
+    C.batch_stats.ensure(((size_t)n_images * 2 + 1) * 4);
     BImg* d_imgs = C.batch_img.as<BImg>();
     IDL_CUDA(cudaMemcpyAsync(d_imgs, pl.imgs.data(), pl.imgs.size() * sizeof(BImg), cudaMemcpyHostToDevice,
                              C.stream));
     IDL_CUDA(cudaMemcpyAsync(C.batch_seed_img.ptr, pl.seed_img.data(), (size_t)n * 4, cudaMemcpyHostToDevice,
-                             C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_rows.ptr, pl.row_img.data(), (size_t)pl.n_rows * 4, cudaMemcpyHostToDevice,
                              C.stream));
     cudaEvent_t ev[5] = {};
     if (timings)
@@ -447,42 +487,49 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     }
 
     // per-image counts, offsets and windows; raster; compose
-    int32_t* cnt = C.batch_stats.as<int32_t>();
-    int32_t* side = cnt + n_images;
+    int32_t* side = C.batch_stats.as<int32_t>();
     int32_t* off = side + n_images;   // n_images + 1
-    IDL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)n_images * 2 * 4, C.stream));
-    k_b_tri_stats<<<C.num_sms * 8, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(),
-                                                       C.xs.as<int32_t>(), C.ys.as<int32_t>(), cnt, side);
-    IDL_LAUNCH();
-    exclusive_scan(C, cnt, off, n_images);
-    C.tgrid.ensure((size_t)pl.n_px * 4);
-    IDL_CUDA(cudaMemsetAsync(C.tgrid.ptr, 0xFF, (size_t)pl.n_px * 4, C.stream));
-    k_b_raster<<<C.num_sms * 16, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(), d_imgs,
-                                                     C.xs.as<int32_t>(), C.ys.as<int32_t>(), side, off,
-                                                     C.tgrid.as<int32_t>());
+    const int64_t nt = C.host_sc->n_triangles;
+    IDL_CUDA(cudaMemsetAsync(side, 0, (size_t)n_images * 4, C.stream));
+    k_b_tri_off<<<nblk(nt + 1), 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(), n_images,
+                                                   off);
     IDL_LAUNCH();
     int32_t* out = d_out;
     if (!out) {
         C.outgrid.ensure((size_t)pl.n_px * 12);
         out = C.outgrid.as<int32_t>();
     }
-    k_b_compose<<<(unsigned)pl.n_rows, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, P, d_imgs,
-                                                          C.batch_rows.as<int32_t>(), C.xs.as<int32_t>(),
-                                                          C.ys.as<int32_t>(), C.tgrid.as<int32_t>(), out);
+    const RasterWork w = raster_work(C, nt, pl.n_tiles);
+    const int32_t* sid = C.batch_sid.as<int32_t>();
+    const int32_t *xs = C.xs.as<int32_t>(), *ys = C.ys.as<int32_t>(), *tris = C.tris.as<int32_t>();
+    if (nt > 0) {
+        k_b_raster_count<<<nblk(nt), 256, 0, C.stream>>>(tris, C.sc(), sid, d_imgs, xs, ys, side, w);
+        IDL_LAUNCH();
+        k_b_raster_fill<<<nblk(nt), 256, 0, C.stream>>>(tris, C.sc(), sid, d_imgs, w);
+        IDL_LAUNCH();
+    } else {
+        IDL_CUDA(cudaMemsetAsync(w.off, 0, ((size_t)pl.n_tiles + 1) * 4, C.stream));
+    }
+    k_b_raster_compose<<<(unsigned)pl.n_tiles, TILE_THREADS, 0, C.stream>>>(w, d_imgs, n_images, off,
+                                                                          C.lab[0].as<int32_t>(), cv.pitch, P, xs, ys,
+                                                                          out);
     IDL_LAUNCH();
+    if (nt > 0) {
+        k_b_raster_rest<<<C.num_sms, 128, 0, C.stream>>>(tris, C.sc(), sid, d_imgs, xs, ys, side, off, out, w);
+        IDL_LAUNCH();
+    }
     k_b_localise<<<C.num_sms * 8, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(),
                                                       d_imgs, P);
     IDL_LAUNCH();
     mark(4);
-    std::vector<int32_t> hc(n_images);
-    IDL_CUDA(cudaMemcpyAsync(hc.data(), cnt, (size_t)n_images * 4, cudaMemcpyDeviceToHost, C.stream));
+    std::vector<int32_t> ho((size_t)n_images + 1);
+    IDL_CUDA(cudaMemcpyAsync(ho.data(), off, ho.size() * 4, cudaMemcpyDeviceToHost, C.stream));
     C.fetch_scalars();
     C.last_n_tri = C.host_sc->n_triangles;
     C.have_result = true;
     if (tri_counts)
-        for (int i = 0; i < n_images; ++i) tri_counts[i] = hc[i];
-    bp->tri_off.assign((size_t)n_images + 1, 0);
-    for (int i = 0; i < n_images; ++i) bp->tri_off[i + 1] = bp->tri_off[i] + hc[i];
+        for (int i = 0; i < n_images; ++i) tri_counts[i] = ho[i + 1] - ho[i];
+    bp->tri_off.assign(ho.begin(), ho.end());
     bp->grids = out;
     bp->full = true;
     if (timings) {

@@ -58,74 +58,6 @@ namespace {
 
 // ---- output composition ------------------------------------------------
 
-// (H, W, 3): seed id and squared distance from the interior window of the
-// detection canvas, triangle id from the assignment (triangulation.cu:391-412).
-// A block composes 256 consecutive pixels of the flattened image in shared
-// memory and stores their 3 KB as 16-byte vectors when the output is 16-byte
-// aligned (each block's slice starts at a multiple of 3 KB), instead of
-// three 4-byte stores 12 bytes apart per pixel.
-constexpr int COMPOSE_PX = 256;
-
-__global__ void __launch_bounds__(COMPOSE_PX)
-k_compose3(const int32_t* __restrict__ lab, int pitch, int P, int W, int64_t n_px, const int32_t* __restrict__ xs,
-           const int32_t* __restrict__ ys, const int32_t* __restrict__ tgrid, int32_t* __restrict__ out, bool vec)
-{
-    __shared__ __align__(16) int32_t stage[COMPOSE_PX * 3];
-    const int64_t i0 = (int64_t)blockIdx.x * COMPOSE_PX;
-    const int64_t i = i0 + threadIdx.x;
-    if (i < n_px) {
-        const int y = (int)(i / W), x = (int)(i - (int64_t)y * W);
-        const int32_t l = lab[(size_t)(y + P) * pitch + x + P];
-        int32_t d = -1;
-        if (l >= 0) {
-            const int32_t dx = x - __ldg(&xs[l]), dy = y - __ldg(&ys[l]);
-            d = dx * dx + dy * dy;
-        }
-        stage[threadIdx.x * 3] = l;
-        stage[threadIdx.x * 3 + 1] = d;
-        stage[threadIdx.x * 3 + 2] = tgrid ? tgrid[i] : -1;
-    }
-    __syncthreads();
-    const int64_t n_here = min((int64_t)COMPOSE_PX, n_px - i0) * 3;   // ints of this block's slice
-    int32_t* dst = out + i0 * 3;
-    if (vec && n_here == COMPOSE_PX * 3) {
-        if (threadIdx.x < COMPOSE_PX * 3 / 4)
-            reinterpret_cast<int4*>(dst)[threadIdx.x] = reinterpret_cast<const int4*>(stage)[threadIdx.x];
-    } else {
-        for (int k = threadIdx.x; k < n_here; k += COMPOSE_PX) dst[k] = stage[k];
-    }
-}
-
-// k_compose3 four pixels of one row per thread, for W and P multiples of 4
-// and a 16-byte aligned output: 16-byte loads of the labels and triangle ids,
-// three 16-byte stores of the four (id, d2, triangle) triples.
-__global__ void __launch_bounds__(256)
-k_compose3x4(const int32_t* __restrict__ lab, int pitch, int P, int W, int64_t n_quads,
-             const int32_t* __restrict__ xs, const int32_t* __restrict__ ys, const int32_t* __restrict__ tgrid,
-             int32_t* __restrict__ out)
-{
-    const int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= n_quads) return;
-    const int64_t i = q * 4;
-    const int y = (int)(i / W), x = (int)(i - (int64_t)y * W);
-    const int4 l4 = *reinterpret_cast<const int4*>(lab + (size_t)(y + P) * pitch + x + P);
-    const int4 t4 = *reinterpret_cast<const int4*>(tgrid + i);
-    const int32_t l[4] = {l4.x, l4.y, l4.z, l4.w};
-    int32_t d[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        d[k] = -1;
-        if (l[k] >= 0) {
-            const int32_t dx = x + k - __ldg(&xs[l[k]]), dy = y - __ldg(&ys[l[k]]);
-            d[k] = dx * dx + dy * dy;
-        }
-    }
-    int4* o = reinterpret_cast<int4*>(out + i * 3);
-    o[0] = make_int4(l[0], d[0], t4.x, l[1]);
-    o[1] = make_int4(d[1], t4.y, l[2], d[2]);
-    o[2] = make_int4(t4.z, l[3], d[3], t4.w);
-}
-
 // (a, b, c) of each (x, y, a, b, c) triangle row.
 __global__ void k_tri_vertices(const int32_t* __restrict__ tris, int64_t n, int32_t* __restrict__ verts)
 {
@@ -269,9 +201,10 @@ bool finish_resolved(Context& C, bool want_passes, int64_t* passes = nullptr)
 }
 
 // Run stages (a) (b) (d) with seeds already in C.seeds_in.  Leaves labels in
-// C.lab[0], triangles in C.tris, pixel ids in C.tgrid; returns triangle count.
+// C.lab[0], triangles in C.tris, the composed (H, W, 3) grid in d_out; returns
+// the triangle count.
 int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgrid_host_or_dev, bool vgrid_on_host,
-                        int P, int mode, float* timings, Canvas& cv_out)
+                        int P, int mode, float* timings, Canvas& cv_out, int32_t* d_out)
 {
     const Canvas cv = make_canvas(W + 2 * P, H + 2 * P);
     cv_out = cv;
@@ -322,9 +255,20 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     // does not change it): no second host round trip here
     const int64_t nt = C.host_sc->n_triangles;
     T.mark(3);
-    C.tgrid.ensure((size_t)W * H * sizeof(int32_t));
-    assign_pixels(C, W, H, C.xs.as<int32_t>(), C.ys.as<int32_t>(), C.tgrid.as<int32_t>(), nt);
-    C.mark(PM_ASSIGN);
+    const int32_t *xs = C.xs.as<int32_t>(), *ys = C.ys.as<int32_t>();
+    if (vgrid_host_or_dev && P == 0) {   // channels 0 and 1 are the caller's
+        C.tgrid.ensure((size_t)W * H * sizeof(int32_t));
+        assign_pixels(C, W, H, xs, ys, C.tgrid.as<int32_t>(), nt);
+        C.mark(PM_ASSIGN);
+        k_compose3_from_grid<<<dim3(ceil_div(W, 256), H), 256, 0, C.stream>>>(C.vgrid.as<int32_t>(), W, H,
+                                                                             C.tgrid.as<int32_t>(), d_out);
+        IDL_LAUNCH();
+        C.mark(PM_COMPOSE);
+    } else {
+        assign_and_compose(C, W, H, xs, ys, nt, C.lab[0].as<int32_t>() + (size_t)P * cv.pitch + P, cv.pitch, d_out);
+        C.mark(PM_ASSIGN);
+        C.mark(PM_COMPOSE);
+    }
     T.mark(4);
     if (timings) {
         IDL_CUDA(cudaEventSynchronize(C.timing.ev[4]));
@@ -337,26 +281,8 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     C.prof.canvas_px = (int64_t)cv.Wd * cv.Hd;
     C.prof.image_px = (int64_t)W * H;
     C.prof.n_triangles = nt;
-    return nt;
-}
-
-void compose_triangulation(Context& C, const Canvas& cv, int W, int H, int P, bool from_grid, int32_t* d_out)
-{
-    dim3 g(ceil_div(W, 256), H);
-    if (from_grid)
-        k_compose3_from_grid<<<g, 256, 0, C.stream>>>(C.vgrid.as<int32_t>(), W, H, C.tgrid.as<int32_t>(), d_out);
-    else if (W % 4 == 0 && P % 4 == 0 && cv.pitch % 4 == 0 && (reinterpret_cast<uintptr_t>(d_out) & 15) == 0) {
-        const int64_t quads = (int64_t)W * H / 4;
-        k_compose3x4<<<(unsigned)ceil_div(quads, (int64_t)256), 256, 0, C.stream>>>(
-            C.lab[0].as<int32_t>(), cv.pitch, P, W, quads, C.xs.as<int32_t>(), C.ys.as<int32_t>(),
-            C.tgrid.as<int32_t>(), d_out);
-    } else
-        k_compose3<<<(unsigned)ceil_div((int64_t)W * H, (int64_t)COMPOSE_PX), COMPOSE_PX, 0, C.stream>>>(
-            C.lab[0].as<int32_t>(), cv.pitch, P, W, (int64_t)W * H, C.xs.as<int32_t>(), C.ys.as<int32_t>(),
-            C.tgrid.as<int32_t>(), d_out, (reinterpret_cast<uintptr_t>(d_out) & 15) == 0);
-    IDL_LAUNCH();
-    C.mark(PM_COMPOSE);
     C.prof.valid = C.prof.enabled;
+    return nt;
 }
 
 void upload_seeds(Context& C, const int32_t* xy, int64_t n, cudaMemcpyKind kind)
@@ -596,11 +522,10 @@ int idl_triangulate(idl_context* ctx, int width, int height, const int32_t* seed
     const int P = resolve_padding(border_padding);
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
     Canvas cv;
-    const bool from_grid = (P == 0 && voronoi_grid != nullptr);
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, voronoi_grid, true, P, mode, timings_out, cv);
     const size_t bytes = (size_t)width * height * 3 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
-    compose_triangulation(C, cv, width, height, P, from_grid, C.outgrid.as<int32_t>());
+    const int64_t nt = run_triangulate(C, width, height, n_seeds, voronoi_grid, true, P, mode, timings_out, cv,
+                                       C.outgrid.as<int32_t>());
     IDL_CUDA(cudaMemcpyAsync(grid_out, C.outgrid.ptr, bytes, cudaMemcpyDeviceToHost, C.stream));
     if (padded_grid_out && P > 0) {
         const size_t pb = (size_t)cv.Wd * cv.Hd * 2 * sizeof(int32_t);
@@ -665,8 +590,7 @@ int idl_triangulate_device(idl_context* ctx, int width, int height, const int32_
     const int P = resolve_padding(border_padding);
     upload_seeds(C, d_seeds_xy, n_seeds, cudaMemcpyDeviceToDevice);
     Canvas cv;
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, false, P, mode, nullptr, cv);
-    compose_triangulation(C, cv, width, height, P, false, d_grid_out);
+    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, false, P, mode, nullptr, cv, d_grid_out);
     if (n_triangles_out) {
         IDL_CUDA(cudaStreamSynchronize(C.stream));
         *n_triangles_out = nt;

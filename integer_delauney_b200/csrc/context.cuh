@@ -98,7 +98,6 @@ struct Scalars {
     int32_t err_dup;          // two seeds share a pixel
     int32_t err_label;        // a caller-supplied label was outside [-1, n)
     int32_t max_side;         // longest triangle side, float-truncated (triangulation.cu:355-368)
-    int32_t n_big;            // tall triangles the raster hands to its block-per-triangle pass
     int32_t n_handoff;        // micro-tiles the last tile round hands to the persistent kernel
     int32_t tile_remaining;   // tiles listed for the tile round after the last one launched
     // resolve.cu, cleared together (RESOLVE_SCALARS values from n_roots on)
@@ -158,7 +157,7 @@ struct Context {
     DevBuf counts;        // per-round list lengths
     DevBuf gsync;         // grid barrier state of the persistent propagation kernel
     DevBuf trace;         // per-pass timestamps of the persistent kernel (profiling only)
-    DevBuf rbig;          // raster: ids of tall triangles
+    DevBuf rbig;          // raster: tile lists and packed triangles (raster.cuh)
     DevBuf bits;          // work-list dedup bitmaps of the persistent propagation kernel
     DevBuf big_tiles;     // tile rounds' last work list, handed to the persistent kernel
     DevBuf cellbits;      // cell-list tile rounds: three last-pass change bitmaps, in rotation
@@ -196,9 +195,8 @@ struct Context {
     // batched triangulation (batch.cu)
     DevBuf batch_img;       // per-image table
     DevBuf batch_seed_img;  // image of each input seed
-    DevBuf batch_rows;      // image of each output row
     DevBuf batch_sid;       // image of each sorted seed
-    DevBuf batch_stats;     // per-image triangle counts, longest sides, triangle offsets
+    DevBuf batch_stats;     // per-image longest sides and triangle offsets
     DevBuf batch_bad;       // first out-of-bounds / duplicate seed index
     DevBuf batch_ximg, batch_colimg, batch_rowimg;  // exact semantics: image table, column / row -> image
 
@@ -230,7 +228,7 @@ struct Context {
                          &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
                          &exact_bands, &sus_bits, &sus_list, &hkeys,
                          &ukeys, &uvals, &cnt, &off, &fill, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
-                         &batch_img, &batch_seed_img, &batch_rows, &batch_sid, &batch_stats, &batch_bad,
+                         &batch_img, &batch_seed_img, &batch_sid, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
         for (DevBuf* b : all) f(*b);
     }
@@ -387,8 +385,11 @@ void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const
                       int shift, cudaEvent_t mid = nullptr, const int32_t* rank = nullptr);
 
 // Stage (d): per-pixel max triangle id over a W x H image (raster.cu).
-void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid,
-                   int64_t max_tri);
+void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri);
+// The same with the (H, W, 3) output (seed id, squared distance, triangle id)
+// composed at once; lab points at the label of pixel (0, 0).
+void assign_and_compose(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri,
+                        const int32_t* lab, int pitch, int32_t* out);
 
 void ensure_scalars(Context& C);
 

@@ -32,65 +32,158 @@
 namespace idl {
 namespace {
 
-__global__ void k_max_side(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc_in,
-                           const int32_t* __restrict__ xs, const int32_t* __restrict__ ys, Scalars* __restrict__ sc)
+template <class TILE>
+__global__ void __launch_bounds__(256)
+k_raster_count(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const int32_t* __restrict__ xs,
+               const int32_t* __restrict__ ys, int W, int H, RasterWork w)
 {
-    const long long nt = sc_in->n_triangles;
-    int best = 0;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < nt;
-         t += (long long)gridDim.x * blockDim.x)
-        best = max(best, tri_max_side(tris + t * 5 + 2, xs, ys));
-    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    if ((threadIdx.x & 31) == 0 && best > 0) atomicMax(&sc->max_side, best);
+    const int tiles_x = (W + TILE::W - 1) / TILE::W;
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    const bool on = t < sc->n_triangles;
+    Tri u{};
+    if (on) u = load_tri(tris + t * 5 + 2, xs, ys);
+    int side = on ? longest_side(u) : 0;
+    raster_count<TILE>(w, on, (int32_t)t, u, W, H, 0, tiles_x);
+    side = __reduce_max_sync(0xFFFFFFFFu, side);
+    if ((threadIdx.x & 31) == 0 && side > __ldcg(&sc->max_side)) atomicMax(&sc->max_side, side);
+    raster_offsets<256>(w);
 }
 
-// A group of RASTER_GROUP lanes per triangle (four triangles per warp: a
-// Delaunay triangle of a dense seed set spans a few rows); lanes take rows.
-constexpr int RASTER_GROUP = 8;
-
+template <class TILE>
 __global__ void __launch_bounds__(256)
-k_raster(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const int32_t* __restrict__ xs,
-         const int32_t* __restrict__ ys, int W, int H, int32_t* __restrict__ tgrid, int32_t* __restrict__ big)
+k_raster_fill(const Scalars* __restrict__ sc, int W, int H, RasterWork w)
 {
-    const long long nt = sc->n_triangles;
-    const int lane = threadIdx.x % RASTER_GROUP;
-    const int wc = max(20, sc->max_side + 3);
-    const long long groups = (long long)gridDim.x * (blockDim.x / RASTER_GROUP);
-    for (long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / RASTER_GROUP; t < nt; t += groups)
-        raster_one<RASTER_GROUP>(tris + t * 5 + 2, (int32_t)t, xs, ys, W, H, wc, tgrid, lane, big, &sc->n_big);
+    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+    if (!w.head->overflow)
+        raster_fill<TILE>(w, t < sc->n_triangles, (int32_t)t, W, H, 0, (W + TILE::W - 1) / TILE::W);
 }
 
-// The tall triangles k_raster set aside: one block per triangle.
-__global__ void __launch_bounds__(256)
-k_raster_big(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, const int32_t* __restrict__ xs,
-             const int32_t* __restrict__ ys, int W, int H, int32_t* __restrict__ tgrid,
-             const int32_t* __restrict__ big)
+template <class TILE>
+__global__ void __launch_bounds__(TILE_THREADS)
+k_raster_tiles(RasterWork w, int W, int H, int32_t* __restrict__ tgrid)
 {
-    const int nb = sc->n_big;
-    for (int i = blockIdx.x; i < nb; i += gridDim.x) {
-        const int32_t t = big[i];
-        raster_rows_block(tris + (size_t)t * 5 + 2, t, xs, ys, W, H, tgrid);
+    __shared__ int32_t pix[TILE::H * TILE::PITCH];
+    const int tiles_x = (W + TILE::W - 1) / TILE::W;
+    const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
+    raster_tile<TILE>(w, pix, blockIdx.x, tx, ty, W, H, 0);
+    const int x = tx * TILE::W + (threadIdx.x % TILE::W);
+    if (x >= W) return;
+    for (int r = threadIdx.x / TILE::W; r < TILE::H && ty * TILE::H + r < H; r += TILE_THREADS / TILE::W)
+        tgrid[(size_t)(ty * TILE::H + r) * W + x] = pix[r * TILE::PITCH + threadIdx.x % TILE::W];
+}
+
+// The same with the (H, W, 3) output composed on the way out, so that the
+// triangle ids never go through memory on their own.
+template <class TILE>
+__global__ void __launch_bounds__(TILE_THREADS)
+k_raster_compose(RasterWork w, int W, int H, const int32_t* __restrict__ lab, int pitch,
+                 const int32_t* __restrict__ xs, const int32_t* __restrict__ ys, int32_t* __restrict__ out)
+{
+    __shared__ int32_t pix[TILE::H * TILE::PITCH];
+    const int tiles_x = (W + TILE::W - 1) / TILE::W;
+    const int tx = blockIdx.x % tiles_x, ty = blockIdx.x / tiles_x;
+    raster_tile<TILE>(w, pix, blockIdx.x, tx, ty, W, H, 0);
+    compose_tile<TILE>(pix, tx, ty, W, H, lab, pitch, xs, ys, 0, out);
+}
+
+// The collinear triangles (the longest side is known by now), and all of them
+// if the tile lists did not fit.
+__global__ void __launch_bounds__(128)
+k_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, const int32_t* __restrict__ xs,
+              const int32_t* __restrict__ ys, int W, int H, int32_t* __restrict__ tgrid, int stride, RasterWork w)
+{
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, warps = (gridDim.x * blockDim.x) >> 5;
+    if (w.head->overflow)
+        for (long long t = warp; t < sc->n_triangles; t += warps) {
+            const Tri u = load_tri(tris + t * 5 + 2, xs, ys);
+            if (!u.line) raster_direct(u, tgrid, stride, W, H, (int32_t)t);
+        }
+    const int n = w.head->n_lines;
+    for (int i = warp; i < n; i += warps) {
+        const int32_t t = w.lines[i];
+        if ((threadIdx.x & 31) == 0)
+            raster_line(load_tri(tris + (size_t)t * 5 + 2, xs, ys), tgrid, stride, W, H, t,
+                        max(20, sc->max_side + 3));
     }
 }
 
 }  // namespace
 
-void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t max_tri)
+RasterWork raster_work(Context& C, int64_t nt, int64_t n_tiles)
 {
-    IDL_CUDA(cudaMemsetAsync(tgrid, 0xFF, (size_t)W * H * sizeof(int32_t), C.stream));
-    if (max_tri <= 0) return;
-    IDL_CUDA(cudaMemsetAsync(&C.sc()->max_side, 0, 2 * sizeof(int32_t), C.stream));   // max_side, n_big
-    C.rbig.ensure((size_t)max_tri * 4);
-    const int g = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(max_tri, 256), C.num_sms * 8));
-    k_max_side<<<g, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), xs, ys, C.sc());
+    // at 200 000 uniform seeds a triangle meets 1.6 tiles; long slivers of
+    // clustered sets meet more, far fewer than this on average
+    const int64_t cap = std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30);
+    const size_t head = 256;
+    const size_t bytes = head + ((size_t)n_tiles * 2 + 1 + (size_t)nt * 4 + (size_t)cap) * 4;
+    C.rbig.ensure(bytes);
+    char* base = C.rbig.as<char>();
+    RasterWork w;
+    w.head = reinterpret_cast<RasterHead*>(base);
+    w.count = reinterpret_cast<int32_t*>(base + head);
+    w.off = w.count + n_tiles;
+    w.lines = w.off + n_tiles + 1;
+    w.xy = reinterpret_cast<uint32_t*>(w.lines + nt);
+    w.list = reinterpret_cast<int32_t*>(w.xy + nt * 3);
+    w.n_tiles = (int32_t)n_tiles;
+    w.list_cap = (int32_t)cap;
+    IDL_CUDA(cudaMemsetAsync(base, 0, head + (size_t)n_tiles * 4, C.stream));
+    return w;
+}
+
+namespace {
+
+// Tile lists of the triangles in C.tris, then draw(tile, tiles, work) and the
+// rest pass on the pixel ids at `ids`, `stride` ints apart.
+template <class TILE, class F>
+void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids,
+                 int stride, F&& draw)
+{
+    const int64_t tiles = (int64_t)ceil_div(W, TILE::W) * ceil_div(H, TILE::H);
+    const RasterWork w = raster_work(C, n_tri, tiles);
+    const int32_t* tris = C.tris.as<int32_t>();
+    if (n_tri > 0) {
+        IDL_CUDA(cudaMemsetAsync(&C.sc()->max_side, 0, sizeof(int32_t), C.stream));
+        const unsigned blocks = (unsigned)ceil_div(n_tri, 256);
+        k_raster_count<TILE><<<blocks, 256, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, w);
+        IDL_LAUNCH();
+        k_raster_fill<TILE><<<blocks, 256, 0, C.stream>>>(C.sc(), W, H, w);
+        IDL_LAUNCH();
+    } else {
+        IDL_CUDA(cudaMemsetAsync(w.off, 0, ((size_t)tiles + 1) * 4, C.stream));
+    }
+    draw(TILE{}, (unsigned)tiles, w);
     IDL_LAUNCH();
-    const int gr = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(max_tri, 256 / RASTER_GROUP),
-                                                                C.num_sms * 16));
-    k_raster<<<gr, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), xs, ys, W, H, tgrid, C.rbig.as<int32_t>());
-    IDL_LAUNCH();
-    k_raster_big<<<C.num_sms * 4, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), xs, ys, W, H, tgrid,
-                                                      C.rbig.as<int32_t>());
-    IDL_LAUNCH();
+    if (n_tri > 0) {
+        k_raster_rest<<<C.num_sms, 128, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, ids, stride, w);
+        IDL_LAUNCH();
+    }
+}
+
+template <class F>
+void raster(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids, int stride,
+            F&& draw)
+{
+    if (small_tiles((int64_t)ceil_div(W, TileLarge::W) * ceil_div(H, TileLarge::H), C.num_sms))
+        raster_with<TileSmall>(C, W, H, xs, ys, n_tri, ids, stride, draw);
+    else raster_with<TileLarge>(C, W, H, xs, ys, n_tri, ids, stride, draw);
+}
+
+}  // namespace
+
+void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri)
+{
+    raster(C, W, H, xs, ys, n_tri, tgrid, 1, [&](auto tile, unsigned tiles, const RasterWork& w) {
+        k_raster_tiles<decltype(tile)><<<tiles, TILE_THREADS, 0, C.stream>>>(w, W, H, tgrid);
+    });
+}
+
+void assign_and_compose(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri,
+                        const int32_t* lab, int pitch, int32_t* out)
+{
+    raster(C, W, H, xs, ys, n_tri, out + 2, 3, [&](auto tile, unsigned tiles, const RasterWork& w) {
+        k_raster_compose<decltype(tile)><<<tiles, TILE_THREADS, 0, C.stream>>>(w, W, H, lab, pitch, xs, ys, out);
+    });
 }
 
 }  // namespace idl

@@ -1,141 +1,429 @@
-// Device helpers of stage (d), shared by the single-image raster
-// (raster.cu) and the batched one (batch.cu).  The rules they implement are
-// documented at the top of raster.cu.
+// Device side of stage (d), shared by the single-image raster (raster.cu) and
+// the batched one (batch.cu).  The rules it implements are documented at the
+// top of raster.cu.
+//
+// Each triangle is listed at every pixel tile it meets, and a
+// block draws one tile in shared memory and stores it once.  Drawn straight
+// into the image instead, every pixel costs an atomic in L2 (an image past L2,
+// like a batch's, a DRAM sector each), and those bounded the stage whatever
+// the mapping of lanes to rows and pixels: 105 to 150 us at 4096 x 4096 /
+// 200 000 seeds, 770 to 890 us for the 59 M pixels of 512 batch images.
 #pragma once
 
 #include "context.cuh"
 
 namespace idl {
 
-__device__ __forceinline__ long long floor_div(long long p, long long q)   // q > 0
-{
-    return p >= 0 ? p / q : -((-p + q - 1) / q);
-}
-__device__ __forceinline__ long long ceil_div_ll(long long p, long long q) { return -floor_div(-p, q); }
+// Tile sizes: 64 x 32, or 32 x 16 for images whose larger tiles would leave the
+// device idle (the tile is then a shorter chain of work).
+template <int W_, int H_>
+struct Tile {
+    static constexpr int W = W_, H = H_;
+    static constexpr int PITCH = W + 1;   // so that the rows of one column fall into different banks
+};
+using TileLarge = Tile<64, 32>;
+using TileSmall = Tile<32, 16>;
+constexpr int TILE_THREADS = 128;
+inline bool small_tiles(int64_t large_tiles, int num_sms) { return large_tiles < (int64_t)num_sms * 8; }
 
 // Longest side of one triangle as triangulation.cu:357-362 computes it: float
 // dx, dy, dx*dx + dy*dy rounded per operation, sqrtf, truncation.
-__device__ __forceinline__ int tri_max_side(const int32_t* v, const int32_t* __restrict__ xs,
-                                            const int32_t* __restrict__ ys)
+__device__ __forceinline__ int side_length(int dx, int dy)
 {
-    const int pa[3] = {0, 0, 1}, pb[3] = {1, 2, 2};
-    int best = 0;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float dx = (float)(xs[v[pa[k]]] - xs[v[pb[k]]]);
-        const float dy = (float)(ys[v[pa[k]]] - ys[v[pb[k]]]);
-        const float s = __fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy));
-        best = max(best, (int)__fsqrt_rn(s));
-    }
-    return best;
+    const float fx = (float)dx, fy = (float)dy;
+    return (int)__fsqrt_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)));
 }
 
-constexpr int BIG_ROWS = 64;
+struct Tri {
+    int x[3], y[3];   // positively oriented, unless collinear
+    bool line;        // collinear
+};
 
-// The x-interval [xl, xr] of row y inside the closed triangle (a, b, c), in
-// exact integers; false if the row misses it.
-__device__ __forceinline__ bool tri_row_span(long long ax, long long ay, long long bx, long long by, long long cx,
-                                             long long cy, long long y, int W, long long& xl, long long& xr)
+__device__ __forceinline__ Tri load_tri(const int32_t* v, const int32_t* __restrict__ xs,
+                                        const int32_t* __restrict__ ys)
 {
-    const long long area2 = (bx - ax) * (cy - ay) - (by - ay) * (cx - ax);
-    const long long sgn = area2 > 0 ? 1 : -1;
-    const long long A[3] = {sgn * (ay - by), sgn * (by - cy), sgn * (cy - ay)};
-    const long long B[3] = {sgn * (bx - ax), sgn * (cx - bx), sgn * (ax - cx)};
-    const long long C0[3] = {sgn * (ax * by - ay * bx), sgn * (bx * cy - by * cx), sgn * (cx * ay - cy * ax)};
-    xl = 0;
-    xr = W - 1;
+    Tri t;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const int32_t s = __ldg(&v[k]);
+        t.x[k] = __ldg(&xs[s]);
+        t.y[k] = __ldg(&ys[s]);
+    }
+    const long long a = (long long)(t.x[1] - t.x[0]) * (t.y[2] - t.y[0]) -
+                        (long long)(t.y[1] - t.y[0]) * (t.x[2] - t.x[0]);
+    t.line = a == 0;
+    if (a < 0) {
+        const int x = t.x[1], y = t.y[1];
+        t.x[1] = t.x[2];
+        t.y[1] = t.y[2];
+        t.x[2] = x;
+        t.y[2] = y;
+    }
+    return t;
+}
+
+__device__ __forceinline__ int longest_side(const Tri& t)
+{
+    return max(side_length(t.x[0] - t.x[1], t.y[0] - t.y[1]),
+               max(side_length(t.x[1] - t.x[2], t.y[1] - t.y[2]), side_length(t.x[2] - t.x[0], t.y[2] - t.y[0])));
+}
+
+// floor(p / q), q > 0, by a float estimate and the remainder: exact while the
+// quotient's estimate is within one, which holds up to 2^20 and more; a larger
+// quotient (a row far from the edge's own rows) may be off by its last digits,
+// but lies beyond every image column either way.
+__device__ __forceinline__ int div_floor(int p, int q)
+{
+    const int d = __float2int_rd(__fdividef((float)p, (float)q));
+    const int r = p - d * q;
+    return d + (r >= q) - (r < 0);
+}
+
+// The x-interval of row y inside the closed triangle, within [xl, xr] on entry;
+// false if empty.  An edge from u to w keeps A (x - ux) + B (y - uy) >= 0 with
+// A = uy - wy, B = wx - ux; differences of coordinates are below 2^15, so
+// every product fits 32 bits.  OUTER: rounded outwards, so that every point of
+// the real interval at y lies in it.
+template <bool OUTER = false>
+__device__ __forceinline__ bool tri_row_span(const Tri& t, int y, int& xl, int& xr)
+{
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
-        const long long c = B[e] * y + C0[e];   // need A*x + c >= 0
-        if (A[e] > 0) xl = max(xl, ceil_div_ll(-c, A[e]));
-        else if (A[e] < 0) xr = min(xr, floor_div(c, -A[e]));
-        else if (c < 0) return false;
+        const int u = e, w = e == 2 ? 0 : e + 1;
+        const int A = t.y[u] - t.y[w], c = (t.x[w] - t.x[u]) * (y - t.y[u]);
+        if (A == 0) {
+            if (c < 0) return false;
+        } else if (A > 0) {   // x - ux >= -c / A
+            xl = max(xl, t.x[u] + (OUTER ? div_floor(-c, A) : -div_floor(c, A)));
+        } else {              // x - ux <= c / -A
+            xr = min(xr, t.x[u] + (OUTER ? -div_floor(-c, -A) : div_floor(c, -A)));
+        }
     }
     return xl <= xr;
 }
 
-// Rasterise one triangle (vertex ids v, coordinates xs/ys) into a W x H grid
-// of triangle ids with atomicMax; a group of G lanes shares the rows (`lane`
-// is the caller's index in its group).  wc: the degenerate-case seed window
-// (max(20, max_side + 3)).  With `big` set, a proper triangle spanning
-// BIG_ROWS rows or more is appended to big (count *n_big) instead, for
-// raster_rows_block.
-template <int G = 32>
-__device__ __forceinline__ void raster_one(const int32_t* v, int32_t tid, const int32_t* __restrict__ xs,
-                                           const int32_t* __restrict__ ys, int W, int H, int wc,
-                                           int32_t* __restrict__ tgrid, int lane, int32_t* big = nullptr,
-                                           int32_t* n_big = nullptr)
+// The tiles of a W x H image (tiles_x to a row, the first one tile_off) that a
+// proper triangle's pixels can lie in: f(t, tile).  A box of a few tiles is taken whole, by its lane; in
+// a larger one each tile row takes the columns the triangle spans there (its
+// extent in a slab is reached at the slab's ends or at a vertex), a lane per
+// tile row: a sliver across the image is hundreds of tiles.  Every lane of the
+// warp calls it; on: the lane brings triangle u, number t, of a W x H image.
+template <class TILE, class F>
+__device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int W, int H, int tile_off, int tiles_x,
+                                          F&& f)
 {
-    const long long ax = xs[v[0]], ay = ys[v[0]], bx = xs[v[1]], by = ys[v[1]], cx = xs[v[2]], cy = ys[v[2]];
-    const long long area2 = (bx - ax) * (cy - ay) - (by - ay) * (cx - ax);
-    if (area2 == 0) {
-        // collinear: supporting line within the reference's seed window
-        if (lane != 0) return;
-        const long long lo_y = max(0ll, min(ay, min(by, cy)) - wc);
-        const long long hi_y = min((long long)H - 1, max(ay, max(by, cy)) + wc);
-        for (long long y = lo_y; y <= hi_y; ++y) {
-            long long x_lo, x_hi;
-            if (by == ay) {
-                if (y != ay) continue;
-                x_lo = 0; x_hi = W - 1;
-            } else {
-                const long long num = (bx - ax) * (y - ay);
-                const long long den = by - ay;
-                if (num % den != 0) continue;
-                x_lo = x_hi = ax + num / den;
-            }
-            for (long long x = max(0ll, x_lo); x <= min((long long)W - 1, x_hi); ++x) {
-                const bool near = (llabs(ax - x) <= wc && llabs(ay - y) <= wc) ||
-                                  (llabs(bx - x) <= wc && llabs(by - y) <= wc) ||
-                                  (llabs(cx - x) <= wc && llabs(cy - y) <= wc);
-                if (near) atomicMax(&tgrid[(size_t)y * W + x], tid);
-            }
-        }
-        return;
-    }
-    const long long sgn = area2 > 0 ? 1 : -1;
-    const long long y0 = max(0ll, min(ay, min(by, cy)));
-    const long long y1 = min((long long)H - 1, max(ay, max(by, cy)));
-    if (big && y1 - y0 >= BIG_ROWS) {   // tall: its rows go to a whole block, lanes along each row
-        if (lane == 0) big[atomicAdd(n_big, 1)] = tid;
-        return;
-    }
-    // d_i(x, y) = A_i * x + B_i * y + C_i for edges (a,b), (b,c), (c,a):
-    // cross(u - p, w - p) = (uy - wy) * px + (wx - ux) * py + (ux*wy - uy*wx)
-    const long long A[3] = {sgn * (ay - by), sgn * (by - cy), sgn * (cy - ay)};
-    const long long B[3] = {sgn * (bx - ax), sgn * (cx - bx), sgn * (ax - cx)};
-    const long long C0[3] = {sgn * (ax * by - ay * bx), sgn * (bx * cy - by * cx), sgn * (cx * ay - cy * ax)};
-    for (long long y = y0 + lane; y <= y1; y += G) {
-        long long xl = 0, xr = W - 1;
-        bool empty = false;
+    const int lane = threadIdx.x & 31;
+    const int x0 = max(0, min(u.x[0], min(u.x[1], u.x[2]))), x1 = min(W - 1, max(u.x[0], max(u.x[1], u.x[2])));
+    const int y0 = max(0, min(u.y[0], min(u.y[1], u.y[2]))), y1 = min(H - 1, max(u.y[0], max(u.y[1], u.y[2])));
+    on = on && x0 <= x1 && y0 <= y1;
+    const int tx0 = x0 / TILE::W, tx1 = x1 / TILE::W, ty0 = y0 / TILE::H, ty1 = y1 / TILE::H;
+    const bool few = on && (tx1 - tx0 + 1) * (ty1 - ty0 + 1) <= 12;
+    if (few)
+        for (int ty = ty0; ty <= ty1; ++ty)
+            for (int tx = tx0; tx <= tx1; ++tx) f(t, tile_off + ty * tiles_x + tx);
+    __syncwarp();
+    for (unsigned m = __ballot_sync(0xFFFFFFFFu, on && !few); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        Tri v;
 #pragma unroll
-        for (int e = 0; e < 3; ++e) {
-            const long long c = B[e] * y + C0[e];   // need A*x + c >= 0
-            if (A[e] > 0) xl = max(xl, ceil_div_ll(-c, A[e]));
-            else if (A[e] < 0) xr = min(xr, floor_div(c, -A[e]));
-            else if (c < 0) empty = true;
+        for (int k = 0; k < 3; ++k) {
+            v.x[k] = __shfl_sync(0xFFFFFFFFu, u.x[k], src);
+            v.y[k] = __shfl_sync(0xFFFFFFFFu, u.y[k], src);
         }
-        if (empty) continue;
-        int32_t* row = tgrid + (size_t)y * W;
-        for (long long x = xl; x <= xr; ++x) atomicMax(&row[x], tid);
+        const int bx0 = __shfl_sync(0xFFFFFFFFu, x0, src), bx1 = __shfl_sync(0xFFFFFFFFu, x1, src),
+                  by0 = __shfl_sync(0xFFFFFFFFu, y0, src), by1 = __shfl_sync(0xFFFFFFFFu, y1, src);
+        const int32_t id = __shfl_sync(0xFFFFFFFFu, t, src);
+        const int first = __shfl_sync(0xFFFFFFFFu, tile_off, src), per_row = __shfl_sync(0xFFFFFFFFu, tiles_x, src);
+        for (int ty = by0 / TILE::H + lane; ty <= by1 / TILE::H; ty += 32) {
+            const int ya = max(by0, ty * TILE::H), yb = min(by1, ty * TILE::H + TILE::H - 1);
+            int lo = bx1 + 1, hi = bx0 - 1;
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                int l = bx0, r = bx1;
+                if (tri_row_span<true>(v, k ? yb : ya, l, r)) {
+                    lo = min(lo, l);
+                    hi = max(hi, r);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+                if (v.y[k] >= ya && v.y[k] <= yb) {
+                    lo = min(lo, max(v.x[k], bx0));
+                    hi = max(hi, min(v.x[k], bx1));
+                }
+            if (lo > hi) continue;
+            for (int tx = lo / TILE::W; tx <= hi / TILE::W; ++tx) f(id, first + ty * per_row + tx);
+        }
+        __syncwarp();
     }
 }
 
-// The rows of one proper triangle split over a whole block: each warp takes a
-// row, its lanes the row's pixels.
-__device__ __forceinline__ void raster_rows_block(const int32_t* v, int32_t tid, const int32_t* __restrict__ xs,
-                                                  const int32_t* __restrict__ ys, int W, int H,
-                                                  int32_t* __restrict__ tgrid)
+// A collinear triangle covers the points of its line within the reference's
+// seed window (Chebyshev distance wc of a vertex); one lane.  Pixel ids are
+// `stride` ints apart.
+__device__ __forceinline__ void raster_line(const Tri& t, int32_t* grid, int stride, int W, int H, int32_t tid, int wc)
 {
-    const long long ax = xs[v[0]], ay = ys[v[0]], bx = xs[v[1]], by = ys[v[1]], cx = xs[v[2]], cy = ys[v[2]];
-    const long long y0 = max(0ll, min(ay, min(by, cy)));
-    const long long y1 = min((long long)H - 1, max(ay, max(by, cy)));
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-    for (long long y = y0 + warp; y <= y1; y += nwarps) {
-        long long xl, xr;
-        if (!tri_row_span(ax, ay, bx, by, cx, cy, y, W, xl, xr)) continue;
-        int32_t* row = tgrid + (size_t)y * W;
-        for (long long x = xl + lane; x <= xr; x += 32) atomicMax(&row[x], tid);
+    const long long ax = t.x[0], ay = t.y[0], bx = t.x[1], by = t.y[1], cx = t.x[2], cy = t.y[2];
+    const long long lo_y = max(0ll, min(ay, min(by, cy)) - wc);
+    const long long hi_y = min((long long)H - 1, max(ay, max(by, cy)) + wc);
+    for (long long y = lo_y; y <= hi_y; ++y) {
+        long long x_lo, x_hi;
+        if (by == ay) {
+            if (y != ay) continue;
+            x_lo = 0; x_hi = W - 1;
+        } else {
+            const long long num = (bx - ax) * (y - ay);
+            const long long den = by - ay;
+            if (num % den != 0) continue;
+            x_lo = x_hi = ax + num / den;
+        }
+        for (long long x = max(0ll, x_lo); x <= min((long long)W - 1, x_hi); ++x) {
+            const bool near = (llabs(ax - x) <= wc && llabs(ay - y) <= wc) ||
+                              (llabs(bx - x) <= wc && llabs(by - y) <= wc) ||
+                              (llabs(cx - x) <= wc && llabs(cy - y) <= wc);
+            if (near) atomicMax(&grid[((size_t)y * W + x) * stride], tid);
+        }
+    }
+}
+
+// The (H, W, 3) output of one tile, from the drawn ids and the label plane:
+// (seed id, squared distance, triangle id) per pixel.  lab and out point at the
+// image's pixel (0, 0); ids are reported relative to first_seed.  A warp stages
+// one row of triples in shared memory and stores it as whole 128-byte lines,
+// whatever the alignment of the row.
+template <class TILE>
+__device__ __forceinline__ void compose_tile(const int32_t* pix, int tx, int ty, int W, int H,
+                                             const int32_t* __restrict__ lab, int pitch,
+                                             const int32_t* __restrict__ xs, const int32_t* __restrict__ ys,
+                                             int32_t first_seed, int32_t* __restrict__ out)
+{
+    __shared__ int32_t stage[TILE_THREADS / 32][TILE::W * 3];
+    int32_t* st = stage[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const int x0 = tx * TILE::W, n = min(TILE::W, W - x0);
+    for (int r = threadIdx.x >> 5; r < TILE::H; r += TILE_THREADS / 32) {
+        const int y = ty * TILE::H + r;
+        if (y >= H) break;
+        int32_t l[TILE::W / 32];
+#pragma unroll
+        for (int k = 0; k < TILE::W / 32; ++k) {
+            const int c = k * 32 + lane;
+            l[k] = c < n ? __ldg(&lab[(size_t)y * pitch + x0 + c]) : -1;
+        }
+#pragma unroll
+        for (int k = 0; k < TILE::W / 32; ++k) {
+            const int c = k * 32 + lane;
+            int32_t d = -1, id = l[k];
+            if (l[k] >= 0) {
+                const int32_t dx = x0 + c - __ldg(&xs[l[k]]), dy = y - __ldg(&ys[l[k]]);
+                d = dx * dx + dy * dy;
+                id = l[k] - first_seed;
+            }
+            st[c * 3] = id;
+            st[c * 3 + 1] = d;
+            st[c * 3 + 2] = pix[r * TILE::PITCH + c];
+        }
+        __syncwarp();
+        int32_t* row = out + ((size_t)y * W + x0) * 3;
+        for (int k = lane; k < n * 3; k += 32) row[k] = st[k];
+        __syncwarp();
+    }
+}
+
+// What the raster kernels share in device memory.
+struct RasterHead {
+    int32_t n_lines;    // collinear triangles
+    int32_t done;       // blocks of the count pass that have finished
+    int32_t overflow;   // the tile lists do not fit: every triangle goes into the image directly
+};
+struct RasterWork {
+    RasterHead* head;
+    int32_t* count;     // triangles per tile
+    int32_t* off;       // first list entry of each tile, n_tiles + 1
+    int32_t* lines;     // the collinear triangles
+    uint32_t* xy;       // three packed corners per triangle
+    int32_t* list;      // triangles by tile
+    int32_t n_tiles, list_cap;
+};
+
+// Lays the work out on C.rbig for nt triangles and n_tiles tiles and clears
+// its head and counts.
+RasterWork raster_work(Context& C, int64_t nt, int64_t n_tiles);
+
+__device__ __forceinline__ Tri unpack_tri(const uint32_t* __restrict__ xy, int32_t t)
+{
+    Tri u;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t p = __ldg(&xy[(size_t)t * 3 + k]);
+        u.x[k] = pos_x(p);
+        u.y[k] = pos_y(p);
+    }
+    u.line = false;
+    return u;
+}
+
+// Count pass, one triangle per lane (on: there is one): its packed corners, and
+// one for each tile it meets (collinear ones are listed apart).
+template <class TILE>
+__device__ __forceinline__ void raster_count(const RasterWork& w, bool on, int32_t t, const Tri& u, int W, int H,
+                                             int tile_off, int tiles_x)
+{
+    if (on) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) w.xy[(size_t)t * 3 + k] = u.line ? 0xFFFFFFFFu : pack_pos(u.x[k], u.y[k]);
+        if (u.line) w.lines[atomicAdd(&w.head->n_lines, 1)] = t;
+    }
+    tri_tiles<TILE>(on && !u.line, u, t, W, H, tile_off, tiles_x,
+              [&](int32_t, int tile) { atomicAdd(&w.count[tile], 1); });
+}
+
+// The last block of the count pass turns the counts into list offsets.  Every
+// thread of the block calls it.
+template <int T>
+__device__ __forceinline__ void raster_offsets(const RasterWork& w)
+{
+    __shared__ int32_t s_last, s_carry, s_warp[T / 32];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(&w.head->done, 1) == (int)gridDim.x - 1;
+        s_carry = 0;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int base = 0; base < w.n_tiles; base += T * 4) {
+        int v[4], sum = 0;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = base + threadIdx.x * 4 + k;
+            v[k] = i < w.n_tiles ? __ldcg(&w.count[i]) : 0;
+            sum += v[k];
+        }
+        int incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) s_warp[warp] = incl;
+        __syncthreads();
+        int at = s_carry + incl - sum, all = 0;
+#pragma unroll
+        for (int k = 0; k < T / 32; ++k) {
+            at += k < warp ? s_warp[k] : 0;
+            all += s_warp[k];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int i = base + threadIdx.x * 4 + k;
+            if (i < w.n_tiles) w.off[i] = at;
+            at += v[k];
+        }
+        __syncthreads();
+        if (threadIdx.x == 0) s_carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        w.off[w.n_tiles] = s_carry;
+        if (s_carry > w.list_cap || s_carry < 0) w.head->overflow = 1;
+    }
+}
+
+// Fill pass: each triangle's entry in each of its tiles' lists; the tile's
+// counter hands back the entry's place.
+template <class TILE>
+__device__ __forceinline__ void raster_fill(const RasterWork& w, bool on, int32_t t, int W, int H, int tile_off,
+                                            int tiles_x)
+{
+    Tri u{};
+    if (on) {
+        on = w.xy[(size_t)t * 3] != 0xFFFFFFFFu;
+        if (on) u = unpack_tri(w.xy, t);
+    }
+    tri_tiles<TILE>(on, u, t, W, H, tile_off, tiles_x, [&](int32_t id, int tile) {
+        w.list[w.off[tile] + atomicSub(&w.count[tile], 1) - 1] = id;
+    });
+}
+
+// The first lane whose inclusive sum exceeds k (sums do not decrease).
+__device__ __forceinline__ int lane_of(int incl, int k)
+{
+    int l = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, incl, l + s - 1) <= k) l += s;
+    return l;
+}
+
+// One tile of a W x H image, by a block: pix[TILE::H * TILE::PITCH] takes the
+// highest id (list entry - first_id) of the tile's triangles at each pixel.  A
+// warp takes 32 triangles, then their rows in the tile 32 at a time, a lane
+// each.  Ends with a barrier.
+template <class TILE>
+__device__ __forceinline__ void raster_tile(const RasterWork& w, int32_t* pix, int tile, int tx, int ty, int W, int H,
+                                            int32_t first_id)
+{
+    for (int i = threadIdx.x; i < TILE::H * TILE::PITCH; i += TILE_THREADS) pix[i] = NO_TRIANGLE;
+    __syncthreads();
+    const int lane = threadIdx.x & 31;
+    const int x0 = tx * TILE::W, y0 = ty * TILE::H;
+    const int x1 = min(W, x0 + TILE::W) - 1, y1 = min(H, y0 + TILE::H) - 1;
+    const bool skip = w.head->overflow != 0;
+    const int b = skip ? 0 : w.off[tile], e = skip ? 0 : w.off[tile + 1];
+    for (int i0 = b + (threadIdx.x & ~31); i0 < e; i0 += TILE_THREADS) {
+        const int i = i0 + lane;
+        int32_t t = 0;
+        uint32_t p[3] = {0, 0, 0};
+        int ya = 0, rows = 0;
+        if (i < e) {
+            t = __ldg(&w.list[i]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) p[k] = __ldg(&w.xy[(size_t)t * 3 + k]);
+            const int a = pos_y(p[0]), c = pos_y(p[1]), d = pos_y(p[2]);
+            ya = max(y0, min(a, min(c, d)));
+            rows = max(min(y1, max(a, max(c, d))) - ya + 1, 0);
+        }
+        int incl = rows;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        const int total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+        const int first = ya - (incl - rows);
+        for (int r0 = 0; r0 < total; r0 += 32) {
+            const int r = r0 + lane;
+            const int src = min(lane_of(incl, r), 31);
+            Tri u;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const uint32_t q = __shfl_sync(0xFFFFFFFFu, p[k], src);
+                u.x[k] = pos_x(q);
+                u.y[k] = pos_y(q);
+            }
+            const int y = r + __shfl_sync(0xFFFFFFFFu, first, src);
+            const int32_t id = __shfl_sync(0xFFFFFFFFu, t, src) - first_id;
+            int xl = x0, xr = x1;
+            if (r < total && tri_row_span(u, y, xl, xr)) {
+                int32_t* row = pix + (y - y0) * TILE::PITCH - x0;
+                for (int x = xl; x <= xr; ++x) atomicMax(&row[x], id);
+            }
+        }
+    }
+    __syncthreads();
+}
+
+// A triangle straight into the image (tile lists that do not fit): a warp.
+__device__ __forceinline__ void raster_direct(const Tri& t, int32_t* grid, int stride, int W, int H, int32_t tid)
+{
+    const int y0 = max(0, min(t.y[0], min(t.y[1], t.y[2]))), y1 = min(H - 1, max(t.y[0], max(t.y[1], t.y[2])));
+    for (int y = y0 + (int)(threadIdx.x & 31); y <= y1; y += 32) {
+        int xl = 0, xr = W - 1;
+        if (!tri_row_span(t, y, xl, xr)) continue;
+        for (int x = xl; x <= xr; ++x) atomicMax(&grid[((size_t)y * W + x) * stride], tid);
     }
 }
 
