@@ -247,7 +247,7 @@ IDL_API int idl_triangles_device(idl_context* ctx, const int32_t** d_tris, const
  * embed the library under an allocator of their own.  Same result as
  * idl_voronoi, but with device pointers, on `stream` (a cudaStream_t, NULL =
  * legacy default stream) and the current device, and all workspace taken
- * from one static device array of about 9.8 MB, which a GPU holds from the
+ * from one static device array of about 9.7 MB, which a GPU holds from the
  * first call on it (when lazy module loading, the CUDA default, loads the
  * array's module there; at context creation under CUDA_MODULE_LOADING=EAGER)
  * until the process exits.  That first call therefore does commit device

@@ -64,12 +64,6 @@ __global__ void k_b_mark(const int32_t* __restrict__ xy, int64_t n, const int32_
     if (atomicOr(&bitmap[bit >> 5], b) & b) atomicMin(&first_bad[1], (unsigned long long)i);
 }
 
-__global__ void k_b_popc(const uint32_t* __restrict__ bitmap, int64_t nwords, int32_t* __restrict__ out)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nwords) out[i] = __popc(bitmap[i]);
-}
-
 __global__ void k_b_rank(const int32_t* __restrict__ xy, int64_t n, const int32_t* __restrict__ seed_img,
                          const BImg* __restrict__ imgs, int P, const uint32_t* __restrict__ bitmap,
                          const int32_t* __restrict__ word_rank, int32_t* __restrict__ xs, int32_t* __restrict__ ys,
@@ -358,6 +352,8 @@ const XImg* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
         pair_img.insert(pair_img.end(), (size_t)(m.Wp + 1) / 2, i);
         row_img.insert(row_img.end(), (size_t)m.Hp, i);
         band_entries += (int64_t)x_bands(m) * m.Wp;
+        m.P = P;
+        m.bit0 = b.px_off;
         max_wp = std::max(max_wp, m.Wp);
         max_hp = std::max(max_hp, m.Hp);
     }
@@ -408,7 +404,6 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     // validate + rank
     const int64_t nwords = (pl.n_px + 31) / 32;
     C.bitmap.ensure((size_t)nwords * 4);
-    C.scan_b.ensure((size_t)nwords * 4);
     C.scan_c.ensure((size_t)(nwords + 1) * 4);
     C.xs.ensure((size_t)n * 4);
     C.ys.ensure((size_t)n * 4);
@@ -428,9 +423,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     if (hb[0] != ~0ull) invalid("image " + std::to_string(image_of(hb[0])) + ": seed coordinate out of bounds");
     if (hb[1] != ~0ull)
         invalid("image " + std::to_string(image_of(hb[1])) + ": duplicate seed positions are not allowed");
-    k_b_popc<<<nblk(nwords), 256, 0, C.stream>>>(C.bitmap.as<uint32_t>(), nwords, C.scan_b.as<int32_t>());
-    IDL_LAUNCH();
-    exclusive_scan(C, C.scan_b.as<int32_t>(), C.scan_c.as<int32_t>(), nwords);
+    exclusive_popc_scan(C, C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nwords);
     k_b_rank<<<nblk(n), 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, C.batch_seed_img.as<int32_t>(), d_imgs, P,
                                            C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), C.xs.as<int32_t>(),
                                            C.ys.as<int32_t>(), C.pos.as<uint32_t>(), C.batch_sid.as<int32_t>());

@@ -34,8 +34,23 @@ void Context::fetch_scalars()
     IDL_CUDA(cudaStreamSynchronize(stream));
 }
 
+void Context::fetch_scalars_begin()
+{
+    IDL_CUDA(cudaMemcpyAsync(host_sc, scalars.ptr, sizeof(Scalars), cudaMemcpyDeviceToHost, stream));
+    if (host_sc_borrowed) return;   // a pageable mirror: the copy is done when the call returns
+    if (!fetched) IDL_CUDA(cudaEventCreateWithFlags(&fetched, cudaEventDisableTiming));
+    IDL_CUDA(cudaEventRecord(fetched, stream));
+}
+
+void Context::fetch_scalars_end()
+{
+    if (host_sc_borrowed) IDL_CUDA(cudaStreamSynchronize(stream));
+    else IDL_CUDA(cudaEventSynchronize(fetched));
+}
+
 Context::~Context()
 {
+    if (fetched) cudaEventDestroy(fetched);
     bool ordered = false;
     each_buf([&](DevBuf& b) { ordered |= b.async; });
     if (ordered) cudaDeviceSynchronize();   // stream-ordered buffers may still be in use
@@ -47,7 +62,10 @@ Context::~Context()
 
 void ensure_scalars(Context& C)
 {
-    C.scalars.ensure(sizeof(Scalars));
+    if (!C.scalars.ptr) {
+        C.scalars.ensure(sizeof(Scalars));
+        IDL_CUDA(cudaMemsetAsync(C.scalars.ptr, 0, sizeof(Scalars), C.stream));
+    }
     if (!C.host_sc) {
         count_alloc();
         IDL_CUDA(cudaMallocHost(reinterpret_cast<void**>(&C.host_sc), sizeof(Scalars)));
@@ -172,17 +190,18 @@ int64_t run_passes(Context& C, int mode, const Canvas& cv, int64_t n)
 // Stage (a) from scratch into C.lab[0].  Returns true if the labels come from
 // resolve_exact: the caller has to look at finish_resolved once the scalars
 // have been read back.  Otherwise *passes (may be nullptr) takes the pass count.
-bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, bool want_passes, int64_t* passes = nullptr)
+bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, int P, bool want_passes,
+                  int64_t* passes = nullptr)
 {
     if (mode == IDL_MODE_REFERENCE && C.direct()) {
         C.prof.pass_ns.clear();
         C.prof.pass_tiles.clear();
-        propagate_exact(C, cv, C.pos.as<uint32_t>(), n);
+        propagate_exact(C, cv, C.pos.as<uint32_t>(), n, P);
         resolve_exact(C, cv, C.pos.as<uint32_t>(), n, want_passes);
         return true;
     }
     int64_t p = 0;
-    if (mode == IDL_MODE_EXACT) propagate_exact(C, cv, C.pos.as<uint32_t>(), n);
+    if (mode == IDL_MODE_EXACT) propagate_exact(C, cv, C.pos.as<uint32_t>(), n, P);
     else p = run_passes(C, mode, cv, n);
     if (passes) *passes = p;
     return false;
@@ -201,13 +220,14 @@ bool finish_resolved(Context& C, bool want_passes, int64_t* passes = nullptr)
 }
 
 // Run stages (a) (b) (d) with seeds already in C.seeds_in.  Leaves labels in
-// C.lab[0], triangles in C.tris, the composed (H, W, 3) grid in d_out; returns
-// the triangle count.
-int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgrid_host_or_dev, bool vgrid_on_host,
-                        int P, int mode, float* timings, Canvas& cv_out, int32_t* d_out)
+// C.lab[0], triangles in C.tris, the composed (H, W, 3) grid in d_out; deliver()
+// queues the copies the caller wants of them.  Returns the triangle count, with
+// the stream's work done.
+template <class F>
+int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgrid, int P, int mode, float* timings,
+                        int32_t* d_out, F&& deliver)
 {
     const Canvas cv = make_canvas(W + 2 * P, H + 2 * P);
-    cv_out = cv;
     C.prof.valid = false;
     for (bool& r : C.prof.recorded) r = false;
     C.prof.rounds = C.prof.tiles = C.prof.passes = 0;
@@ -216,15 +236,14 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     sort_seeds_device(C, W, H, n, P);
     C.mark(PM_SEEDS);
 
-    StageTimer T(C, timings != nullptr);
+    const bool from_grid = vgrid && P == 0;
     bool resolved = false;
-    if (P > 0 || !vgrid_host_or_dev) {
-        resolved = start_labels(C, mode, cv, n, C.prof.enabled);
+    if (!from_grid) {
+        resolved = start_labels(C, mode, cv, n, P, C.prof.enabled);
     } else {
         const size_t gbytes = (size_t)W * H * 2 * sizeof(int32_t);
         C.vgrid.ensure(gbytes);
-        IDL_CUDA(cudaMemcpyAsync(C.vgrid.ptr, vgrid_host_or_dev, gbytes,
-                                 vgrid_on_host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, C.stream));
+        IDL_CUDA(cudaMemcpyAsync(C.vgrid.ptr, vgrid, gbytes, cudaMemcpyHostToDevice, C.stream));
         C.lab[0].ensure((size_t)cv.pitch * cv.Hd * 4);
         IDL_CUDA(cudaMemsetAsync(&C.sc()->err_label, 0, sizeof(int32_t), C.stream));
         dim3 g(ceil_div(W, 256), H);
@@ -236,42 +255,58 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     }
     C.mark(PM_PROPAGATE);
 
-    T.mark(0);
-    // detect_ms covers the fused detect + hash insert kernel, dedup_ms the
-    // enumeration and canonical ranking (the reference's thrust sort/unique)
-    detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, P,
-                     T.on ? C.timing.ev[1] : nullptr);
+    StageTimer T(C, timings != nullptr);
+    const int32_t *xs = C.xs.as<int32_t>(), *ys = C.ys.as<int32_t>();
+    auto detect = [&](int64_t cap) {
+        T.mark(0);
+        // detect_ms covers the fused detect + hash insert kernel, dedup_ms the
+        // enumeration and canonical ranking (the reference's thrust sort/unique)
+        detect_launch(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, P, cap, T.on ? C.timing.ev[1] : nullptr);
+        T.mark(2);
+        C.mark(PM_DEDUP);
+    };
+    auto assign = [&](int64_t n_tri) {
+        T.mark(3);
+        if (from_grid) {   // channels 0 and 1 are the caller's
+            C.tgrid.ensure((size_t)W * H * sizeof(int32_t));
+            assign_pixels(C, W, H, xs, ys, C.tgrid.as<int32_t>(), n_tri);
+            C.mark(PM_ASSIGN);
+            k_compose3_from_grid<<<dim3(ceil_div(W, 256), H), 256, 0, C.stream>>>(C.vgrid.as<int32_t>(), W, H,
+                                                                                 C.tgrid.as<int32_t>(), d_out);
+            IDL_LAUNCH();
+        } else {
+            assign_and_compose(C, W, H, xs, ys, n_tri, C.lab[0].as<int32_t>() + (size_t)P * cv.pitch + P, cv.pitch,
+                               d_out);
+            C.mark(PM_ASSIGN);
+        }
+        C.mark(PM_COMPOSE);
+        T.mark(4);
+        deliver(cv);
+        C.fetch_scalars();
+    };
+    // Everything goes out before anything is read back, with the usual bounds
+    // on the table and the triangle count (under 2n); one wait at the end tells
+    // whether they held and whether the exact diagram decided the labels.  What
+    // failed is run again, each time with room for what is known by then.
+    int64_t cap = detect_capacity(C, n);
+    int64_t bound = 2 * n + 64;
+    detect(cap);
+    assign(bound);
     if (resolved && !finish_resolved(C, C.prof.enabled)) {
-        // the exact diagram did not decide the fixed point: run the passes
         run_passes(C, mode, cv, n);
         C.mark(PM_PROPAGATE);
-        T.mark(0);
-        detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, P,
-                         T.on ? C.timing.ev[1] : nullptr);
+        detect(cap);
+        assign(bound);
     }
-    T.mark(2);
-    C.mark(PM_DEDUP);
-    // the triangle count came back with detection's own read-back (ranking
-    // does not change it): no second host round trip here
+    for (int attempt = 0; !detect_done(C, cap); ++attempt) {
+        if (attempt >= 6) throw Error(IDL_ERR_INTERNAL, "triangle hash table overflow");
+        cap *= 4;
+        detect(cap);
+        assign(bound);
+    }
     const int64_t nt = C.host_sc->n_triangles;
-    T.mark(3);
-    const int32_t *xs = C.xs.as<int32_t>(), *ys = C.ys.as<int32_t>();
-    if (vgrid_host_or_dev && P == 0) {   // channels 0 and 1 are the caller's
-        C.tgrid.ensure((size_t)W * H * sizeof(int32_t));
-        assign_pixels(C, W, H, xs, ys, C.tgrid.as<int32_t>(), nt);
-        C.mark(PM_ASSIGN);
-        k_compose3_from_grid<<<dim3(ceil_div(W, 256), H), 256, 0, C.stream>>>(C.vgrid.as<int32_t>(), W, H,
-                                                                             C.tgrid.as<int32_t>(), d_out);
-        IDL_LAUNCH();
-        C.mark(PM_COMPOSE);
-    } else {
-        assign_and_compose(C, W, H, xs, ys, nt, C.lab[0].as<int32_t>() + (size_t)P * cv.pitch + P, cv.pitch, d_out);
-        C.mark(PM_ASSIGN);
-        C.mark(PM_COMPOSE);
-    }
-    T.mark(4);
+    if (nt > bound) assign(nt);
     if (timings) {
-        IDL_CUDA(cudaEventSynchronize(C.timing.ev[4]));
         timings[IDL_T_DETECT_MS] = T.ms(0, 1);
         timings[IDL_T_DEDUP_MS] = T.ms(1, 2);
         timings[IDL_T_ASSIGN_MS] = T.ms(3, 4);
@@ -485,7 +520,7 @@ int idl_voronoi(idl_context* ctx, int width, int height, const int32_t* seeds_xy
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
     sort_seeds_device(C, width, height, n_seeds, 0);
     int64_t passes = 0;
-    const bool resolved = start_labels(C, mode, cv, n_seeds, passes_out != nullptr, &passes);
+    const bool resolved = start_labels(C, mode, cv, n_seeds, 0, passes_out != nullptr, &passes);
     const size_t bytes = (size_t)width * height * 2 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
     auto deliver = [&] {
@@ -521,22 +556,21 @@ int idl_triangulate(idl_context* ctx, int width, int height, const int32_t* seed
     C.have_result = false;
     const int P = resolve_padding(border_padding);
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
-    Canvas cv;
     const size_t bytes = (size_t)width * height * 3 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, voronoi_grid, true, P, mode, timings_out, cv,
-                                       C.outgrid.as<int32_t>());
-    IDL_CUDA(cudaMemcpyAsync(grid_out, C.outgrid.ptr, bytes, cudaMemcpyDeviceToHost, C.stream));
-    if (padded_grid_out && P > 0) {
-        const size_t pb = (size_t)cv.Wd * cv.Hd * 2 * sizeof(int32_t);
-        C.padded.ensure(pb);
-        dim3 gp(ceil_div(cv.Wd, 256), cv.Hd);
-        k_compose2<<<gp, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, cv.Wd, cv.Hd, C.pos.as<uint32_t>(),
-                                             C.padded.as<int32_t>());
-        IDL_LAUNCH();
-        IDL_CUDA(cudaMemcpyAsync(padded_grid_out, C.padded.ptr, pb, cudaMemcpyDeviceToHost, C.stream));
-    }
-    IDL_CUDA(cudaStreamSynchronize(C.stream));
+    const int64_t nt = run_triangulate(
+        C, width, height, n_seeds, voronoi_grid, P, mode, timings_out, C.outgrid.as<int32_t>(), [&](const Canvas& cv) {
+            IDL_CUDA(cudaMemcpyAsync(grid_out, C.outgrid.ptr, bytes, cudaMemcpyDeviceToHost, C.stream));
+            if (padded_grid_out && P > 0) {
+                const size_t pb = (size_t)cv.Wd * cv.Hd * 2 * sizeof(int32_t);
+                C.padded.ensure(pb);
+                dim3 gp(ceil_div(cv.Wd, 256), cv.Hd);
+                k_compose2<<<gp, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, cv.Wd, cv.Hd,
+                                                     C.pos.as<uint32_t>(), C.padded.as<int32_t>());
+                IDL_LAUNCH();
+                IDL_CUDA(cudaMemcpyAsync(padded_grid_out, C.padded.ptr, pb, cudaMemcpyDeviceToHost, C.stream));
+            }
+        });
     if (n_triangles_out) *n_triangles_out = nt;
     IDL_API_END
 }
@@ -589,12 +623,9 @@ int idl_triangulate_device(idl_context* ctx, int width, int height, const int32_
     C.have_result = false;
     const int P = resolve_padding(border_padding);
     upload_seeds(C, d_seeds_xy, n_seeds, cudaMemcpyDeviceToDevice);
-    Canvas cv;
-    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, false, P, mode, nullptr, cv, d_grid_out);
-    if (n_triangles_out) {
-        IDL_CUDA(cudaStreamSynchronize(C.stream));
-        *n_triangles_out = nt;
-    }
+    const int64_t nt = run_triangulate(C, width, height, n_seeds, nullptr, P, mode, nullptr, d_grid_out,
+                                       [](const Canvas&) {});
+    if (n_triangles_out) *n_triangles_out = nt;
     IDL_API_END
 }
 

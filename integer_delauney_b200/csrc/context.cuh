@@ -94,8 +94,9 @@ struct Scalars {
     int32_t n_blocks;         // 2 x 2 blocks detection leaves to its second pass
     int32_t overflow;         // hash table over its load limit or probe bound
     int64_t last_change;      // last propagation step (0-based) that changed a cell
-    int32_t err_oob;          // a seed lay outside the canvas
+    int32_t err_oob;          // a seed lay outside the canvas (cleared with the next two)
     int32_t err_dup;          // two seeds share a pixel
+    int32_t scan_done;        // blocks of a scan that have finished (0 between scans)
     int32_t err_label;        // a caller-supplied label was outside [-1, n)
     int32_t max_side;         // longest triangle side, float-truncated (triangulation.cu:355-368)
     int32_t n_handoff;        // micro-tiles the last tile round hands to the persistent kernel
@@ -148,7 +149,7 @@ struct Context {
     DevBuf xs, ys;        // sorted seed coordinates (image space)
     DevBuf pos;           // sorted seed positions on the detection canvas, packed
     DevBuf bitmap;        // canvas occupancy bits, column major, for the (x, y) sort
-    DevBuf scan_a, scan_b, scan_c;  // scan scratch
+    DevBuf scan_a, scan_c;  // scan scratch; ranks of the occupancy bits' words
 
     // propagation
     DevBuf lab[2];        // label planes, pitch x Hd int32, ping-pong
@@ -181,7 +182,7 @@ struct Context {
     // topology
     DevBuf hkeys;         // hash table of triangle keys -> first witness (key, value interleaved)
     DevBuf ukeys, uvals;  // compacted unique keys
-    DevBuf cnt, off, fill, grp;  // group-by-smallest-vertex ranking
+    DevBuf cnt, off, grp;  // group-by-smallest-vertex ranking
     DevBuf tris;          // n_tri x 5 int32 (x, y, a, b, c)
     DevBuf verts;         // n_tri x 3 int32 (a, b, c) staged for idl_get_triangle_vertices
     int64_t hash_cap = 0;
@@ -224,10 +225,10 @@ struct Context {
     template <class F>
     void each_buf(F&& f)
     {
-        DevBuf* all[] = {&seeds_in, &xs, &ys, &pos, &bitmap, &scan_a, &scan_b, &scan_c, &lab[0], &lab[1],
+        DevBuf* all[] = {&seeds_in, &xs, &ys, &pos, &bitmap, &scan_a, &scan_c, &lab[0], &lab[1],
                          &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
                          &exact_bands, &sus_bits, &sus_list, &hkeys,
-                         &ukeys, &uvals, &cnt, &off, &fill, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
+                         &ukeys, &uvals, &cnt, &off, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
                          &batch_img, &batch_seed_img, &batch_sid, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
         for (DevBuf* b : all) f(*b);
@@ -242,6 +243,10 @@ struct Context {
     Scalars* sc() const { return scalars.as<Scalars>(); }
     size_t workspace_bytes() const;
     void fetch_scalars();        // D2H of the Scalars block + stream sync
+    // The same in two halves: what is queued between them does not delay the wait.
+    void fetch_scalars_begin();
+    void fetch_scalars_end();
+    cudaEvent_t fetched = nullptr;
     ~Context();
 };
 
@@ -266,6 +271,8 @@ struct DeviceGuard {
 // Exclusive scan of n int32 values in place semantics: out[i] = sum(in[0..i)),
 // and out[n] = total.  `out` must hold n + 1 values.  Uses ctx scan scratch.
 void exclusive_scan(Context& C, const int32_t* in, int32_t* out, int64_t n);
+// The same over the popcounts of n words.
+void exclusive_popc_scan(Context& C, const uint32_t* words, int32_t* out, int64_t n);
 
 // Validate and sort seeds on the device (seeds.cu).  Reads C.seeds_in (n x 2),
 // writes C.xs / C.ys (sorted, image space) and C.pos (detection canvas, shifted
@@ -342,16 +349,18 @@ void grid_barrier_selftest(Context& C, int missing_arrivals, unsigned spin_limit
 
 // Stage (a), exact semantics (exact.cu): nearest seed, ties to the higher id,
 // for the n (x, y)-sorted seeds `pos` of the canvas; labels into C.lab[0]
-// (C.lab[1] holds the column pass's offsets, C.exact_bands its table).
+// (C.lab[1] holds the column pass's offsets, C.exact_bands its table).  P: the
+// canvas's padding; C.bitmap and C.scan_c hold these seeds' occupancy bits and
+// their ranks, as sort_seeds_device and rank_seeds_device leave them.
 struct XImg;
-void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n);
+void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P);
 // The same for the images of a batch atlas (exact.cu): device tables of the
 // images, of each column pair's and each row's image; C.lab[0] and C.lab[1]
 // hold planes of the atlas.
 void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, const int32_t* pair_img, int n_pairs,
                   const int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries);
 // The one image of a single canvas with n seeds.
-XImg whole_canvas(const Canvas& cv, int64_t n);
+XImg whole_canvas(const Canvas& cv, int64_t n, int P);
 
 // Turns the exact labels propagate_exact left in C.lab[0] (and the column
 // plane in C.lab[1]) into the reference semantics' fixed point from scratch
@@ -383,8 +392,17 @@ void init_labels(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n);
 // keys, numbering and the recorded vertex ids use rank[label] instead.
 void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n,
                       int shift, cudaEvent_t mid = nullptr, const int32_t* rank = nullptr);
+// The same without the read-back: detect_launch queues it on a table of `cap`
+// slots (detect_capacity to begin with); once the scalars have been read back,
+// detect_done tells whether the table was large enough.
+int64_t detect_capacity(const Context& C, int64_t n);
+void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
+                   int64_t cap, cudaEvent_t mid = nullptr, const int32_t* rank = nullptr);
+bool detect_done(Context& C, int64_t cap);
 
-// Stage (d): per-pixel max triangle id over a W x H image (raster.cu).
+// Stage (d): per-pixel max triangle id over a W x H image (raster.cu), of the
+// triangles in C.tris, whose number is read on the device; n_tri is the
+// host's copy of it or an upper bound (triangles from n_tri on are not drawn).
 void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri);
 // The same with the (H, W, 3) output (seed id, squared distance, triangle id)
 // composed at once; lab points at the label of pixel (0, 0).

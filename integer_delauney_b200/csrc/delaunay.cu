@@ -976,7 +976,7 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
         d->spos.ensure((size_t)d->N * 4);
         k_pack_pos<<<blocks(d->N), 256, 0, C.stream>>>(d->sx, d->sy, d->N, 0, d->spos.as<uint32_t>());
         IDL_LAUNCH();
-        propagate_exact(C, d->canvas(), d->spos.as<uint32_t>(), d->N);
+        propagate_exact(C, d->canvas(), d->spos.as<uint32_t>(), d->N, d->P);
         k_exact_planes<<<dim3(blocks(d->Wd), (unsigned)d->Hd), 256, 0, C.stream>>>(
             d->planes, d->planes + (size_t)d->pitch * d->Hd, d->pitch, d->Wd, d->inv);
         IDL_LAUNCH();

@@ -29,21 +29,21 @@ namespace idl {
 namespace {
 
 __global__ void __launch_bounds__(64)
-k_column_off(const uint32_t* __restrict__ pos, XImg m, int pitch, int16_t* __restrict__ off,
+k_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, XImg m, int pitch, int16_t* __restrict__ off,
              int32_t* __restrict__ bands)
 {
     const int c = (blockIdx.x * 64 + threadIdx.x) * 2;
-    if (c < m.Wp) x_column_pair(pos, m, c, blockIdx.y, pitch, off, bands);
+    if (c < m.Wp) x_column_pair(pos, ranks, m, c, blockIdx.y, pitch, off, bands);
 }
 
 __global__ void __launch_bounds__(64)
-k_bx_column_off(const uint32_t* __restrict__ pos, const XImg* __restrict__ xi, const int32_t* __restrict__ pair_img,
+k_bx_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, const XImg* __restrict__ xi, const int32_t* __restrict__ pair_img,
                 int n_pairs, int pitch, int16_t* __restrict__ off, int32_t* __restrict__ bands)
 {
     const int g = blockIdx.x * 64 + threadIdx.x;
     if (g >= n_pairs) return;
     const XImg m = xi[pair_img[g]];
-    if ((int)blockIdx.y < x_bands(m)) x_column_pair(pos, m, (g - m.pair_off) * 2, blockIdx.y, pitch, off, bands);
+    if ((int)blockIdx.y < x_bands(m)) x_column_pair(pos, ranks, m, (g - m.pair_off) * 2, blockIdx.y, pitch, off, bands);
 }
 
 template <int T>
@@ -99,25 +99,27 @@ void rows_for_width(Context& C, int width, unsigned rows, A... args)
 
 }  // namespace
 
-XImg whole_canvas(const Canvas& cv, int64_t n)
+XImg whole_canvas(const Canvas& cv, int64_t n, int P)
 {
     XImg m{};
     m.Wp = cv.Wd;
     m.Hp = cv.Hd;
     m.s1 = (int)n;
+    m.P = P;
     return m;
 }
 
-void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n)
+void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P)
 {
     const size_t plane = (size_t)cv.pitch * cv.Hd * 4;
     C.lab[0].ensure(plane);
     C.lab[1].ensure(plane);
-    const XImg m = whole_canvas(cv, n);
+    const XImg m = whole_canvas(cv, n, P);
     C.exact_bands.ensure((size_t)x_bands(m) * cv.Wd * 4);
     int16_t* off = C.lab[1].as<int16_t>();
     int32_t* bands = C.exact_bands.as<int32_t>();
-    k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, m, cv.pitch, off,
+    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>()};
+    k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, ranks, m, cv.pitch, off,
                                                                                                bands);
     IDL_LAUNCH();
     rows_for_width<false>(C, cv.Wd, (unsigned)cv.Hd, (const int16_t*)off, m, cv.pitch, pos, (const int32_t*)bands,
@@ -138,8 +140,9 @@ void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, co
     C.exact_bands.ensure((size_t)band_entries * 4);
     int16_t* off = C.lab[1].as<int16_t>();
     int32_t* bands = C.exact_bands.as<int32_t>();
+    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>()};
     k_bx_column_off<<<dim3((unsigned)ceil_div(n_pairs, 64), (unsigned)ceil_div(max_hp, BAND)), 64, 0, C.stream>>>(
-        pos, xi, pair_img, n_pairs, pitch, off, bands);
+        pos, ranks, xi, pair_img, n_pairs, pitch, off, bands);
     IDL_LAUNCH();
     rows_for_width<true>(C, max_wp, (unsigned)n_rows, (const int16_t*)off, xi, row_img, pitch, pos,
                          (const int32_t*)bands, C.lab[0].as<int32_t>());

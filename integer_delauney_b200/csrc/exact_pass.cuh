@@ -18,6 +18,8 @@ struct XImg {
     int row_off;           // first entry in the row table
     int band_off;          // first entry in the band table
     int s0, s1;            // its seeds: ids [s0, s1), (x, y)-sorted
+    int P;                 // padding around the image proper
+    long long bit0;        // its first occupancy bit (column-major over the image proper)
 };
 
 constexpr int BAND = 64;                       // rows a thread of the column pass walks
@@ -25,18 +27,26 @@ constexpr int16_t NO_SEED = (int16_t)-32768;   // a column without seeds
 
 __host__ __device__ inline int x_bands(const XImg& m) { return (m.Hp + BAND - 1) / BAND; }
 
-// First of the image's seeds at or after (x, y) in (x, y) order.
-__device__ __forceinline__ int x_lower_bound(const uint32_t* __restrict__ pos, const XImg& m, int x, int y)
+// The seeds' occupancy bits, column-major image after image, and the number of
+// seeds before each word (seeds.cu): a seed's rank is the number before its bit.
+struct SeedRanks {
+    const uint32_t* bits;
+    const int32_t* before;
+};
+
+// First of the image's seeds at or after (x, y) in (x, y) order: two loads,
+// where a search of the sorted seeds takes one round trip to L2 per halving
+// (most of the column pass's time on a small image).
+__device__ __forceinline__ int x_lower_bound(const SeedRanks& R, const XImg& m, int x, int y)
 {
-    int lo = m.s0, hi = m.s1;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        const uint32_t p = __ldg(&pos[mid]);
-        const int px = pos_x(p);
-        if (px < x || (px == x && (int)pos_y(p) < y)) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
+    const int W = m.Wp - 2 * m.P, H = m.Hp - 2 * m.P;
+    const int c = x - m.ox - m.P;
+    if (c < 0) return m.s0;
+    if (c >= W) return m.s1;
+    const long long bit = m.bit0 + (long long)c * H + min(max(y - m.oy - m.P, 0), H);
+    if (bit >= m.bit0 + (long long)W * H) return m.s1;
+    const uint32_t below = __ldg(&R.bits[bit >> 5]) & ((1u << (bit & 31)) - 1u);
+    return __ldg(&R.before[bit >> 5]) + __popc(below);
 }
 
 // Id of the seed at (x, y) of the plane, which must exist: bands holds, per
@@ -51,10 +61,10 @@ __device__ __forceinline__ int32_t x_seed_at(const uint32_t* __restrict__ pos, c
 
 // One thread walks two adjacent columns (the pair starting at image column c)
 // through the rows of one band, so that a warp writes 128 bytes of a row at
-// once; its place in each column's seeds comes from one search of the sorted
-// seeds.  Two bytes per cell is all that is written (the planes of 4-byte ids
+// once; its place in each column's seeds comes from the seeds' ranks.  Two bytes per cell is all that is written (the planes of 4-byte ids
 // and distances this replaces took four times the traffic).
-__device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, const XImg& m, int c, int band,
+__device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, const SeedRanks& ranks,
+                                              const XImg& m, int c, int band,
                                               int pitch, int16_t* __restrict__ off, int32_t* __restrict__ bands)
 {
     const int y0 = band * BAND, y1 = min(m.Hp, y0 + BAND);
@@ -69,7 +79,7 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
         a[k] = 0;
         if (c + k < m.Wp) {
             const int x = m.ox + c + k;
-            a[k] = x_lower_bound(pos, m, x, m.oy + y0);
+            a[k] = x_lower_bound(ranks, m, x, m.oy + y0);
             bands[m.band_off + band * m.Wp + c + k] = a[k];
             if (a[k] < m.s1) {
                 const uint32_t p = __ldg(&pos[a[k]]);

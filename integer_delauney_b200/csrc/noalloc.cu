@@ -52,7 +52,7 @@ constexpr size_t align256(size_t b) { return (b + 255) & ~size_t(255); }
 
 constexpr size_t NA_SCRATCH_BYTES =
     3 * align256(NA_SEEDS) +                                  // xs, ys, pos
-    3 * align256(NA_BITS_WORDS * 4 + 4) +                     // occupancy bitmap, popcounts, ranks
+    2 * align256(NA_BITS_WORDS * 4 + 4) +                     // occupancy bitmap, ranks
     align256(NA_SCAN_ARENA * 4) +                             // scan block sums
     2 * align256(NA_PLANE) +                                  // label planes
     2 * align256(NA_TILES * 4) +                              // work lists
@@ -64,7 +64,7 @@ constexpr size_t NA_SCRATCH_BYTES =
 }  // namespace
 }  // namespace idl
 
-// The workspace itself (about 9.8 MB); a device holds it once this module is loaded there.
+// The workspace itself (about 9.7 MB); a device holds it once this module is loaded there.
 static __device__ __align__(256) unsigned char g_noalloc_scratch[idl::NA_SCRATCH_BYTES];
 
 namespace idl {
@@ -103,7 +103,6 @@ Context& noalloc_context(int dev)
     take(C.ys, NA_SEEDS);
     take(C.pos, NA_SEEDS);
     take(C.bitmap, NA_BITS_WORDS * 4 + 4);
-    take(C.scan_b, NA_BITS_WORDS * 4 + 4);
     take(C.scan_c, NA_BITS_WORDS * 4 + 4);
     take(C.scan_a, NA_SCAN_ARENA * 4);
     take(C.lab[0], NA_PLANE);

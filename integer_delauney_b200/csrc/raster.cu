@@ -39,7 +39,7 @@ k_raster_count(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const
 {
     const int tiles_x = (W + TILE::W - 1) / TILE::W;
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
-    const bool on = t < sc->n_triangles;
+    const bool on = t < min(sc->n_triangles, (int64_t)w.max_tri);
     Tri u{};
     if (on) u = load_tri(tris + t * 5 + 2, xs, ys);
     int side = on ? longest_side(u) : 0;
@@ -55,7 +55,7 @@ k_raster_fill(const Scalars* __restrict__ sc, int W, int H, RasterWork w)
 {
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     if (!w.head->overflow)
-        raster_fill<TILE>(w, t < sc->n_triangles, (int32_t)t, W, H, 0, (W + TILE::W - 1) / TILE::W);
+        raster_fill<TILE>(w, t < min(sc->n_triangles, (int64_t)w.max_tri), (int32_t)t, W, H, 0, (W + TILE::W - 1) / TILE::W);
 }
 
 template <class TILE>
@@ -127,6 +127,7 @@ RasterWork raster_work(Context& C, int64_t nt, int64_t n_tiles)
     w.list = reinterpret_cast<int32_t*>(w.xy + nt * 3);
     w.n_tiles = (int32_t)n_tiles;
     w.list_cap = (int32_t)cap;
+    w.max_tri = (int32_t)nt;
     IDL_CUDA(cudaMemsetAsync(base, 0, head + (size_t)n_tiles * 4, C.stream));
     return w;
 }

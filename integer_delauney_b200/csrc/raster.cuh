@@ -244,6 +244,7 @@ struct RasterWork {
     uint32_t* xy;       // three packed corners per triangle
     int32_t* list;      // triangles by tile
     int32_t n_tiles, list_cap;
+    int32_t max_tri;    // triangles there is room for
 };
 
 // Lays the work out on C.rbig for nt triangles and n_tiles tiles and clears

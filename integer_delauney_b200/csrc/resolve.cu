@@ -661,7 +661,7 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     IDL_CUDA(cudaMemsetAsync(sus, 0, bits, C.stream));
     IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
     const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), C.exact_bands.as<int32_t>(), pos, sus, images,
-                 seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n)};
+                 seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n, 0)};
     const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 4 * ROOT_ROWS));
     if (passes)
         k_roots<true><<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());

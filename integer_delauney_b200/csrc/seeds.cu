@@ -15,8 +15,10 @@
 namespace idl {
 
 // ---------------------------------------------------------------------------
-// exclusive scan (int32), 3-phase: per-block scan, scan of block totals,
-// add-back.  4096 items per block.
+// exclusive scan (int32, or of the popcounts of 32-bit words): per-block sums,
+// scanned by the block that finishes last, then the blocks' own scans on top.
+// Two launches, one for up to SCAN_TILE items: on a small image the launches
+// of a scan level by level cost more than the scan.
 // ---------------------------------------------------------------------------
 namespace {
 
@@ -24,120 +26,112 @@ constexpr int SCAN_THREADS = 512;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
-__global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_block(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n,
-             int32_t* __restrict__ block_sums)
+template <bool POPC>
+__device__ __forceinline__ int32_t scan_item(const int32_t* __restrict__ in, int64_t j, int64_t n)
 {
-    __shared__ int32_t warp_tot[SCAN_THREADS / 32];
-    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    int32_t v[SCAN_ITEMS];
-    int32_t run = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const int64_t j = base + i;
-        v[i] = j < n ? in[j] : 0;
-        const int32_t t = v[i];
-        v[i] = run;          // exclusive within the thread
-        run += t;
-    }
-    // inclusive warp scan of thread totals
+    if (j >= n) return 0;
+    return POPC ? __popc((uint32_t)in[j]) : in[j];
+}
+
+// Exclusive prefix of v over the block's threads; *total: their sum.
+__device__ __forceinline__ int32_t block_prefix(int32_t v, int32_t* total)
+{
+    __shared__ int32_t warp_sum[SCAN_THREADS / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int32_t x = run;
+    int32_t x = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
-    if (lane == 31) warp_tot[warp] = x;
+    if (lane == 31) warp_sum[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-        int32_t w = lane < SCAN_THREADS / 32 ? warp_tot[lane] : 0;
+    int32_t before = 0, all = 0;
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= o) w += y;
-        }
-        if (lane < SCAN_THREADS / 32) warp_tot[lane] = w;   // inclusive
+    for (int k = 0; k < SCAN_THREADS / 32; ++k) {
+        const int32_t w = warp_sum[k];
+        before += k < warp ? w : 0;
+        all += w;
     }
     __syncthreads();
-    const int32_t warp_excl = warp > 0 ? warp_tot[warp - 1] : 0;
-    const int32_t thread_excl = warp_excl + x - run;
+    *total = all;
+    return before + x - v;
+}
+
+template <bool POPC>
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_scan_sums(const int32_t* __restrict__ in, int64_t n, int32_t* __restrict__ sums, int32_t* __restrict__ total,
+            int32_t* __restrict__ done)
+{
+    __shared__ bool last;
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE;
+    int32_t v = 0, all;
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i) v += scan_item<POPC>(in, base + i * SCAN_THREADS + threadIdx.x, n);
+    block_prefix(v, &all);
+    if (threadIdx.x == 0) {
+        sums[blockIdx.x] = all;
+        __threadfence();
+        last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    int32_t carry = 0;
+    for (unsigned b0 = 0; b0 < gridDim.x; b0 += SCAN_THREADS) {
+        const unsigned b = b0 + threadIdx.x;
+        const int32_t s = b < gridDim.x ? __ldcg(&sums[b]) : 0;
+        const int32_t before = block_prefix(s, &all);
+        if (b < gridDim.x) sums[b] = carry + before;
+        carry += all;
+    }
+    if (threadIdx.x == 0) {
+        *total = carry;
+        *done = 0;   // for the next scan on this context
+    }
+}
+
+template <bool POPC>
+__global__ void __launch_bounds__(SCAN_THREADS)
+k_scan_write(const int32_t* __restrict__ in, int32_t* __restrict__ out, int64_t n, const int32_t* __restrict__ sums)
+{
+    const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
+    int32_t v[SCAN_ITEMS];
+    int32_t run = 0, all;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const int64_t j = base + i;
-        if (j < n) out[j] = thread_excl + v[i];
+        v[i] = run;
+        run += scan_item<POPC>(in, base + i, n);
     }
-    if (threadIdx.x == SCAN_THREADS - 1) block_sums[blockIdx.x] = thread_excl + run;
+    const int32_t before = (sums ? sums[blockIdx.x] : 0) + block_prefix(run, &all);
+#pragma unroll
+    for (int i = 0; i < SCAN_ITEMS; ++i)
+        if (base + i < n) out[base + i] = before + v[i];
+    if (!sums && threadIdx.x == 0) out[n] = all;
 }
 
-__global__ void k_scan_add(int32_t* __restrict__ out, int64_t n, const int32_t* __restrict__ offs)
+template <bool POPC>
+void scan(Context& C, const int32_t* in, int32_t* out, int64_t n)
 {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < n) out[j] += offs[j / SCAN_TILE];
-}
-
-__global__ void k_set_total(int32_t* __restrict__ out, int64_t n, const int32_t* __restrict__ total)
-{
-    out[n] = *total;
+    const int64_t nb = std::max<int64_t>(1, (n + SCAN_TILE - 1) / SCAN_TILE);
+    int32_t* sums = nullptr;
+    if (nb > 1) {
+        C.scan_a.ensure((size_t)nb * sizeof(int32_t));
+        sums = C.scan_a.as<int32_t>();
+        k_scan_sums<POPC><<<(unsigned)nb, SCAN_THREADS, 0, C.stream>>>(in, n, sums, out + n, &C.sc()->scan_done);
+        IDL_LAUNCH();
+    }
+    k_scan_write<POPC><<<(unsigned)nb, SCAN_THREADS, 0, C.stream>>>(in, out, n, sums);
+    IDL_LAUNCH();
 }
 
 }  // namespace
 
-void exclusive_scan(Context& C, const int32_t* in, int32_t* out, int64_t n)
-{
-    // level sizes (fixed-size bookkeeping: no host allocation on this path;
-    // 4096^8 items is far beyond any int32 count)
-    constexpr int MAX_LEVELS = 8;
-    int64_t lens[MAX_LEVELS];
-    int nlev = 0;
-    int64_t m = n;
-    for (;;) {
-        const int64_t nb = (m + SCAN_TILE - 1) / SCAN_TILE;
-        if (nlev == MAX_LEVELS) throw Error(IDL_ERR_INTERNAL, "scan too large");
-        lens[nlev++] = nb > 0 ? nb : 1;
-        if (nb <= 1) break;
-        m = nb;
-    }
-    // scratch: per level, block sums (nb) and their scan (nb + 1)
-    size_t need = 0;
-    for (int l = 0; l < nlev; ++l) need += size_t(2 * lens[l] + 1);
-    C.scan_a.ensure(need * sizeof(int32_t));
-    int32_t* arena = C.scan_a.as<int32_t>();
+void exclusive_scan(Context& C, const int32_t* in, int32_t* out, int64_t n) { scan<false>(C, in, out, n); }
 
-    int32_t* sums[MAX_LEVELS];
-    int32_t* scans[MAX_LEVELS];
-    size_t at = 0;
-    for (int l = 0; l < nlev; ++l) {
-        sums[l] = arena + at;  at += lens[l];
-        scans[l] = arena + at; at += lens[l] + 1;
-    }
-    // down: scan each level's input into its output
-    const int32_t* lin = in;
-    int32_t* lout = out;
-    int64_t len = n;
-    for (int l = 0; l < nlev; ++l) {
-        const int64_t nb = lens[l];
-        k_scan_block<<<(unsigned)nb, SCAN_THREADS, 0, C.stream>>>(lin, lout, len, sums[l]);
-        IDL_LAUNCH();
-        if (nb <= 1) {
-            k_set_total<<<1, 1, 0, C.stream>>>(lout, len, sums[l]);
-            IDL_LAUNCH();
-            break;
-        }
-        lin = sums[l];
-        lout = scans[l];
-        len = nb;
-    }
-    // up: add scanned block offsets back, deepest first
-    for (int l = nlev - 2; l >= 0; --l) {
-        int32_t* target = (l == 0) ? out : scans[l - 1];
-        const int64_t tlen = (l == 0) ? n : lens[l - 1];
-        k_scan_add<<<(unsigned)((tlen + 255) / 256), 256, 0, C.stream>>>(target, tlen, scans[l]);
-        IDL_LAUNCH();
-        // total of this level = last entry of scans[l]
-        k_set_total<<<1, 1, 0, C.stream>>>(target, tlen, scans[l] + lens[l]);
-        IDL_LAUNCH();
-    }
+void exclusive_popc_scan(Context& C, const uint32_t* words, int32_t* out, int64_t n)
+{
+    scan<true>(C, reinterpret_cast<const int32_t*>(words), out, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -159,12 +153,6 @@ __global__ void k_seed_mark(const int32_t* __restrict__ xy, int64_t n, int W, in
     const uint32_t m = 1u << (bit & 31);
     const uint32_t old = atomicOr(&bitmap[bit >> 5], m);
     if (old & m) atomicOr(&sc->err_dup, 1);
-}
-
-__global__ void k_popc(const uint32_t* __restrict__ bitmap, int64_t nwords, int32_t* __restrict__ out)
-{
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < nwords) out[i] = __popc(bitmap[i]);
 }
 
 __global__ void k_seed_rank(const int32_t* __restrict__ xy, int64_t n, int W, int H, int P,
@@ -216,16 +204,12 @@ void rank_seeds_device(Context& C, int W, int H, const int32_t* xs, const int32_
     if (n <= 0) return;
     const int64_t nwords = ((int64_t)W * H + 31) / 32;
     C.bitmap.ensure(size_t(nwords) * 4);
-    C.scan_b.ensure(size_t(nwords) * 4);
     C.scan_c.ensure(size_t(nwords + 1) * 4);
     IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, size_t(nwords) * 4, C.stream));
     const unsigned gs = (unsigned)((n + 255) / 256);
     k_mark_xy<<<gs, 256, 0, C.stream>>>(xs, ys, n, H, C.bitmap.as<uint32_t>());
     IDL_LAUNCH();
-    k_popc<<<(unsigned)((nwords + 255) / 256), 256, 0, C.stream>>>(C.bitmap.as<uint32_t>(), nwords,
-                                                                  C.scan_b.as<int32_t>());
-    IDL_LAUNCH();
-    exclusive_scan(C, C.scan_b.as<int32_t>(), C.scan_c.as<int32_t>(), nwords);
+    exclusive_popc_scan(C, C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nwords);
     k_rank_xy<<<gs, 256, 0, C.stream>>>(xs, ys, n, H, C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), off, rank,
                                         inv, xs_sorted, ys_sorted);
     IDL_LAUNCH();
@@ -236,29 +220,27 @@ void sort_seeds_device(Context& C, int W, int H, int64_t n, int P)
     const int64_t bits = (int64_t)W * H;
     const int64_t nwords = (bits + 31) / 32;
     C.bitmap.ensure(size_t(nwords) * 4);
-    C.scan_b.ensure(size_t(nwords) * 4);
     C.scan_c.ensure(size_t(nwords + 1) * 4);
     C.xs.ensure(size_t(n) * 4);
     C.ys.ensure(size_t(n) * 4);
     C.pos.ensure(size_t(n) * 4);
 
     IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, size_t(nwords) * 4, C.stream));
-    IDL_CUDA(cudaMemsetAsync(&C.sc()->err_oob, 0, 2 * sizeof(int32_t), C.stream));
+    IDL_CUDA(cudaMemsetAsync(&C.sc()->err_oob, 0, 3 * sizeof(int32_t), C.stream));
     const unsigned gs = (unsigned)((n + 255) / 256);
     k_seed_mark<<<gs, 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, W, H, C.bitmap.as<uint32_t>(), C.sc());
     IDL_LAUNCH();
-    C.fetch_scalars();
-    if (C.host_sc->err_oob) invalid("seed coordinate out of bounds");
-    if (C.host_sc->err_dup) invalid("duplicate seed positions are not allowed");
-
-    k_popc<<<(unsigned)((nwords + 255) / 256), 256, 0, C.stream>>>(C.bitmap.as<uint32_t>(), nwords,
-                                                                  C.scan_b.as<int32_t>());
-    IDL_LAUNCH();
-    exclusive_scan(C, C.scan_b.as<int32_t>(), C.scan_c.as<int32_t>(), nwords);
+    C.fetch_scalars_begin();
+    exclusive_popc_scan(C, C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nwords);
     k_seed_rank<<<gs, 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, W, H, P, C.bitmap.as<uint32_t>(),
                                           C.scan_c.as<int32_t>(), C.xs.as<int32_t>(), C.ys.as<int32_t>(),
                                           C.pos.as<uint32_t>());
     IDL_LAUNCH();
+    // the flags are waited for with the ranking already queued behind them (it
+    // stays in bounds on seeds that are about to be refused)
+    C.fetch_scalars_end();
+    if (C.host_sc->err_oob) invalid("seed coordinate out of bounds");
+    if (C.host_sc->err_dup) invalid("duplicate seed positions are not allowed");
 }
 
 }  // namespace idl

@@ -380,72 +380,86 @@ __global__ void k_rank(const unsigned long long* __restrict__ ukeys, const unsig
 
 }  // namespace
 
-void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n,
-                      int shift, cudaEvent_t mid, const int32_t* rank)
+int64_t detect_capacity(const Context& C, int64_t n)
 {
     // Unique triangles of a planar triangulation number under 2n; the table
     // starts at four times that (a table half that size probes longer: 70 us
-    // against 53 us of detection at 200 000 seeds), and on the rare probe overflow it grows and
-    // the detection is redone.  The occupied slots are counted while they are
-    // compacted (one atomic per block), not while they are inserted, where a
-    // single counter would serialise every new key.
-    int64_t cap = std::max<int64_t>(next_pow2(8 * n + 1024), C.hash_cap);
-    C.cnt.ensure((size_t)(n + 1) * 4);
-    C.off.ensure((size_t)(n + 2) * 4);
-    C.fill.ensure((size_t)(n + 1) * 4);
-    for (int attempt = 0;; ++attempt) {
-        C.hkeys.ensure((size_t)cap * 16);
-        C.ukeys.ensure((size_t)cap * 8);
-        C.uvals.ensure((size_t)cap * 8);
-        // grouping and ranking follow with no read-back between: their
-        // buffers hold as many triangles as the table has slots, and their
-        // count comes from the device
-        C.grp.ensure((size_t)cap * 4);
-        C.tris.ensure((size_t)cap * 5 * 4);
-        IDL_CUDA(cudaMemsetAsync(C.hkeys.ptr, 0xFF, (size_t)cap * 16, C.stream));
-        // the blocks left to k_detect_rest wait in the grouping buffer, free until then
-        uint32_t* rest = C.grp.as<uint32_t>();
-        static_assert(offsetof(Scalars, overflow) == 12 && offsetof(Scalars, n_blocks) == 8, "cleared together");
-        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
-        IDL_CUDA(cudaMemsetAsync(C.cnt.ptr, 0, (size_t)(n + 1) * 4, C.stream));
+    // against 53 us of detection at 200 000 seeds), and on the rare probe
+    // overflow it grows and the detection is redone.  The occupied slots are
+    // counted while they are compacted (one atomic per block), not while they
+    // are inserted, where a single counter would serialise every new key.
+    return std::max<int64_t>(next_pow2(8 * n + 1024), C.hash_cap);
+}
 
-        const int strips = ceil_div(std::max(cv.Wd - 1, 1), DET_COLS);
-        const bool small = strips * ceil_div(cv.Hd, DET_ROWS) < C.num_sms * 16;
-        const dim3 grd(strips, ceil_div(std::max(cv.Hd - 1, 1), (small ? DET_ROWS_SMALL : DET_ROWS) * DET_WARPS));
-        auto* detect = small ? k_detect<DET_ROWS_SMALL> : k_detect<DET_ROWS>;
-        detect<<<grd, DET_WARPS * 32, 0, C.stream>>>(labels, cv.pitch, cv.Wd, cv.Hd, pos, rank,
-                                                     C.hkeys.as<unsigned long long>(), (unsigned long long)(cap - 1),
-                                                     C.sc(), rest, (int)cap);
-        IDL_LAUNCH();
-        k_detect_rest<<<C.num_sms * 4, 128, 0, C.stream>>>(labels, cv.pitch, cv.Wd, pos, rank,
-                                                          C.hkeys.as<unsigned long long>(),
-                                                          (unsigned long long)(cap - 1), C.sc(), rest, (int)cap);
-        IDL_LAUNCH();
-        if (mid) IDL_CUDA(cudaEventRecord(mid, C.stream));
-        C.mark(PM_DETECT);
-        const int g1 = (int)std::min<int64_t>(ceil_div(cap, 256), C.num_sms * 16);
-        k_enumerate<<<g1, ENUM_THREADS, 0, C.stream>>>(C.hkeys.as<unsigned long long>(), cap,
-                                              C.ukeys.as<unsigned long long>(),
-                                              C.uvals.as<unsigned long long>(), C.cnt.as<int32_t>(), C.sc());
-        IDL_LAUNCH();
-        IDL_CUDA(cudaMemsetAsync(C.fill.ptr, 0, (size_t)(n + 1) * 4, C.stream));
-        exclusive_scan(C, C.cnt.as<int32_t>(), C.off.as<int32_t>(), n);
-        const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(2 * n + 2, 256), C.num_sms * 16));
-        k_group<<<g2, 256, 0, C.stream>>>(C.ukeys.as<unsigned long long>(), C.sc(), C.off.as<int32_t>(),
-                                          C.fill.as<int32_t>(), C.grp.as<int32_t>());
-        IDL_LAUNCH();
-        k_rank<<<g2, 256, 0, C.stream>>>(C.ukeys.as<unsigned long long>(), C.uvals.as<unsigned long long>(), C.sc(),
-                                         C.off.as<int32_t>(), C.grp.as<int32_t>(), cv.Wd, shift, C.tris.as<int32_t>());
-        IDL_LAUNCH();
+void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
+                   int64_t cap, cudaEvent_t mid, const int32_t* rank)
+{
+    C.cnt.ensure((size_t)(n + 1) * 2 * 4);   // counts, then fill positions: cleared together
+    C.off.ensure((size_t)(n + 2) * 4);
+    int32_t* cnt = C.cnt.as<int32_t>();
+    int32_t* fill = cnt + n + 1;
+    C.hkeys.ensure((size_t)cap * 16);
+    C.ukeys.ensure((size_t)cap * 8);
+    C.uvals.ensure((size_t)cap * 8);
+    // grouping and ranking follow with no read-back between: their
+    // buffers hold as many triangles as the table has slots, and their
+    // count comes from the device
+    C.grp.ensure((size_t)cap * 4);
+    C.tris.ensure((size_t)cap * 5 * 4);
+    unsigned long long* table = C.hkeys.as<unsigned long long>();
+    unsigned long long* ukeys = C.ukeys.as<unsigned long long>();
+    unsigned long long* uvals = C.uvals.as<unsigned long long>();
+    IDL_CUDA(cudaMemsetAsync(table, 0xFF, (size_t)cap * 16, C.stream));
+    // the blocks left to k_detect_rest wait in the grouping buffer, free until then
+    uint32_t* rest = C.grp.as<uint32_t>();
+    static_assert(offsetof(Scalars, overflow) == 12 && offsetof(Scalars, n_blocks) == 8, "cleared together");
+    IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
+    IDL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(n + 1) * 2 * 4, C.stream));
+
+    const int strips = ceil_div(std::max(cv.Wd - 1, 1), DET_COLS);
+    const bool small = strips * ceil_div(cv.Hd, DET_ROWS) < C.num_sms * 16;
+    const dim3 grd(strips, ceil_div(std::max(cv.Hd - 1, 1), (small ? DET_ROWS_SMALL : DET_ROWS) * DET_WARPS));
+    auto* detect = small ? k_detect<DET_ROWS_SMALL> : k_detect<DET_ROWS>;
+    detect<<<grd, DET_WARPS * 32, 0, C.stream>>>(labels, cv.pitch, cv.Wd, cv.Hd, pos, rank, table,
+                                                 (unsigned long long)(cap - 1), C.sc(), rest, (int)cap);
+    IDL_LAUNCH();
+    k_detect_rest<<<C.num_sms * 4, 128, 0, C.stream>>>(labels, cv.pitch, cv.Wd, pos, rank, table,
+                                                      (unsigned long long)(cap - 1), C.sc(), rest, (int)cap);
+    IDL_LAUNCH();
+    if (mid) IDL_CUDA(cudaEventRecord(mid, C.stream));
+    C.mark(PM_DETECT);
+    const int g1 = (int)std::min<int64_t>(ceil_div(cap, 256), C.num_sms * 16);
+    k_enumerate<<<g1, ENUM_THREADS, 0, C.stream>>>(table, cap, ukeys, uvals, cnt, C.sc());
+    IDL_LAUNCH();
+    exclusive_scan(C, cnt, C.off.as<int32_t>(), n);
+    const int g2 = (int)std::max<int64_t>(1, std::min<int64_t>(ceil_div(2 * n + 2, 256), C.num_sms * 16));
+    k_group<<<g2, 256, 0, C.stream>>>(ukeys, C.sc(), C.off.as<int32_t>(), fill, C.grp.as<int32_t>());
+    IDL_LAUNCH();
+    k_rank<<<g2, 256, 0, C.stream>>>(ukeys, uvals, C.sc(), C.off.as<int32_t>(), C.grp.as<int32_t>(), cv.Wd, shift,
+                                     C.tris.as<int32_t>());
+    IDL_LAUNCH();
+}
+
+bool detect_done(Context& C, int64_t cap)
+{
+    if (C.host_sc->overflow) return false;
+    // keep the next run's table at most half full
+    C.hash_cap = C.host_sc->n_triangles > cap / 2 ? cap * 4 : cap;
+    return true;
+}
+
+void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n,
+                      int shift, cudaEvent_t mid, const int32_t* rank)
+{
+    int64_t cap = detect_capacity(C, n);
+    for (int attempt = 0;; ++attempt) {
+        detect_launch(C, cv, labels, pos, n, shift, cap, mid, rank);
         // one read-back: overflow (then all of it again, with a larger table) and the count
         C.fetch_scalars();
-        if (!C.host_sc->overflow) break;
+        if (detect_done(C, cap)) break;
         if (attempt >= 6) throw Error(IDL_ERR_INTERNAL, "triangle hash table overflow");
         cap *= 4;
     }
-    const int64_t nu = C.host_sc->n_triangles;
-    if (nu > cap / 2) cap *= 4;          // keep the next run's table at most half full
-    C.hash_cap = cap;
 }
 
 }  // namespace idl
