@@ -79,6 +79,16 @@ __device__ __forceinline__ void best_of4_keys(int32_t& b, int32_t n0, int32_t n1
     relax_key(b, bd, n3, x, y);
 }
 
+// relax() with the candidate's position at hand, without branches.
+__device__ __forceinline__ void relax_pos(int32_t& bl, int32_t& bd, uint32_t& bp, int32_t n, uint32_t np, int x, int y)
+{
+    const int32_t nd = dist2(x, y, np);
+    const bool better = n >= 0 && (nd < bd || (nd == bd && n > bl));
+    bl = better ? n : bl;
+    bd = better ? nd : bd;
+    bp = better ? np : bp;
+}
+
 // Per-block staging of next-pass list entries.  Groups reserve slots with
 // atomicAdd on *n; a group whose slots would run past STAGE goes to the global
 // list instead and lowers *cut to its first slot, so that only the prefix
@@ -275,6 +285,12 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
         const int gx = gx0 + j;
         c[j] = (row_in && gx >= 0 && gx < Wd) ? __ldcg(cur + (size_t)gy * pitch + gx) : OUTSIDE;
     }
+    // ids: their seeds' positions, gathered once and handed on with the labels
+    // (looked up candidate by candidate, the passes of a lone micro-tile were a
+    // chain of loads)
+    uint32_t cp[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cp[j] = !KEYS && c[j] >= 0 ? __ldg(&pos[c[j]]) : 0u;
     // this lane's inner cells: region rows RK .. RK + MT - 1, columns RK .. RK + MT - 1
     const bool inner_row = r >= RK && r < RK + MT;
     // (registers are indexed statically: h picks c[0..3] or c[4..7])
@@ -286,7 +302,10 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
 #pragma unroll 1
     for (int p = 0; p < RK; ++p) {
         const int32_t lft = __shfl_up_sync(FULL, c[7], 1), rgt = __shfl_down_sync(FULL, c[0], 1);
+        const uint32_t lft_p = KEYS ? 0u : __shfl_up_sync(FULL, cp[7], 1);
+        const uint32_t rgt_p = KEYS ? 0u : __shfl_down_sync(FULL, cp[0], 1);
         int32_t nv[8];
+        uint32_t np[8];
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
             const int32_t up = __shfl_up_sync(FULL, c[j], 2), dn = __shfl_down_sync(FULL, c[j], 2);
@@ -299,18 +318,35 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
                 int32_t k = b;
                 best_of4_keys(k, L, R, U, D, gx0 + j, gy);
                 b = b >= UNDEF ? k : b;
-            } else if (b >= UNDEF && (L != b || R != b || U != b || D != b)) {
-                best_of4(b, L, R, U, D, gx0 + j, gy, pos);
+                np[j] = 0u;
+            } else {
+                const uint32_t Up = __shfl_up_sync(FULL, cp[j], 2), Dp = __shfl_down_sync(FULL, cp[j], 2);
+                const uint32_t Lp = j > 0 ? cp[j - 1] : lft_p, Rp = j < 7 ? cp[j + 1] : rgt_p;
+                int32_t k = b, d = b >= 0 ? dist2(gx0 + j, gy, cp[j]) : FAR;
+                uint32_t kp = cp[j];
+                relax_pos(k, d, kp, L, Lp, gx0 + j, gy);
+                relax_pos(k, d, kp, R, Rp, gx0 + j, gy);
+                relax_pos(k, d, kp, U, Up, gx0 + j, gy);
+                relax_pos(k, d, kp, D, Dp, gx0 + j, gy);
+                np[j] = b >= UNDEF ? kp : cp[j];
+                b = b >= UNDEF ? k : b;
             }
             nv[j] = b;
         }
+        bool moved = false;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) moved = moved || nv[j] != c[j];
         ch = false;
 #pragma unroll
         for (int q = 0; q < 4; ++q) ch = ch || (h ? nv[q] != c[q] : nv[4 + q] != c[4 + q]);
         ch = ch && inner_row;
         if (__any_sync(FULL, ch)) last = p;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) c[j] = nv[j];
+        for (int j = 0; j < 8; ++j) {
+            c[j] = nv[j];
+            cp[j] = np[j];
+        }
+        if (!__any_sync(FULL, moved)) break;   // nor will the next passes change the region
     }
     if (inner_row && gy < Hd) {
         const int gxi = mx * MT + 4 * h;
@@ -369,7 +405,7 @@ template <bool KEYS>
 __global__ void __launch_bounds__(SJ_THREADS, 1)
 k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
                 uint32_t* bits0, uint32_t* bits1, int32_t* list0, int32_t* list1, int32_t* counts, int max_steps,
-                int mt_x, int mt_y, int rounds_below, GridSync* gs, unsigned long long* trace)
+                int mt_x, int mt_y, int rounds_below, int start_rounds, GridSync* gs, unsigned long long* trace)
 {
     // trace (profiling only): the global timer at the start and after each
     // generation, and from trace[max_steps + 2] on the passes each advanced
@@ -385,7 +421,7 @@ k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, con
     int t = 0;              // passes done
     int g = 0;              // generation
     int par = 0;            // plane holding the current state
-    bool rounds = false;
+    bool rounds = start_rounds != 0;   // the first list is one for the round mode
     bool converged = false;
     for (; t < max_steps; ++g) {
         const int n = *reinterpret_cast<volatile int32_t*>(&counts[g]);
@@ -479,24 +515,24 @@ __global__ void k_iota_list(int32_t* __restrict__ list, int n, int mt_x, int32_t
     if (i == 0) *count = n;
 }
 
-// Initial work list of a continued propagation: the micro-tiles holding a new
-// seed cell or one of its 4 neighbours (the only cells pass 0 can change).
-__global__ void k_seed_tiles(const uint32_t* __restrict__ seed_pos, int n_new, int Wd, int Hd, int mt_x,
+// Initial work list of a continued propagation: the micro-tiles with a cell
+// within `reach` steps of a new seed (1: the cells the first pass can change;
+// RK: those of the first round).
+__global__ void k_seed_tiles(const uint32_t* __restrict__ seed_pos, int n_new, int mt_x, int mt_y, int reach,
                              uint32_t* __restrict__ bits, int32_t* __restrict__ list, int32_t* __restrict__ count)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_new) return;
-    const uint32_t p = seed_pos[i];
+    if (i >= n_new * 9) return;
+    const uint32_t p = seed_pos[i / 9];
     const int x = pos_x(p), y = pos_y(p);
-    const int dx[5] = {0, -1, 1, 0, 0}, dy[5] = {0, 0, 0, -1, 1};
-#pragma unroll
-    for (int j = 0; j < 5; ++j) {
-        const int cx = x + dx[j], cy = y + dy[j];
-        if (cx < 0 || cy < 0 || cx >= Wd || cy >= Hd) continue;
-        const int mt = (cy / MT) * mt_x + cx / MT;
-        const uint32_t bit = 1u << (mt & 31);
-        if (!(atomicOr(&bits[mt >> 5], bit) & bit)) list[atomicAdd(count, 1)] = pack_mt(cx / MT, cy / MT);
-    }
+    const int dx = i % 9 % 3 - 1, dy = i % 9 / 3 - 1;
+    const int mx = x / MT + dx, my = y / MT + dy;
+    if (mx < 0 || my < 0 || mx >= mt_x || my >= mt_y) return;
+    const int sx = dx < 0 ? x % MT + 1 : dx > 0 ? MT - x % MT : 0, sy = dy < 0 ? y % MT + 1 : dy > 0 ? MT - y % MT : 0;
+    if (sx + sy > reach) return;
+    const int mt = my * mt_x + mx;
+    const uint32_t bit = 1u << (mt & 31);
+    if (!(atomicOr(&bits[mt >> 5], bit) & bit)) list[atomicAdd(count, 1)] = pack_mt(mx, my);
 }
 
 __global__ void k_fill_bits(uint32_t* __restrict__ bits, int n_words, int n_items)
@@ -609,6 +645,7 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
     int32_t* counts = C.counts.as<int32_t>();
     int32_t* l0 = C.tiles[0].as<int32_t>();
     int32_t* l1 = C.tiles[1].as<int32_t>();
+    int start_rounds = 0;
     if (st.marked) {
         // the hand-off list (capacity n_mt) serves as the first list itself;
         // its length comes from the device (an empty one ends the kernel at
@@ -626,8 +663,11 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
     } else if (st.seed_pos) {
         if (st.n_new == 0) return 0;
         IDL_CUDA(cudaMemsetAsync(b0, 0, (size_t)n_words * 2 * 4, C.stream));
-        k_seed_tiles<<<(unsigned)((st.n_new + 255) / 256), 256, 0, C.stream>>>(st.seed_pos, (int)st.n_new, cv.Wd,
-                                                                               cv.Hd, mt_x, b0, l0, counts);
+        // few seeds: straight into the round mode, whose reach is known here
+        // (entering it on the device lists all eight neighbours of each micro-tile)
+        start_rounds = st.n_new <= std::max(C.tail_rounds_below, 0);
+        k_seed_tiles<<<(unsigned)((st.n_new * 9 + 255) / 256), 256, 0, C.stream>>>(
+            st.seed_pos, (int)st.n_new, mt_x, mt_y, start_rounds ? RK : 1, b0, l0, counts);
         IDL_LAUNCH();
     } else {
         k_fill_bits<<<(unsigned)((n_words + 255) / 256), 256, 0, C.stream>>>(b0, n_words, n_mt);
@@ -648,13 +688,13 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
     int32_t* p1 = C.lab[1].as<int32_t>();
     GridSync* gs = C.gsync.as<GridSync>();
     int pitch = cv.pitch, Wd = cv.Wd, Hd = cv.Hd, ms = max_steps, mx = mt_x, my = mt_y;
-    int rb = std::max(C.tail_rounds_below, 0);
+    int rb = std::max(C.tail_rounds_below, 0), sr = start_rounds;
     unsigned long long* trace = nullptr;
     if (C.prof.enabled) {
         C.trace.ensure(((size_t)max_steps + 2) * 2 * 8);   // timestamps, then passes per generation
         trace = C.trace.as<unsigned long long>();
     }
-    void* args[] = {&p0, &p1, &pitch, &Wd, &Hd, (void*)&pos, &b0, &b1, &l0, &l1, &counts, &ms, &mx, &my, &rb, &gs,
+    void* args[] = {&p0, &p1, &pitch, &Wd, &Hd, (void*)&pos, &b0, &b1, &l0, &l1, &counts, &ms, &mx, &my, &rb, &sr, &gs,
                     &trace};
     GridSync h{};
     {
