@@ -266,11 +266,35 @@ constexpr int RK = 4;
 constexpr int RR = MT + 2 * RK;
 static_assert(RR == 16 && MT == 8 && RK == MT / 2, "lane layout: 16 rows of two 8-cell halves");
 
+// Block rounds (below): passes, and reach, of one.
+constexpr int BK = 12;
+constexpr int BR = MT + 2 * BK;
+static_assert(BR == 32 && SJ_THREADS == BR * BR, "one thread per cell, one warp per region row");
+constexpr int BLOCK_BELOW = 384;    // list length from which a round's next list is one for block rounds
+constexpr int BLOCK_LIMIT = 1536;   // and above which such a list is run in ordinary rounds again
+
+// Lists the micro-tile itself and, if any inner cell changed in the round's
+// last pass (columns x0..x1, rows y0..y1 of the micro-tile bound them), the
+// micro-tiles within BK steps of them.  Warp-wide.
+__device__ __forceinline__ void list_reach(bool any, int x0, int x1, int y0, int y1, int mx, int my, int mt_x,
+                                           int mt_y, uint32_t* bout, int32_t* lout, int32_t* count_out, Stage st,
+                                           int lane)
+{
+    static_assert(BK <= 2 * MT, "two micro-tiles to each side");
+    const int dx = lane % 5 - 2, dy = lane / 5 - 2;
+    const int nx = mx + dx, ny = my + dy;
+    const int sx = dx < 0 ? x0 + 1 + (-dx - 1) * MT : dx > 0 ? MT - x1 + (dx - 1) * MT : 0;
+    const int sy = dy < 0 ? y0 + 1 + (-dy - 1) * MT : dy > 0 ? MT - y1 + (dy - 1) * MT : 0;
+    const bool want = lane < 25 && ((dx == 0 && dy == 0) || (any && sx + sy <= BK)) && nx >= 0 && nx < mt_x &&
+                      ny >= 0 && ny < mt_y;
+    append_fresh(want, ny * mt_x + nx, pack_mt(nx, ny), bout, lout, count_out, st, lane);
+}
+
 template <bool KEYS>
 __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t* nxt, int pitch, int Wd, int Hd,
                                          int mt_x, int mt_y, const uint32_t* __restrict__ pos, uint32_t* bin,
                                          uint32_t* bout, int32_t* lout, int32_t* count_out, Stage st, int lane,
-                                         int pass0, int& last_pass)
+                                         int pass0, int reach, int& last_pass)
 {
     const int mx = id & 0xFFFF, my = id >> 16;
     const int mt = my * mt_x + mx;
@@ -362,24 +386,111 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
     // quadrants of the inner tile with a change in the last pass: lanes 8..15
     // hold its top half, 16..23 the bottom; even lanes the left half
     const unsigned lb = __ballot_sync(FULL, ch);   // ch: changes of the last pass
-    const bool tl = lb & 0x00005500u, tr = lb & 0x0000AA00u, bl = lb & 0x00550000u, br = lb & 0x00AA0000u;
-    int dx = 0, dy = 0;
-    bool want = false;
-    switch (lane) {
-    case 0: want = true; break;
-    case 1: dx = -1; want = tl || bl; break;
-    case 2: dx = 1; want = tr || br; break;
-    case 3: dy = -1; want = tl || tr; break;
-    case 4: dy = 1; want = bl || br; break;
-    case 5: dx = -1; dy = -1; want = tl; break;
-    case 6: dx = 1; dy = -1; want = tr; break;
-    case 7: dx = -1; dy = 1; want = bl; break;
-    case 8: dx = 1; dy = 1; want = br; break;
-    default: break;
+    if (reach == RK) {
+        const bool tl = lb & 0x00005500u, tr = lb & 0x0000AA00u, bl = lb & 0x00550000u, br = lb & 0x00AA0000u;
+        int dx = 0, dy = 0;
+        bool want = false;
+        switch (lane) {
+        case 0: want = true; break;
+        case 1: dx = -1; want = tl || bl; break;
+        case 2: dx = 1; want = tr || br; break;
+        case 3: dy = -1; want = tl || tr; break;
+        case 4: dy = 1; want = bl || br; break;
+        case 5: dx = -1; dy = -1; want = tl; break;
+        case 6: dx = 1; dy = -1; want = tr; break;
+        case 7: dx = -1; dy = 1; want = bl; break;
+        case 8: dx = 1; dy = 1; want = br; break;
+        default: break;
+        }
+        const int nx = mx + dx, ny = my + dy;
+        want = want && nx >= 0 && nx < mt_x && ny >= 0 && ny < mt_y;
+        append_fresh(want, ny * mt_x + nx, pack_mt(nx, ny), bout, lout, count_out, st, lane);
+    } else {
+        // rows and (by halves) columns of the inner cells that changed last
+        const unsigned rows = lb >> 8;   // lane pairs 4 .. 11
+        const int y0 = rows ? (__ffs(rows) - 1) >> 1 : 0, y1 = rows ? (31 - __clz(rows)) >> 1 : 0;
+        list_reach(lb != 0, (lb & 0x55555555u) ? 0 : 4, (lb & 0xAAAAAAAAu) ? 7 : 3, y0, y1, mx, my, mt_x, mt_y, bout,
+                   lout, count_out, st, lane);
     }
-    const int nx = mx + dx, ny = my + dy;
-    want = want && nx >= 0 && nx < mt_x && ny >= 0 && ny < mt_y;
-    append_fresh(want, ny * mt_x + nx, pack_mt(nx, ny), bout, lout, count_out, st, lane);
+}
+
+// Block rounds.  Once the list is down to a few hundred micro-tiles, a round's
+// time is the latency of its passes: 2 us each in one warp with eight cells a
+// lane.  A block then takes a micro-tile with a BK-cell halo, one cell per
+// thread in shared memory, and runs BK passes at about 0.2 us each.  Same
+// rules as above, with reach BK.
+template <bool KEYS>
+__device__ __forceinline__ void round_block(int32_t id, const int32_t* cur, int32_t* nxt, int pitch, int Wd, int Hd,
+                                            int mt_x, int mt_y, const uint32_t* __restrict__ pos, uint32_t* bin,
+                                            uint32_t* bout, int32_t* lout, int32_t* count_out, Stage st, int pass0,
+                                            int* s_last)
+{
+    __shared__ int32_t lab[2][BR][BR];
+    __shared__ uint32_t at[KEYS ? 1 : 2][KEYS ? 1 : BR][KEYS ? 1 : BR];
+    __shared__ unsigned row_now[MT];    // inner cells that changed in the last pass, by row
+    __shared__ int row_last[MT], row_moved[MT];
+    const int mx = id & 0xFFFF, my = id >> 16;
+    const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+    const int gx = mx * MT - BK + lane, gy = my * MT - BK + row;
+    const bool inner_row = row >= BK && row < BK + MT, inner = inner_row && lane >= BK && lane < BK + MT;
+    if (threadIdx.x == 0) {
+        const int mt = my * mt_x + mx;
+        atomicAnd(&bin[mt >> 5], ~(1u << (mt & 31)));
+    }
+    int32_t c = (gx >= 0 && gx < Wd && gy >= 0 && gy < Hd) ? __ldcg(cur + (size_t)gy * pitch + gx) : OUTSIDE;
+    uint32_t cp = !KEYS && c >= 0 ? __ldg(&pos[c]) : 0u;
+    const int32_t c0 = c;
+    lab[0][row][lane] = c;
+    if (!KEYS) at[0][row][lane] = cp;
+    __syncthreads();
+    int last = -1;
+    unsigned now = 0;
+    for (int p = 0; p < BK; ++p) {
+        const int f = p & 1;
+        int32_t k = c;
+        if (c >= UNDEF) {
+            const int32_t L = lane > 0 ? lab[f][row][lane - 1] : OUTSIDE, R = lane < BR - 1 ? lab[f][row][lane + 1] : OUTSIDE;
+            const int32_t U = row > 0 ? lab[f][row - 1][lane] : OUTSIDE, D = row < BR - 1 ? lab[f][row + 1][lane] : OUTSIDE;
+            if (KEYS) {
+                best_of4_keys(k, L, R, U, D, gx, gy);
+            } else {
+                int32_t d = c >= 0 ? dist2(gx, gy, cp) : FAR;
+                if (lane > 0) relax_pos(k, d, cp, L, at[f][row][lane - 1], gx, gy);
+                if (lane < BR - 1) relax_pos(k, d, cp, R, at[f][row][lane + 1], gx, gy);
+                if (row > 0) relax_pos(k, d, cp, U, at[f][row - 1][lane], gx, gy);
+                if (row < BR - 1) relax_pos(k, d, cp, D, at[f][row + 1][lane], gx, gy);
+            }
+        }
+        const bool ch = k != c;
+        c = k;
+        lab[f ^ 1][row][lane] = c;
+        if (!KEYS) at[f ^ 1][row][lane] = cp;
+        now = __ballot_sync(FULL, ch && inner);
+        if (now) last = p;
+        if (!__syncthreads_or(ch)) {   // nor will the next passes change the region
+            now = 0;
+            break;
+        }
+    }
+    if (inner && gx < Wd && gy < Hd) nxt[(size_t)gy * pitch + gx] = c;
+    const bool moved = __any_sync(FULL, inner && c != c0);
+    if (inner_row && lane == 0) {
+        row_now[row - BK] = now >> BK;
+        row_last[row - BK] = last;
+        row_moved[row - BK] = moved;
+    }
+    __syncthreads();
+    if (row == 0) {
+        const unsigned bits = lane < MT ? row_now[lane] : 0u;
+        const unsigned rows = __ballot_sync(FULL, bits != 0), cols = __reduce_or_sync(FULL, bits);
+        const int newest = __reduce_max_sync(FULL, lane < MT ? row_last[lane] : -1);
+        if (__any_sync(FULL, lane < MT && row_moved[lane])) {
+            if (lane == 0 && newest >= 0) *s_last = max(*s_last, pass0 + newest);
+            list_reach(rows != 0, rows ? __ffs(cols) - 1 : 0, rows ? 31 - __clz(cols) : 0, rows ? __ffs(rows) - 1 : 0,
+                       rows ? 31 - __clz(rows) : 0, mx, my, mt_x, mt_y, bout, lout, count_out, st, lane);
+        }
+    }
+    __syncthreads();   // the buffers are filled anew by the next micro-tile
 }
 
 // Entering the round mode: the list holds the micro-tiles that can change in
@@ -399,8 +510,9 @@ __device__ __forceinline__ void dilate_mt(int32_t id, int mt_x, int mt_y, uint32
 // counts[g]: micro-tiles listed for work-list generation g, which runs list
 // g%2 and appends generation g+1's micro-tiles to list (g+1)%2.  A generation
 // is one pass while the list is longer than rounds_below, then (once) the
-// dilation into the round mode, then rounds of RK passes.  The mode is the
-// same in every block: it depends only on the list lengths all of them read.
+// dilation into the round mode, then rounds of RK passes, and on lists of a few
+// hundred micro-tiles block rounds of BK passes.  The mode is the same in every
+// block: it depends only on the list lengths all of them read.
 template <bool KEYS>
 __global__ void __launch_bounds__(SJ_THREADS, 1)
 k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
@@ -422,6 +534,7 @@ k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, con
     int g = 0;              // generation
     int par = 0;            // plane holding the current state
     bool rounds = start_rounds != 0;   // the first list is one for the round mode
+    bool blocks = false;    // the list is one for block rounds
     bool converged = false;
     for (; t < max_steps; ++g) {
         const int n = *reinterpret_cast<volatile int32_t*>(&counts[g]);
@@ -429,9 +542,12 @@ k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, con
             converged = true;
             break;
         }
-        int kind = 0;   // 0: one pass, 1: dilation into the round mode, 2: a round of RK passes
+        // 0: one pass, 1: dilation into the round mode, 2: a round of RK passes,
+        // 3: a block round of BK passes
+        int kind = 0;
         if (rounds) {
-            kind = 2;
+            kind = blocks && n <= BLOCK_LIMIT ? 3 : 2;
+            blocks = kind == 3 || n <= BLOCK_BELOW;   // what the list made now is for
         } else if (n <= rounds_below) {
             kind = 1;
             rounds = true;
@@ -463,11 +579,15 @@ k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, con
             if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(&gs->last1, t);
             for (int i = gwarp; i < n; i += nwarps)
                 dilate_mt(__ldcg(&lin[i]), mt_x, mt_y, bin, bout, lout, counts + g + 1, stg, lane);
+        } else if (kind == 3) {
+            for (int i = blockIdx.x; i < n; i += gridDim.x)
+                round_block<KEYS>(__ldcg(&lin[i]), cur, nxt, pitch, Wd, Hd, mt_x, mt_y, pos, bin, bout, lout,
+                                  counts + g + 1, stg, t, &s_last);
         } else {
             int last = -1;
             for (int i = gwarp; i < n; i += nwarps)
                 round_mt<KEYS>(__ldcg(&lin[i]), cur, nxt, pitch, Wd, Hd, mt_x, mt_y, pos, bin, bout, lout,
-                               counts + g + 1, stg, lane, t, last);
+                               counts + g + 1, stg, lane, t, blocks ? BK : RK, last);
             if (lane == 0 && last >= 0) atomicMax(&s_last, last);
         }
         __syncthreads();
@@ -479,7 +599,7 @@ k_sparse_jacobi(int32_t* plane0, int32_t* plane1, int pitch, int Wd, int Hd, con
         }
         __syncthreads();
         for (int i = threadIdx.x; i < s_m; i += blockDim.x) lout[s_base + i] = s_list[i];
-        const int advanced = kind == 0 ? 1 : (kind == 2 ? RK : 0);
+        const int advanced = kind == 0 ? 1 : kind == 2 ? RK : kind == 3 ? BK : 0;
         t += advanced;
         if (advanced) par ^= 1;
         if (!grid_sync(gs, gridDim.x, gen_local)) return;
