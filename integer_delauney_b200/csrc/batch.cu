@@ -47,6 +47,17 @@ struct BImg {
     int tiles_x;         // raster tiles per row
 };
 
+// Image of each seed (ids of an image are contiguous, in input and in sorted
+// order); a block per image.  Filled here: as host tables, these and the
+// column and row tables below took 0.4 ms of a 512-image call to build and
+// upload.
+__global__ void k_b_seed_image(const BImg* __restrict__ imgs, int n_images, long long n, int32_t* __restrict__ seed_img)
+{
+    const int im = blockIdx.x;
+    const long long end = im + 1 < n_images ? imgs[im + 1].seed_off : n;
+    for (long long i = imgs[im].seed_off + threadIdx.x; i < end; i += blockDim.x) seed_img[i] = im;
+}
+
 __global__ void k_b_mark(const int32_t* __restrict__ xy, int64_t n, const int32_t* __restrict__ seed_img,
                          const BImg* __restrict__ imgs, uint32_t* __restrict__ bitmap,
                          unsigned long long* __restrict__ first_bad)
@@ -67,7 +78,7 @@ __global__ void k_b_mark(const int32_t* __restrict__ xy, int64_t n, const int32_
 __global__ void k_b_rank(const int32_t* __restrict__ xy, int64_t n, const int32_t* __restrict__ seed_img,
                          const BImg* __restrict__ imgs, int P, const uint32_t* __restrict__ bitmap,
                          const int32_t* __restrict__ word_rank, int32_t* __restrict__ xs, int32_t* __restrict__ ys,
-                         uint32_t* __restrict__ pos, int32_t* __restrict__ sid_img)
+                         uint32_t* __restrict__ pos)
 {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -79,7 +90,6 @@ __global__ void k_b_rank(const int32_t* __restrict__ xy, int64_t n, const int32_
     xs[r] = x;
     ys[r] = y;
     pos[r] = pack_pos(m.ox + P + x, m.oy + P + y);
-    sid_img[r] = im;
 }
 
 // Each image's padded canvas starts UNDEF (the rest of the atlas is WALL).
@@ -239,7 +249,6 @@ inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)std::max<int64_t
 
 struct Plan {
     std::vector<BImg> imgs;
-    std::vector<int32_t> seed_img;
     int AW = 0, AH = 0;
     int64_t n_seeds = 0, n_px = 0, n_tiles = 0;
 };
@@ -302,10 +311,6 @@ Plan make_plan(int n_images, const int32_t* dims, const int64_t* counts, int P)
     if (AH > MAX_CANVAS_SIDE) invalid("batch too large for one atlas: split it into smaller batches");
     pl.AW = AW;
     pl.AH = (int)AH;
-    pl.seed_img.resize(pl.n_seeds);
-    for (int i = 0; i < n_images; ++i) {
-        std::fill(pl.seed_img.begin() + pl.imgs[i].seed_off, pl.seed_img.begin() + pl.imgs[i].seed_off + counts[i], i);
-    }
     return pl;
 }
 
@@ -334,7 +339,7 @@ const XImg* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
 {
     const int n_images = (int)pl.imgs.size();
     std::vector<XImg> xi(n_images);
-    std::vector<int32_t> pair_img, row_img;
+    int n_pairs = 0, n_rows = 0;
     int max_wp = 0, max_hp = 0;
     int64_t band_entries = 0;
     for (int i = 0; i < n_images; ++i) {
@@ -344,13 +349,13 @@ const XImg* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
         m.oy = b.oy;
         m.Wp = b.W + 2 * P;
         m.Hp = b.H + 2 * P;
-        m.pair_off = (int)pair_img.size();
-        m.row_off = (int)row_img.size();
+        m.pair_off = n_pairs;
+        m.row_off = n_rows;
         m.band_off = (int)band_entries;
         m.s0 = (int)b.seed_off;
         m.s1 = (int)(i + 1 < n_images ? pl.imgs[i + 1].seed_off : pl.n_seeds);
-        pair_img.insert(pair_img.end(), (size_t)(m.Wp + 1) / 2, i);
-        row_img.insert(row_img.end(), (size_t)m.Hp, i);
+        n_pairs += (m.Wp + 1) / 2;
+        n_rows += m.Hp;
         band_entries += (int64_t)x_bands(m) * m.Wp;
         m.P = P;
         m.bit0 = b.px_off;
@@ -358,17 +363,13 @@ const XImg* exact_atlas(Context& C, const Plan& pl, int P, const Canvas& cv)
         max_hp = std::max(max_hp, m.Hp);
     }
     C.batch_ximg.ensure(xi.size() * sizeof(XImg));
-    C.batch_colimg.ensure(pair_img.size() * 4);
-    C.batch_rowimg.ensure(row_img.size() * 4);
+    C.batch_colimg.ensure((size_t)n_pairs * 4);
+    C.batch_rowimg.ensure((size_t)n_rows * 4);
     IDL_CUDA(cudaMemcpyAsync(C.batch_ximg.ptr, xi.data(), xi.size() * sizeof(XImg), cudaMemcpyHostToDevice,
                              C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_colimg.ptr, pair_img.data(), pair_img.size() * 4, cudaMemcpyHostToDevice,
-                             C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_rowimg.ptr, row_img.data(), row_img.size() * 4, cudaMemcpyHostToDevice,
-                             C.stream));
     const XImg* d_xi = C.batch_ximg.as<XImg>();
-    exact_images(C, cv.pitch, C.pos.as<uint32_t>(), d_xi, C.batch_colimg.as<int32_t>(), (int)pair_img.size(),
-                 C.batch_rowimg.as<int32_t>(), (int)row_img.size(), max_wp, max_hp, band_entries);
+    exact_images(C, cv.pitch, C.pos.as<uint32_t>(), d_xi, n_images, C.batch_colimg.as<int32_t>(), n_pairs,
+                 C.batch_rowimg.as<int32_t>(), n_rows, max_wp, max_hp, band_entries);
     return d_xi;
 }
 
@@ -379,13 +380,12 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     const int64_t n = pl.n_seeds;
     C.batch_img.ensure(pl.imgs.size() * sizeof(BImg));
     C.batch_seed_img.ensure((size_t)n * 4);
-    C.batch_sid.ensure((size_t)n * 4);
     C.batch_stats.ensure(((size_t)n_images * 2 + 1) * 4);
     BImg* d_imgs = C.batch_img.as<BImg>();
     IDL_CUDA(cudaMemcpyAsync(d_imgs, pl.imgs.data(), pl.imgs.size() * sizeof(BImg), cudaMemcpyHostToDevice,
                              C.stream));
-    IDL_CUDA(cudaMemcpyAsync(C.batch_seed_img.ptr, pl.seed_img.data(), (size_t)n * 4, cudaMemcpyHostToDevice,
-                             C.stream));
+    k_b_seed_image<<<(unsigned)n_images, 256, 0, C.stream>>>(d_imgs, n_images, n, C.batch_seed_img.as<int32_t>());
+    IDL_LAUNCH();
     cudaEvent_t ev[5] = {};
     if (timings)
         for (auto& e : ev) IDL_CUDA(cudaEventCreate(&e));
@@ -419,14 +419,18 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     unsigned long long hb[2] = {0, 0};
     IDL_CUDA(cudaMemcpyAsync(hb, bad, 16, cudaMemcpyDeviceToHost, C.stream));
     IDL_CUDA(cudaStreamSynchronize(C.stream));
-    auto image_of = [&](unsigned long long i) { return (int)pl.seed_img[(size_t)i]; };
+    auto image_of = [&](unsigned long long i) {
+        return (int)(std::upper_bound(pl.imgs.begin(), pl.imgs.end(), (long long)i,
+                                      [](long long v, const BImg& m) { return v < m.seed_off; }) -
+                     pl.imgs.begin()) - 1;
+    };
     if (hb[0] != ~0ull) invalid("image " + std::to_string(image_of(hb[0])) + ": seed coordinate out of bounds");
     if (hb[1] != ~0ull)
         invalid("image " + std::to_string(image_of(hb[1])) + ": duplicate seed positions are not allowed");
     exclusive_popc_scan(C, C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nwords);
     k_b_rank<<<nblk(n), 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, C.batch_seed_img.as<int32_t>(), d_imgs, P,
                                            C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), C.xs.as<int32_t>(),
-                                           C.ys.as<int32_t>(), C.pos.as<uint32_t>(), C.batch_sid.as<int32_t>());
+                                           C.ys.as<int32_t>(), C.pos.as<uint32_t>());
     IDL_LAUNCH();
 
     const Canvas cv{pl.AW, pl.AH, (pl.AW + 31) / 32 * 32};
@@ -452,7 +456,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
         // them are read by the block rule (and by resolve_exact) in plane 0 only
         IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
         const XImg* xi = exact_atlas(C, pl, P, cv);
-        if (direct) resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, xi, C.batch_sid.as<int32_t>());
+        if (direct) resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, xi, C.batch_seed_img.as<int32_t>());
     } else {
         run_passes();
     }
@@ -484,7 +488,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     int32_t* off = side + n_images;   // n_images + 1
     const int64_t nt = C.host_sc->n_triangles;
     IDL_CUDA(cudaMemsetAsync(side, 0, (size_t)n_images * 4, C.stream));
-    k_b_tri_off<<<nblk(nt + 1), 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(), n_images,
+    k_b_tri_off<<<nblk(nt + 1), 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_seed_img.as<int32_t>(), n_images,
                                                    off);
     IDL_LAUNCH();
     int32_t* out = d_out;
@@ -493,7 +497,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
         out = C.outgrid.as<int32_t>();
     }
     const RasterWork w = raster_work(C, nt, pl.n_tiles);
-    const int32_t* sid = C.batch_sid.as<int32_t>();
+    const int32_t* sid = C.batch_seed_img.as<int32_t>();
     const int32_t *xs = C.xs.as<int32_t>(), *ys = C.ys.as<int32_t>(), *tris = C.tris.as<int32_t>();
     if (nt > 0) {
         k_b_raster_count<<<nblk(nt), 256, 0, C.stream>>>(tris, C.sc(), sid, d_imgs, xs, ys, side, w);
@@ -511,7 +515,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
         k_b_raster_rest<<<C.num_sms, 128, 0, C.stream>>>(tris, C.sc(), sid, d_imgs, xs, ys, side, off, out, w);
         IDL_LAUNCH();
     }
-    k_b_localise<<<C.num_sms * 8, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_sid.as<int32_t>(),
+    k_b_localise<<<C.num_sms * 8, 256, 0, C.stream>>>(C.tris.as<int32_t>(), C.sc(), C.batch_seed_img.as<int32_t>(),
                                                       d_imgs, P);
     IDL_LAUNCH();
     mark(4);

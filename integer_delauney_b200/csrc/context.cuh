@@ -195,8 +195,7 @@ struct Context {
 
     // batched triangulation (batch.cu)
     DevBuf batch_img;       // per-image table
-    DevBuf batch_seed_img;  // image of each input seed
-    DevBuf batch_sid;       // image of each sorted seed
+    DevBuf batch_seed_img;  // image of each seed
     DevBuf batch_stats;     // per-image longest sides and triangle offsets
     DevBuf batch_bad;       // first out-of-bounds / duplicate seed index
     DevBuf batch_ximg, batch_colimg, batch_rowimg;  // exact semantics: image table, column / row -> image
@@ -229,7 +228,7 @@ struct Context {
                          &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
                          &exact_bands, &sus_bits, &sus_list, &hkeys,
                          &ukeys, &uvals, &cnt, &off, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
-                         &batch_img, &batch_seed_img, &batch_sid, &batch_stats, &batch_bad,
+                         &batch_img, &batch_seed_img, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
         for (DevBuf* b : all) f(*b);
     }
@@ -354,11 +353,11 @@ void grid_barrier_selftest(Context& C, int missing_arrivals, unsigned spin_limit
 // their ranks, as sort_seeds_device and rank_seeds_device leave them.
 struct XImg;
 void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P);
-// The same for the images of a batch atlas (exact.cu): device tables of the
-// images, of each column pair's and each row's image; C.lab[0] and C.lab[1]
-// hold planes of the atlas.
-void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, const int32_t* pair_img, int n_pairs,
-                  const int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries);
+// The same for the images of a batch atlas (exact.cu): the device table of the
+// images, room for each column pair's and each row's image; C.lab[0] and
+// C.lab[1] hold planes of the atlas.
+void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, int n_images, int32_t* pair_img,
+                  int n_pairs, int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries);
 // The one image of a single canvas with n seeds.
 XImg whole_canvas(const Canvas& cv, int64_t n, int P);
 

@@ -46,6 +46,14 @@ k_bx_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, const XImg* _
     if ((int)blockIdx.y < x_bands(m)) x_column_pair(pos, ranks, m, (g - m.pair_off) * 2, blockIdx.y, pitch, off, bands);
 }
 
+// Image of each column pair and row of the batch; a block per image.
+__global__ void k_bx_tables(const XImg* __restrict__ xi, int32_t* __restrict__ pair_img, int32_t* __restrict__ row_img)
+{
+    const XImg& m = xi[blockIdx.x];
+    for (int i = threadIdx.x; i < (m.Wp + 1) / 2; i += blockDim.x) pair_img[m.pair_off + i] = blockIdx.x;
+    for (int i = threadIdx.x; i < m.Hp; i += blockDim.x) row_img[m.row_off + i] = blockIdx.x;
+}
+
 template <int T>
 __global__ void __launch_bounds__(T)
 k_row_win(const int16_t* __restrict__ off, XImg m, int pitch, const uint32_t* __restrict__ pos,
@@ -85,7 +93,7 @@ template <bool BATCH, class... A>
 void rows_for_width(Context& C, int width, unsigned rows, A... args)
 {
     static std::atomic<uint64_t> opted[4];
-    const int threads = row_pass_threads(width);
+    const int threads = row_pass_threads(width, rows);
     const size_t smem = row_pass_smem(width);
     auto go = [&](auto single, auto batch, int slot) {
         if constexpr (BATCH) launch_rows(C, batch, opted[slot], rows, threads, smem, args..., row_list_bytes(width));
@@ -134,9 +142,11 @@ void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t 
     }
 }
 
-void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, const int32_t* pair_img, int n_pairs,
-                  const int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries)
+void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, int n_images, int32_t* pair_img,
+                  int n_pairs, int32_t* row_img, int n_rows, int max_wp, int max_hp, int64_t band_entries)
 {
+    k_bx_tables<<<(unsigned)n_images, 256, 0, C.stream>>>(xi, pair_img, row_img);
+    IDL_LAUNCH();
     C.exact_bands.ensure((size_t)band_entries * 4);
     int16_t* off = C.lab[1].as<int16_t>();
     int32_t* bands = C.exact_bands.as<int32_t>();
@@ -144,7 +154,7 @@ void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, co
     k_bx_column_off<<<dim3((unsigned)ceil_div(n_pairs, 64), (unsigned)ceil_div(max_hp, BAND)), 64, 0, C.stream>>>(
         pos, ranks, xi, pair_img, n_pairs, pitch, off, bands);
     IDL_LAUNCH();
-    rows_for_width<true>(C, max_wp, (unsigned)n_rows, (const int16_t*)off, xi, row_img, pitch, pos,
+    rows_for_width<true>(C, max_wp, (unsigned)n_rows, (const int16_t*)off, xi, (const int32_t*)row_img, pitch, pos,
                          (const int32_t*)bands, C.lab[0].as<int32_t>());
 }
 
