@@ -535,7 +535,7 @@ IDL_API int64_t idl_server_clock_ns(void);
 IDL_API int idl_server_create(int device, int64_t budget_bytes, int slots, int border_padding, int mode,
                               idl_server** out);
 /* Propagation schedules (idl_context_set_schedule) of every slot: of the
- * grouped new diagrams (group_rounds, default 1) and of inserts (insert_rounds,
+ * grouped new diagrams (group_rounds, default IDL_SCHEDULE_DIRECT) and of inserts (insert_rounds,
  * default -1: tile rounds from the new seeds' tiles, plain launches that
  * overlap other slots' work; 0 or more: the device-wide persistent kernel).
  * Before the first request; IDL_ERR_STATE after it. */

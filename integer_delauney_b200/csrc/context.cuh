@@ -168,7 +168,8 @@ struct Context {
     // propagation schedule from scratch (resolve.cu, propagate.cu; idl_context_set_schedule)
     int dense_rounds = IDL_SCHEDULE_DIRECT;
     bool direct() const { return dense_rounds == IDL_SCHEDULE_DIRECT; }
-    int rounds_schedule() const { return direct() ? 3 : dense_rounds; }   // when the passes are run after all
+    int passes_rounds = 3;   // the schedule when IDL_SCHEDULE_DIRECT has to run the passes after all
+    int rounds_schedule() const { return direct() ? passes_rounds : dense_rounds; }
     int key_tile = 9;      // tile shape of the owner-key tile round (propagate.cu; idl_context_set_tile)
     // The persistent kernel advances several passes per grid barrier once its
     // work list holds at most this many micro-tiles (sparse_jacobi.cu; 0:

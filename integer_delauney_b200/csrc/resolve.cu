@@ -227,7 +227,8 @@ k_suspects(View V, uint32_t* sus, int32_t* list, int cap, Scalars* sc)
 
 constexpr int RES_WARPS = 4;
 constexpr int MAX_CAND = 16;    // candidates of one suspect, rivals at one cell (2 at most at the sizes above)
-constexpr int MAX_SEARCH = 64;  // cells of a "no" search before the "yes" rule is tried
+constexpr int MAX_SEARCH = 64;  // cells of a "no" search
+constexpr int SHORT_SEARCH = 16;
 constexpr int MAX_FRONT = 4;    // line cells per step (2 are reached)
 // Disc columns (in warp strides) a suspect may look at: a few thousand are
 // reached with clustered seeds; beyond it the suspect stays undecided, so that
@@ -250,17 +251,24 @@ __device__ __forceinline__ void for_better(const View& V, int x, int y, int32_t 
 {
     const int R = isqrt(d);
     const int lo = max(b.ox, x - R), hi = min(b.ox + b.Wp - 1, x + R);
-    for (int xx = lo + lane; xx <= hi; xx += 32) {
-        const int o = __ldg(&V.off[(size_t)y * V.pitch + xx]);
-        if (o == NO_SEED || (long long)o * o + (long long)(xx - x) * (xx - x) > d) continue;
-        const int32_t c = x_seed_at(V.pos, V.bands, b, xx, y + o);
-        for (int step = 1; step >= -1; step -= 2) {
-            for (int32_t m = step > 0 ? c : c - 1; m >= b.s0 && m < b.s1; m += step) {
-                const uint32_t p = __ldg(&V.pos[m]);
-                if ((int)pos_x(p) != xx) break;   // past the column's run
-                const int32_t dm = dist2(x, y, p);
-                if (dm > d) break;
-                if (m != s && beats(dm, m, d, s) && !f(m, p)) return;
+    const int16_t* row = V.off + (size_t)y * V.pitch;
+    for (int x0 = lo + lane; x0 <= hi; x0 += 128) {
+        int o[4];   // four columns' loads in flight: a disc of the empty parts of a clustered set has a thousand
+#pragma unroll
+        for (int j = 0; j < 4; ++j) o[j] = x0 + 32 * j <= hi ? __ldg(&row[x0 + 32 * j]) : NO_SEED;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int xx = x0 + 32 * j;
+            if (o[j] == NO_SEED || (long long)o[j] * o[j] + (long long)(xx - x) * (xx - x) > d) continue;
+            const int32_t c = x_seed_at(V.pos, V.bands, b, xx, y + o[j]);
+            for (int step = 1; step >= -1; step -= 2) {
+                for (int32_t m = step > 0 ? c : c - 1; m >= b.s0 && m < b.s1; m += step) {
+                    const uint32_t p = __ldg(&V.pos[m]);
+                    if ((int)pos_x(p) != xx) break;   // past the column's run
+                    const int32_t dm = dist2(x, y, p);
+                    if (dm > d) break;
+                    if (m != s && beats(dm, m, d, s) && !f(m, p)) return;
+                }
             }
         }
     }
@@ -313,7 +321,8 @@ __device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int 
 }
 
 template <int LEVEL>
-__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane);
+__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane,
+                      int cap = MAX_SEARCH);
 
 // Rule "yes": k certainly arrives at (px, py), at its L1 distance.  LEVEL 1: a
 // rival that never arrives at a cell does not count there.  Warp-wide.
@@ -354,19 +363,26 @@ __device__ bool arrives(const View& V, WarpScratch& S, int px, int py, int32_t k
 
 // Rule "no": k certainly never arrives at (px, py).  LEVEL 1: a cell where a
 // rival of k certainly arrives no later than k can is closed to k.  Warp-wide.
+// The search takes eight cells at a time, four lanes each; it gives up beyond
+// `cap` cells.
 template <int LEVEL>
-__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane)
+__device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, const XImg& b, int lane, int cap)
 {
     uint32_t* seen = S.seen[LEVEL];
     int ns = 1, head = 0;
     __syncwarp();
     if (lane == 0) seen[0] = pack_pos(px, py);
     __syncwarp();
+    const int dir = lane & 3;
     while (head < ns) {
-        const uint32_t q = seen[head++];
+        const int at = head + (lane >> 2);
+        head = min(head + 8, ns);
         bool src = false, add = false;
-        const int x = (int)pos_x(q) + (lane == 0) - (lane == 1), y = (int)pos_y(q) + (lane == 2) - (lane == 3);
-        if (lane < 4) {
+        int x = 0, y = 0;
+        if (at < head) {
+            const uint32_t q = seen[at];
+            x = (int)pos_x(q) + (dir == 0) - (dir == 1);
+            y = (int)pos_y(q) + (dir == 2) - (dir == 3);
             const int32_t l = label_at(V, x, y);
             if (l >= 0) {
                 const bool su = suspect_at(V, x, y);
@@ -379,19 +395,21 @@ __device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, 
             }
         }
         if (__any_sync(FULL, src)) return false;
-        unsigned ab = __ballot_sync(FULL, add);
+        // a cell two of them lead to is taken once
+        const unsigned same = __match_any_sync(FULL, add ? pack_pos(x, y) : 0xFFFFFFFFu);
+        unsigned ab = __ballot_sync(FULL, add && lane == __ffs(same) - 1);
         if (LEVEL > 0) {
-            for (int j = 0; j < 4; ++j) {
-                if (!((ab >> j) & 1u)) continue;
-                const int rx = (int)pos_x(q) + (j == 0) - (j == 1), ry = (int)pos_y(q) + (j == 2) - (j == 3);
+            for (unsigned m = ab; m; m &= m - 1) {
+                const int j = __ffs(m) - 1;
+                const int rx = __shfl_sync(FULL, x, j), ry = __shfl_sync(FULL, y, j);
                 const int nr = rivals<LEVEL>(V, S, rx, ry, k, b, lane);
                 if (nr > MAX_CAND) return false;
                 bool closed = false;
-                for (int m = 0; !closed && m < nr; ++m) closed = arrives<0>(V, S, rx, ry, S.rival[LEVEL][m], b, lane);
+                for (int c = 0; !closed && c < nr; ++c) closed = arrives<0>(V, S, rx, ry, S.rival[LEVEL][c], b, lane);
                 if (closed) ab &= ~(1u << j);
             }
         }
-        if (ns + __popc(ab) > MAX_SEARCH) return false;
+        if (ns + __popc(ab) > cap) return false;
         if ((ab >> lane) & 1u) seen[ns + __popc(ab & ((1u << lane) - 1u))] = pack_pos(x, y);
         ns += __popc(ab);
         __syncwarp();
@@ -463,9 +481,10 @@ k_resolve(View V, const int32_t* __restrict__ list, int cap, int32_t* __restrict
                 }
                 last = k;
                 last_d = kd;
-                if (never<0>(V, S, px, py, k, b, lane)) continue;
+                // a short search, then the line, which is quick where it succeeds
+                if (never<0>(V, S, px, py, k, b, lane, SHORT_SEARCH)) continue;
                 const bool yes = arrives<0>(V, S, px, py, k, b, lane);
-                if (!yes && never<1>(V, S, px, py, k, b, lane)) continue;
+                if (!yes && (never<0>(V, S, px, py, k, b, lane) || never<1>(V, S, px, py, k, b, lane))) continue;
                 if (yes || arrives<1>(V, S, px, py, k, b, lane)) {
                     out = k;
                     t_hi = l1_to(V, px, py, k);

@@ -426,11 +426,10 @@ int idl_server_create(int device, int64_t budget_bytes, int slots, int border_pa
             // workers' work, where the persistent kernel would hold the whole
             // device (measured: twice the insert throughput with 8 workers)
             check_status(idl_context_set_schedule(sl.ws, -1));
-            // grouped new diagrams likewise, as cell-list tile rounds (48 x 48
-            // tiles, 8 passes per round) to convergence: measured 3 329 req/s
-            // on the saturated stream against 2 853 with one tile round and
-            // the persistent kernel for the tail
-            check_status(idl_context_set_schedule(sl.batch, -1));
+            // grouped new diagrams by the default schedule, whose launches are
+            // plain too; what it leaves undecided runs as cell-list tile rounds
+            // (48 x 48 tiles, 8 passes per round) to convergence
+            sl.batch->passes_rounds = -1;
             check_status(idl_context_set_tile(sl.batch, 8, nullptr));
         }
         for (int i = 0; i < slots; ++i) s->workers.emplace_back(worker_loop, s, i);
