@@ -74,6 +74,63 @@ void ensure_scalars(Context& C)
 
 namespace {
 
+struct ClearList {
+    static constexpr int MAX = 6;
+    uint4* p[MAX];
+    long long n[MAX];     // 16-byte units
+    uint32_t word[MAX];
+    int count;
+};
+
+__global__ void __launch_bounds__(256) k_clear(ClearList l)
+{
+    const long long step = (long long)gridDim.x * blockDim.x;
+    for (int k = 0; k < l.count; ++k) {
+        const uint32_t v = l.word[k];
+        for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < l.n[k]; i += step)
+            l.p[k][i] = make_uint4(v, v, v, v);
+    }
+}
+
+}  // namespace
+
+void clear_for_run(Context& C, const Canvas& cv, int W, int H, int64_t n, bool suspects, int64_t cap, int64_t n_tri)
+{
+    ClearList l{};
+    long long units = 0;
+    // buffers are whole multiples of 256 bytes, so the last unit may run past `bytes`
+    auto add = [&](const DevBuf& b, size_t bytes, uint32_t word) {
+        l.p[l.count] = b.as<uint4>();
+        l.n[l.count] = (long long)((bytes + 15) / 16);
+        l.word[l.count] = word;
+        units = std::max(units, l.n[l.count]);
+        ++l.count;
+    };
+    const size_t bitmap = ((size_t)W * H + 31) / 32 * 4;
+    C.bitmap.ensure(bitmap);
+    add(C.scalars, sizeof(Scalars), 0);
+    add(C.bitmap, bitmap, 0);
+    if (suspects) add(C.sus_bits, resolve_reserve(C, cv), 0);
+    if (cap > 0) {
+        detect_reserve(C, n, cap);
+        add(C.hkeys, (size_t)cap * 16, 0xFFFFFFFFu);
+        add(C.cnt, (size_t)(n + 1) * 2 * 4, 0);
+        add(C.rbig, raster_reserve(C, W, H, n_tri), 0);
+    }
+    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((units + 255) / 256, C.num_sms * 16));
+    k_clear<<<blocks, 256, 0, C.stream>>>(l);
+    IDL_LAUNCH();
+    C.precleared = true;
+}
+
+namespace {
+
+// Ends a run's use of cleared buffers, however the run ends.
+struct Precleared {
+    Context& C;
+    ~Precleared() { C.precleared = false; }
+};
+
 // ---- output composition ------------------------------------------------
 
 // (a, b, c) of each (x, y, a, b, c) triangle row.
@@ -232,11 +289,16 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     for (bool& r : C.prof.recorded) r = false;
     C.prof.rounds = C.prof.tiles = C.prof.passes = 0;
     C.prof.prop_bytes = 0;
+    // the usual bounds on the hash table and the triangle count (under 2n)
+    int64_t cap = detect_capacity(C, n);
+    int64_t bound = 2 * n + 64;
+    const bool from_grid = vgrid && P == 0;
     C.mark(PM_START);
+    const Precleared guard{C};
+    clear_for_run(C, cv, W, H, n, !from_grid && mode == IDL_MODE_REFERENCE && C.direct(), cap, bound);
     sort_seeds_device(C, W, H, n, P);
     C.mark(PM_SEEDS);
 
-    const bool from_grid = vgrid && P == 0;
     bool resolved = false;
     if (!from_grid) {
         resolved = start_labels(C, mode, cv, n, P, C.prof.enabled);
@@ -284,14 +346,13 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         deliver(cv);
         C.fetch_scalars();
     };
-    // Everything goes out before anything is read back, with the usual bounds
-    // on the table and the triangle count (under 2n); one wait at the end tells
-    // whether they held and whether the exact diagram decided the labels.  What
-    // failed is run again, each time with room for what is known by then.
-    int64_t cap = detect_capacity(C, n);
-    int64_t bound = 2 * n + 64;
+    // Everything goes out before anything is read back; one wait at the end
+    // tells whether the bounds held and whether the exact diagram decided the
+    // labels.  What failed is run again, each time with room for what is known
+    // by then.
     detect(cap);
     assign(bound);
+    C.precleared = false;
     if (resolved && !finish_resolved(C, C.prof.enabled)) {
         run_passes(C, mode, cv, n);
         C.mark(PM_PROPAGATE);
@@ -518,8 +579,10 @@ int idl_voronoi(idl_context* ctx, int width, int height, const int32_t* seeds_xy
     Context& C = *ctx;
     const Canvas cv = make_canvas(width, height);
     upload_seeds(C, seeds_xy, n_seeds, cudaMemcpyHostToDevice);
-    sort_seeds_device(C, width, height, n_seeds, 0);
     int64_t passes = 0;
+    const Precleared guard{C};
+    clear_for_run(C, cv, width, height, n_seeds, mode == IDL_MODE_REFERENCE && C.direct(), 0, 0);
+    sort_seeds_device(C, width, height, n_seeds, 0);
     const bool resolved = start_labels(C, mode, cv, n_seeds, 0, passes_out != nullptr, &passes);
     const size_t bytes = (size_t)width * height * 2 * sizeof(int32_t);
     C.outgrid.ensure(bytes);

@@ -167,6 +167,9 @@ struct Context {
     int32_t stamp_epoch = 0;
     // propagation schedule from scratch (resolve.cu, propagate.cu; idl_context_set_schedule)
     int dense_rounds = IDL_SCHEDULE_DIRECT;
+    // Set while the buffers a single-image run starts from are known to be
+    // cleared (clear_for_run): the stages then leave their own memsets out.
+    bool precleared = false;
     bool direct() const { return dense_rounds == IDL_SCHEDULE_DIRECT; }
     int passes_rounds = 3;   // the schedule when IDL_SCHEDULE_DIRECT has to run the passes after all
     int rounds_schedule() const { return direct() ? passes_rounds : dense_rounds; }
@@ -396,9 +399,21 @@ void detect_triangles(Context& C, const Canvas& cv, const int32_t* labels, const
 // slots (detect_capacity to begin with); once the scalars have been read back,
 // detect_done tells whether the table was large enough.
 int64_t detect_capacity(const Context& C, int64_t n);
+void detect_reserve(Context& C, int64_t n, int64_t cap);
 void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
                    int64_t cap, cudaEvent_t mid = nullptr, const int32_t* rank = nullptr);
 bool detect_done(Context& C, int64_t cap);
+
+// One launch clears what the stages of a single-image run clear one by one
+// (occupancy bits, counters, suspect bits, hash table, group counts, tile
+// counts), reserving the buffers for it; sets C.precleared.  With cap 0 only
+// what stage (a) needs.  n_tri: the raster's bound on the triangle count.
+void clear_for_run(Context& C, const Canvas& cv, int W, int H, int64_t n, bool suspects, int64_t cap, int64_t n_tri);
+// The raster's workspace for a W x H image (raster.cu): reserves it and tells
+// the bytes at its start that have to be zero.
+size_t raster_reserve(Context& C, int W, int H, int64_t n_tri);
+// Likewise resolve_exact's suspect bits.
+size_t resolve_reserve(Context& C, const Canvas& cv);
 
 // Stage (d): per-pixel max triangle id over a W x H image (raster.cu), of the
 // triangles in C.tris, whose number is read on the device; n_tri is the

@@ -109,26 +109,49 @@ k_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, 
 
 }  // namespace
 
+namespace {
+
+constexpr size_t HEAD_BYTES = 256;
+
+// at 200 000 uniform seeds a triangle meets 1.6 tiles; long slivers of
+// clustered sets meet more, far fewer than this on average
+int64_t list_capacity(int64_t nt, int64_t n_tiles)
+{
+    return std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30);
+}
+
+size_t work_reserve(Context& C, int64_t nt, int64_t n_tiles)
+{
+    C.rbig.ensure(HEAD_BYTES + ((size_t)n_tiles * 2 + 1 + (size_t)nt * 4 + (size_t)list_capacity(nt, n_tiles)) * 4);
+    return HEAD_BYTES + (size_t)n_tiles * 4;
+}
+
+template <class TILE>
+int64_t tile_count(int W, int H) { return (int64_t)ceil_div(W, TILE::W) * ceil_div(H, TILE::H); }
+
+}  // namespace
+
+size_t raster_reserve(Context& C, int W, int H, int64_t n_tri)
+{
+    const int64_t large = tile_count<TileLarge>(W, H);
+    return work_reserve(C, n_tri, small_tiles(large, C.num_sms) ? tile_count<TileSmall>(W, H) : large);
+}
+
 RasterWork raster_work(Context& C, int64_t nt, int64_t n_tiles)
 {
-    // at 200 000 uniform seeds a triangle meets 1.6 tiles; long slivers of
-    // clustered sets meet more, far fewer than this on average
-    const int64_t cap = std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30);
-    const size_t head = 256;
-    const size_t bytes = head + ((size_t)n_tiles * 2 + 1 + (size_t)nt * 4 + (size_t)cap) * 4;
-    C.rbig.ensure(bytes);
+    const size_t zero = work_reserve(C, nt, n_tiles);
     char* base = C.rbig.as<char>();
     RasterWork w;
     w.head = reinterpret_cast<RasterHead*>(base);
-    w.count = reinterpret_cast<int32_t*>(base + head);
+    w.count = reinterpret_cast<int32_t*>(base + HEAD_BYTES);
     w.off = w.count + n_tiles;
     w.lines = w.off + n_tiles + 1;
     w.xy = reinterpret_cast<uint32_t*>(w.lines + nt);
     w.list = reinterpret_cast<int32_t*>(w.xy + nt * 3);
     w.n_tiles = (int32_t)n_tiles;
-    w.list_cap = (int32_t)cap;
+    w.list_cap = (int32_t)list_capacity(nt, n_tiles);
     w.max_tri = (int32_t)nt;
-    IDL_CUDA(cudaMemsetAsync(base, 0, head + (size_t)n_tiles * 4, C.stream));
+    if (!C.precleared) IDL_CUDA(cudaMemsetAsync(base, 0, zero, C.stream));
     return w;
 }
 
@@ -140,11 +163,11 @@ template <class TILE, class F>
 void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids,
                  int stride, F&& draw)
 {
-    const int64_t tiles = (int64_t)ceil_div(W, TILE::W) * ceil_div(H, TILE::H);
+    const int64_t tiles = tile_count<TILE>(W, H);
     const RasterWork w = raster_work(C, n_tri, tiles);
     const int32_t* tris = C.tris.as<int32_t>();
     if (n_tri > 0) {
-        IDL_CUDA(cudaMemsetAsync(&C.sc()->max_side, 0, sizeof(int32_t), C.stream));
+        if (!C.precleared) IDL_CUDA(cudaMemsetAsync(&C.sc()->max_side, 0, sizeof(int32_t), C.stream));
         const unsigned blocks = (unsigned)ceil_div(n_tri, 256);
         k_raster_count<TILE><<<blocks, 256, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, w);
         IDL_LAUNCH();
@@ -165,7 +188,7 @@ template <class F>
 void raster(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids, int stride,
             F&& draw)
 {
-    if (small_tiles((int64_t)ceil_div(W, TileLarge::W) * ceil_div(H, TileLarge::H), C.num_sms))
+    if (small_tiles(tile_count<TileLarge>(W, H), C.num_sms))
         raster_with<TileSmall>(C, W, H, xs, ys, n_tri, ids, stride, draw);
     else raster_with<TileLarge>(C, W, H, xs, ys, n_tri, ids, stride, draw);
 }

@@ -689,22 +689,30 @@ __global__ void k_resolve_apply(int32_t* __restrict__ lab, int pitch, const int3
 
 }  // namespace
 
+size_t resolve_reserve(Context& C, const Canvas& cv)
+{
+    const size_t bits = (size_t)ceil_div(cv.Wd, 32) * cv.Hd * 4;
+    C.sus_bits.ensure(bits);
+    return bits;
+}
+
 void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes, const XImg* images,
                    const int32_t* seed_img)
 {
     const int words = ceil_div(cv.Wd, 32);
-    const size_t bits = (size_t)words * cv.Hd * 4;
+    const size_t bits = resolve_reserve(C, cv);
     // suspects: 0.02 % of the cells at the usual densities (at most 0.4 % in
     // the densest sets measured); beyond the lists the iteration takes over
     const int cap = (int)std::min<int64_t>((int64_t)cv.Wd * cv.Hd / 64 + 4096, 1 << 22);
-    C.sus_bits.ensure(bits);
     C.sus_list.ensure((size_t)cap * 3 * 4);
     int32_t* list = C.sus_list.as<int32_t>();
     int32_t* res = list + cap;
     int32_t* open = res + cap;
     uint32_t* sus = C.sus_bits.as<uint32_t>();
-    IDL_CUDA(cudaMemsetAsync(sus, 0, bits, C.stream));
-    IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
+    if (!C.precleared) {
+        IDL_CUDA(cudaMemsetAsync(sus, 0, bits, C.stream));
+        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
+    }
     const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), C.exact_bands.as<int32_t>(), pos, sus, images,
                  seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n, 0)};
     const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 4 * ROOT_ROWS));

@@ -225,8 +225,10 @@ void sort_seeds_device(Context& C, int W, int H, int64_t n, int P)
     C.ys.ensure(size_t(n) * 4);
     C.pos.ensure(size_t(n) * 4);
 
-    IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, size_t(nwords) * 4, C.stream));
-    IDL_CUDA(cudaMemsetAsync(&C.sc()->err_oob, 0, 3 * sizeof(int32_t), C.stream));
+    if (!C.precleared) {
+        IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, size_t(nwords) * 4, C.stream));
+        IDL_CUDA(cudaMemsetAsync(&C.sc()->err_oob, 0, 3 * sizeof(int32_t), C.stream));
+    }
     const unsigned gs = (unsigned)((n + 255) / 256);
     k_seed_mark<<<gs, 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, W, H, C.bitmap.as<uint32_t>(), C.sc());
     IDL_LAUNCH();

@@ -391,13 +391,10 @@ int64_t detect_capacity(const Context& C, int64_t n)
     return std::max<int64_t>(next_pow2(8 * n + 1024), C.hash_cap);
 }
 
-void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
-                   int64_t cap, cudaEvent_t mid, const int32_t* rank)
+void detect_reserve(Context& C, int64_t n, int64_t cap)
 {
     C.cnt.ensure((size_t)(n + 1) * 2 * 4);   // counts, then fill positions: cleared together
     C.off.ensure((size_t)(n + 2) * 4);
-    int32_t* cnt = C.cnt.as<int32_t>();
-    int32_t* fill = cnt + n + 1;
     C.hkeys.ensure((size_t)cap * 16);
     C.ukeys.ensure((size_t)cap * 8);
     C.uvals.ensure((size_t)cap * 8);
@@ -406,15 +403,25 @@ void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const ui
     // count comes from the device
     C.grp.ensure((size_t)cap * 4);
     C.tris.ensure((size_t)cap * 5 * 4);
+}
+
+void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
+                   int64_t cap, cudaEvent_t mid, const int32_t* rank)
+{
+    detect_reserve(C, n, cap);
+    int32_t* cnt = C.cnt.as<int32_t>();
+    int32_t* fill = cnt + n + 1;
     unsigned long long* table = C.hkeys.as<unsigned long long>();
     unsigned long long* ukeys = C.ukeys.as<unsigned long long>();
     unsigned long long* uvals = C.uvals.as<unsigned long long>();
-    IDL_CUDA(cudaMemsetAsync(table, 0xFF, (size_t)cap * 16, C.stream));
     // the blocks left to k_detect_rest wait in the grouping buffer, free until then
     uint32_t* rest = C.grp.as<uint32_t>();
     static_assert(offsetof(Scalars, overflow) == 12 && offsetof(Scalars, n_blocks) == 8, "cleared together");
-    IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
-    IDL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(n + 1) * 2 * 4, C.stream));
+    if (!C.precleared) {
+        IDL_CUDA(cudaMemsetAsync(table, 0xFF, (size_t)cap * 16, C.stream));
+        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
+        IDL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(n + 1) * 2 * 4, C.stream));
+    }
 
     const int strips = ceil_div(std::max(cv.Wd - 1, 1), DET_COLS);
     const bool small = strips * ceil_div(cv.Hd, DET_ROWS) < C.num_sms * 16;
