@@ -465,7 +465,7 @@ __global__ void k_score_keys(const float* __restrict__ scores, int64_t n, float 
 // canvas, rounded half to even (lrint) and clamped to the image
 // (midpoints_from_sorted_kernel, delaunay_scalar_field.cu:129-160): the padded
 // pixel index, or -1 where the pixel already holds a seed (its cell's label
-// is a seed at that very position).
+// is a seed at that very position) or the edge is not eligible.
 __global__ void k_midpoints(const unsigned long long* __restrict__ sorted, int take,
                             const unsigned long long* __restrict__ edge_keys, int64_t n_seeds,
                             const int32_t* __restrict__ x, const int32_t* __restrict__ y, int P, int Wd, int Hd,
@@ -474,6 +474,10 @@ __global__ void k_midpoints(const unsigned long long* __restrict__ sorted, int t
 {
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= take) return;
+    if ((sorted[r] >> 32) == 0xFFFFFFFFull) {   // not eligible, nor is any after it
+        out[r] = -1;
+        return;
+    }
     const uint32_t e = (uint32_t)(sorted[r] & 0xFFFFFFFFull);
     const unsigned long long k = edge_keys[e];
     const int32_t a = (int32_t)(k / (unsigned long long)n_seeds), b = (int32_t)(k % (unsigned long long)n_seeds);
@@ -1258,20 +1262,16 @@ int idl_delaunay_select_midpoints(idl_delaunay* d, double min_length, int count,
                                                   d->score_keys.as<unsigned long long>());
     IDL_LAUNCH();
     size_t need = 0;
+    // by the score alone: the sort is stable and the edge indices below ascend
+    // already (half the passes of sorting whole keys)
     IDL_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, need, d->score_keys.as<unsigned long long>(),
-                                            d->score_sorted.as<unsigned long long>(), (int)E, 0, 64, C.stream));
+                                            d->score_sorted.as<unsigned long long>(), (int)E, 32, 64, C.stream));
     d->sort_tmp.ensure(need);
     size_t tb = d->sort_tmp.bytes;
     IDL_CUDA(cub::DeviceRadixSort::SortKeys(d->sort_tmp.ptr, tb, d->score_keys.as<unsigned long long>(),
-                                            d->score_sorted.as<unsigned long long>(), (int)E, 0, 64, C.stream));
-    // the eligible edges sort first; take at most `count` of them
-    const int64_t look = std::min<int64_t>(count, E);
-    std::vector<unsigned long long> head((size_t)look);
-    IDL_CUDA(cudaMemcpyAsync(head.data(), d->score_sorted.ptr, (size_t)look * 8, cudaMemcpyDeviceToHost, C.stream));
-    IDL_CUDA(cudaStreamSynchronize(C.stream));
-    int take = 0;
-    while (take < look && (head[take] >> 32) != 0xFFFFFFFFull) ++take;
-    if (take == 0) return IDL_OK;
+                                            d->score_sorted.as<unsigned long long>(), (int)E, 32, 64, C.stream));
+    // the eligible edges sort first; at most `count` of them
+    const int take = (int)std::min<int64_t>(count, E);
     d->stage.ensure((size_t)take * 8);
     k_midpoints<<<blocks(take), 256, 0, C.stream>>>(d->score_sorted.as<unsigned long long>(), take,
                                                     d->edge_keys.as<unsigned long long>(), d->N, d->ix, d->iy, d->P,
