@@ -354,9 +354,11 @@ void grid_barrier_selftest(Context& C, int missing_arrivals, unsigned spin_limit
 // for the n (x, y)-sorted seeds `pos` of the canvas; labels into C.lab[0]
 // (C.lab[1] holds the column pass's offsets, C.exact_bands its table).  P: the
 // canvas's padding; C.bitmap and C.scan_c hold these seeds' occupancy bits and
-// their ranks, as sort_seeds_device and rank_seeds_device leave them.
+// their ranks, as sort_seeds_device and rank_seeds_device leave them.  label:
+// each rank's label, which the plane takes and ties go by (null: the rank).
 struct XImg;
-void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P);
+void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P,
+                     const int32_t* label = nullptr);
 // The same for the images of a batch atlas (exact.cu): the device table of the
 // images, room for each column pair's and each row's image; C.lab[0] and
 // C.lab[1] hold planes of the atlas.
@@ -370,9 +372,11 @@ XImg whole_canvas(const Canvas& cv, int64_t n, int P);
 // (resolve.cu).  Reads nothing back: C.sc()->resolve_fail, with the scalars'
 // next read-back, tells whether the passes have to be run instead.  `passes`:
 // also what resolved_passes needs.  Batch atlas: `images` is the table
-// exact_images used, `seed_img` the image of each seed.
+// exact_images used, `seed_img` the image of each seed.  Labels that are not
+// ranks: `pos` by label, `sorted` by rank and the `label` table propagate_exact had.
 void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes,
-                   const XImg* images = nullptr, const int32_t* seed_img = nullptr);
+                   const XImg* images = nullptr, const int32_t* seed_img = nullptr,
+                   const uint32_t* sorted = nullptr, const int32_t* label = nullptr);
 // The iteration's pass count from the scalars read back after resolve_exact
 // with `passes`, or -1 if they do not determine it.
 inline int64_t resolved_passes(const Scalars& s)

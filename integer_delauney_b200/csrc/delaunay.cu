@@ -985,10 +985,27 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
             d->planes, d->planes + (size_t)d->pitch * d->Hd, d->pitch, d->Wd, d->inv);
         IDL_LAUNCH();
     } else {
-        k_put_seeds<<<gk, 256, 0, C.stream>>>(d->planes, d->planes + (size_t)d->pitch * d->Hd, d->pitch,
-                                              d->pos + n0, k, n0);
-        IDL_LAUNCH();
-        passes = propagate(C, d->mode, d->canvas(), d->pos, n0 + k, d->pos + n0, k);
+        const size_t plane = (size_t)d->pitch * d->Hd;
+        bool done = false;
+        if (n0 == 0 && C.direct() && !timings) {
+            // into an empty object the propagation is one from scratch: read its
+            // fixed point off the exact diagram (ties by insertion id)
+            ensure_rank(*d);
+            d->spos.ensure((size_t)d->N * 4);
+            k_pack_pos<<<blocks(d->N), 256, 0, C.stream>>>(d->sx, d->sy, d->N, 0, d->spos.as<uint32_t>());
+            IDL_LAUNCH();
+            propagate_exact(C, d->canvas(), d->spos.as<uint32_t>(), d->N, d->P, d->inv);
+            resolve_exact(C, d->canvas(), d->pos, d->N, false, nullptr, nullptr, d->spos.as<uint32_t>(), d->inv);
+            IDL_CUDA(cudaMemcpyAsync(d->planes + plane, d->planes, plane * 4, cudaMemcpyDeviceToDevice, C.stream));
+            C.fetch_scalars();
+            done = !C.host_sc->resolve_fail;
+            if (!done) IDL_CUDA(cudaMemsetAsync(d->planes, 0xFF, plane * 8, C.stream));   // empty again
+        }
+        if (!done) {
+            k_put_seeds<<<gk, 256, 0, C.stream>>>(d->planes, d->planes + plane, d->pitch, d->pos + n0, k, n0);
+            IDL_LAUNCH();
+            passes = propagate(C, d->mode, d->canvas(), d->pos, n0 + k, d->pos + n0, k);
+        }
     }
     const float bfs = T.stop();
     if (timings) {

@@ -24,6 +24,7 @@
 #include "exact_pass.cuh"
 
 #include <atomic>
+#include <type_traits>
 
 namespace idl {
 namespace {
@@ -54,13 +55,14 @@ __global__ void k_bx_tables(const XImg* __restrict__ xi, int32_t* __restrict__ p
     for (int i = threadIdx.x; i < m.Hp; i += blockDim.x) row_img[m.row_off + i] = blockIdx.x;
 }
 
-template <int T>
+template <int T, bool LABELS>
 __global__ void __launch_bounds__(T)
 k_row_win(const int16_t* __restrict__ off, XImg m, int pitch, const uint32_t* __restrict__ pos,
-          const int32_t* __restrict__ bands, int32_t* __restrict__ lab, int list_bytes)
+          const int32_t* __restrict__ bands, const int32_t* __restrict__ label, int32_t* __restrict__ lab,
+          int list_bytes)
 {
     const int y = blockIdx.x;
-    x_row<T>(off + (size_t)y * pitch, y, m, pos, bands, lab + (size_t)y * pitch, list_bytes);
+    x_row<T, LABELS>(off + (size_t)y * pitch, y, m, pos, bands, label, lab + (size_t)y * pitch, list_bytes);
 }
 
 template <int T>
@@ -72,7 +74,7 @@ k_bx_row_win(const int16_t* __restrict__ off, const XImg* __restrict__ xi, const
     const XImg m = xi[row_img[blockIdx.x]];
     const int y = m.oy + (int)blockIdx.x - m.row_off;
     const size_t o = (size_t)y * pitch + m.ox;
-    x_row<T>(off + o, y, m, pos, bands, lab + o, list_bytes);
+    x_row<T, false>(off + o, y, m, pos, bands, nullptr, lab + o, list_bytes);
 }
 
 template <class K, class... A>
@@ -88,21 +90,20 @@ void launch_rows(Context& C, K kernel, std::atomic<uint64_t>& opted, unsigned ro
     IDL_LAUNCH();
 }
 
-// One instantiation per row width class (row_pass_threads).
-template <bool BATCH, class... A>
-void rows_for_width(Context& C, int width, unsigned rows, A... args)
+// One instantiation per row width class (row_pass_threads): which(threads)
+// names the kernel.
+template <class W, class... A>
+void rows_for_width(Context& C, int width, unsigned rows, std::atomic<uint64_t>* opted, W&& which, A... args)
 {
-    static std::atomic<uint64_t> opted[4];
     const int threads = row_pass_threads(width, rows);
     const size_t smem = row_pass_smem(width);
-    auto go = [&](auto single, auto batch, int slot) {
-        if constexpr (BATCH) launch_rows(C, batch, opted[slot], rows, threads, smem, args..., row_list_bytes(width));
-        else launch_rows(C, single, opted[slot], rows, threads, smem, args..., row_list_bytes(width));
+    auto go = [&](auto tag, int slot) {
+        launch_rows(C, which(tag), opted[slot], rows, threads, smem, args..., row_list_bytes(width));
     };
-    if (threads == 32) go(k_row_win<32>, k_bx_row_win<32>, 0);
-    else if (threads == 64) go(k_row_win<64>, k_bx_row_win<64>, 1);
-    else if (threads == 128) go(k_row_win<128>, k_bx_row_win<128>, 2);
-    else go(k_row_win<256>, k_bx_row_win<256>, 3);
+    if (threads == 32) go(std::integral_constant<int, 32>{}, 0);
+    else if (threads == 64) go(std::integral_constant<int, 64>{}, 1);
+    else if (threads == 128) go(std::integral_constant<int, 128>{}, 2);
+    else go(std::integral_constant<int, 256>{}, 3);
 }
 
 }  // namespace
@@ -117,7 +118,7 @@ XImg whole_canvas(const Canvas& cv, int64_t n, int P)
     return m;
 }
 
-void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P)
+void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, int P, const int32_t* label)
 {
     const size_t plane = (size_t)cv.pitch * cv.Hd * 4;
     C.lab[0].ensure(plane);
@@ -126,12 +127,19 @@ void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t 
     C.exact_bands.ensure((size_t)x_bands(m) * cv.Wd * 4);
     int16_t* off = C.lab[1].as<int16_t>();
     int32_t* bands = C.exact_bands.as<int32_t>();
-    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>()};
+    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), label};
     k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, ranks, m, cv.pitch, off,
                                                                                                bands);
     IDL_LAUNCH();
-    rows_for_width<false>(C, cv.Wd, (unsigned)cv.Hd, (const int16_t*)off, m, cv.pitch, pos, (const int32_t*)bands,
-                          C.lab[0].as<int32_t>());
+    static std::atomic<uint64_t> opted[2][4];
+    const int16_t* o = off;
+    const int32_t* t = bands;
+    if (label)
+        rows_for_width(C, cv.Wd, (unsigned)cv.Hd, opted[1], [](auto T) { return k_row_win<T(), true>; }, o, m, cv.pitch,
+                       pos, t, label, C.lab[0].as<int32_t>());
+    else
+        rows_for_width(C, cv.Wd, (unsigned)cv.Hd, opted[0], [](auto T) { return k_row_win<T(), false>; }, o, m,
+                       cv.pitch, pos, t, label, C.lab[0].as<int32_t>());
     if (C.prof.enabled) {
         C.prof.passes = 0;
         C.prof.rounds = 2;
@@ -150,12 +158,13 @@ void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, in
     C.exact_bands.ensure((size_t)band_entries * 4);
     int16_t* off = C.lab[1].as<int16_t>();
     int32_t* bands = C.exact_bands.as<int32_t>();
-    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>()};
+    const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nullptr};
     k_bx_column_off<<<dim3((unsigned)ceil_div(n_pairs, 64), (unsigned)ceil_div(max_hp, BAND)), 64, 0, C.stream>>>(
         pos, ranks, xi, pair_img, n_pairs, pitch, off, bands);
     IDL_LAUNCH();
-    rows_for_width<true>(C, max_wp, (unsigned)n_rows, (const int16_t*)off, xi, (const int32_t*)row_img, pitch, pos,
-                         (const int32_t*)bands, C.lab[0].as<int32_t>());
+    static std::atomic<uint64_t> opted[4];
+    rows_for_width(C, max_wp, (unsigned)n_rows, opted, [](auto T) { return k_bx_row_win<T()>; }, (const int16_t*)off, xi,
+                   (const int32_t*)row_img, pitch, pos, (const int32_t*)bands, C.lab[0].as<int32_t>());
 }
 
 }  // namespace idl

@@ -32,6 +32,7 @@ __host__ __device__ inline int x_bands(const XImg& m) { return (m.Hp + BAND - 1)
 struct SeedRanks {
     const uint32_t* bits;
     const int32_t* before;
+    const int32_t* label;   // label of each rank, ties going to the higher label; null: the rank itself
 };
 
 // First of the image's seeds at or after (x, y) in (x, y) order: two loads,
@@ -106,8 +107,11 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
                     if ((int)pos_x(p) == m.ox + c + k) next_y[k] = (int)pos_y(p) - m.oy;
                 }
             }
-            const int below = next_y[k] - y, above = y - prev_y[k];   // tie: the larger y, the higher id
-            v[k] = any[k] ? (below <= above ? below : -above) : NO_SEED;
+            const int below = next_y[k] - y, above = y - prev_y[k];   // tie: the larger y, the higher rank
+            bool down = below <= above;
+            if (ranks.label && below == above && any[k])
+                down = __ldg(&ranks.label[a[k]]) > __ldg(&ranks.label[a[k] - 1]);
+            v[k] = any[k] ? (down ? below : -above) : NO_SEED;
         }
         if (paired) {
             *reinterpret_cast<short2*>(dst) = make_short2((short)v[0], (short)v[1]);
@@ -159,7 +163,7 @@ inline int row_list_bytes(int W) { return W > ROW_WIDE ? 2 : 4; }   // per colum
 inline size_t row_pass_smem(int W)
 {
     const size_t w = (size_t)(W + 7) / 4 * 4;
-    return w * (4 + row_list_bytes(W)) + (size_t)(W / ROW_STEP + 3) * 2 + 16;
+    return w * (4 + row_list_bytes(W)) + (size_t)(W / ROW_STEP + 3) * 4 + 16;
 }
 // Threads per row: warps of at most ROW_SHARE columns, up to 8 (twice that
 // where there are rows enough to fill the device with fewer warps each: 2 % of
@@ -171,11 +175,14 @@ inline int row_pass_threads(int W, unsigned rows)
 }
 
 // Steps 2 and 3 of the row pass over a list of n columns; cost(k, t) is
-// F - 2 t x of its entry k.
-template <int T, class Cost>
+// F - 2 t x of its entry k.  LABELS: ties between columns go to the higher
+// label, whichever side it lies on; a cell's bounds are then the first minimum
+// at the anchor before and the last one at the anchor after.
+template <int T, bool LABELS, class Cost>
 __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* listx, uint16_t* buf, uint16_t* hx,
-                                           uint16_t* win, const int16_t* off, int n, int W, int y, const XImg& m,
-                                           const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
+                                           uint16_t* win, uint16_t* win_lo, const int16_t* off, int n, int W, int y,
+                                           const XImg& m, const uint32_t* __restrict__ pos,
+                                           const int32_t* __restrict__ bands, const int32_t* __restrict__ label,
                                            int32_t* __restrict__ out, Cost cost, bool packed)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -184,86 +191,98 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         if (T == 32) __syncwarp();
         else __syncthreads();
     };
-    auto best_in = [&](int t, int lo, int hi) {
-        int arg = lo;
-        int32_t best = cost(lo, t);
-        for (int k = lo + 1; k <= hi; ++k) {
-            const int32_t c = cost(k, t);
-            if (c <= best) {
-                best = c;
-                arg = k;
-            }
-        }
-        return arg;
-    };
-    auto by_warp = [&](int t, int lo, int hi) {
+    auto name = [&](int32_t rank) { return LABELS ? __ldg(&label[rank]) : rank; };
+    auto by_warp = [&](int i, int lo, int hi) {
+        const int t = i * ROW_STEP;
         int32_t best = 0x7FFFFFFF;
-        int arg = lo;
+        int arg = lo, first = 0x7FFFFFFF;
         for (int k = lo + lane; k <= hi; k += 32) {
             const int32_t c = cost(k, t);
+            if (LABELS && c < best) first = k;
             if (c <= best) {
                 best = c;
                 arg = k;
             }
         }
         const int32_t low = __reduce_min_sync(0xFFFFFFFFu, best);
-        return (int)__reduce_max_sync(0xFFFFFFFFu, best == low ? arg : -1);
+        const int last = (int)__reduce_max_sync(0xFFFFFFFFu, best == low ? arg : -1);
+        if (lane == 0) win[i] = (uint16_t)last;
+        if (LABELS) {
+            const int f = (int)__reduce_min_sync(0xFFFFFFFFu, best == low ? first : 0x7FFFFFFF);
+            if (lane == 0) win_lo[i] = (uint16_t)f;
+        }
     };
+    const uint16_t* low = LABELS ? win_lo : win;
 
     // 2. winners of the cells ROW_TOP, ROW_MID and ROW_STEP apart
     const int steps = (W + ROW_STEP - 1) / ROW_STEP;
     constexpr int TOP = ROW_TOP / ROW_STEP, MID = ROW_MID / ROW_STEP;
-    for (int i = warp * TOP; i < steps; i += NW * TOP) {
-        const int a = by_warp(i * ROW_STEP, 0, n - 1);
-        if (lane == 0) win[i] = (uint16_t)a;
-    }
+    for (int i = warp * TOP; i < steps; i += NW * TOP) by_warp(i, 0, n - 1);
     if (tid == 0) win[steps] = (uint16_t)(n - 1);
     sync();
     for (int i = warp * MID; i < steps; i += NW * MID) {
         if (i % TOP == 0) continue;
         const int up = i / TOP * TOP;
-        const int a = by_warp(i * ROW_STEP, win[up], win[min(up + TOP, steps)]);
-        if (lane == 0) win[i] = (uint16_t)a;
+        by_warp(i, low[up], win[min(up + TOP, steps)]);
     }
     sync();
     for (int i = tid; i < steps; i += T) {
         if (i % MID == 0) continue;
-        const int up = i / MID * MID;
-        win[i] = (uint16_t)best_in(i * ROW_STEP, win[up], win[min(up + MID, steps)]);
+        const int up = i / MID * MID, hi = win[min(up + MID, steps)], t = i * ROW_STEP;
+        int arg = low[up], first = arg;
+        int32_t best = cost(arg, t);
+        for (int k = arg + 1; k <= hi; ++k) {
+            const int32_t c = cost(k, t);
+            if (LABELS && c < best) first = k;
+            if (c <= best) {
+                best = c;
+                arg = k;
+            }
+        }
+        win[i] = (uint16_t)arg;
+        if (LABELS) win_lo[i] = (uint16_t)first;
     }
     if (packed) {
-        // ids of the listed columns' seeds: the offsets move aside first, then
-        // buf and hx take the ids' halves (each list entry is one thread's)
+        // labels of the listed columns' seeds: the offsets move aside first,
+        // then buf and hx take the labels' halves (each list entry is one thread's)
         for (int k = tid; k < n; k += T) hx[k] = (uint16_t)off[list2[k].y / -2];
         sync();
         for (int k = tid; k < n; k += T) {
-            const int32_t id = x_seed_at(pos, bands, m, m.ox + list2[k].y / -2, y + (int16_t)hx[k]);
+            const int32_t id = name(x_seed_at(pos, bands, m, m.ox + list2[k].y / -2, y + (int16_t)hx[k]));
             buf[k] = (uint16_t)(id & 0xFFFF);
             hx[k] = (uint16_t)(id >> 16);
         }
     }
     sync();
+    auto label_of = [&](int k) -> int32_t {
+        if (packed) return (int32_t)buf[k] | (int32_t)hx[k] << 16;
+        const int x = listx[k];
+        return name(x_seed_at(pos, bands, m, m.ox + x, y + off[x]));
+    };
 
     // 3. every cell, from the list between its interval's bounds
     for (int i = warp; i < steps; i += NW) {
         const int t = i * ROW_STEP + lane;
-        const int arg = best_in(t, win[i], win[i + 1]);
-        if (t >= W) continue;
-        if (packed) {
-            out[t] = (int32_t)buf[arg] | (int32_t)hx[arg] << 16;
-        } else {
-            const int x = listx[arg];
-            out[t] = x_seed_at(pos, bands, m, m.ox + x, y + off[x]);
+        const int hi = win[i + 1];
+        int arg = low[i];
+        int32_t best = cost(arg, t);
+        for (int k = arg + 1; k <= hi; ++k) {
+            const int32_t c = cost(k, t);
+            if (LABELS ? c < best || (c == best && label_of(k) > label_of(arg)) : c <= best) {
+                best = c;
+                arg = k;
+            }
         }
+        if (t < W) out[t] = label_of(arg);
     }
 }
 
 // row: the row's offsets; y: its row on the plane; out: its labels;
 // list_bytes: row_list_bytes of the launch.
-template <int T>
+template <int T, bool LABELS>
 __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, const XImg& m,
                                       const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-                                      int32_t* __restrict__ out, int list_bytes)
+                                      const int32_t* __restrict__ label, int32_t* __restrict__ out, int list_bytes)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
     __shared__ int s_sum[T / 32 + 1];
@@ -275,6 +294,8 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
     uint16_t* buf = reinterpret_cast<uint16_t*>(row_smem + (size_t)w * list_bytes);   // offsets, then id low halves
     uint16_t* hx = buf + w;                                        // columns kept, then id high halves
     uint16_t* win = hx + w;                                        // winner at each 32nd cell
+    uint16_t* win_lo = win + (W / ROW_STEP + 3);                   // LABELS: the first of the tied ones
+    constexpr int TIE = LABELS ? 1 : 0;   // columns that could still tie are kept
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = T / 32;
     auto sync = [] {
@@ -326,8 +347,8 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
             const uint32_t d = q[4 + c], dd = 2u * d;
-            keep[c] = x + c < s1 && d != NO_SQUARE && q[3 + c] + q[5 + c] + 2u > dd &&
-                      q[2 + c] + q[6 + c] + 8u > dd && q[c] + q[8 + c] + 32u > dd;
+            keep[c] = x + c < s1 && d != NO_SQUARE && q[3 + c] + q[5 + c] + 2u + TIE > dd &&
+                      q[2 + c] + q[6 + c] + 8u + TIE > dd && q[c] + q[8 + c] + 32u + TIE > dd;
         }
         const unsigned k0 = __ballot_sync(0xFFFFFFFFu, keep[0]), k1 = __ballot_sync(0xFFFFFFFFu, keep[1]);
         const int at0 = s0 + kept + __popc(k0 & below) + __popc(k1 & below);
@@ -349,7 +370,7 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
                 if (i > 0 && i + 1 < kept) {
                     const int xl = hx[s0 + i - 1], xr = hx[s0 + i + 1];
                     const int32_t f = value(x), fl = value(xl), fr = value(xr);
-                    keep = (long long)(x - xl) * (fr - f) > (long long)(f - fl) * (xr - x);
+                    keep = (long long)(x - xl) * (fr - f) + TIE > (long long)(f - fl) * (xr - x);
                 }
             }
             const unsigned k = __ballot_sync(0xFFFFFFFFu, keep);
@@ -387,12 +408,14 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
         return;
     }
     if (packed) {
-        x_row_fill<T>(list2, listx, buf, hx, win, off, n, W, y, m, pos, bands, out, [&](int k, int t) {
+        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, pos, bands, label, out,
+                              [&](int k, int t) {
             const int2 c = list2[k];
             return c.x + t * c.y;
         }, true);
     } else {
-        x_row_fill<T>(list2, listx, buf, hx, win, off, n, W, y, m, pos, bands, out, [&](int k, int t) {
+        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, pos, bands, label, out,
+                              [&](int k, int t) {
             const int x = listx[k];
             return value(x) - 2 * t * x;
         }, false);

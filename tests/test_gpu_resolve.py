@@ -115,3 +115,27 @@ def test_exact_rows(W, H, n):
     seeds = random_seeds(W, H, n, 5)
     want, _ = oracle.voronoi("exact", W, H, oracle.sort_seeds(seeds, W, H))
     np.testing.assert_array_equal(cu.Voronoi().compute(W, H, seeds, voronoi_mode="exact"), want)
+
+
+@pytest.mark.parametrize("W,H", [(129, 17), (127, 131), (417, 301)])
+@pytest.mark.parametrize("kind", ["uniform", "sparse", "dense", "clustered", "lattice", "line", "circle", "disc"])
+def test_first_insert_in_insertion_order(ctx, kind, W, H):
+    """A first insert (ids, and so ties, in the order given) against the same
+    insert through the passes, and a second insert on top of each."""
+    for seed in (1, 2, 3):
+        seeds = _layout(kind, W, H, seed)
+        np.random.default_rng(seed).shuffle(seeds)
+        taken = np.sort(seeds[:, 1].astype(np.int64) * W + seeds[:, 0])
+        from integer_delauney_b200.workloads import fresh_points
+        more = fresh_points(W, H, 5, taken, seed)
+        ctx.set_schedule(0)
+        got, want = (cu.Delaunay(W, H, len(seeds) + 5, 8) for _ in range(2))
+        want.use_workspace(ctx)
+        for batch in (seeds, more):
+            if not len(batch):
+                continue
+            got.insert_deferred(batch)
+            want.insert_deferred(batch)
+            msg = f"{kind} {W}x{H} seed {seed}"
+            np.testing.assert_array_equal(got.get_voronoi_grid(), want.get_voronoi_grid(), err_msg=msg)
+            np.testing.assert_array_equal(got.get_triangles(), want.get_triangles(), err_msg=msg)
