@@ -74,14 +74,6 @@ void ensure_scalars(Context& C)
 
 namespace {
 
-struct ClearList {
-    static constexpr int MAX = 6;
-    uint4* p[MAX];
-    long long n[MAX];     // 16-byte units
-    uint32_t word[MAX];
-    int count;
-};
-
 __global__ void __launch_bounds__(256) k_clear(ClearList l)
 {
     const long long step = (long long)gridDim.x * blockDim.x;
@@ -94,32 +86,34 @@ __global__ void __launch_bounds__(256) k_clear(ClearList l)
 
 }  // namespace
 
-void clear_for_run(Context& C, const Canvas& cv, int W, int H, int64_t n, bool suspects, int64_t cap, int64_t n_tri)
+void clear_buffers(Context& C, const ClearList& l)
 {
-    ClearList l{};
-    long long units = 0;
-    // buffers are whole multiples of 256 bytes, so the last unit may run past `bytes`
-    auto add = [&](const DevBuf& b, size_t bytes, uint32_t word) {
-        l.p[l.count] = b.as<uint4>();
-        l.n[l.count] = (long long)((bytes + 15) / 16);
-        l.word[l.count] = word;
-        units = std::max(units, l.n[l.count]);
-        ++l.count;
-    };
-    const size_t bitmap = ((size_t)W * H + 31) / 32 * 4;
-    C.bitmap.ensure(bitmap);
-    add(C.scalars, sizeof(Scalars), 0);
-    add(C.bitmap, bitmap, 0);
-    if (suspects) add(C.sus_bits, resolve_reserve(C, cv), 0);
-    if (cap > 0) {
-        detect_reserve(C, n, cap);
-        add(C.hkeys, (size_t)cap * 16, 0xFFFFFFFFu);
-        add(C.cnt, (size_t)(n + 1) * 2 * 4, 0);
-        add(C.rbig, raster_reserve(C, W, H, n_tri), 0);
-    }
-    const unsigned blocks = (unsigned)std::max<long long>(1, std::min<long long>((units + 255) / 256, C.num_sms * 16));
+    long long units = 1;
+    for (int k = 0; k < l.count; ++k) units = std::max(units, l.n[k]);
+    const unsigned blocks = (unsigned)std::min<long long>((units + 255) / 256, C.num_sms * 16);
     k_clear<<<blocks, 256, 0, C.stream>>>(l);
     IDL_LAUNCH();
+}
+
+void clear_for_run(Context& C, const Canvas& cv, int W, int H, int64_t n, bool suspects, int64_t cap, int64_t n_tri)
+{
+    ClearList l;
+    const size_t bitmap = ((size_t)W * H + 31) / 32 * 4;
+    C.bitmap.ensure(bitmap);
+    l.add(C.scalars.ptr, sizeof(Scalars), 0);
+    l.add(C.bitmap.ptr, bitmap, 0);
+    if (suspects) {
+        const size_t bits = resolve_reserve(C, cv);
+        l.add(C.sus_bits.ptr, bits, 0);
+    }
+    if (cap > 0) {
+        detect_reserve(C, n, cap);
+        l.add(C.hkeys.ptr, (size_t)cap * 16, 0xFFFFFFFFu);
+        l.add(C.cnt.ptr, (size_t)(n + 1) * 2 * 4, 0);
+        const size_t head = raster_reserve(C, W, H, n_tri);
+        l.add(C.rbig.ptr, head, 0);
+    }
+    clear_buffers(C, l);
     C.precleared = true;
 }
 

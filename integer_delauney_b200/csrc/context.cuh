@@ -98,7 +98,6 @@ struct Scalars {
     int32_t err_dup;          // two seeds share a pixel
     int32_t scan_done;        // blocks of a scan that have finished (0 between scans)
     int32_t err_label;        // a caller-supplied label was outside [-1, n)
-    int32_t max_side;         // longest triangle side, float-truncated (triangulation.cu:355-368)
     int32_t n_handoff;        // micro-tiles the last tile round hands to the persistent kernel
     int32_t tile_remaining;   // tiles listed for the tile round after the last one launched
     // resolve.cu, cleared together (RESOLVE_SCALARS values from n_roots on)
@@ -407,6 +406,23 @@ void detect_reserve(Context& C, int64_t n, int64_t cap);
 void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const uint32_t* pos, int64_t n, int shift,
                    int64_t cap, cudaEvent_t mid = nullptr, const int32_t* rank = nullptr);
 bool detect_done(Context& C, int64_t cap);
+
+// Fills up to six buffers in one launch, each with one word: whole 16-byte
+// units from a 16-byte aligned start (buffers are multiples of 256 bytes).
+struct ClearList {
+    static constexpr int MAX = 6;
+    uint4* p[MAX];
+    long long n[MAX];
+    uint32_t word[MAX];
+    int count = 0;
+    void add(void* ptr, size_t bytes, uint32_t w)
+    {
+        p[count] = static_cast<uint4*>(ptr);
+        n[count] = (long long)((bytes + 15) / 16);
+        word[count++] = w;
+    }
+};
+void clear_buffers(Context& C, const ClearList& l);
 
 // One launch clears what the stages of a single-image run clear one by one
 // (occupancy bits, counters, suspect bits, hash table, group counts, tile

@@ -191,6 +191,24 @@ __global__ void k_put_seeds(int32_t* __restrict__ a, int32_t* __restrict__ b, in
     b[o] = (int32_t)(first_id + i);
 }
 
+// A batch in the order given: its coordinates, its packed canvas positions and,
+// with planes, its cells (k_put_seeds), in one launch.
+__global__ void k_append(const int32_t* __restrict__ xy, int64_t k, int P, int32_t* __restrict__ ix,
+                         int32_t* __restrict__ iy, uint32_t* __restrict__ pos, int32_t* __restrict__ a,
+                         int32_t* __restrict__ b, int pitch, int64_t first_id)
+{
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= k) return;
+    const int32_t x = xy[2 * i], y = xy[2 * i + 1];
+    ix[i] = x;
+    iy[i] = y;
+    pos[i] = pack_pos(x + P, y + P);
+    if (!a) return;
+    const size_t o = (size_t)(y + P) * pitch + x + P;
+    a[o] = (int32_t)(first_id + i);
+    b[o] = (int32_t)(first_id + i);
+}
+
 // ---- batch validation (before any change), on the raster as scratch ----
 // Out-of-bounds seeds are recorded and skipped; each in-bounds seed's cell
 // is reset to "no seed yet".
@@ -928,16 +946,23 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
 
     ++d->generation;
     // coordinates in insertion order, or (order 1) this batch in (x, y) order
+    const size_t plane = (size_t)d->pitch * d->Hd;
+    // into an empty object the propagation is one from scratch: its fixed point
+    // is read off the exact diagram (ties by insertion id)
+    const bool direct = d->mode == IDL_MODE_REFERENCE && n0 == 0 && C.direct() && !timings;
+    bool put = false;   // the seeds' cells are written
     if (order == 0) {
-        k_split<<<gk, 256, 0, C.stream>>>(b_xy, k, d->ix + n0, d->iy + n0);
+        put = d->mode == IDL_MODE_REFERENCE && !direct;
+        k_append<<<gk, 256, 0, C.stream>>>(b_xy, k, d->P, d->ix + n0, d->iy + n0, d->pos + n0,
+                                           put ? d->planes : nullptr, d->planes + plane, d->pitch, n0);
         IDL_LAUNCH();
     } else {
         k_split<<<gk, 256, 0, C.stream>>>(b_xy, k, b_tx, b_ty);
         IDL_LAUNCH();
         rank_seeds_device(C, d->W, d->H, b_tx, b_ty, k, 0, b_rank, b_inv, d->ix + n0, d->iy + n0);
+        k_pack_pos<<<gk, 256, 0, C.stream>>>(d->ix + n0, d->iy + n0, k, d->P, d->pos + n0);
+        IDL_LAUNCH();
     }
-    k_pack_pos<<<gk, 256, 0, C.stream>>>(d->ix + n0, d->iy + n0, k, d->P, d->pos + n0);
-    IDL_LAUNCH();
     const size_t hn = d->hx.size();
     d->hx.resize(hn + k);
     d->hy.resize(hn + k);
@@ -985,11 +1010,8 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
             d->planes, d->planes + (size_t)d->pitch * d->Hd, d->pitch, d->Wd, d->inv);
         IDL_LAUNCH();
     } else {
-        const size_t plane = (size_t)d->pitch * d->Hd;
         bool done = false;
-        if (n0 == 0 && C.direct() && !timings) {
-            // into an empty object the propagation is one from scratch: read its
-            // fixed point off the exact diagram (ties by insertion id)
+        if (direct) {
             ensure_rank(*d);
             d->spos.ensure((size_t)d->N * 4);
             k_pack_pos<<<blocks(d->N), 256, 0, C.stream>>>(d->sx, d->sy, d->N, 0, d->spos.as<uint32_t>());
@@ -1002,8 +1024,10 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
             if (!done) IDL_CUDA(cudaMemsetAsync(d->planes, 0xFF, plane * 8, C.stream));   // empty again
         }
         if (!done) {
-            k_put_seeds<<<gk, 256, 0, C.stream>>>(d->planes, d->planes + plane, d->pitch, d->pos + n0, k, n0);
-            IDL_LAUNCH();
+            if (!put) {
+                k_put_seeds<<<gk, 256, 0, C.stream>>>(d->planes, d->planes + plane, d->pitch, d->pos + n0, k, n0);
+                IDL_LAUNCH();
+            }
             passes = propagate(C, d->mode, d->canvas(), d->pos, n0 + k, d->pos + n0, k);
         }
     }

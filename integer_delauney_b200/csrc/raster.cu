@@ -45,7 +45,7 @@ k_raster_count(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const
     int side = on ? longest_side(u) : 0;
     raster_count<TILE>(w, on, (int32_t)t, u, W, H, 0, tiles_x);
     side = __reduce_max_sync(0xFFFFFFFFu, side);
-    if ((threadIdx.x & 31) == 0 && side > __ldcg(&sc->max_side)) atomicMax(&sc->max_side, side);
+    if ((threadIdx.x & 31) == 0 && side > __ldcg(&w.head->max_side)) atomicMax(&w.head->max_side, side);
     raster_offsets<256>(w);
 }
 
@@ -103,7 +103,7 @@ k_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, 
         const int32_t t = w.lines[i];
         if ((threadIdx.x & 31) == 0)
             raster_line(load_tri(tris + (size_t)t * 5 + 2, xs, ys), tgrid, stride, W, H, t,
-                        max(20, sc->max_side + 3));
+                        max(20, w.head->max_side + 3));
     }
 }
 
@@ -167,7 +167,6 @@ void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys,
     const RasterWork w = raster_work(C, n_tri, tiles);
     const int32_t* tris = C.tris.as<int32_t>();
     if (n_tri > 0) {
-        if (!C.precleared) IDL_CUDA(cudaMemsetAsync(&C.sc()->max_side, 0, sizeof(int32_t), C.stream));
         const unsigned blocks = (unsigned)ceil_div(n_tri, 256);
         k_raster_count<TILE><<<blocks, 256, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, w);
         IDL_LAUNCH();

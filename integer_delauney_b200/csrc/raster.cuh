@@ -235,6 +235,7 @@ struct RasterHead {
     int32_t n_lines;    // collinear triangles
     int32_t done;       // blocks of the count pass that have finished
     int32_t overflow;   // the tile lists do not fit: every triangle goes into the image directly
+    int32_t max_side;   // longest triangle side, float-truncated (triangulation.cu:355-368); single images
 };
 struct RasterWork {
     RasterHead* head;

@@ -761,7 +761,12 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
     uint32_t* b0 = C.bits.as<uint32_t>();
     uint32_t* b1 = b0 + n_words;
     C.counts.ensure(((size_t)max_steps + 2) * 4);
-    IDL_CUDA(cudaMemsetAsync(C.counts.ptr, 0, ((size_t)max_steps + 2) * 4, C.stream));
+    C.gsync.ensure(sizeof(GridSync));
+    ClearList zero;
+    zero.add(C.counts.ptr, ((size_t)max_steps + 2) * 4, 0);
+    zero.add(C.gsync.ptr, sizeof(GridSync), 0);
+    if (!st.marked) zero.add(b0, (size_t)n_words * 2 * 4, 0);
+    clear_buffers(C, zero);
     int32_t* counts = C.counts.as<int32_t>();
     int32_t* l0 = C.tiles[0].as<int32_t>();
     int32_t* l1 = C.tiles[1].as<int32_t>();
@@ -776,13 +781,11 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
         IDL_CUDA(cudaMemcpyAsync(counts, &C.sc()->n_handoff, 4, cudaMemcpyDeviceToDevice, C.stream));
     } else if (st.big_list) {
         if (st.n_big == 0) return 0;
-        IDL_CUDA(cudaMemsetAsync(b0, 0, (size_t)n_words * 2 * 4, C.stream));
         k_expand_tiles<<<(unsigned)st.n_big, 64, 0, C.stream>>>(st.big_list, st.big_tiles_x, st.sub_x, st.sub_y, mt_x,
                                                                 mt_y, b0, l0, counts);
         IDL_LAUNCH();
     } else if (st.seed_pos) {
         if (st.n_new == 0) return 0;
-        IDL_CUDA(cudaMemsetAsync(b0, 0, (size_t)n_words * 2 * 4, C.stream));
         // few seeds: straight into the round mode, whose reach is known here
         // (entering it on the device lists all eight neighbours of each micro-tile)
         start_rounds = st.n_new <= std::max(C.tail_rounds_below, 0);
@@ -792,12 +795,9 @@ int64_t propagate_sparse_impl(Context& C, const Canvas& cv, const uint32_t* pos,
     } else {
         k_fill_bits<<<(unsigned)((n_words + 255) / 256), 256, 0, C.stream>>>(b0, n_words, n_mt);
         IDL_LAUNCH();
-        IDL_CUDA(cudaMemsetAsync(b1, 0, (size_t)n_words * 4, C.stream));
         k_iota_list<<<(unsigned)((n_mt + 255) / 256), 256, 0, C.stream>>>(l0, n_mt, mt_x, counts);
         IDL_LAUNCH();
     }
-    C.gsync.ensure(sizeof(GridSync));
-    IDL_CUDA(cudaMemsetAsync(C.gsync.ptr, 0, sizeof(GridSync), C.stream));
 
     int per_sm = 0;
     const void* kernel = keys ? (const void*)k_sparse_jacobi<true> : (const void*)k_sparse_jacobi<false>;

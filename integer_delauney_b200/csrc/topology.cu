@@ -418,9 +418,11 @@ void detect_launch(Context& C, const Canvas& cv, const int32_t* labels, const ui
     uint32_t* rest = C.grp.as<uint32_t>();
     static_assert(offsetof(Scalars, overflow) == 12 && offsetof(Scalars, n_blocks) == 8, "cleared together");
     if (!C.precleared) {
-        IDL_CUDA(cudaMemsetAsync(table, 0xFF, (size_t)cap * 16, C.stream));
-        IDL_CUDA(cudaMemsetAsync(&C.sc()->n_triangles, 0, 16, C.stream));   // n_triangles, n_blocks, overflow
-        IDL_CUDA(cudaMemsetAsync(cnt, 0, (size_t)(n + 1) * 2 * 4, C.stream));
+        ClearList l;
+        l.add(table, (size_t)cap * 16, 0xFFFFFFFFu);
+        l.add(C.scalars.ptr, 16, 0);   // n_triangles, n_blocks, overflow
+        l.add(cnt, (size_t)(n + 1) * 2 * 4, 0);
+        clear_buffers(C, l);
     }
 
     const int strips = ceil_div(std::max(cv.Wd - 1, 1), DET_COLS);
