@@ -251,8 +251,7 @@ __device__ __forceinline__ void append_fresh(bool want, int target, int32_t pack
 
 // Round mode.  Once the work list is short, the kernel advances RK passes per
 // grid barrier: a warp takes one micro-tile with an RK-cell halo (a 16 x 16
-// region; lane l holds region row l / 2, columns 8 (l % 2) .. + 7, in
-// registers) and runs RK Jacobi passes on it, neighbours by shuffles and
+// region; lane l holds half of region row l / 2 in registers) and runs RK Jacobi passes on it, neighbours by shuffles and
 // region cells beyond the canvas OUTSIDE.  Errors from the region's frozen
 // edge travel one cell per pass, so after RK passes the inner 8 x 8 cells are
 // exact (the light cone of the tile rounds); they go to the other plane.
@@ -299,14 +298,18 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
     const int mx = id & 0xFFFF, my = id >> 16;
     const int mt = my * mt_x + mx;
     if (lane == 0) atomicAnd(&bin[mt >> 5], ~(1u << (mt & 31)));
+    // A lane's cells run from the region's outer edge inwards: columns 0 .. 7 of
+    // the left half, 15 .. 8 of the right one.  Cell j is then right after pass
+    // p only for j > p and needed only there, in both halves: the passes step 7,
+    // 6, 5 and 4 of the 8.
     const int r = lane >> 1, h = lane & 1;
     const int gy = my * MT - RK + r;
-    const int gx0 = mx * MT - RK + 8 * h;
+    const int gx0 = mx * MT - RK + (h ? RR - 1 : 0), step = h ? -1 : 1;
     const bool row_in = gy >= 0 && gy < Hd;
     int32_t c[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-        const int gx = gx0 + j;
+        const int gx = gx0 + step * j;
         c[j] = (row_in && gx >= 0 && gx < Wd) ? __ldcg(cur + (size_t)gy * pitch + gx) : OUTSIDE;
     }
     // ids: their seeds' positions, gathered once and handed on with the labels
@@ -315,72 +318,66 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
     uint32_t cp[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) cp[j] = !KEYS && c[j] >= 0 ? __ldg(&pos[c[j]]) : 0u;
-    // this lane's inner cells: region rows RK .. RK + MT - 1, columns RK .. RK + MT - 1
+    // this lane's inner cells: j = 4 .. 7 of rows RK .. RK + MT - 1
     const bool inner_row = r >= RK && r < RK + MT;
-    // (registers are indexed statically: h picks c[0..3] or c[4..7])
     int32_t c0[4];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) c0[q] = h ? c[q] : c[4 + q];
+    for (int q = 0; q < 4; ++q) c0[q] = c[4 + q];
     int last = -1;
     bool ch = false;   // an inner cell of this lane changed in the latest pass
-#pragma unroll 1
+#pragma unroll
     for (int p = 0; p < RK; ++p) {
-        const int32_t lft = __shfl_up_sync(FULL, c[7], 1), rgt = __shfl_down_sync(FULL, c[0], 1);
-        const uint32_t lft_p = KEYS ? 0u : __shfl_up_sync(FULL, cp[7], 1);
-        const uint32_t rgt_p = KEYS ? 0u : __shfl_down_sync(FULL, cp[0], 1);
-        int32_t nv[8];
-        uint32_t np[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int32_t up = __shfl_up_sync(FULL, c[j], 2), dn = __shfl_down_sync(FULL, c[j], 2);
-            const int32_t L = j > 0 ? c[j - 1] : (h ? lft : OUTSIDE);
-            const int32_t R = j < 7 ? c[j + 1] : (h ? OUTSIDE : rgt);
-            const int32_t U = r > 0 ? up : OUTSIDE;
-            const int32_t D = r < RR - 1 ? dn : OUTSIDE;
-            int32_t b = c[j];
-            if (KEYS) {
-                int32_t k = b;
-                best_of4_keys(k, L, R, U, D, gx0 + j, gy);
-                b = b >= UNDEF ? k : b;
-                np[j] = 0u;
-            } else {
-                const uint32_t Up = __shfl_up_sync(FULL, cp[j], 2), Dp = __shfl_down_sync(FULL, cp[j], 2);
-                const uint32_t Lp = j > 0 ? cp[j - 1] : lft_p, Rp = j < 7 ? cp[j + 1] : rgt_p;
-                int32_t k = b, d = b >= 0 ? dist2(gx0 + j, gy, cp[j]) : FAR;
-                uint32_t kp = cp[j];
-                relax_pos(k, d, kp, L, Lp, gx0 + j, gy);
-                relax_pos(k, d, kp, R, Rp, gx0 + j, gy);
-                relax_pos(k, d, kp, U, Up, gx0 + j, gy);
-                relax_pos(k, d, kp, D, Dp, gx0 + j, gy);
-                np[j] = b >= UNDEF ? kp : cp[j];
-                b = b >= UNDEF ? k : b;
-            }
-            nv[j] = b;
-        }
+        const int32_t mid = __shfl_xor_sync(FULL, c[7], 1);   // across the middle
+        const uint32_t mid_p = KEYS ? 0u : __shfl_xor_sync(FULL, cp[7], 1);
+        int32_t out = c[p];          // the next cell outwards, before this pass
+        uint32_t out_p = cp[p];
         bool moved = false;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) moved = moved || nv[j] != c[j];
         ch = false;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) ch = ch || (h ? nv[q] != c[q] : nv[4 + q] != c[4 + q]);
+        for (int j = p + 1; j < 8; ++j) {
+            const int32_t up = __shfl_up_sync(FULL, c[j], 2), dn = __shfl_down_sync(FULL, c[j], 2);
+            const int32_t in = j < 7 ? c[j + 1] : mid;
+            const int32_t U = r > 0 ? up : OUTSIDE;
+            const int32_t D = r < RR - 1 ? dn : OUTSIDE;
+            const int32_t b = c[j];
+            const int gx = gx0 + step * j;
+            int32_t k = b;
+            if (KEYS) {
+                best_of4_keys(k, out, in, U, D, gx, gy);
+                k = b >= UNDEF ? k : b;
+            } else {
+                const uint32_t bp = cp[j];
+                const uint32_t Up = __shfl_up_sync(FULL, bp, 2), Dp = __shfl_down_sync(FULL, bp, 2);
+                const uint32_t in_p = j < 7 ? cp[j + 1] : mid_p;
+                int32_t d = b >= 0 ? dist2(gx, gy, bp) : FAR;
+                uint32_t kp = bp;
+                relax_pos(k, d, kp, out, out_p, gx, gy);
+                relax_pos(k, d, kp, in, in_p, gx, gy);
+                relax_pos(k, d, kp, U, Up, gx, gy);
+                relax_pos(k, d, kp, D, Dp, gx, gy);
+                k = b >= UNDEF ? k : b;
+                cp[j] = b >= UNDEF ? kp : bp;
+                out_p = bp;
+            }
+            c[j] = k;
+            out = b;
+            moved = moved || k != b;
+            if (j >= 4) ch = ch || k != b;
+        }
         ch = ch && inner_row;
         if (__any_sync(FULL, ch)) last = p;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            c[j] = nv[j];
-            cp[j] = np[j];
-        }
-        if (!__any_sync(FULL, moved)) break;   // nor will the next passes change the region
+        if (!__any_sync(FULL, moved)) break;   // nor will the next passes change what they step
     }
     if (inner_row && gy < Hd) {
-        const int gxi = mx * MT + 4 * h;
 #pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (gxi + q < Wd) nxt[(size_t)gy * pitch + gxi + q] = h ? c[q] : c[4 + q];
+        for (int q = 0; q < 4; ++q) {
+            const int gx = gx0 + step * (4 + q);
+            if (gx < Wd) nxt[(size_t)gy * pitch + gx] = c[4 + q];
+        }
     }
     bool moved = false;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) moved = moved || (h ? c[q] : c[4 + q]) != c0[q];
+    for (int q = 0; q < 4; ++q) moved = moved || c[4 + q] != c0[q];
     if (!__any_sync(FULL, moved && inner_row)) return;
     last_pass = max(last_pass, pass0 + last);
     // quadrants of the inner tile with a change in the last pass: lanes 8..15
