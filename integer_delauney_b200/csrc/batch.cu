@@ -223,7 +223,7 @@ k_b_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc
         int32_t* ids = out + m.px_off * 3 + 2;
         const int32_t id = t - tri_off[im];
         if (!u.line) raster_direct(u, ids, 3, m.W, m.H, id);
-        else if ((threadIdx.x & 31) == 0) raster_line(u, ids, 3, m.W, m.H, id, max(20, side[im] + 3));
+        else raster_line(u, ids, 3, m.W, m.H, id, max(20, side[im] + 3));
     }
 }
 

@@ -101,9 +101,7 @@ k_raster_rest(const int32_t* __restrict__ tris, const Scalars* __restrict__ sc, 
     const int n = w.head->n_lines;
     for (int i = warp; i < n; i += warps) {
         const int32_t t = w.lines[i];
-        if ((threadIdx.x & 31) == 0)
-            raster_line(load_tri(tris + (size_t)t * 5 + 2, xs, ys), tgrid, stride, W, H, t,
-                        max(20, w.head->max_side + 3));
+        raster_line(load_tri(tris + (size_t)t * 5 + 2, xs, ys), tgrid, stride, W, H, t, max(20, w.head->max_side + 3));
     }
 }
 

@@ -159,30 +159,30 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
 }
 
 // A collinear triangle covers the points of its line within the reference's
-// seed window (Chebyshev distance wc of a vertex); one lane.  Pixel ids are
-// `stride` ints apart.
+// seed window (Chebyshev distance wc of a vertex).  A warp, its lanes along the
+// line (a lane alone walked hundreds of rows, 70 us for one such triangle).
+// Pixel ids are `stride` ints apart.
 __device__ __forceinline__ void raster_line(const Tri& t, int32_t* grid, int stride, int W, int H, int32_t tid, int wc)
 {
-    const long long ax = t.x[0], ay = t.y[0], bx = t.x[1], by = t.y[1], cx = t.x[2], cy = t.y[2];
-    const long long lo_y = max(0ll, min(ay, min(by, cy)) - wc);
-    const long long hi_y = min((long long)H - 1, max(ay, max(by, cy)) + wc);
-    for (long long y = lo_y; y <= hi_y; ++y) {
-        long long x_lo, x_hi;
-        if (by == ay) {
-            if (y != ay) continue;
-            x_lo = 0; x_hi = W - 1;
-        } else {
-            const long long num = (bx - ax) * (y - ay);
-            const long long den = by - ay;
-            if (num % den != 0) continue;
-            x_lo = x_hi = ax + num / den;
-        }
-        for (long long x = max(0ll, x_lo); x <= min((long long)W - 1, x_hi); ++x) {
-            const bool near = (llabs(ax - x) <= wc && llabs(ay - y) <= wc) ||
-                              (llabs(bx - x) <= wc && llabs(by - y) <= wc) ||
-                              (llabs(cx - x) <= wc && llabs(cy - y) <= wc);
-            if (near) atomicMax(&grid[((size_t)y * W + x) * stride], tid);
-        }
+    const int lane = threadIdx.x & 31;
+    const int ax = t.x[0], ay = t.y[0], bx = t.x[1], by = t.y[1], cx = t.x[2], cy = t.y[2];
+    auto put = [&](int x, int y) {
+        const bool near = (abs(ax - x) <= wc && abs(ay - y) <= wc) || (abs(bx - x) <= wc && abs(by - y) <= wc) ||
+                          (abs(cx - x) <= wc && abs(cy - y) <= wc);
+        if (near) atomicMax(&grid[((size_t)y * W + x) * stride], tid);
+    };
+    if (by == ay) {
+        if (ay < 0 || ay >= H) return;
+        const int lo = max(0, min(ax, min(bx, cx)) - wc), hi = min(W - 1, max(ax, max(bx, cx)) + wc);
+        for (int x = lo + lane; x <= hi; x += 32) put(x, ay);
+        return;
+    }
+    const int lo = max(0, min(ay, min(by, cy)) - wc), hi = min(H - 1, max(ay, max(by, cy)) + wc);
+    for (int y = lo + lane; y <= hi; y += 32) {
+        const int num = (bx - ax) * (y - ay), den = by - ay;   // below 2^30
+        const int q = num / den;
+        const int x = ax + q;
+        if (q * den == num && x >= 0 && x < W) put(x, y);
     }
 }
 
