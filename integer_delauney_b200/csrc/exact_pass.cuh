@@ -323,38 +323,38 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
     const int s0 = min(W, warp * share), s1 = min(W, s0 + share);
     const unsigned below = (1u << lane) - 1u;
     int kept = 0;
-    // the first test, two columns a lane, against the columns 1, 2 and 4 to
+    // the first test, four columns a lane, against the columns 1, 2 and 4 to
     // either side (at equal distances k it is d_l^2 + d_r^2 + 2 k^2 <= 2 d_x^2)
-    for (int base = s0; base < s1; base += 64) {
-        const int x = base + 2 * lane;
-        uint32_t q[10];   // squares of columns x - 4 .. x + 5; beyond the warp's 64: not there
+    for (int base = s0; base < s1; base += 128) {
+        const int x = base + 4 * lane;
+        uint32_t q[12];   // squares of columns x - 4 .. x + 7; beyond the warp's 128: not there
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < 4; ++c) {
             const int d = x + c < W ? off[x + c] : NO_SEED;
             q[4 + c] = d == NO_SEED ? NO_SQUARE : (uint32_t)(d * d);
         }
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-#pragma unroll
-            for (int j = 1; j <= 2; ++j) {
-                const uint32_t l = __shfl_up_sync(0xFFFFFFFFu, q[4 + c], j);
-                const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, q[4 + c], j);
-                q[4 + c - 2 * j] = lane >= j ? l : NO_SQUARE;
-                q[4 + c + 2 * j] = lane + j < 32 ? r : NO_SQUARE;
-            }
+        for (int c = 0; c < 4; ++c) {
+            const uint32_t l = __shfl_up_sync(0xFFFFFFFFu, q[4 + c], 1);
+            const uint32_t r = __shfl_down_sync(0xFFFFFFFFu, q[4 + c], 1);
+            q[c] = lane > 0 ? l : NO_SQUARE;
+            q[8 + c] = lane < 31 ? r : NO_SQUARE;
         }
-        bool keep[2];
+        int at = s0 + kept, total = 0;
+        bool keep[4];
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
+        for (int c = 0; c < 4; ++c) {
             const uint32_t d = q[4 + c], dd = 2u * d;
             keep[c] = x + c < s1 && d != NO_SQUARE && q[3 + c] + q[5 + c] + 2u + TIE > dd &&
                       q[2 + c] + q[6 + c] + 8u + TIE > dd && q[c] + q[8 + c] + 32u + TIE > dd;
+            const unsigned k = __ballot_sync(0xFFFFFFFFu, keep[c]);
+            at += __popc(k & below);
+            total += __popc(k);
         }
-        const unsigned k0 = __ballot_sync(0xFFFFFFFFu, keep[0]), k1 = __ballot_sync(0xFFFFFFFFu, keep[1]);
-        const int at0 = s0 + kept + __popc(k0 & below) + __popc(k1 & below);
-        if (keep[0]) hx[at0] = (uint16_t)x;
-        if (keep[1]) hx[at0 + (keep[0] ? 1 : 0)] = (uint16_t)(x + 1);
-        kept += __popc(k0) + __popc(k1);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+            if (keep[c]) hx[at++] = (uint16_t)(x + c);
+        kept += total;
     }
     __syncwarp();
     for (int pass = 1; pass < ROW_THIN && kept > 2; ++pass) {
