@@ -140,7 +140,8 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
 //     1024 apart, then 256 apart, then 32 apart bound those in between: the
 //     first two by a warp over the list range, the last by a lane each.
 //  3. A warp takes 32 cells and tests the list between its two bounds, a
-//     broadcast load and four instructions per column.
+//     broadcast load and four instructions per column (unrolled by four, 2 %
+//     of an image over the compiler's choice; by one or two was no better).
 // The work is O(W) per row whatever the seed layout (the ranges of one step
 // add up to the list and one column per cell looked at).  It is bound by
 // instruction issue; a monotone chain per thread in step 1 (its pops diverge)
@@ -196,6 +197,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         const int t = i * ROW_STEP;
         int32_t best = 0x7FFFFFFF;
         int arg = lo, first = 0x7FFFFFFF;
+#pragma unroll 4
         for (int k = lo + lane; k <= hi; k += 32) {
             const int32_t c = cost(k, t);
             if (LABELS && c < best) first = k;
@@ -231,6 +233,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         const int up = i / MID * MID, hi = win[min(up + MID, steps)], t = i * ROW_STEP;
         int arg = low[up], first = arg;
         int32_t best = cost(arg, t);
+#pragma unroll 4
         for (int k = arg + 1; k <= hi; ++k) {
             const int32_t c = cost(k, t);
             if (LABELS && c < best) first = k;
@@ -266,6 +269,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         const int hi = win[i + 1];
         int arg = low[i];
         int32_t best = cost(arg, t);
+#pragma unroll 4
         for (int k = arg + 1; k <= hi; ++k) {
             const int32_t c = cost(k, t);
             if (LABELS ? c < best || (c == best && label_of(k) > label_of(arg)) : c <= best) {
