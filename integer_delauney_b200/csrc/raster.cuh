@@ -83,23 +83,22 @@ __device__ __forceinline__ int div_floor(int p, int q)
 // false if empty.  An edge from u to w keeps A (x - ux) + B (y - uy) >= 0 with
 // A = uy - wy, B = wx - ux; differences of coordinates are below 2^15, so
 // every product fits 32 bits.  OUTER: rounded outwards, so that every point of
-// the real interval at y lies in it.
+// the real interval at y lies in it.  One division per edge whichever side it
+// bounds: lanes of both signs of A share it.
 template <bool OUTER = false>
 __device__ __forceinline__ bool tri_row_span(const Tri& t, int y, int& xl, int& xr)
 {
+    bool in = true;
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
         const int u = e, w = e == 2 ? 0 : e + 1;
         const int A = t.y[u] - t.y[w], c = (t.x[w] - t.x[u]) * (y - t.y[u]);
-        if (A == 0) {
-            if (c < 0) return false;
-        } else if (A > 0) {   // x - ux >= -c / A
-            xl = max(xl, t.x[u] + (OUTER ? div_floor(-c, A) : -div_floor(c, A)));
-        } else {              // x - ux <= c / -A
-            xr = min(xr, t.x[u] + (OUTER ? -div_floor(-c, -A) : div_floor(c, -A)));
-        }
+        const int q = OUTER ? -div_floor(-c, max(abs(A), 1)) : div_floor(c, max(abs(A), 1));
+        if (A > 0) xl = max(xl, t.x[u] - q);    // x - ux >= -c / A
+        if (A < 0) xr = min(xr, t.x[u] + q);    // x - ux <= c / -A
+        in = in && (A != 0 || c >= 0);
     }
-    return xl <= xr;
+    return in && xl <= xr;
 }
 
 // The tiles of a W x H image (tiles_x to a row, the first one tile_off) that a
