@@ -11,7 +11,7 @@
 //
 // Here each triangle rasterises itself instead: for every row its vertices
 // span, the exact integer x-interval of the closed triangle is found from the
-// three edge functions in int64, and atomicMax writes the triangle id into
+// three edge functions in integers, and atomicMax writes the triangle id into
 // every pixel of it.  The window never excludes a pixel of a non-degenerate
 // triangle (any vertex of a triangle is within its longest side of every
 // point inside it, and window_cap exceeds every side), so the result is the
@@ -20,8 +20,8 @@
 // Two details keep it bit-equal:
 //  * The reference's test is float.  For pixel and seed coordinates in
 //    [0, 4096) every product in it is an exact float below 2^24 and the sign
-//    of the difference is exact, so float and int64 agree; beyond that the
-//    int64 test is the exact one.
+//    of the difference is exact, so float and integers agree; beyond that the
+//    integer test is the exact one.
 //  * A degenerate (collinear) triangle passes the closed test at every point
 //    of its supporting line (all three cross products are 0) and nowhere else.
 //    The reference then reaches it only through the window, so such a triangle

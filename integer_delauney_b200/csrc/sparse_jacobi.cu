@@ -415,7 +415,10 @@ __device__ __forceinline__ void round_mt(int32_t id, const int32_t* cur, int32_t
 // time is the latency of its passes: 2 us each in one warp with eight cells a
 // lane.  A block then takes a micro-tile with a BK-cell halo, one cell per
 // thread in shared memory, and runs BK passes at about 0.2 us each.  Same
-// rules as above, with reach BK.
+// rules as above, with reach BK.  An insert of 1 000 seeds into 2 048^2 spends
+// 125 us in this kernel, bound by its chain of rounds (18 of 30 cycles per
+// instruction at a barrier); with these rounds, the positions carried along and
+// the round mode from the start the whole insert takes 217 us instead of 359.
 template <bool KEYS>
 __device__ __forceinline__ void round_block(int32_t id, const int32_t* cur, int32_t* nxt, int pitch, int Wd, int Hd,
                                             int mt_x, int mt_y, const uint32_t* __restrict__ pos, uint32_t* bin,

@@ -189,6 +189,8 @@ __device__ __forceinline__ void detect_block(const int32_t* __restrict__ lab, in
 // a whole warp for the one or two lanes that have a vertex.  A strip with more
 // than DET_OWN of them (a dense blob) leaves the others to k_detect_rest, which
 // spreads them over the device.
+// 46 us at that size (126 with a thread per block), bound by the latency of the
+// loads and of the table's round trips: 25 % of HBM bandwidth, 49 % issue.
 // Canvases too small to fill the device with such strips use shorter ones.
 constexpr int DET_COLS = 128, DET_ROWS = 16, DET_ROWS_SMALL = 4, DET_WARPS = 4, DET_OWN = 96;
 static_assert(DET_ROWS * 4 == 64, "a lane's blocks are the bits of one 64-bit mask");
@@ -383,8 +385,8 @@ __global__ void k_rank(const unsigned long long* __restrict__ ukeys, const unsig
 int64_t detect_capacity(const Context& C, int64_t n)
 {
     // Unique triangles of a planar triangulation number under 2n; the table
-    // starts at four times that (a table half that size probes longer: 70 us
-    // against 53 us of detection at 200 000 seeds), and on the rare probe
+    // starts at four times that (a table half that size probes longer: 17 us
+    // more at 200 000 seeds), and on the rare probe
     // overflow it grows and the detection is redone.  The occupied slots are
     // counted while they are compacted (one atomic per block), not while they
     // are inserted, where a single counter would serialise every new key.
