@@ -139,3 +139,37 @@ def test_first_insert_in_insertion_order(ctx, kind, W, H):
             msg = f"{kind} {W}x{H} seed {seed}"
             np.testing.assert_array_equal(got.get_voronoi_grid(), want.get_voronoi_grid(), err_msg=msg)
             np.testing.assert_array_equal(got.get_triangles(), want.get_triangles(), err_msg=msg)
+
+
+@pytest.mark.parametrize("W,H,kind", [(31, 15, "uniform"), (32, 16, "dense"), (33, 17, "lattice"), (64, 32, "uniform"),
+                                      (65, 33, "dense"), (129, 47, "dense"), (260, 97, "line"), (417, 301, "circle"),
+                                      (1601, 1537, "sparse")])
+def test_detection_strips_and_raster_tiles(W, H, kind):
+    """Triangles and their pixels at the edges of the detection's strips and
+    the raster's tiles (32 x 16, from 1 184 of them up 64 x 32): strips with
+    more vertex blocks than they keep, slivers across many tiles."""
+    seeds = _layout(kind, W, H, 1)
+    tris, grid, _ = oracle.triangulate(W, H, oracle.sort_seeds(seeds, W, H), 8, "reference")
+    verts, got = cu.triangulate(W, H, seeds, border_padding=8, as_arrays=True)
+    np.testing.assert_array_equal(verts, tris[:, 2:5])
+    np.testing.assert_array_equal(got, grid)
+
+
+@pytest.mark.parametrize("dx,dy", [(1, 0), (0, 1), (1, 1), (2, 1), (1, -2), (3, 5)])
+def test_collinear_triangle(dx, dy):
+    """A collinear triangle covers its line within the seed window, whatever
+    the line's direction: a caller's grid in which one block sees three seeds
+    of one line."""
+    W, H = 201, 163
+    x0, y0 = 100 - 10 * dx, 80 - 10 * dy
+    seeds = np.array([(x0, y0), (x0 + 10 * dx, y0 + 10 * dy), (x0 + 18 * dx, y0 + 18 * dy), (199, 161)], np.int32)
+    s = oracle.sort_seeds(seeds, W, H)
+    vg = np.zeros((H, W, 2), np.int32)
+    vg[..., 0] = 2
+    vg[:70, :90, 0] = 0
+    vg[:70, 90:, 0] = 1
+    o_tris, o_grid, _ = oracle.triangulate(W, H, s, 0, "numpy", vgrid=vg)
+    assert len(o_tris) == 1 and (o_grid[..., 2] == 0).sum() > 10
+    tm, grid = cu.GridTriangulation().compute(vg, seeds, 0)
+    assert len(tm) == 1
+    np.testing.assert_array_equal(grid, o_grid)
