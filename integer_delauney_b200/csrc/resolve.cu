@@ -58,9 +58,9 @@
 // Cost at 4096 x 4096, 200 000 uniform seeds: one read of the label plane for
 // the roots (39 us, bound by the latency of its loads), the suspects 12 us, their
 // decisions 30 us (a chain of dependent loads per suspect, 3 034 of them), the
-// writes 4 us.  With the exact diagram's 170 us that is 0.31 ms of
+// writes 4 us.  With the exact diagram's 167 us that is 0.30 ms of
 // propagation; the 51 passes took 1.18 ms.  With 200 000 clustered seeds
-// 0.35 ms, the 1 100 passes 7.8 ms.
+// 0.34 ms, the 1 100 passes 7.8 ms.
 #include "context.cuh"
 #include "exact_pass.cuh"
 #include "stencil.cuh"
