@@ -410,8 +410,11 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     C.pos.ensure((size_t)n * 4);
     C.batch_bad.ensure(16);
     unsigned long long* bad = C.batch_bad.as<unsigned long long>();
-    IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, (size_t)nwords * 4, C.stream));
-    IDL_CUDA(cudaMemsetAsync(bad, 0xFF, 16, C.stream));
+    ClearList zero;
+    zero.add(C.bitmap.ptr, (size_t)nwords * 4, 0);
+    zero.add(bad, 16, 0xFFFFFFFFu);
+    zero.add(reinterpret_cast<char*>(C.sc()) + SCAN_UNIT, 16, 0);
+    clear_buffers(C, zero);
     mark(0);
     k_b_mark<<<nblk(n), 256, 0, C.stream>>>(C.seeds_in.as<int32_t>(), n, C.batch_seed_img.as<int32_t>(), d_imgs,
                                            C.bitmap.as<uint32_t>(), bad);

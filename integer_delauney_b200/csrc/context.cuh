@@ -10,6 +10,7 @@
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <memory>
 #include <mutex>
@@ -109,6 +110,11 @@ struct Scalars {
     int32_t sus_far;          // longest owner distance among the n_more suspects
 };
 constexpr int RESOLVE_SCALARS = 7;
+// The 16-byte unit that holds scan_done, for a clear with other buffers; what
+// else lies in it is set by the runs that read it.
+constexpr size_t SCAN_UNIT = offsetof(Scalars, scan_done);
+static_assert(SCAN_UNIT % 16 == 0 && SCAN_UNIT + 16 == offsetof(Scalars, n_roots),
+              "scan_done, err_label, n_handoff, tile_remaining");
 
 struct Timing {
     cudaEvent_t ev[8] = {};

@@ -97,7 +97,6 @@ struct DelaunayState {
     Context& ctx()
     {
         Context& c = ws ? *ws : own;
-        if (!ws && !own.scalars.ptr) ensure_scalars(own);
         if (c.stream != stream) {
             // the context's last user queued work on another stream: let it
             // finish before this object's work (and stream-ordered frees of
@@ -105,6 +104,9 @@ struct DelaunayState {
             if (ws) IDL_CUDA(cudaStreamSynchronize(c.stream));
             c.stream = stream;
         }
+        // on the object's stream by now: the counters are allocated and cleared
+        // there, ahead of the work that uses them
+        if (!ws && !own.scalars.ptr) ensure_scalars(own);
         if (bound != &c) {
             unbind();
             saved[0] = c.lab[0];

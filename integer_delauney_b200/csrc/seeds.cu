@@ -205,7 +205,11 @@ void rank_seeds_device(Context& C, int W, int H, const int32_t* xs, const int32_
     const int64_t nwords = ((int64_t)W * H + 31) / 32;
     C.bitmap.ensure(size_t(nwords) * 4);
     C.scan_c.ensure(size_t(nwords + 1) * 4);
-    IDL_CUDA(cudaMemsetAsync(C.bitmap.ptr, 0, size_t(nwords) * 4, C.stream));
+    // with the bits, the scan's counter, so that no earlier state of it matters
+    ClearList zero;
+    zero.add(C.bitmap.ptr, size_t(nwords) * 4, 0);
+    zero.add(reinterpret_cast<char*>(C.sc()) + SCAN_UNIT, 16, 0);
+    clear_buffers(C, zero);
     const unsigned gs = (unsigned)((n + 255) / 256);
     k_mark_xy<<<gs, 256, 0, C.stream>>>(xs, ys, n, H, C.bitmap.as<uint32_t>());
     IDL_LAUNCH();
