@@ -15,6 +15,7 @@
 #pragma once
 
 #include "context.cuh"
+#include "held_sum.h"
 
 namespace idl {
 
@@ -284,7 +285,8 @@ __device__ __forceinline__ void raster_count(const RasterWork& w, bool on, int32
 }
 
 // The last block of the count pass turns the counts into list offsets.  Every
-// thread of the block calls it.
+// thread of the block calls it.  The sums are held at SUM_CEILING, above every
+// list_cap: a sum that wrapped round could pass for one that fits.
 template <int T>
 __device__ __forceinline__ void raster_offsets(const RasterWork& w)
 {
@@ -305,35 +307,36 @@ __device__ __forceinline__ void raster_offsets(const RasterWork& w)
         for (int k = 0; k < 4; ++k) {
             const int i = base + threadIdx.x * 4 + k;
             v[k] = i < w.n_tiles ? __ldcg(&w.count[i]) : 0;
-            sum += v[k];
+            sum = held_sum(sum, v[k]);
         }
         int incl = sum;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int u = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-            if (lane >= o) incl += u;
+            if (lane >= o) incl = held_sum(incl, u);
         }
         if (lane == 31) s_warp[warp] = incl;
+        const int before = __shfl_up_sync(0xFFFFFFFFu, incl, 1);
         __syncthreads();
-        int at = s_carry + incl - sum, all = 0;
+        int at = held_sum(s_carry, lane > 0 ? before : 0), all = 0;
 #pragma unroll
         for (int k = 0; k < T / 32; ++k) {
-            at += k < warp ? s_warp[k] : 0;
-            all += s_warp[k];
+            at = held_sum(at, k < warp ? s_warp[k] : 0);
+            all = held_sum(all, s_warp[k]);
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
             const int i = base + threadIdx.x * 4 + k;
             if (i < w.n_tiles) w.off[i] = at;
-            at += v[k];
+            at = held_sum(at, v[k]);
         }
         __syncthreads();
-        if (threadIdx.x == 0) s_carry += all;
+        if (threadIdx.x == 0) s_carry = held_sum(s_carry, all);
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         w.off[w.n_tiles] = s_carry;
-        if (s_carry > w.list_cap || s_carry < 0) w.head->overflow = 1;
+        if (s_carry > w.list_cap) w.head->overflow = 1;
     }
 }
 
