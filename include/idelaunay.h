@@ -99,6 +99,24 @@ IDL_API long long idl_alloc_count(void);
  * usable. */
 IDL_API int idl_selftest_grid_barrier(idl_context* ctx, int missing_arrivals, unsigned int spin_limit);
 
+/* Self-test of what happens where a workspace bound is met.  No counterpart in
+ * the reference.  Sets one of the context's bounds to at most `limit` (0: back
+ * to its own, which grows with the input), so that a small input meets it.
+ * Results do not depend on it. */
+#define IDL_LIMIT_SUSPECTS 0   /* cells resolve.cu lists */
+#define IDL_LIMIT_TRIANGLES 1  /* triangles drawn before their number is known */
+#define IDL_LIMIT_TABLE 2      /* slots detection's hash table starts with */
+#define IDL_LIMIT_TILE_LISTS 3 /* entries of the raster's tile lists */
+#define IDL_LIMIT_COUNT 4
+IDL_API int idl_selftest_limit(idl_context* ctx, int which, int64_t limit);
+/* What the context's runs with IDL_SCHEDULE_DIRECT came to since it was made:
+ * out[IDL_COUNT_*], n = number of slots to fill. */
+#define IDL_COUNT_DIRECT 0  /* stage (a) read off the exact diagram */
+#define IDL_COUNT_PASSES 1  /* not decided: the passes were run */
+#define IDL_COUNT_WINDOWS 2 /* cells decided by iterating a window around them */
+#define IDL_COUNTED 3
+IDL_API int idl_selftest_counts(idl_context* ctx, int64_t* out, int n);
+
 /* ---- context: device, stream, persistent workspace ------------------ */
 /* The reference allocates and frees device buffers on every call
  * (src/cuda/voronoi.cu:87-91, todo.txt); a context owns grow-only workspace

@@ -49,6 +49,8 @@ SIGNATURES = {
     "idl_launch_count": (ctypes.c_longlong, []),
     "idl_alloc_count": (ctypes.c_longlong, []),
     "idl_selftest_grid_barrier": (_i32, [_vp, _i32, ctypes.c_uint]),
+    "idl_selftest_limit": (_i32, [_vp, _i32, _i64]),
+    "idl_selftest_counts": (_i32, [_vp, _pi64, _i32]),
     "idl_context_create": (_i32, [_i32, ctypes.POINTER(_vp)]),
     "idl_context_destroy": (_i32, [_vp]),
     "idl_context_set_stream": (_i32, [_vp, _vp]),

@@ -474,12 +474,12 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
     if (labels_only) {
         if (direct) {
             C.fetch_scalars();
-            if (C.host_sc->resolve_fail) run_passes();
+            if (!resolved(C)) run_passes();
         }
         return;
     }
     detect_triangles(C, cv, C.lab[0].as<int32_t>(), C.pos.as<uint32_t>(), n, 0, timings ? ev[3] : nullptr);
-    if (direct && C.host_sc->resolve_fail) {
+    if (direct && !resolved(C)) {
         // the exact diagram did not decide some image's fixed point: run the passes
         run_passes();
         mark(2);

@@ -262,7 +262,7 @@ bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, int P, bool
 // its pass count, where wanted, is known).
 bool finish_resolved(Context& C, bool want_passes, int64_t* passes = nullptr)
 {
-    if (C.host_sc->resolve_fail) return false;
+    if (!resolved(C)) return false;
     if (!want_passes) return true;
     const int64_t p = resolved_passes(*C.host_sc);
     C.prof.passes = p;
@@ -285,7 +285,7 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     C.prof.prop_bytes = 0;
     // the usual bounds on the hash table and the triangle count (under 2n)
     int64_t cap = detect_capacity(C, n);
-    int64_t bound = 2 * n + 64;
+    const int64_t bound = C.selftest.bound(IDL_LIMIT_TRIANGLES, 2 * n + 64);
     const bool from_grid = vgrid && P == 0;
     C.mark(PM_START);
     const Precleared guard{C};
@@ -411,6 +411,24 @@ int idl_selftest_grid_barrier(idl_context* ctx, int missing_arrivals, unsigned i
     if (!ctx) invalid("context must not be NULL");
     DeviceGuard g(ctx->device);
     grid_barrier_selftest(*ctx, missing_arrivals, spin_limit);
+    IDL_API_END
+}
+
+int idl_selftest_limit(idl_context* ctx, int which, int64_t limit)
+{
+    IDL_API_BEGIN
+    if (!ctx) invalid("context must not be NULL");
+    if (which < 0 || which >= IDL_LIMIT_COUNT) invalid("no such limit");
+    if (limit < 0) invalid("limit must not be negative");
+    ctx->selftest.limit[which] = limit;
+    IDL_API_END
+}
+
+int idl_selftest_counts(idl_context* ctx, int64_t* out, int n)
+{
+    IDL_API_BEGIN
+    if (!ctx || !out) invalid("arguments must not be NULL");
+    for (int i = 0; i < n && i < IDL_COUNTED; ++i) out[i] = ctx->selftest.count[i];
     IDL_API_END
 }
 

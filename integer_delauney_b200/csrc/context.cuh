@@ -121,6 +121,16 @@ struct Timing {
     bool on = false;
 };
 
+// Workspace bounds set smaller than their own by idl_selftest_limit (0: their
+// own), and what idl_selftest_counts reports of the runs since the context was
+// made: how often stage (a) was read off the exact diagram, how often it ran the
+// passes after all, and how many cells the window kernel decided.
+struct SelfTest {
+    int64_t limit[IDL_LIMIT_COUNT] = {};
+    int64_t count[IDL_COUNTED] = {};
+    int64_t bound(int which, int64_t own) const { return limit[which] > 0 ? std::min(limit[which], own) : own; }
+};
+
 // Stage boundaries of the last pipeline run, recorded on the context's stream
 // when profiling is enabled (idl_context_set_profiling).
 enum ProfMark { PM_START = 0, PM_SEEDS, PM_PROPAGATE, PM_DETECT, PM_DEDUP, PM_ASSIGN, PM_COMPOSE, PM_COUNT };
@@ -220,6 +230,7 @@ struct Context {
 
     Timing timing;
     Profile prof;
+    SelfTest selftest;
 
     void mark(ProfMark m)
     {
@@ -382,6 +393,8 @@ XImg whole_canvas(const Canvas& cv, int64_t n, int P);
 void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes,
                    const XImg* images = nullptr, const int32_t* seed_img = nullptr,
                    const uint32_t* sorted = nullptr, const int32_t* label = nullptr);
+// After a read-back of the scalars: whether resolve_exact's labels stand.
+bool resolved(Context& C);
 // The iteration's pass count from the scalars read back after resolve_exact
 // with `passes`, or -1 if they do not determine it.
 inline int64_t resolved_passes(const Scalars& s)

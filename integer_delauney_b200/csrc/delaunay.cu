@@ -1022,7 +1022,7 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
             resolve_exact(C, d->canvas(), d->pos, d->N, false, nullptr, nullptr, d->spos.as<uint32_t>(), d->inv);
             IDL_CUDA(cudaMemcpyAsync(d->planes + plane, d->planes, plane * 4, cudaMemcpyDeviceToDevice, C.stream));
             C.fetch_scalars();
-            done = !C.host_sc->resolve_fail;
+            done = resolved(C);
             if (!done) IDL_CUDA(cudaMemsetAsync(d->planes, 0xFF, plane * 8, C.stream));   // empty again
         }
         if (!done) {

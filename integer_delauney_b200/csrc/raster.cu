@@ -113,14 +113,14 @@ constexpr size_t HEAD_BYTES = 256;
 
 // at 200 000 uniform seeds a triangle meets 1.6 tiles; long slivers of
 // clustered sets meet more, far fewer than this on average
-int64_t list_capacity(int64_t nt, int64_t n_tiles)
+int64_t list_capacity(const Context& C, int64_t nt, int64_t n_tiles)
 {
-    return std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30);
+    return C.selftest.bound(IDL_LIMIT_TILE_LISTS, std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30));
 }
 
 size_t work_reserve(Context& C, int64_t nt, int64_t n_tiles)
 {
-    C.rbig.ensure(HEAD_BYTES + ((size_t)n_tiles * 2 + 1 + (size_t)nt * 4 + (size_t)list_capacity(nt, n_tiles)) * 4);
+    C.rbig.ensure(HEAD_BYTES + ((size_t)n_tiles * 2 + 1 + (size_t)nt * 4 + (size_t)list_capacity(C, nt, n_tiles)) * 4);
     return HEAD_BYTES + (size_t)n_tiles * 4;
 }
 
@@ -147,7 +147,7 @@ RasterWork raster_work(Context& C, int64_t nt, int64_t n_tiles)
     w.xy = reinterpret_cast<uint32_t*>(w.lines + nt);
     w.list = reinterpret_cast<int32_t*>(w.xy + nt * 3);
     w.n_tiles = (int32_t)n_tiles;
-    w.list_cap = (int32_t)list_capacity(nt, n_tiles);
+    w.list_cap = (int32_t)list_capacity(C, nt, n_tiles);
     w.max_tri = (int32_t)nt;
     if (!C.precleared) IDL_CUDA(cudaMemsetAsync(base, 0, zero, C.stream));
     return w;

@@ -696,6 +696,15 @@ __global__ void k_resolve_apply(int32_t* __restrict__ lab, int pitch, const int3
 
 }  // namespace
 
+bool resolved(Context& C)
+{
+    const Scalars& s = *C.host_sc;
+    int64_t* count = C.selftest.count;
+    ++count[s.resolve_fail ? IDL_COUNT_PASSES : IDL_COUNT_DIRECT];
+    if (!s.resolve_fail) count[IDL_COUNT_WINDOWS] += s.n_open;
+    return !s.resolve_fail;
+}
+
 size_t resolve_reserve(Context& C, const Canvas& cv)
 {
     const size_t bits = (size_t)ceil_div(cv.Wd, 32) * cv.Hd * 4;
@@ -710,7 +719,8 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     const size_t bits = resolve_reserve(C, cv);
     // suspects: 0.02 % of the cells at the usual densities (at most 0.4 % in
     // the densest sets measured); beyond the lists the iteration takes over
-    const int cap = (int)std::min<int64_t>((int64_t)cv.Wd * cv.Hd / 64 + 4096, 1 << 22);
+    const int cap = (int)C.selftest.bound(IDL_LIMIT_SUSPECTS,
+                                          std::min<int64_t>((int64_t)cv.Wd * cv.Hd / 64 + 4096, 1 << 22));
     C.sus_list.ensure((size_t)cap * 3 * 4);
     int32_t* list = C.sus_list.as<int32_t>();
     int32_t* res = list + cap;

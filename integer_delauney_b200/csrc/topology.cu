@@ -390,7 +390,8 @@ int64_t detect_capacity(const Context& C, int64_t n)
     // overflow it grows and the detection is redone.  The occupied slots are
     // counted while they are compacted (one atomic per block), not while they
     // are inserted, where a single counter would serialise every new key.
-    return std::max<int64_t>(next_pow2(8 * n + 1024), C.hash_cap);
+    const int64_t cap = std::max<int64_t>(next_pow2(8 * n + 1024), C.hash_cap);
+    return next_pow2(C.selftest.bound(IDL_LIMIT_TABLE, cap));
 }
 
 void detect_reserve(Context& C, int64_t n, int64_t cap)
