@@ -37,6 +37,22 @@ def random_seeds(W, H, n, seed, margin=0):
     return _uniform(W, H, n, seed, margin)
 
 
+@pytest.fixture(autouse=True)
+def shared_context_defaults(request):
+    """After a GPU test, the process-wide contexts are back at their defaults,
+    whatever the test left on them: the tests that follow run the default
+    schedule."""
+    yield
+    if request.node.get_closest_marker("gpu") is None:
+        return
+    from integer_delauney_b200 import _capi
+    for c in _capi._contexts.values():
+        c.set_schedule(_capi.SCHEDULE_DIRECT)
+        c.set_tile(9)
+        c.set_tail_rounds(4096)
+        c.set_profiling(False)
+
+
 @pytest.fixture(scope="session")
 def golden_dir():
     return os.path.join(ROOT, "tests", "golden")
