@@ -107,7 +107,8 @@ IDL_API int idl_selftest_grid_barrier(idl_context* ctx, int missing_arrivals, un
 #define IDL_LIMIT_TRIANGLES 1  /* triangles drawn before their number is known */
 #define IDL_LIMIT_TABLE 2      /* slots detection's hash table starts with */
 #define IDL_LIMIT_TILE_LISTS 3 /* entries of the raster's tile lists */
-#define IDL_LIMIT_COUNT 4
+#define IDL_LIMIT_OPEN 4       /* cells left to windows around them */
+#define IDL_LIMIT_COUNT 5
 IDL_API int idl_selftest_limit(idl_context* ctx, int which, int64_t limit);
 /* What the context's runs with IDL_SCHEDULE_DIRECT came to since it was made:
  * out[IDL_COUNT_*], n = number of slots to fill. */

@@ -50,7 +50,8 @@
 //      cells whose label can still matter to p at a time when it is not known
 //      (k_resolve_window).  If such cells reach the
 //      window's edge, or a list overflows, resolve_fail is raised and the
-//      caller runs the pass-by-pass propagation instead.
+//      caller runs the pass-by-pass propagation instead; the kernels that
+//      follow, and what is left of the one at work, then end at once.
 //
 // Rules (1) and (2) are checked against the iteration on uniform, clustered,
 // lattice, line and circle seed sets by the tests, on the CPU and the GPU.
@@ -219,7 +220,11 @@ k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32
 __global__ void __launch_bounds__(128)
 k_suspects(View V, uint32_t* sus, int32_t* list, int cap, Scalars* sc)
 {
-    const int n = min(sc->n_roots, cap);
+    const int n = sc->n_roots;
+    if (n > cap) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) sc->resolve_fail = 1;
+        return;
+    }
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         constexpr int DEPTH = 24;
         uint32_t stack[DEPTH];
@@ -246,10 +251,13 @@ k_suspects(View V, uint32_t* sus, int32_t* list, int cap, Scalars* sc)
                 if (atomicOr(&sus[(size_t)y * V.words + (x >> 5)], bit) & bit) continue;
                 __threadfence();
                 const int k = n + atomicAdd(&sc->n_more, 1);
-                if (k < cap) list[k] = (int32_t)pack_pos(x, y);
+                if (k < cap && top < DEPTH) {
+                    list[k] = (int32_t)pack_pos(x, y);
+                    stack[top++] = pack_pos(x, y);
+                } else {
+                    sc->resolve_fail = 1;
+                }
                 atomicMax(&sc->sus_far, abs(x - pos_x(p)) + abs(y - pos_y(p)));
-                if (top < DEPTH) stack[top++] = pack_pos(x, y);
-                else sc->resolve_fail = 1;
             }
         }
     }
@@ -266,6 +274,13 @@ constexpr int MAX_FRONT = 4;    // line cells per step (2 are reached)
 // reached with clustered seeds; beyond it the suspect stays undecided, so that
 // no seed set makes a warp run long.
 constexpr int BUDGET = 1 << 14;
+
+// resolve_fail as it is now, the same for all lanes of the warp.
+__device__ __forceinline__ bool raised(const Scalars* sc, int lane)
+{
+    const int v = lane == 0 ? __ldcg(&sc->resolve_fail) : 0;
+    return __shfl_sync(FULL, v, 0) != 0;
+}
 
 struct WarpScratch {
     int32_t cand[MAX_CAND], rival[2][MAX_CAND];
@@ -451,17 +466,20 @@ __device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, 
 }
 
 // One warp per suspect.  res[i] takes the final label, or -1 with i appended
-// to `open` for the window kernel.  The time of p's last change is at least
+// to `open` (at most open_cap) for the window kernel.  The time of p's last change is at least
 // its label's L1 distance (sc->arrive_max) and at most sc->late_max.
 __global__ void __launch_bounds__(RES_WARPS * 32)
-k_resolve(View V, const int32_t* __restrict__ list, int cap, int32_t* __restrict__ res, int32_t* __restrict__ open,
-          Scalars* __restrict__ sc)
+k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, int32_t* __restrict__ open,
+          int open_cap, Scalars* __restrict__ sc)
 {
     __shared__ WarpScratch scratch[RES_WARPS];
     WarpScratch& S = scratch[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    const int n = min(sc->n_roots + sc->n_more, cap);
-    for (int i = blockIdx.x * RES_WARPS + (threadIdx.x >> 5); i < n; i += gridDim.x * RES_WARPS) {
+    if (raised(sc, lane)) return;
+    const int n = sc->n_roots + sc->n_more;
+    const int first = blockIdx.x * RES_WARPS + (threadIdx.x >> 5);
+    for (int i = first; i < n; i += gridDim.x * RES_WARPS) {
+        if (i != first && raised(sc, lane)) return;
         const uint32_t pk = (uint32_t)list[i];
         const int px = pos_x(pk), py = pos_y(pk);
         const XImg b = image_of(V, label_at(V, px, py));
@@ -534,7 +552,9 @@ k_resolve(View V, const int32_t* __restrict__ list, int cap, int32_t* __restrict
                 atomicMax(&sc->arrive_max, t_lo);
                 atomicMax(&sc->late_max, t_hi);
             } else {
-                open[atomicAdd(&sc->n_open, 1)] = i;
+                const int at = atomicAdd(&sc->n_open, 1);
+                if (at < open_cap) open[at] = i;
+                else sc->resolve_fail = 1;
             }
         }
         __syncwarp();
@@ -556,7 +576,7 @@ constexpr size_t WIN_SMEM = (size_t)WIN_N * (4 * 4 + 2 * 2);
 constexpr int32_t FOREVER = 1 << 28;
 
 __global__ void __launch_bounds__(WIN_THREADS)
-k_resolve_window(View V, const int32_t* __restrict__ list, const int32_t* __restrict__ open, int cap,
+k_resolve_window(View V, const int32_t* __restrict__ list, const int32_t* __restrict__ open,
                  int32_t* __restrict__ res, Scalars* __restrict__ sc)
 {
     extern __shared__ __align__(16) int32_t win[];
@@ -566,9 +586,12 @@ k_resolve_window(View V, const int32_t* __restrict__ list, const int32_t* __rest
     volatile int32_t* need = st1 + WIN_N;
     uint16_t* arr = reinterpret_cast<uint16_t*>(st1 + 2 * WIN_N);   // A, 0xFFFF for a suspect
     uint16_t* first = arr + WIN_N;      // no label before this time
-    __shared__ int s_t0, s_t1, s_bad;
-    const int n = min(sc->n_open, cap);
+    __shared__ int s_t0, s_t1, s_bad, s_stop;
+    const int n = sc->n_open;   // beyond the list only with resolve_fail raised
     for (int it = blockIdx.x; it < n; it += gridDim.x) {
+        if (threadIdx.x == 0) s_stop = __ldcg(&sc->resolve_fail);
+        __syncthreads();
+        if (s_stop) return;
         const int i = open[it];
         const uint32_t pk = (uint32_t)list[i];
         const int ox = (int)pos_x(pk) - WIN / 2, oy = (int)pos_y(pk) - WIN / 2;
@@ -683,11 +706,10 @@ k_resolve_window(View V, const int32_t* __restrict__ list, const int32_t* __rest
 }
 
 __global__ void k_resolve_apply(int32_t* __restrict__ lab, int pitch, const int32_t* __restrict__ list,
-                                const int32_t* __restrict__ res, int cap, Scalars* __restrict__ sc)
+                                const int32_t* __restrict__ res, const Scalars* __restrict__ sc)
 {
-    const int total = sc->n_roots + sc->n_more;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && total > cap) sc->resolve_fail = 1;
-    const int n = min(total, cap);
+    if (sc->resolve_fail) return;
+    const int n = sc->n_roots + sc->n_more;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t p = (uint32_t)list[i];
         if (res[i] >= 0) lab[(size_t)pos_y(p) * pitch + pos_x(p)] = res[i];
@@ -742,8 +764,11 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     const int gs = std::max(1, std::min(ceil_div(cap, 128), C.num_sms));
     k_suspects<<<gs, 128, 0, C.stream>>>(V, sus, list, cap, C.sc());
     IDL_LAUNCH();
-    k_resolve<<<std::min(ceil_div(cap, RES_WARPS), C.num_sms * 8), RES_WARPS * 32, 0, C.stream>>>(V, list, cap, res,
-                                                                                              open, C.sc());
+    // a window takes up to a millisecond, the passes a few at most: beyond four
+    // windows per SM the passes take over
+    const int open_cap = (int)C.selftest.bound(IDL_LIMIT_OPEN, std::min(cap, C.num_sms * 4));
+    k_resolve<<<std::min(ceil_div(cap, RES_WARPS), C.num_sms * 8), RES_WARPS * 32, 0, C.stream>>>(V, list, res, open,
+                                                                                              open_cap, C.sc());
     IDL_LAUNCH();
     static std::atomic<uint64_t> opted{0};   // the shared-memory opt-in is per device
     const uint64_t bit = 1ull << (C.device & 63);
@@ -752,9 +777,9 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
                                       (int)WIN_SMEM));
         opted.fetch_or(bit, std::memory_order_acq_rel);
     }
-    k_resolve_window<<<std::min(cap, C.num_sms), WIN_THREADS, WIN_SMEM, C.stream>>>(V, list, open, cap, res, C.sc());
+    k_resolve_window<<<std::min(open_cap, C.num_sms), WIN_THREADS, WIN_SMEM, C.stream>>>(V, list, open, res, C.sc());
     IDL_LAUNCH();
-    k_resolve_apply<<<gs, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, list, res, cap, C.sc());
+    k_resolve_apply<<<gs, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, list, res, C.sc());
     IDL_LAUNCH();
 }
 

@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
 cu = pytest.importorskip("integer_delauney_b200._delauney_cuda")
 from integer_delauney_b200 import _capi  # noqa: E402
 
-SUSPECTS, TRIANGLES, TABLE, TILE_LISTS = range(4)
+SUSPECTS, TRIANGLES, TABLE, TILE_LISTS, OPEN = range(5)
 W, H, P = 301, 203, 8
 
 
@@ -178,3 +178,29 @@ def test_windows_decide_cells(ctx, radius):
         assert windows > 0 and passes == 0
     else:
         assert passes > 0
+
+
+def test_too_many_windows_run_the_passes(ctx):
+    """Circles that leave more than one cell to windows, with room for one."""
+    lib = _capi.load()
+    several = 0
+    for n in range(40, 400, 9):
+        a = np.linspace(0, 2 * np.pi, n, endpoint=False)
+        p = np.stack([np.rint(70 + 40 * np.cos(a)), np.rint(70 + 40 * np.sin(a))], 1).astype(np.int32)
+        seeds = np.ascontiguousarray(np.unique(p, axis=0))
+        want, _ = oracle.voronoi("reference", 141, 141, oracle.sort_seeds(seeds, 141, 141))
+        got = np.empty((141, 141, 2), np.int32)
+        for limit in (0, 1):
+            _limit(ctx, OPEN, limit)
+            before = np.array(_counts(ctx))
+            _capi.check(lib.idl_voronoi(ctx.handle, 141, 141, seeds.ctypes.data, len(seeds), _capi.MODE_REFERENCE,
+                                        got.ctypes.data, None))
+            np.testing.assert_array_equal(got, want, err_msg=f"{n} {limit}")
+            direct, passes, windows = np.array(_counts(ctx)) - before
+            if limit == 0:
+                open_cells = windows
+                assert passes == 0
+            else:
+                assert passes == (open_cells > 1) and windows == (open_cells if open_cells <= 1 else 0)
+        several += open_cells > 1
+    assert several > 0
