@@ -177,7 +177,7 @@ struct Context {
     DevBuf bits;          // work-list dedup bitmaps of the persistent propagation kernel
     DevBuf big_tiles;     // tile rounds' last work list, handed to the persistent kernel
     DevBuf cellbits;      // cell-list tile rounds: three last-pass change bitmaps, in rotation
-    DevBuf exact_bands;   // exact mode: per band of rows and column, its first seed (exact_pass.cuh)
+    DevBuf exact_bands;   // exact diagram: per band of rows and column, its seeds (exact_pass.cuh)
     DevBuf sus_bits, sus_list;  // resolve.cu: suspect bits, suspect list with results and open indices
     int32_t stamp_epoch = 0;
     // propagation schedule from scratch (resolve.cu, propagate.cu; idl_context_set_schedule)

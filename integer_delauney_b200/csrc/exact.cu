@@ -32,15 +32,16 @@ namespace {
 
 __global__ void __launch_bounds__(64)
 k_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, XImg m, int pitch, int16_t* __restrict__ off,
-             int32_t* __restrict__ bands)
+             uint4* __restrict__ bands)
 {
     const int c = (blockIdx.x * 64 + threadIdx.x) * 2;
     if (c < m.Wp) x_column_pair(pos, ranks, m, c, blockIdx.y, pitch, off, bands);
 }
 
 __global__ void __launch_bounds__(64)
-k_bx_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, const XImg* __restrict__ xi, const int32_t* __restrict__ pair_img,
-                int n_pairs, int pitch, int16_t* __restrict__ off, int32_t* __restrict__ bands)
+k_bx_column_off(const uint32_t* __restrict__ pos, SeedRanks ranks, const XImg* __restrict__ xi,
+                const int32_t* __restrict__ pair_img, int n_pairs, int pitch, int16_t* __restrict__ off,
+                uint4* __restrict__ bands)
 {
     const int g = blockIdx.x * 64 + threadIdx.x;
     if (g >= n_pairs) return;
@@ -58,24 +59,22 @@ __global__ void k_bx_tables(const XImg* __restrict__ xi, int32_t* __restrict__ p
 
 template <int T, bool LABELS>
 __global__ void __launch_bounds__(T)
-k_row_win(const int16_t* __restrict__ off, XImg m, int pitch, const uint32_t* __restrict__ pos,
-          const int32_t* __restrict__ bands, const int32_t* __restrict__ label, int32_t* __restrict__ lab,
+k_row_win(const int16_t* __restrict__ off, XImg m, int pitch, SeedBands seeds, int32_t* __restrict__ lab,
           int list_bytes)
 {
     const int y = blockIdx.x;
-    x_row<T, LABELS>(off + (size_t)y * pitch, y, m, pos, bands, label, lab + (size_t)y * pitch, list_bytes);
+    x_row<T, LABELS>(off + (size_t)y * pitch, y, m, seeds, lab + (size_t)y * pitch, list_bytes);
 }
 
 template <int T>
 __global__ void __launch_bounds__(T)
 k_bx_row_win(const int16_t* __restrict__ off, const XImg* __restrict__ xi, const int32_t* __restrict__ row_img,
-             int pitch, const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-             int32_t* __restrict__ lab, int list_bytes)
+             int pitch, SeedBands seeds, int32_t* __restrict__ lab, int list_bytes)
 {
     const XImg m = xi[row_img[blockIdx.x]];
     const int y = m.oy + (int)blockIdx.x - m.row_off;
     const size_t o = (size_t)y * pitch + m.ox;
-    x_row<T, false>(off + o, y, m, pos, bands, nullptr, lab + o, list_bytes);
+    x_row<T, false>(off + o, y, m, seeds, lab + o, list_bytes);
 }
 
 template <class K, class... A>
@@ -84,7 +83,7 @@ void launch_rows(Context& C, K kernel, std::atomic<uint64_t>& opted, unsigned ro
     // the shared-memory opt-in is per device
     const uint64_t bit = 1ull << (C.device & 63);
     if (!(opted.load(std::memory_order_acquire) & bit)) {
-        IDL_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 64));
+        IDL_CUDA(cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - 256));
         opted.fetch_or(bit, std::memory_order_acq_rel);
     }
     kernel<<<rows, threads, smem, C.stream>>>(args...);
@@ -125,22 +124,22 @@ void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t 
     C.lab[0].ensure(plane);
     C.lab[1].ensure(plane);
     const XImg m = whole_canvas(cv, n, P);
-    C.exact_bands.ensure((size_t)x_bands(m) * cv.Wd * 4);
+    C.exact_bands.ensure((size_t)x_bands(m) * cv.Wd * sizeof(uint4));
     int16_t* off = C.lab[1].as<int16_t>();
-    int32_t* bands = C.exact_bands.as<int32_t>();
+    uint4* bands = C.exact_bands.as<uint4>();
     const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), label};
-    k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, ranks, m, cv.pitch, off,
-                                                                                               bands);
+    const SeedBands seeds{bands, label};
+    k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, ranks, m, cv.pitch,
+                                                                                               off, bands);
     IDL_LAUNCH();
     static std::atomic<uint64_t> opted[2][4];
     const int16_t* o = off;
-    const int32_t* t = bands;
     if (label)
         rows_for_width(C, cv.Wd, (unsigned)cv.Hd, opted[1], [](auto T) { return k_row_win<T(), true>; }, o, m, cv.pitch,
-                       pos, t, label, C.lab[0].as<int32_t>());
+                       seeds, C.lab[0].as<int32_t>());
     else
         rows_for_width(C, cv.Wd, (unsigned)cv.Hd, opted[0], [](auto T) { return k_row_win<T(), false>; }, o, m,
-                       cv.pitch, pos, t, label, C.lab[0].as<int32_t>());
+                       cv.pitch, seeds, C.lab[0].as<int32_t>());
     if (C.prof.enabled) {
         C.prof.passes = 0;
         C.prof.rounds = 2;
@@ -156,16 +155,17 @@ void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, in
 {
     k_bx_tables<<<(unsigned)n_images, 256, 0, C.stream>>>(xi, pair_img, row_img);
     IDL_LAUNCH();
-    C.exact_bands.ensure((size_t)band_entries * 4);
     int16_t* off = C.lab[1].as<int16_t>();
-    int32_t* bands = C.exact_bands.as<int32_t>();
+    C.exact_bands.ensure((size_t)band_entries * sizeof(uint4));
+    uint4* bands = C.exact_bands.as<uint4>();
     const SeedRanks ranks{C.bitmap.as<uint32_t>(), C.scan_c.as<int32_t>(), nullptr};
+    const SeedBands seeds{bands, nullptr};
     k_bx_column_off<<<dim3((unsigned)ceil_div(n_pairs, 64), (unsigned)ceil_div(max_hp, BAND)), 64, 0, C.stream>>>(
         pos, ranks, xi, pair_img, n_pairs, pitch, off, bands);
     IDL_LAUNCH();
     static std::atomic<uint64_t> opted[4];
     rows_for_width(C, max_wp, (unsigned)n_rows, opted, [](auto T) { return k_bx_row_win<T()>; }, (const int16_t*)off, xi,
-                   (const int32_t*)row_img, pitch, pos, (const int32_t*)bands, C.lab[0].as<int32_t>());
+                   (const int32_t*)row_img, pitch, seeds, C.lab[0].as<int32_t>());
 }
 
 }  // namespace idl

@@ -4,7 +4,7 @@
 //
 // Column pass: each cell's signed row offset to the nearest seed of its own
 // column (ties to the lower one, the higher id), two bytes per cell, and a
-// small table that turns (column, row of a seed) into the seed's id.
+// table that turns (column, row of a seed) into the seed's id.
 // Row pass: each cell's winner among its row's column candidates, and its id.
 #pragma once
 
@@ -35,63 +35,83 @@ struct SeedRanks {
     const int32_t* label;   // label of each rank, ties going to the higher label; null: the rank itself
 };
 
-// First of the image's seeds at or after (x, y) in (x, y) order: two loads,
-// where a search of the sorted seeds takes one round trip to L2 per halving
-// (most of the column pass's time on a small image).
-__device__ __forceinline__ int x_lower_bound(const SeedRanks& R, const XImg& m, int x, int y)
-{
-    const int W = m.Wp - 2 * m.P, H = m.Hp - 2 * m.P;
-    const int c = x - m.ox - m.P;
-    if (c < 0) return m.s0;
-    if (c >= W) return m.s1;
-    const long long bit = m.bit0 + (long long)c * H + min(max(y - m.oy - m.P, 0), H);
-    if (bit >= m.bit0 + (long long)W * H) return m.s1;
-    const uint32_t below = __ldg(&R.bits[bit >> 5]) & ((1u << (bit & 31)) - 1u);
-    return __ldg(&R.before[bit >> 5]) + __popc(below);
-}
+// Per band of rows and column: its seeds in the band as a 64-bit mask of the
+// rows (z, w) and the rank of the first of them (x).
+struct SeedBands {
+    const uint4* band;
+    const int32_t* label;   // as in SeedRanks
+};
 
-// Id of the seed at (x, y) of the plane, which must exist: bands holds, per
-// band of rows and column, the first seed at or below the band's first row.
-__device__ __forceinline__ int32_t x_seed_at(const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-                                             const XImg& m, int x, int y)
+// Rank of the seed at (x, y) of the plane, which must exist.  One load however
+// dense the seeds: a walk along the column's seeds from the band's first one
+// took ten loads in a row per cell at one seed in three cells (row pass of
+// 2048 x 2048: 291 us, now 88; at 200 000 seeds in 4096 x 4096 134 and 130
+// us), and the occupancy bits and their ranks, two loads from column-major
+// tables, 147 us there.
+__device__ __forceinline__ int32_t x_seed_at(const SeedBands& B, const XImg& m, int x, int y)
 {
-    int32_t a = __ldg(&bands[m.band_off + (y - m.oy) / BAND * m.Wp + (x - m.ox)]);
-    while (a < m.s1 - 1 && (int)pos_y(__ldg(&pos[a])) < y) ++a;
-    return a;
+    const unsigned row = (unsigned)(y - m.oy), k = row % BAND;
+    const uint4 e = __ldg(&B.band[m.band_off + (int)(row / BAND) * m.Wp + (x - m.ox)]);
+    const uint32_t low = k < 32 ? (1u << k) - 1u : 0xFFFFFFFFu, high = k > 32 ? (1u << (k - 32)) - 1u : 0u;
+    return (int32_t)e.x + __popc(e.z & low) + __popc(e.w & high);
 }
 
 // One thread walks two adjacent columns (the pair starting at image column c)
 // through the rows of one band, so that a warp writes 128 bytes of a row at
-// once; its place in each column's seeds comes from the seeds' ranks.  Two bytes per cell is all that is written (the planes of 4-byte ids
-// and distances this replaces took four times the traffic).
+// once.  The band's seeds of a column come as a 64-bit mask from the occupancy
+// bits, the seeds before and after the band by their ranks: the walk itself
+// loads nothing (dense columns: 24 us instead of 44 at 2048 x 2048, one seed in
+// three cells).  Two bytes per cell and a table entry per 64 are written.
 __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, const SeedRanks& ranks,
                                               const XImg& m, int c, int band,
-                                              int pitch, int16_t* __restrict__ off, int32_t* __restrict__ bands)
+                                              int pitch, int16_t* __restrict__ off, uint4* __restrict__ bands)
 {
+    static_assert(BAND == 64, "a column's rows of a band are the bits of one 64-bit mask");
     const int y0 = band * BAND, y1 = min(m.Hp, y0 + BAND);
-    int a[2], next_y[2], prev_y[2];
+    const int W = m.Wp - 2 * m.P, H = m.Hp - 2 * m.P;
+    const int r0 = min(max(y0 - m.P, 0), H), r1 = min(max(y1 - m.P, 0), H);   // the band's rows of the image proper
+    int a[2], next_y[2], prev_y[2], after_y[2];
+    unsigned long long left[2];   // seeds of the band not passed yet, a bit per row
     bool any[2];
     constexpr int FAR_BELOW = 0x3FFFFFFF, FAR_ABOVE = -0x3FFFFFFF;
 #pragma unroll
     for (int k = 0; k < 2; ++k) {
-        next_y[k] = FAR_BELOW;
+        after_y[k] = FAR_BELOW;
         prev_y[k] = FAR_ABOVE;
-        any[k] = false;
+        left[k] = 0;
         a[k] = 0;
-        if (c + k < m.Wp) {
-            const int x = m.ox + c + k;
-            a[k] = x_lower_bound(ranks, m, x, m.oy + y0);
-            bands[m.band_off + band * m.Wp + c + k] = a[k];
-            if (a[k] < m.s1) {
-                const uint32_t p = __ldg(&pos[a[k]]);
-                if ((int)pos_x(p) == x) next_y[k] = (int)pos_y(p) - m.oy;
+        const int col = c + k - m.P;
+        if (col >= 0 && col < W) {
+            const long long b0 = m.bit0 + (long long)col * H + r0;
+            const long long w0 = b0 >> 5;
+            const int shift = (int)(b0 & 31), n = r1 - r0;
+            if (r0 < H) {
+                const uint32_t first = __ldg(&ranks.bits[w0]);
+                a[k] = __ldg(&ranks.before[w0]) + __popc(first & ((1u << shift) - 1u));
+                unsigned long long v = first >> shift;
+                if (n + shift > 32) v |= (unsigned long long)__ldg(&ranks.bits[w0 + 1]) << (32 - shift);
+                if (n + shift > 64) v |= (unsigned long long)__ldg(&ranks.bits[w0 + 2]) << (64 - shift);
+                if (n < 64) v &= (1ull << n) - 1ull;
+                left[k] = v << (m.P + r0 - y0 & 63);   // n rows from there on: none if the band lies above the image
+            } else {   // below the image proper: the column's seeds are all above
+                const long long end = m.bit0 + (long long)(col + 1) * H - 1, w = end >> 5;
+                a[k] = __ldg(&ranks.before[w]) + __popc(__ldg(&ranks.bits[w]) & (0xFFFFFFFFu >> (31 - (int)(end & 31))));
+            }
+            const int x = m.ox + c + k, b = a[k] + __popcll(left[k]);
+            if (b < m.s1) {
+                const uint32_t p = __ldg(&pos[b]);
+                if ((int)pos_x(p) == x) after_y[k] = (int)pos_y(p) - m.oy;
             }
             if (a[k] > m.s0) {
                 const uint32_t p = __ldg(&pos[a[k] - 1]);
                 if ((int)pos_x(p) == x) prev_y[k] = (int)pos_y(p) - m.oy;
             }
-            any[k] = next_y[k] != FAR_BELOW || prev_y[k] != FAR_ABOVE;
         }
+        if (c + k < m.Wp)
+            bands[m.band_off + band * m.Wp + c + k] =
+                make_uint4((uint32_t)a[k], 0u, (uint32_t)left[k], (uint32_t)(left[k] >> 32));
+        next_y[k] = left[k] ? y0 + __ffsll((long long)left[k]) - 1 : after_y[k];
+        any[k] = next_y[k] != FAR_BELOW || prev_y[k] != FAR_ABOVE;
     }
     int16_t* dst = off + (size_t)(m.oy + y0) * pitch + m.ox + c;
     const bool paired = c + 1 < m.Wp && ((m.ox | pitch) & 1) == 0;   // c is even
@@ -99,13 +119,11 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
         int v[2];
 #pragma unroll
         for (int k = 0; k < 2; ++k) {
-            while (next_y[k] < y) {   // the seed below was passed: it becomes the one above
+            if (next_y[k] < y) {   // the seed below was passed: it becomes the one above
                 prev_y[k] = next_y[k];
-                next_y[k] = FAR_BELOW;
-                if (++a[k] < m.s1) {
-                    const uint32_t p = __ldg(&pos[a[k]]);
-                    if ((int)pos_x(p) == m.ox + c + k) next_y[k] = (int)pos_y(p) - m.oy;
-                }
+                left[k] &= left[k] - 1;
+                next_y[k] = left[k] ? y0 + __ffsll((long long)left[k]) - 1 : after_y[k];
+                ++a[k];
             }
             const int below = next_y[k] - y, above = y - prev_y[k];   // tie: the larger y, the higher rank
             bool down = below <= above;
@@ -149,9 +167,12 @@ __device__ __forceinline__ void x_column_pair(const uint32_t* __restrict__ pos, 
 // idle.
 // Shared memory is 8 bytes per column, so that enough rows share an SM: the
 // offsets, the columns' list, and room for W / 2 list entries with their F; a
-// longer list (seed sets denser than one in ten cells) holds columns only and
-// works F out again each time.  Rows of more than ROW_WIDE columns get 6 bytes
-// per column, room for W / 4 entries.
+// longer list (seed sets denser than one in ten cells, or a line of seeds across
+// the image) keeps F and the columns in arrays of their own, and each cell looks
+// its id up for itself (with F worked out again each time, 88 us instead of 71 at
+// 2048 x 2048, one seed in three cells).  Rows of more than ROW_WIDE columns get 6 bytes per
+// column, room for W / 4 entries; their longer lists hold columns only and work
+// F out again each time.
 constexpr int ROW_STEP = 32, ROW_MID = 256, ROW_TOP = 1024;
 constexpr int ROW_THIN = 5;    // thinning passes at most
 constexpr int ROW_WIDE = 27000;
@@ -182,9 +203,8 @@ inline int row_pass_threads(int W, unsigned rows)
 template <int T, bool LABELS, class Cost>
 __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* listx, uint16_t* buf, uint16_t* hx,
                                            uint16_t* win, uint16_t* win_lo, const int16_t* off, int n, int W, int y,
-                                           const XImg& m, const uint32_t* __restrict__ pos,
-                                           const int32_t* __restrict__ bands, const int32_t* __restrict__ label,
-                                           int32_t* __restrict__ out, Cost cost, bool packed)
+                                           const XImg& m, const SeedBands& seeds, int32_t* __restrict__ out,
+                                           Cost cost, bool packed)
 {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = T / 32;
@@ -192,7 +212,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         if (T == 32) __syncwarp();
         else __syncthreads();
     };
-    auto name = [&](int32_t rank) { return LABELS ? __ldg(&label[rank]) : rank; };
+    auto name = [&](int32_t rank) { return LABELS ? __ldg(&seeds.label[rank]) : rank; };
     auto by_warp = [&](int i, int lo, int hi) {
         const int t = i * ROW_STEP;
         int32_t best = 0x7FFFFFFF;
@@ -251,7 +271,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
         for (int k = tid; k < n; k += T) hx[k] = (uint16_t)off[list2[k].y / -2];
         sync();
         for (int k = tid; k < n; k += T) {
-            const int32_t id = name(x_seed_at(pos, bands, m, m.ox + list2[k].y / -2, y + (int16_t)hx[k]));
+            const int32_t id = name(x_seed_at(seeds, m, m.ox + list2[k].y / -2, y + (int16_t)hx[k]));
             buf[k] = (uint16_t)(id & 0xFFFF);
             hx[k] = (uint16_t)(id >> 16);
         }
@@ -260,7 +280,7 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
     auto label_of = [&](int k) -> int32_t {
         if (packed) return (int32_t)buf[k] | (int32_t)hx[k] << 16;
         const int x = listx[k];
-        return name(x_seed_at(pos, bands, m, m.ox + x, y + off[x]));
+        return name(x_seed_at(seeds, m, m.ox + x, y + off[x]));
     };
 
     // 3. every cell, from the list between its interval's bounds
@@ -284,9 +304,8 @@ __device__ __forceinline__ void x_row_fill(const int2* list2, const uint16_t* li
 // row: the row's offsets; y: its row on the plane; out: its labels;
 // list_bytes: row_list_bytes of the launch.
 template <int T, bool LABELS>
-__device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, const XImg& m,
-                                      const uint32_t* __restrict__ pos, const int32_t* __restrict__ bands,
-                                      const int32_t* __restrict__ label, int32_t* __restrict__ out, int list_bytes)
+__device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, const XImg& m, const SeedBands& seeds,
+                                      int32_t* __restrict__ out, int list_bytes)
 {
     extern __shared__ __align__(16) unsigned char row_smem[];
     __shared__ int s_sum[T / 32 + 1];
@@ -412,13 +431,21 @@ __device__ __forceinline__ void x_row(const int16_t* __restrict__ row, int y, co
         return;
     }
     if (packed) {
-        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, pos, bands, label, out,
+        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, seeds, out,
                               [&](int k, int t) {
             const int2 c = list2[k];
             return c.x + t * c.y;
         }, true);
+    } else if (list_bytes == 4) {   // room for any list: the columns move on to hx, F takes their place
+        int32_t* listf = reinterpret_cast<int32_t*>(row_smem);
+        for (int k = tid; k < n; k += T) hx[k] = listx[k];
+        sync();
+        for (int k = tid; k < n; k += T) listf[k] = value(hx[k]);
+        sync();
+        x_row_fill<T, LABELS>(list2, hx, buf, hx, win, win_lo, off, n, W, y, m, seeds, out,
+                              [&](int k, int t) { return listf[k] - 2 * t * (int)hx[k]; }, false);
     } else {
-        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, pos, bands, label, out,
+        x_row_fill<T, LABELS>(list2, listx, buf, hx, win, win_lo, off, n, W, y, m, seeds, out,
                               [&](int k, int t) {
             const int x = listx[k];
             return value(x) - 2 * t * x;

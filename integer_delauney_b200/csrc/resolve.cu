@@ -74,10 +74,9 @@ namespace {
 struct View {
     const int32_t* lab;      // exact labels
     const int16_t* off;      // column pass: row offset to the nearest seed of the cell's column
-    const int32_t* bands;    // and its table
+    SeedBands seeds;         // and its table
     const uint32_t* pos;     // seed positions by label
     const uint32_t* sorted;  // and by (x, y) rank
-    const int32_t* label;    // label of each rank; null: the rank itself
     const uint32_t* sus;     // suspect bits, rows of `words` words
     const XImg* images;      // batch: image table, else null
     const int32_t* seed_img; // batch: image of each seed
@@ -307,14 +306,14 @@ __device__ __forceinline__ void for_better(const View& V, int x, int y, int32_t 
         for (int j = 0; j < 4; ++j) {
             const int xx = x0 + 32 * j;
             if (o[j] == NO_SEED || (long long)o[j] * o[j] + (long long)(xx - x) * (xx - x) > d) continue;
-            const int32_t c = x_seed_at(V.sorted, V.bands, b, xx, y + o[j]);
+            const int32_t c = x_seed_at(V.seeds, b, xx, y + o[j]);
             for (int step = 1; step >= -1; step -= 2) {
                 for (int32_t r = step > 0 ? c : c - 1; r >= b.s0 && r < b.s1; r += step) {
                     const uint32_t p = __ldg(&V.sorted[r]);
                     if ((int)pos_x(p) != xx) break;   // past the column's run
                     const int32_t dm = dist2(x, y, p);
                     if (dm > d) break;
-                    const int32_t m = V.label ? __ldg(&V.label[r]) : r;
+                    const int32_t m = V.seeds.label ? __ldg(&V.seeds.label[r]) : r;
                     if (m != s && beats(dm, m, d, s) && !f(m, p)) return;
                 }
             }
@@ -752,8 +751,8 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
         IDL_CUDA(cudaMemsetAsync(sus, 0, bits, C.stream));
         IDL_CUDA(cudaMemsetAsync(&C.sc()->n_roots, 0, RESOLVE_SCALARS * sizeof(int32_t), C.stream));
     }
-    const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), C.exact_bands.as<int32_t>(), pos,
-                 sorted ? sorted : pos, label, sus, images,
+    const View V{C.lab[0].as<int32_t>(), C.lab[1].as<int16_t>(), SeedBands{C.exact_bands.as<uint4>(), label}, pos,
+                 sorted ? sorted : pos, sus, images,
                  seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n, 0)};
     const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 4 * ROOT_ROWS));
     if (passes)
