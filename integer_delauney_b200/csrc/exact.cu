@@ -103,7 +103,8 @@ void rows_for_width(Context& C, int width, unsigned rows, std::atomic<uint64_t>*
     if (threads == 32) go(std::integral_constant<int, 32>{}, 0);
     else if (threads == 64) go(std::integral_constant<int, 64>{}, 1);
     else if (threads == 128) go(std::integral_constant<int, 128>{}, 2);
-    else go(std::integral_constant<int, 256>{}, 3);
+    else if (threads == 256) go(std::integral_constant<int, 256>{}, 3);
+    else go(std::integral_constant<int, 1024>{}, 4);
 }
 
 }  // namespace
@@ -132,7 +133,7 @@ void propagate_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t 
     k_column_off<<<dim3((unsigned)ceil_div(cv.Wd, 128), (unsigned)x_bands(m)), 64, 0, C.stream>>>(pos, ranks, m, cv.pitch,
                                                                                                off, bands);
     IDL_LAUNCH();
-    static std::atomic<uint64_t> opted[2][4];
+    static std::atomic<uint64_t> opted[2][5];
     const int16_t* o = off;
     if (label)
         rows_for_width(C, cv.Wd, (unsigned)cv.Hd, opted[1], [](auto T) { return k_row_win<T(), true>; }, o, m, cv.pitch,
@@ -163,7 +164,7 @@ void exact_images(Context& C, int pitch, const uint32_t* pos, const XImg* xi, in
     k_bx_column_off<<<dim3((unsigned)ceil_div(n_pairs, 64), (unsigned)ceil_div(max_hp, BAND)), 64, 0, C.stream>>>(
         pos, ranks, xi, pair_img, n_pairs, pitch, off, bands);
     IDL_LAUNCH();
-    static std::atomic<uint64_t> opted[4];
+    static std::atomic<uint64_t> opted[5];
     rows_for_width(C, max_wp, (unsigned)n_rows, opted, [](auto T) { return k_bx_row_win<T()>; }, (const int16_t*)off, xi,
                    (const int32_t*)row_img, pitch, seeds, C.lab[0].as<int32_t>());
 }

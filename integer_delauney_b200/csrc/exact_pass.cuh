@@ -187,12 +187,16 @@ inline size_t row_pass_smem(int W)
     const size_t w = (size_t)(W + 7) / 4 * 4;
     return w * (4 + row_list_bytes(W)) + (size_t)(W / ROW_STEP + 3) * 4 + 16;
 }
+// Wide rows too few to fill the device take 32 warps each (one row of 32 767
+// columns: 37 us against 72 with 8; 40 rows of 32 703: 43 against 86).
+constexpr unsigned ROW_FEW = 148;
 // Threads per row: warps of at most ROW_SHARE columns, up to 8 (twice that
 // where there are rows enough to fill the device with fewer warps each: 2 % of
 // a 512-image batch; 192 against 216 us the other way at 4 128 rows).
 inline int row_pass_threads(int W, unsigned rows)
 {
     const int share = rows >= 32768 ? 2 * ROW_SHARE : ROW_SHARE;
+    if (rows <= ROW_FEW && W > 8 * ROW_SHARE) return 1024;
     return W <= share ? 32 : W <= 2 * share ? 64 : W <= 4 * share ? 128 : 256;
 }
 

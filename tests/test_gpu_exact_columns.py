@@ -58,3 +58,13 @@ def test_bands_with_ties_by_insertion(W, H):
         np.testing.assert_array_equal(got.get_triangles(), want.get_triangles())
         del want
     ctx.close()
+
+
+@pytest.mark.parametrize("W,H", [(4224, 148), (4225, 148), (4225, 149), (4300, 1), (27001, 2)])
+@pytest.mark.parametrize("n", [1, 900, 3500])
+def test_wide_rows_that_are_few(W, H, n):
+    """Rows of more than 4 224 columns, up to 148 of them: a block of 32 warps
+    each; one more row or one column less: 8 warps."""
+    seeds = random_seeds(W, H, n, 3)
+    want, _ = oracle.voronoi("exact", W, H, oracle.sort_seeds(seeds, W, H))
+    np.testing.assert_array_equal(cu.Voronoi().compute(W, H, seeds, voronoi_mode="exact"), want)
