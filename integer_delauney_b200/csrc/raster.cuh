@@ -29,6 +29,7 @@ struct Tile {
 using TileLarge = Tile<64, 32>;
 using TileSmall = Tile<32, 16>;
 constexpr int TILE_THREADS = 128;
+constexpr int TILE_FEW = 12;   // tiles of a box a lane lists alone
 inline bool small_tiles(int64_t large_tiles, int num_sms) { return large_tiles < (int64_t)num_sms * 8; }
 
 // Longest side of one triangle as triangulation.cu:357-362 computes it: float
@@ -106,12 +107,37 @@ __device__ __forceinline__ bool tri_row_span(const Tri& t, int y, int& xl, int& 
     return in && xl <= xr;
 }
 
+// The first lane whose inclusive sum exceeds k (sums do not decrease).
+__device__ __forceinline__ int lane_of(int incl, int k)
+{
+    int l = 0;
+#pragma unroll
+    for (int s = 16; s > 0; s >>= 1)
+        if (__shfl_sync(0xFFFFFFFFu, incl, l + s - 1) <= k) l += s;
+    return l;
+}
+
+// Inclusive sum over the warp's lanes.
+__device__ __forceinline__ int warp_prefix(int v)
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xFFFFFFFFu, v, o);
+        if (lane >= o) v += u;
+    }
+    return v;
+}
+
 // The tiles of a W x H image (tiles_x to a row, the first one tile_off) that a
-// proper triangle's pixels can lie in: f(t, tile).  A box of a few tiles is taken whole, by its lane; in
-// a larger one each tile row takes the columns the triangle spans there (its
-// extent in a slab is reached at the slab's ends or at a vertex), a lane per
-// tile row: a sliver across the image is hundreds of tiles.  Every lane of the
-// warp calls it; on: the lane brings triangle u, number t, of a W x H image.
+// proper triangle's pixels can lie in: f(t, tile).  A box of a few tiles is
+// taken whole, by its lane.  In a larger one each tile row takes the columns the
+// triangle spans there (its extent in a slab is reached at the slab's ends or at
+// a vertex); a warp works off the tile rows of its larger triangles 32 at a
+// time, then the tiles of those rows 32 at a time: slivers across the image are
+// hundreds of tiles each, and f waits for memory (one triangle after another,
+// 88 seeds 64 pixels apart took 23 + 36 us to list, now 5 + 4; slivers from side
+// to side of 2048 x 2048 106 us to count, now 8).  Every lane of the warp calls it; on: the lane brings triangle u, number t, of a W x H image.
 template <class TILE, class F>
 __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int W, int H, int tile_off, int tiles_x,
                                           F&& f)
@@ -121,13 +147,17 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
     const int y0 = max(0, min(u.y[0], min(u.y[1], u.y[2]))), y1 = min(H - 1, max(u.y[0], max(u.y[1], u.y[2])));
     on = on && x0 <= x1 && y0 <= y1;
     const int tx0 = x0 / TILE::W, tx1 = x1 / TILE::W, ty0 = y0 / TILE::H, ty1 = y1 / TILE::H;
-    const bool few = on && (tx1 - tx0 + 1) * (ty1 - ty0 + 1) <= 12;
+    const bool few = on && (tx1 - tx0 + 1) * (ty1 - ty0 + 1) <= TILE_FEW;
     if (few)
         for (int ty = ty0; ty <= ty1; ++ty)
             for (int tx = tx0; tx <= tx1; ++tx) f(t, tile_off + ty * tiles_x + tx);
     __syncwarp();
-    for (unsigned m = __ballot_sync(0xFFFFFFFFu, on && !few); m; m &= m - 1) {
-        const int src = __ffs(m) - 1;
+    const int rows = on && !few ? ty1 - ty0 + 1 : 0;
+    if (!__any_sync(0xFFFFFFFFu, rows > 0)) return;
+    const int rows_incl = warp_prefix(rows), total = __shfl_sync(0xFFFFFFFFu, rows_incl, 31);
+    const int first_row = ty0 - (rows_incl - rows);
+    for (int r0 = 0; r0 < total; r0 += 32) {
+        const int r = r0 + lane, src = min(lane_of(rows_incl, r), 31);
         Tri v;
 #pragma unroll
         for (int k = 0; k < 3; ++k) {
@@ -138,15 +168,16 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
                   by0 = __shfl_sync(0xFFFFFFFFu, y0, src), by1 = __shfl_sync(0xFFFFFFFFu, y1, src);
         const int32_t id = __shfl_sync(0xFFFFFFFFu, t, src);
         const int first = __shfl_sync(0xFFFFFFFFu, tile_off, src), per_row = __shfl_sync(0xFFFFFFFFu, tiles_x, src);
-        for (int ty = by0 / TILE::H + lane; ty <= by1 / TILE::H; ty += 32) {
+        const int ty = r + __shfl_sync(0xFFFFFFFFu, first_row, src);
+        int lo = bx1 + 1, hi = bx0 - 1;
+        if (r < total) {
             const int ya = max(by0, ty * TILE::H), yb = min(by1, ty * TILE::H + TILE::H - 1);
-            int lo = bx1 + 1, hi = bx0 - 1;
 #pragma unroll
             for (int k = 0; k < 2; ++k) {
-                int l = bx0, r = bx1;
-                if (tri_row_span<true>(v, k ? yb : ya, l, r)) {
+                int l = bx0, q = bx1;
+                if (tri_row_span<true>(v, k ? yb : ya, l, q)) {
                     lo = min(lo, l);
-                    hi = max(hi, r);
+                    hi = max(hi, q);
                 }
             }
 #pragma unroll
@@ -155,10 +186,16 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
                     lo = min(lo, max(v.x[k], bx0));
                     hi = max(hi, min(v.x[k], bx1));
                 }
-            if (lo > hi) continue;
-            for (int tx = lo / TILE::W; tx <= hi / TILE::W; ++tx) f(id, first + ty * per_row + tx);
         }
-        __syncwarp();
+        const int tiles = lo <= hi ? hi / TILE::W - lo / TILE::W + 1 : 0;
+        const int tiles_incl = warp_prefix(tiles), all = __shfl_sync(0xFFFFFFFFu, tiles_incl, 31);
+        const int first_tile = first + ty * per_row + lo / TILE::W - (tiles_incl - tiles);
+        for (int e0 = 0; e0 < all; e0 += 32) {
+            const int e = e0 + lane, from = min(lane_of(tiles_incl, e), 31);
+            const int32_t of = __shfl_sync(0xFFFFFFFFu, id, from);
+            const int tile = e + __shfl_sync(0xFFFFFFFFu, first_tile, from);
+            if (e < all) f(of, tile);
+        }
     }
 }
 
@@ -354,16 +391,6 @@ __device__ __forceinline__ void raster_fill(const RasterWork& w, bool on, int32_
     tri_tiles<TILE>(on, u, t, W, H, tile_off, tiles_x, [&](int32_t id, int tile) {
         w.list[w.off[tile] + atomicSub(&w.count[tile], 1) - 1] = id;
     });
-}
-
-// The first lane whose inclusive sum exceeds k (sums do not decrease).
-__device__ __forceinline__ int lane_of(int incl, int k)
-{
-    int l = 0;
-#pragma unroll
-    for (int s = 16; s > 0; s >>= 1)
-        if (__shfl_sync(0xFFFFFFFFu, incl, l + s - 1) <= k) l += s;
-    return l;
 }
 
 // One tile of a W x H image, by a block: pix[TILE::H * TILE::PITCH] takes the
