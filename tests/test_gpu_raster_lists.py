@@ -42,3 +42,31 @@ def test_triangles_across_many_tiles(W, H, kind):
     seeds = np.unique(seeds.astype(np.int32), axis=0)
     np.random.default_rng(1).shuffle(seeds)
     _check(W, H, np.ascontiguousarray(seeds))
+
+
+@pytest.mark.parametrize("side,n,limit", [(64, 40, 0), (64, 40, 1), (200, 300, 0), (200, 300, 700)])
+def test_overlapping_triangles_of_a_callers_grid(side, n, limit):
+    """A grid of labelled squares in no order: more triangles than twice the
+    seeds, on top of each other, drawn by their lists and (limit) without."""
+    import ctypes
+    from integer_delauney_b200 import _capi
+    rng = np.random.default_rng(side)
+    seeds = random_seeds(side, side, n, 2)
+    s = oracle.sort_seeds(seeds, side, side)
+    vg = np.zeros((side, side, 2), np.int32)
+    vg[..., 0] = rng.integers(0, n, (side // 4 + 1, side // 4 + 1)).repeat(4, 0).repeat(4, 1)[:side, :side]
+    o_tris, o_grid, _ = oracle.triangulate(side, side, s, 0, "numpy", vgrid=vg)
+    assert len(o_tris) > 2 * n + 64
+    ctx = _capi.Context(0)
+    lib = _capi.load()
+    _capi.check(lib.idl_selftest_limit(ctx.handle, 3, limit))
+    grid = np.empty((side, side, 3), np.int32)
+    count = ctypes.c_int64()
+    for _ in range(2):
+        _capi.check(lib.idl_triangulate(ctx.handle, side, side, seeds.ctypes.data, n, vg.ctypes.data, 0,
+                                        _capi.MODE_REFERENCE, grid.ctypes.data, ctypes.byref(count), None, None))
+        np.testing.assert_array_equal(grid, o_grid)
+        tris = np.empty((count.value, 5), np.int32)
+        _capi.check(lib.idl_get_triangles(ctx.handle, tris.ctypes.data, count.value))
+        np.testing.assert_array_equal(tris, o_tris)
+    ctx.close()
