@@ -273,6 +273,7 @@ constexpr int MAX_FRONT = 4;    // line cells per step (2 are reached)
 // reached with clustered seeds; beyond it the suspect stays undecided, so that
 // no seed set makes a warp run long.
 constexpr int BUDGET = 1 << 14;
+constexpr int LONG_SPENT = 256;
 
 // resolve_fail as it is now, the same for all lanes of the warp.
 __device__ __forceinline__ bool raised(const Scalars* sc, int lane)
@@ -285,6 +286,7 @@ struct WarpScratch {
     int32_t cand[MAX_CAND], rival[2][MAX_CAND];
     uint32_t seen[2][MAX_SEARCH];
     int n, n_rival, budget;
+    const Scalars* sc;
 };
 
 // Offers every seed m of the image that beats (d, s) at (x, y) to f(m); a lane
@@ -354,6 +356,8 @@ __device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int 
     if (lane == 0) {
         S.n_rival = 0;
         S.budget -= 1 + (isqrt(d) >> 4);
+        // a long decision (3 % of them with clustered seeds) ends with the others
+        if (S.budget < BUDGET - LONG_SPENT && __ldcg(&S.sc->resolve_fail)) S.budget = -1;
     }
     __syncwarp();
     if (S.budget < 0) return MAX_CAND + 1;
@@ -476,9 +480,31 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
     const int lane = threadIdx.x & 31;
     if (raised(sc, lane)) return;
     const int n = sc->n_roots + sc->n_more;
-    const int first = blockIdx.x * RES_WARPS + (threadIdx.x >> 5);
-    for (int i = first; i < n; i += gridDim.x * RES_WARPS) {
-        if (i != first && raised(sc, lane)) return;
+    const int first = blockIdx.x * RES_WARPS + (threadIdx.x >> 5), warps = gridDim.x * RES_WARPS;
+    if (lane == 0) S.sc = sc;
+    auto leave_open = [&](int i) {
+        const int at = atomicAdd(&sc->n_open, 1);
+        if (at < open_cap) open[at] = i;
+        else sc->resolve_fail = 1;
+    };
+    // More suspects than warps: those without a settled neighbour go first, since
+    // too many of them end the run.
+    const bool ahead = n > warps;
+    if (ahead) {
+        for (int i = first * 32 + lane; i < n; i += warps * 32) {
+            const uint32_t pk = (uint32_t)list[i];
+            bool settled = false;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int x = (int)pos_x(pk) + (j == 0) - (j == 1), y = (int)pos_y(pk) + (j == 2) - (j == 3);
+                settled = settled || (label_at(V, x, y) >= 0 && !suspect_at(V, x, y));
+            }
+            if (!settled) leave_open(i);
+        }
+        __syncwarp();
+    }
+    for (int i = first; i < n; i += warps) {
+        if (ahead && raised(sc, lane)) return;
         const uint32_t pk = (uint32_t)list[i];
         const int px = pos_x(pk), py = pos_y(pk);
         const XImg b = image_of(V, label_at(V, px, py));
@@ -550,10 +576,8 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
                 const int t_lo = l1_to(V, px, py, out);
                 atomicMax(&sc->arrive_max, t_lo);
                 atomicMax(&sc->late_max, t_hi);
-            } else {
-                const int at = atomicAdd(&sc->n_open, 1);
-                if (at < open_cap) open[at] = i;
-                else sc->resolve_fail = 1;
+            } else if (f >= 0 || !ahead) {
+                leave_open(i);
             }
         }
         __syncwarp();
@@ -570,6 +594,7 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
 // their owner from A on and nothing before, which is right whenever asked.
 constexpr int WIN = 96;
 constexpr int WIN_THREADS = 512;
+static_assert(4 * WIN <= WIN_THREADS, "a thread per cell of the window's sides");
 constexpr int WIN_N = WIN * WIN;
 constexpr size_t WIN_SMEM = (size_t)WIN_N * (4 * 4 + 2 * 2);
 constexpr int32_t FOREVER = 1 << 28;
@@ -635,6 +660,17 @@ k_resolve_window(View V, const int32_t* __restrict__ list, const int32_t* __rest
                 }
             }
             if (!__syncthreads_or(ch)) break;
+            if (sweep % 8 == 7) {   // a stepped cell at the window's edge: found again below, no need to go on
+                bool edge = threadIdx.x == 0 && __ldcg(&sc->resolve_fail);
+                if (threadIdx.x < 4 * WIN) {
+                    const int side = threadIdx.x / WIN, at = threadIdx.x % WIN;
+                    const int cx = side == 0 ? 0 : side == 1 ? WIN - 1 : at, cy = side == 2 ? 0 : side == 3 ? WIN - 1 : at;
+                    edge = edge || (need[cy * WIN + cx] >= 0 &&
+                                    label_at(V, ox + cx + (side == 1) - (side == 0),
+                                             oy + cy + (side == 3) - (side == 2)) >= 0);
+                }
+                if (__syncthreads_or(edge)) break;
+            }
         }
         // the stepped cells must lie inside the window; their time span
         for (int c = threadIdx.x; c < WIN_N; c += WIN_THREADS) {
@@ -763,9 +799,10 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     const int gs = std::max(1, std::min(ceil_div(cap, 128), C.num_sms));
     k_suspects<<<gs, 128, 0, C.stream>>>(V, sus, list, cap, C.sc());
     IDL_LAUNCH();
-    // a window takes up to a millisecond, the passes a few at most: beyond four
-    // windows per SM the passes take over
-    const int open_cap = (int)C.selftest.bound(IDL_LIMIT_OPEN, std::min(cap, C.num_sms * 4));
+    // a window takes up to a millisecond, the passes a few at most: a batch gets
+    // four windows per SM; an image with more than a few (seeds on a wide circle,
+    // a hundred and more) does not fit them either
+    const int open_cap = (int)C.selftest.bound(IDL_LIMIT_OPEN, std::min(cap, images ? C.num_sms * 4 : 64));
     k_resolve<<<std::min(ceil_div(cap, RES_WARPS), C.num_sms * 8), RES_WARPS * 32, 0, C.stream>>>(V, list, res, open,
                                                                                               open_cap, C.sc());
     IDL_LAUNCH();

@@ -204,3 +204,26 @@ def test_too_many_windows_run_the_passes(ctx):
                 assert passes == (open_cells > 1) and windows == (open_cells if open_cells <= 1 else 0)
         several += open_cells > 1
     assert several > 0
+
+
+@pytest.mark.parametrize("kind", ["lines", "circle"])
+def test_more_suspects_than_warps(ctx, kind):
+    """Tens of thousands of cells cut off: between slanted lines of seeds, all
+    decided; in a wide circle, many of them without a settled neighbour."""
+    W, H = 900, 800
+    if kind == "lines":
+        t = np.arange(W)
+        p = np.concatenate([np.stack([t, np.rint(t * 0.37 + k * H / 6)], 1) for k in range(6)])
+    else:
+        a = np.linspace(0, 2 * np.pi, 8000, endpoint=False)
+        p = np.stack([np.rint(W / 2 + 350 * np.cos(a)), np.rint(H / 2 + 350 * np.sin(a))], 1)
+    p = p[(p[:, 0] >= 0) & (p[:, 0] < W) & (p[:, 1] >= 0) & (p[:, 1] < H)]
+    seeds = np.ascontiguousarray(np.unique(p.astype(np.int32), axis=0))
+    want, want_passes = oracle.voronoi("reference", W, H, oracle.sort_seeds(seeds, W, H))
+    got = np.empty((H, W, 2), np.int32)
+    passes = ctypes.c_int64()
+    _capi.check(_capi.load().idl_voronoi(ctx.handle, W, H, seeds.ctypes.data, len(seeds), _capi.MODE_REFERENCE,
+                                         got.ctypes.data, ctypes.byref(passes)))
+    np.testing.assert_array_equal(got, want)
+    assert passes.value == want_passes
+    assert _counts(ctx)[:2] == ((1, 0) if kind == "lines" else (0, 1))
