@@ -247,7 +247,7 @@ struct Context {
         DevBuf* all[] = {&seeds_in, &xs, &ys, &pos, &bitmap, &scan_a, &scan_c, &lab[0], &lab[1],
                          &tiles[0], &tiles[1], &stamps, &counts, &gsync, &trace, &rbig, &bits, &big_tiles, &cellbits,
                          &exact_bands, &sus_bits, &sus_list, &hkeys,
-                         &ukeys, &uvals, &cnt, &off, &grp, &tris, &tgrid, &vgrid, &outgrid, &padded,
+                         &ukeys, &uvals, &cnt, &off, &grp, &tris, &verts, &tgrid, &vgrid, &outgrid, &padded,
                          &batch_img, &batch_seed_img, &batch_stats, &batch_bad,
                          &batch_ximg, &batch_colimg, &batch_rowimg, &scalars};
         for (DevBuf* b : all) f(*b);
