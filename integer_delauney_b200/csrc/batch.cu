@@ -377,6 +377,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
                float* timings, bool labels_only = false, int mode = IDL_MODE_REFERENCE)
 {
     C.batch_plan.reset();
+    C.owner = nullptr;
     const int64_t n = pl.n_seeds;
     C.batch_img.ensure(pl.imgs.size() * sizeof(BImg));
     C.batch_seed_img.ensure((size_t)n * 4);

@@ -97,6 +97,7 @@ void clear_buffers(Context& C, const ClearList& l)
 
 void clear_for_run(Context& C, const Canvas& cv, int W, int H, int64_t n, bool suspects, int64_t cap, int64_t n_tri)
 {
+    C.owner = nullptr;   // the counters are the run's from here on
     ClearList l;
     const size_t bitmap = ((size_t)W * H + 31) / 32 * 4;
     C.bitmap.ensure(bitmap);

@@ -223,7 +223,9 @@ struct Context {
     Scalars* host_sc = nullptr;  // pinned mirror
     bool host_sc_borrowed = false;  // host_sc points at static storage, not cudaMallocHost memory
 
-    const void* owner = nullptr; // object whose intermediates the buffers hold (shared workspaces)
+    // Object whose triangle rows and count the buffers hold (shared workspaces);
+    // every other run on the context clears it.
+    const void* owner = nullptr;
     std::shared_ptr<void> batch_plan;  // layout of the last batch (batch.cu)
     int64_t last_n_tri = 0;      // triangles of the last triangulation (host copy)
     bool have_result = false;

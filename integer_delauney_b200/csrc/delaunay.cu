@@ -615,6 +615,7 @@ void ensure_topology(DelaunayState& D, float* timings)
     if (D.N < 3) {
         D.n_tri = 0;
     } else {
+        C.have_result = false;   // a triangulation's rows on a shared workspace are overwritten
         cudaEvent_t e[3] = {};
         if (timings)
             for (auto& ev : e) IDL_CUDA(cudaEventCreate(&ev));

@@ -30,3 +30,48 @@ def test_vertex_triples_are_part_of_the_workspace():
     _capi.check(_capi.load().idl_get_triangle_vertices(ctx.handle, verts.ctypes.data, n))
     assert ctx.workspace_bytes() >= before + 12 * n
     ctx.close()
+
+
+def test_calls_on_a_context_between_calls_of_an_object_that_borrows_it():
+    """The triangles and counters an object left on the context are not taken
+    for its own after the context has served another call, nor the other way
+    round."""
+    lib = _capi.load()
+    ctx = _capi.Context(0)
+    W, H = 300, 200
+    seeds = random_seeds(W, H, 700, 3)
+    ref = cu.Delaunay(W, H, 1000, 16)
+    ref.insert_deferred(seeds)
+    want_tris, want_grid = ref.get_triangles(), ref.finalise(as_arrays=True)[1]
+    other = random_seeds(120, 90, 50, 4)
+    vor = np.empty((90, 120, 2), np.int32)
+    dims, counts = np.array([[120, 90]], np.int32), np.array([50], np.int64)
+
+    def voronoi():
+        _capi.check(lib.idl_voronoi(ctx.handle, 120, 90, other.ctypes.data, 50, _capi.MODE_REFERENCE, vor.ctypes.data,
+                                    None))
+
+    def batch():
+        _capi.check(lib.idl_triangulate_batch(ctx.handle, 1, dims.ctypes.data, counts.ctypes.data, other.ctypes.data,
+                                              16, _capi.MODE_REFERENCE, None, None, None))
+
+    def labels():
+        _capi.check(lib.idl_voronoi_batch(ctx.handle, 1, dims.ctypes.data, counts.ctypes.data, other.ctypes.data, 16,
+                                          _capi.MODE_REFERENCE))
+
+    for between in (voronoi, lambda: _triangulate(ctx, 120, 90, 50), batch, labels):
+        d = cu.Delaunay(W, H, 1000, 16)
+        d.use_workspace(ctx)
+        d.insert_deferred(seeds)
+        np.testing.assert_array_equal(d.get_triangles(), want_tris)
+        between()
+        np.testing.assert_array_equal(d.finalise(as_arrays=True)[1], want_grid)
+        between()
+        np.testing.assert_array_equal(d.get_triangles(), want_tris)
+    # the rows on the context are the object's by now
+    _triangulate(ctx, 120, 90, 50)
+    d.get_triangles()
+    rows = np.empty((200, 5), np.int32)
+    assert lib.idl_get_triangles(ctx.handle, rows.ctypes.data, 200) == _capi.IDL_ERR_STATE
+    del d
+    ctx.close()
