@@ -460,7 +460,7 @@ void run_batch(Context& C, const Plan& pl, int P, int n_images, int32_t* d_out, 
         // them are read by the block rule (and by resolve_exact) in plane 0 only
         IDL_CUDA(cudaMemsetAsync(C.lab[0].ptr, 0xFE, plane, C.stream));
         const XImg* xi = exact_atlas(C, pl, P, cv);
-        if (direct) resolve_exact(C, cv, C.pos.as<uint32_t>(), n, false, xi, C.batch_seed_img.as<int32_t>());
+        if (direct) resolve_exact(C, cv, C.pos.as<uint32_t>(), n, xi, C.batch_seed_img.as<int32_t>());
     } else {
         run_passes();
     }

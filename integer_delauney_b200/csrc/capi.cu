@@ -240,16 +240,15 @@ int64_t run_passes(Context& C, int mode, const Canvas& cv, int64_t n)
 }
 
 // Stage (a) from scratch into C.lab[0].  Returns true if the labels come from
-// resolve_exact: the caller has to look at finish_resolved once the scalars
-// have been read back.  Otherwise *passes (may be nullptr) takes the pass count.
-bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, int P, bool want_passes,
-                  int64_t* passes = nullptr)
+// resolve_exact: the caller has to look at resolved() once the scalars have been
+// read back.  Otherwise *passes (may be nullptr) takes the pass count.
+bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, int P, int64_t* passes = nullptr)
 {
     if (mode == IDL_MODE_REFERENCE && C.direct()) {
         C.prof.pass_ns.clear();
         C.prof.pass_tiles.clear();
         propagate_exact(C, cv, C.pos.as<uint32_t>(), n, P);
-        resolve_exact(C, cv, C.pos.as<uint32_t>(), n, want_passes);
+        resolve_exact(C, cv, C.pos.as<uint32_t>(), n);
         return true;
     }
     int64_t p = 0;
@@ -259,16 +258,19 @@ bool start_labels(Context& C, int mode, const Canvas& cv, int64_t n, int P, bool
     return false;
 }
 
-// After a read-back of the scalars: whether resolve_exact's labels stand (and
-// its pass count, where wanted, is known).
-bool finish_resolved(Context& C, bool want_passes, int64_t* passes = nullptr)
+// The pass count of labels that stand, after resolve_arrivals and a read-back of
+// the scalars.  Where those do not determine it, the passes are run after all;
+// they reach the same labels, and a profile keeps what it has recorded.
+int64_t count_passes(Context& C, int mode, const Canvas& cv, int64_t n)
 {
-    if (!resolved(C)) return false;
-    if (!want_passes) return true;
-    const int64_t p = resolved_passes(*C.host_sc);
-    C.prof.passes = p;
-    if (passes) *passes = p;
-    return p >= 0;
+    int64_t p = resolved_passes(*C.host_sc);
+    if (p < 0) {
+        const Profile kept = C.prof;
+        C.prof.enabled = false;
+        p = run_passes(C, mode, cv, n);
+        C.prof = kept;
+    }
+    return p;
 }
 
 // Run stages (a) (b) (d) with seeds already in C.seeds_in.  Leaves labels in
@@ -296,7 +298,7 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
 
     bool resolved = false;
     if (!from_grid) {
-        resolved = start_labels(C, mode, cv, n, P, C.prof.enabled);
+        resolved = start_labels(C, mode, cv, n, P);
     } else {
         const size_t gbytes = (size_t)W * H * 2 * sizeof(int32_t);
         C.vgrid.ensure(gbytes);
@@ -338,6 +340,7 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         }
         C.mark(PM_COMPOSE);
         T.mark(4);
+        if (resolved && C.prof.enabled) resolve_arrivals(C, cv, C.pos.as<uint32_t>());
         deliver(cv);
         C.fetch_scalars();
     };
@@ -349,7 +352,8 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     detect(cap);
     assign(bound);
     C.precleared = false;
-    if (resolved && !finish_resolved(C, C.prof.enabled)) {
+    if (resolved && !idl::resolved(C)) {
+        resolved = false;
         run_passes(C, mode, cv, n);
         C.mark(PM_PROPAGATE);
         detect(cap);
@@ -363,6 +367,7 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
     }
     if (C.host_sc->n_triangles > bound) assign(C.host_sc->n_triangles);
     const int64_t nt = C.host_sc->n_triangles;
+    if (resolved && C.prof.enabled) C.prof.passes = count_passes(C, mode, cv, n);
     if (timings) {
         timings[IDL_T_DETECT_MS] = T.ms(0, 1);
         timings[IDL_T_DEDUP_MS] = T.ms(1, 2);
@@ -597,7 +602,7 @@ int idl_voronoi(idl_context* ctx, int width, int height, const int32_t* seeds_xy
     const Precleared guard{C};
     clear_for_run(C, cv, width, height, n_seeds, mode == IDL_MODE_REFERENCE && C.direct(), 0, 0);
     sort_seeds_device(C, width, height, n_seeds, 0);
-    const bool resolved = start_labels(C, mode, cv, n_seeds, 0, passes_out != nullptr, &passes);
+    const bool resolved = start_labels(C, mode, cv, n_seeds, 0, &passes);
     const size_t bytes = (size_t)width * height * 2 * sizeof(int32_t);
     C.outgrid.ensure(bytes);
     auto deliver = [&] {
@@ -609,10 +614,13 @@ int idl_voronoi(idl_context* ctx, int width, int height, const int32_t* seeds_xy
         if (resolved) C.fetch_scalars();
         else IDL_CUDA(cudaStreamSynchronize(C.stream));
     };
+    if (resolved && passes_out) resolve_arrivals(C, cv, C.pos.as<uint32_t>());
     deliver();
-    if (resolved && !finish_resolved(C, passes_out != nullptr, &passes)) {
+    if (resolved && !idl::resolved(C)) {
         passes = run_passes(C, mode, cv, n_seeds);
         deliver();
+    } else if (resolved && passes_out) {
+        passes = count_passes(C, mode, cv, n_seeds);
     }
     if (passes_out) *passes_out = passes;
     IDL_API_END

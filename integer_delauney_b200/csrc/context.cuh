@@ -107,9 +107,8 @@ struct Scalars {
     int32_t resolve_fail;     // the fixed point was not decided: iterate instead
     int32_t arrive_max;       // latest last change known exactly (passes done by then)
     int32_t late_max;         // latest upper bound of a decided suspect's last change
-    int32_t sus_far;          // longest owner distance among the n_more suspects
 };
-constexpr int RESOLVE_SCALARS = 7;
+constexpr int RESOLVE_SCALARS = 6;
 // The 16-byte unit that holds scan_done, for a clear with other buffers; what
 // else lies in it is set by the runs that read it.
 constexpr size_t SCAN_UNIT = offsetof(Scalars, scan_done);
@@ -388,21 +387,22 @@ XImg whole_canvas(const Canvas& cv, int64_t n, int P);
 // Turns the exact labels propagate_exact left in C.lab[0] (and the column
 // plane in C.lab[1]) into the reference semantics' fixed point from scratch
 // (resolve.cu).  Reads nothing back: C.sc()->resolve_fail, with the scalars'
-// next read-back, tells whether the passes have to be run instead.  `passes`:
-// also what resolved_passes needs.  Batch atlas: `images` is the table
+// next read-back, tells whether the passes have to be run instead.  Batch atlas: `images` is the table
 // exact_images used, `seed_img` the image of each seed.  Labels that are not
 // ranks: `pos` by label, `sorted` by rank and the `label` table propagate_exact had.
-void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes,
+void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
                    const XImg* images = nullptr, const int32_t* seed_img = nullptr,
                    const uint32_t* sorted = nullptr, const int32_t* label = nullptr);
 // After a read-back of the scalars: whether resolve_exact's labels stand.
 bool resolved(Context& C);
-// The iteration's pass count from the scalars read back after resolve_exact
-// with `passes`, or -1 if they do not determine it.
+// What the pass count needs besides, by a read of the finished labels: only
+// where the count is wanted, after what is timed.
+void resolve_arrivals(Context& C, const Canvas& cv, const uint32_t* pos);
+// The iteration's pass count from the scalars read back after resolve_arrivals,
+// or -1 if they do not determine it.
 inline int64_t resolved_passes(const Scalars& s)
 {
-    const bool sure = !s.resolve_fail && s.late_max <= s.arrive_max && (s.n_more == 0 || s.sus_far < s.arrive_max);
-    return sure ? (int64_t)s.arrive_max + 1 : -1;
+    return !s.resolve_fail && s.late_max <= s.arrive_max ? (int64_t)s.arrive_max + 1 : -1;
 }
 
 // Reserve a range of per-item stamp values for `steps` steps (propagate.cu).

@@ -952,7 +952,7 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
     const size_t plane = (size_t)d->pitch * d->Hd;
     // into an empty object the propagation is one from scratch: its fixed point
     // is read off the exact diagram (ties by insertion id)
-    const bool direct = d->mode == IDL_MODE_REFERENCE && n0 == 0 && C.direct() && !timings;
+    const bool direct = d->mode == IDL_MODE_REFERENCE && n0 == 0 && C.direct();
     bool put = false;   // the seeds' cells are written
     if (order == 0) {
         put = d->mode == IDL_MODE_REFERENCE && !direct;
@@ -999,7 +999,10 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
     d->pending = true;
 
     Timer T(C, timings != nullptr);
+    float bfs = 0.f;
     int64_t passes = 0;
+    bool count = false;       // the pass count is still to be found
+    bool have_time = false;   // bfs is set
     if (d->mode == IDL_MODE_EXACT) {
         // history-independent: the exact diagram of the whole seed set, in
         // (x, y) ranks (plane 1, which detection reads) and as insertion ids
@@ -1020,21 +1023,29 @@ int idl_delaunay_insert_ordered(idl_delaunay* d, const int32_t* xy, int64_t k, c
             k_pack_pos<<<blocks(d->N), 256, 0, C.stream>>>(d->sx, d->sy, d->N, 0, d->spos.as<uint32_t>());
             IDL_LAUNCH();
             propagate_exact(C, d->canvas(), d->spos.as<uint32_t>(), d->N, d->P, d->inv);
-            resolve_exact(C, d->canvas(), d->pos, d->N, false, nullptr, nullptr, d->spos.as<uint32_t>(), d->inv);
+            resolve_exact(C, d->canvas(), d->pos, d->N, nullptr, nullptr, d->spos.as<uint32_t>(), d->inv);
             IDL_CUDA(cudaMemcpyAsync(d->planes + plane, d->planes, plane * 4, cudaMemcpyDeviceToDevice, C.stream));
             C.fetch_scalars();
             done = resolved(C);
-            if (!done) IDL_CUDA(cudaMemsetAsync(d->planes, 0xFF, plane * 8, C.stream));   // empty again
+            if (done && timings) {   // the time is the insert's; the count comes after it
+                bfs = T.stop();
+                resolve_arrivals(C, d->canvas(), d->pos);
+                C.fetch_scalars();
+                passes = resolved_passes(*C.host_sc);
+                count = passes < 0;
+            }
+            if (!done || count) IDL_CUDA(cudaMemsetAsync(d->planes, 0xFF, plane * 8, C.stream));   // empty again
         }
-        if (!done) {
+        if (!done || count) {
             if (!put) {
                 k_put_seeds<<<gk, 256, 0, C.stream>>>(d->planes, d->planes + plane, d->pitch, d->pos + n0, k, n0);
                 IDL_LAUNCH();
             }
             passes = propagate(C, d->mode, d->canvas(), d->pos, n0 + k, d->pos + n0, k);
         }
+        have_time = done && timings;
     }
-    const float bfs = T.stop();
+    if (!have_time) bfs = T.stop();
     if (timings) {
         timings[IDL_T_BFS_MS] = bfs;
         timings[IDL_T_BFS_ITERS] = (float)passes;

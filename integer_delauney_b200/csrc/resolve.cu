@@ -125,11 +125,9 @@ __device__ __forceinline__ int isqrt(int32_t v)   // floor, v >= 0
 
 // A warp takes 128 columns (four per lane) by ROOT_ROWS rows, loaded at once
 // with the rows above and below; cells that their neighbours' owners rule out
-// are skipped without a seed-table load.  PASSES: also the largest A of a
-// linked cell (sc->arrive_max) for the pass count.
+// are skipped without a seed-table load.
 constexpr int ROOT_ROWS = 8;
 
-template <bool PASSES>
 __global__ void __launch_bounds__(128)
 k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
         uint32_t* __restrict__ sus, int words, int32_t* __restrict__ list, int cap, Scalars* __restrict__ sc)
@@ -155,7 +153,6 @@ k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32
     // on the segment between them, inside the owner's region.  So a root has a
     // differing neighbour both across and up or down; of those (a quarter of
     // the cells at 200 000 seeds in 4096 x 4096) the owner's direction decides.
-    int far = 0;
     unsigned maybe = 0;   // bit 4 row + column of the lane's cells
 #pragma unroll
     for (int j = 1; j <= ROOT_ROWS; ++j) {
@@ -169,7 +166,7 @@ k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32
         for (int c = 0; c < 4; ++c) {
             const int32_t s = row[c + 1];
             const bool across = row[c] != s || row[c + 2] != s, along = above[c] != s || below[c] != s;
-            if (s >= 0 && (PASSES || (across && along))) maybe |= 1u << (4 * (j - 1) + c);
+            if (s >= 0 && across && along) maybe |= 1u << (4 * (j - 1) + c);
         }
     }
     const int valid = min(max(Wd - x0, 0), 4);
@@ -202,14 +199,27 @@ k_roots(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32
             atomicOr(&sus[(size_t)y * words + (x >> 5)], 1u << (x & 31));
             const int k = atomicAdd(&sc->n_roots, 1);
             if (k < cap) list[k] = (int32_t)pack_pos(x, y);
-        } else if (PASSES) {
-            far = max(far, abs(dx) + abs(dy));
         }
     }
-    if (PASSES) {
-        far = __reduce_max_sync(FULL, far);
-        if (lane == 0) atomicMax(&sc->arrive_max, far);
-    }
+}
+
+// For the pass count: the largest A of a settled cell into sc->arrive_max.  On
+// the finished labels, of which the settled cells' are their exact owners still.
+__global__ void __launch_bounds__(256)
+k_arrivals(const int32_t* __restrict__ lab, int pitch, int Wd, int Hd, const uint32_t* __restrict__ pos,
+           const uint32_t* __restrict__ sus, int words, Scalars* __restrict__ sc)
+{
+    int far = 0;
+    for (int y = blockIdx.x; y < Hd; y += gridDim.x)
+        for (int x = threadIdx.x; x < Wd; x += 256) {
+            const int32_t l = __ldg(&lab[(size_t)y * pitch + x]);
+            const uint32_t w = __ldg(&sus[(size_t)y * words + (x >> 5)]);
+            if (l < 0 || ((w >> (x & 31)) & 1u)) continue;
+            const uint32_t p = __ldg(&pos[l]);
+            far = max(far, abs((int)pos_x(p) - x) + abs((int)pos_y(p) - y));
+        }
+    far = __reduce_max_sync(FULL, far);
+    if ((threadIdx.x & 31) == 0) atomicMax(&sc->arrive_max, far);
 }
 
 // The cells that reach their owner only through roots.  A cell is suspect
@@ -256,7 +266,6 @@ k_suspects(View V, uint32_t* sus, int32_t* list, int cap, Scalars* sc)
                 } else {
                     sc->resolve_fail = 1;
                 }
-                atomicMax(&sc->sus_far, abs(x - pos_x(p)) + abs(y - pos_y(p)));
             }
         }
     }
@@ -769,7 +778,7 @@ size_t resolve_reserve(Context& C, const Canvas& cv)
     return bits;
 }
 
-void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, bool passes, const XImg* images,
+void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, const XImg* images,
                    const int32_t* seed_img, const uint32_t* sorted, const int32_t* label)
 {
     const int words = ceil_div(cv.Wd, 32);
@@ -791,10 +800,7 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
                  sorted ? sorted : pos, sus, images,
                  seed_img, cv.pitch, cv.Wd, cv.Hd, words, whole_canvas(cv, n, 0)};
     const dim3 g((unsigned)ceil_div(cv.Wd, 128), (unsigned)ceil_div(cv.Hd, 4 * ROOT_ROWS));
-    if (passes)
-        k_roots<true><<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
-    else
-        k_roots<false><<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
+    k_roots<<<g, 128, 0, C.stream>>>(V.lab, cv.pitch, cv.Wd, cv.Hd, pos, sus, words, list, cap, C.sc());
     IDL_LAUNCH();
     const int gs = std::max(1, std::min(ceil_div(cap, 128), C.num_sms));
     k_suspects<<<gs, 128, 0, C.stream>>>(V, sus, list, cap, C.sc());
@@ -816,6 +822,14 @@ void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n,
     k_resolve_window<<<std::min(open_cap, C.num_sms), WIN_THREADS, WIN_SMEM, C.stream>>>(V, list, open, res, C.sc());
     IDL_LAUNCH();
     k_resolve_apply<<<gs, 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, list, res, C.sc());
+    IDL_LAUNCH();
+}
+
+void resolve_arrivals(Context& C, const Canvas& cv, const uint32_t* pos)
+{
+    k_arrivals<<<std::min(cv.Hd, C.num_sms * 8), 256, 0, C.stream>>>(C.lab[0].as<int32_t>(), cv.pitch, cv.Wd, cv.Hd, pos,
+                                                                    C.sus_bits.as<uint32_t>(), ceil_div(cv.Wd, 32),
+                                                                    C.sc());
     IDL_LAUNCH();
 }
 
