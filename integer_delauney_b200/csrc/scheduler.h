@@ -70,27 +70,38 @@ inline Capacity capacity(int W, int H, int64_t max_seeds, int P)
 }
 
 // Scratch a context grows to triangulate a canvas of Wd x Hd with `seeds`
-// seeds: micro-tile lists and bitmaps, hash table, work lists, triangle rows.
+// seeds, besides its label planes and the staged output: hash table and triangle
+// rows, seed arrays, the exact diagram's tables, the raster's tile lists, and the
+// micro-tile lists and bitmaps of the passes.
 inline int64_t scratch_bytes(int64_t Wd, int64_t Hd, int64_t seeds)
 {
     const int64_t n_mt = ((Wd + 7) / 8) * ((Hd + 7) / 8);
     int64_t hash = 1024;
     while (hash < 8 * seeds + 1024) hash <<= 1;
+    // raster tiles: 64 x 32, or 32 x 16 on canvases with few of those
+    int64_t tiles = ((Wd + 63) / 64) * ((Hd + 31) / 32);
+    if (tiles < 148 * 8) tiles = ((Wd + 31) / 32) * ((Hd + 15) / 16);
+    const int64_t tris = 2 * seeds + 64;
+    const int64_t lists = 4 * (130 * tiles + 8 * tris + 65536);
+    // per 64 rows and column its seeds; the suspects, listed three times
+    const int64_t exact = 16 * ((Hd + 63) / 64) * Wd + 12 * (Wd * Hd / 64 + 4096);
     // hash table (32 B a slot) and the grouping and triangle rows sized by it
-    // (24 B a slot); the tile rounds' three change bitmaps
-    return n_mt * 8 + n_mt / 4 + 16 * (Wd + Hd) + 56 * hash + 48 * seeds + Wd * Hd / 8 +
-           3 * ((Wd + 127) / 32 + 1) * 4 * Hd;
+    // (24 B a slot); the seeds' occupancy bits, their ranks and the suspects'
+    // bits; the tile rounds' three change bitmaps
+    return n_mt * 8 + n_mt / 4 + 16 * (Wd + Hd) + 56 * hash + 48 * seeds + 3 * (Wd * Hd / 8) +
+           3 * ((Wd + 127) / 32 + 1) * 4 * Hd + lists + exact;
 }
 
-// Memory one worker slot holds at most: its diagram workspace, and its batch
+// Memory one worker slot is charged: its diagram workspace, and its batch
 // context triangulating a full group (one atlas of MAX_SIDE^2 padded, its
-// label planes, raster and composed grids, seed arrays).
+// label planes, composed grids, seed arrays).  A fetched insert stages its grid
+// (12 bytes per pixel) on top of it.
 inline int64_t slot_reserve(int P)
 {
     const int64_t Wd = MAX_SIDE + 2 * P, Hd = Wd;
     const int64_t pitch = (Wd + 31) / 32 * 32;
     const int64_t px = (int64_t)MAX_SIDE * MAX_SIDE;
-    return 2 * scratch_bytes(Wd, Hd, MAX_REQUEST_SEEDS) + pitch * Hd * 8 + px * 16 + 32 * MAX_REQUEST_SEEDS;
+    return 2 * scratch_bytes(Wd, Hd, MAX_REQUEST_SEEDS) + pitch * Hd * 8 + px * 12 + 32 * MAX_REQUEST_SEEDS;
 }
 
 struct Request {

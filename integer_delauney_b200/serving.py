@@ -65,7 +65,8 @@ def _class_dims(width: int, height: int):
 def estimate_bytes(width: int, height: int, max_seeds: int, padding: int, workspace: bool = True) -> int:
     """Device footprint of a diagram: label planes, padded raster, pixel
     outputs and seed arrays, plus (``workspace``) the scratch a triangulation
-    of it grows (micro-tile lists and bitmaps, hash table, triangle rows).
+    of it grows (scratch_bytes() of csrc/scheduler.h: hash table, triangle
+    rows, tables of the exact diagram, tile lists, micro-tile lists).
     Without the workspace this is what the server charges for a fresh object
     (capacity() of csrc/scheduler.h)."""
     Wd, Hd = width + 2 * padding, height + 2 * padding
@@ -75,8 +76,13 @@ def estimate_bytes(width: int, height: int, max_seeds: int, padding: int, worksp
         return int(fixed)
     n_mt = ((Wd + 7) // 8) * ((Hd + 7) // 8)
     hash_cap = 1 << max(10, int(8 * max_seeds + 1024 - 1).bit_length())
-    work = (n_mt * 8 + n_mt // 4 + 16 * (Wd + Hd) + 56 * hash_cap + 48 * max_seeds + Wd * Hd // 8 +
-            3 * ((Wd + 127) // 32 + 1) * 4 * Hd)
+    tiles = ((Wd + 63) // 64) * ((Hd + 31) // 32)
+    if tiles < 148 * 8:
+        tiles = ((Wd + 31) // 32) * ((Hd + 15) // 16)
+    lists = 4 * (130 * tiles + 8 * (2 * max_seeds + 64) + 65536)
+    exact = 16 * ((Hd + 63) // 64) * Wd + 12 * (Wd * Hd // 64 + 4096)
+    work = (n_mt * 8 + n_mt // 4 + 16 * (Wd + Hd) + 56 * hash_cap + 48 * max_seeds + 3 * (Wd * Hd // 8) +
+            3 * ((Wd + 127) // 32 + 1) * 4 * Hd + lists + exact)
     return int(fixed + work)
 
 
@@ -88,13 +94,13 @@ MAX_REQUEST_SEEDS = 200_000
 def slot_reserve(padding: int) -> int:
     """Budget the server reserves per worker slot (slot_reserve() of
     csrc/scheduler.h): a diagram workspace, and a batch context triangulating
-    a full group (one atlas of MAX_SIDE^2 padded: label planes, raster,
-    composed grids, seed arrays)."""
+    a full group (one atlas of MAX_SIDE^2 padded: label planes, composed
+    grids, seed arrays)."""
     Wd = Hd = MAX_SIDE + 2 * padding
     pitch = (Wd + 31) // 32 * 32
     scratch = (estimate_bytes(MAX_SIDE, MAX_SIDE, MAX_REQUEST_SEEDS, padding) -
                estimate_bytes(MAX_SIDE, MAX_SIDE, MAX_REQUEST_SEEDS, padding, workspace=False))
-    return 2 * scratch + pitch * Hd * 8 + MAX_SIDE * MAX_SIDE * 16 + 32 * MAX_REQUEST_SEEDS
+    return 2 * scratch + pitch * Hd * 8 + MAX_SIDE * MAX_SIDE * 12 + 32 * MAX_REQUEST_SEEDS
 
 
 _KIND = {0: "new", 1: "insert"}

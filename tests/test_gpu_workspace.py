@@ -75,3 +75,17 @@ def test_calls_on_a_context_between_calls_of_an_object_that_borrows_it():
     assert lib.idl_get_triangles(ctx.handle, rows.ctypes.data, 200) == _capi.IDL_ERR_STATE
     del d
     ctx.close()
+
+
+@pytest.mark.parametrize("side,n", [(64, 20), (256, 300), (1024, 10000), (2048, 50000)])
+def test_estimates_cover_what_a_context_grows_to(side, n):
+    """Besides the label planes and the staged output: what the server's
+    budget and estimate_bytes charge for scratch."""
+    from integer_delauney_b200.serving import estimate_bytes
+    ctx = _capi.Context(0)
+    _triangulate(ctx, side, side, n)
+    wd = side + 32
+    planes, staged = (wd + 31) // 32 * 32 * wd * 8, side * side * 12
+    scratch = estimate_bytes(side, side, n, 16) - estimate_bytes(side, side, n, 16, workspace=False)
+    assert ctx.workspace_bytes() - planes - staged <= scratch
+    ctx.close()
