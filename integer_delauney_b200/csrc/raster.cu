@@ -33,17 +33,19 @@ namespace idl {
 namespace {
 
 // Triangles of one image to the lanes of the list kernels: `per` lanes of every
-// warp, four consecutive triangles at a time, so that the large triangles around
+// warp, eight consecutive triangles at a time, so that the large triangles around
 // one seed, consecutive by their numbers, fall to many warps (a disc of 84 000
-// seeds and five far ones: 72 + 91 us with 32 consecutive ones to a warp, 47 + 46
-// with four, 56 + 53 with eight; 28 + 17 and 30 + 17 at 200 000 uniform seeds).
-constexpr int CHUNK = 4;
+// seeds and five far ones: 72 + 91 us with 32 consecutive ones to a warp, 56 + 53
+// with eight, 47 + 46 with four).  Eight rows, and eight triangles' corners, are
+// whole 32-byte sectors; with four, 200 000 uniform seeds took 2 to 10 us more,
+// by the device.
+constexpr int LEAST = 4, CHUNK = 8;
 
 __device__ __forceinline__ long long triangle_of_lane(int per)
 {
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, chunk = per < CHUNK ? per : CHUNK;
     const long long warps = (long long)gridDim.x * 8, warp = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-    return lane < per ? (lane / CHUNK * warps + warp) * CHUNK + lane % CHUNK : 0x7FFFFFFFFFFFFFFFll;
+    return lane < per ? (lane / CHUNK * warps + warp) * chunk + lane % CHUNK : 0x7FFFFFFFFFFFFFFFll;
 }
 
 // Triangles to draw: none if there is no room for all of them, since the caller
@@ -195,7 +197,7 @@ void raster_with(Context& C, int W, int H, const int32_t* xs, const int32_t* ys,
     if (n_tri > 0) {
         // few triangles: fewer to a warp, so that every SM has some
         int per = 32;
-        while (per > CHUNK && n_tri < (int64_t)C.num_sms * 8 * per) per /= 2;
+        while (per > LEAST && n_tri < (int64_t)C.num_sms * 8 * per) per /= 2;
         const unsigned blocks = (unsigned)ceil_div(n_tri, 8 * per);
         k_raster_count<TILE><<<blocks, 256, 0, C.stream>>>(tris, C.sc(), xs, ys, W, H, w, per);
         IDL_LAUNCH();

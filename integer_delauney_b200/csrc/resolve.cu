@@ -477,10 +477,18 @@ __device__ bool never(const View& V, WarpScratch& S, int px, int py, int32_t k, 
     return true;
 }
 
+// Appends suspect i to the open ones.
+__device__ __forceinline__ void leave_open(int i, int32_t* open, int open_cap, Scalars* sc)
+{
+    const int at = atomicAdd(&sc->n_open, 1);
+    if (at < open_cap) open[at] = i;
+    else sc->resolve_fail = 1;
+}
+
 // One warp per suspect.  res[i] takes the final label, or -1 with i appended
 // to `open` (at most open_cap) for the window kernel.  The time of p's last change is at least
 // its label's L1 distance (sc->arrive_max) and at most sc->late_max.
-__global__ void __launch_bounds__(RES_WARPS * 32)
+__global__ void __launch_bounds__(RES_WARPS * 32, 4)
 k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, int32_t* __restrict__ open,
           int open_cap, Scalars* __restrict__ sc)
 {
@@ -489,18 +497,11 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
     const int lane = threadIdx.x & 31;
     if (raised(sc, lane)) return;
     const int n = sc->n_roots + sc->n_more;
-    const int first = blockIdx.x * RES_WARPS + (threadIdx.x >> 5), warps = gridDim.x * RES_WARPS;
     if (lane == 0) S.sc = sc;
-    auto leave_open = [&](int i) {
-        const int at = atomicAdd(&sc->n_open, 1);
-        if (at < open_cap) open[at] = i;
-        else sc->resolve_fail = 1;
-    };
     // More suspects than warps: those without a settled neighbour go first, since
     // too many of them end the run.
-    const bool ahead = n > warps;
-    if (ahead) {
-        for (int i = first * 32 + lane; i < n; i += warps * 32) {
+    if (n > (int)gridDim.x * RES_WARPS) {
+        for (int i = blockIdx.x * RES_WARPS * 32 + threadIdx.x; i < n; i += gridDim.x * RES_WARPS * 32) {
             const uint32_t pk = (uint32_t)list[i];
             bool settled = false;
 #pragma unroll
@@ -508,12 +509,12 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
                 const int x = (int)pos_x(pk) + (j == 0) - (j == 1), y = (int)pos_y(pk) + (j == 2) - (j == 3);
                 settled = settled || (label_at(V, x, y) >= 0 && !suspect_at(V, x, y));
             }
-            if (!settled) leave_open(i);
+            if (!settled) leave_open(i, open, open_cap, sc);
         }
         __syncwarp();
     }
-    for (int i = first; i < n; i += warps) {
-        if (ahead && raised(sc, lane)) return;
+    for (int i = blockIdx.x * RES_WARPS + (threadIdx.x >> 5); i < n; i += gridDim.x * RES_WARPS) {
+        if (n > (int)gridDim.x * RES_WARPS && raised(sc, lane)) return;
         const uint32_t pk = (uint32_t)list[i];
         const int px = pos_x(pk), py = pos_y(pk);
         const XImg b = image_of(V, label_at(V, px, py));
@@ -585,8 +586,8 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
                 const int t_lo = l1_to(V, px, py, out);
                 atomicMax(&sc->arrive_max, t_lo);
                 atomicMax(&sc->late_max, t_hi);
-            } else if (f >= 0 || !ahead) {
-                leave_open(i);
+            } else if (out >= 0 || n <= (int)gridDim.x * RES_WARPS) {   // without a settled neighbour: open already
+                leave_open(i, open, open_cap, sc);
             }
         }
         __syncwarp();
