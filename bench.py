@@ -25,9 +25,10 @@ no collective on the data path); the time is the max over ranks.
 
 `--impl reference` times the reference's own CUDA triangulate, compiled from
 its sources for sm_100a (oracle/_ref), through its stock host path on the same
-full workload, on rank 0 only (the oracle port on the host cores if that build
-is absent).  The same measurement appears on this arm's line as `ref_cuda`,
-beside `cpu_baseline` (the oracle port on all host cores: the 512 x 512 CPU
+full workload, on rank 0 only; if that build is absent, its line says
+"unavailable".  The same measurement appears on this arm's line as `ref_cuda`
+(null without the build), beside `cpu_baseline` (the oracle port on all host
+cores: the 512 x 512 CPU
 configuration measured outright, the 4096 x 4096 image extrapolated from a
 sample of assignment rows and marked so).
 """
@@ -220,32 +221,24 @@ REF_CUDA_DESC = ("the reference's own triangulate compiled from its sources for 
 
 def run_reference(args, rank, world):
     """The reference arm: the reference's own CUDA path on the full
-    4096 x 4096 / 200 000-seed workload, every step measured (no sample);
-    the oracle port on the host cores when the reference build is absent."""
+    4096 x 4096 / 200 000-seed workload, every step measured (no sample).
+    Where its build is absent there is nothing to measure, and the line says so."""
     if rank != 0:
+        return
+    import oracle
+    if not oracle.ref_available():
+        print(json.dumps({"impl": "reference",
+                          "unavailable": "the reference's CUDA code is not built here (oracle/build_ref.sh needs its "
+                                         "sources)"}), flush=True)
         return
     from integer_delauney_b200.workloads import uniform
     seeds = uniform(W, H, N_SEEDS, seed=0)
-    r = ref_cuda_baseline(seeds, args.steps, args.warmup)
-    if r is not None:
-        ms_list, n_tri = r
-        ms = statistics.median(ms_list)
-        value = W * H / (ms / 1e3) / 1e6
-        base = {"value": value, "unit": "Mpixel/s", "cores": 1, "kind": "reference",
-                "sample": f"full workload every step ({args.steps} steps); " + REF_CUDA_DESC,
-                "ms_per_call": ms_list, "triangles": n_tri}
-    else:
-        vals, secs = [], []
-        base = {}
-        for _ in range(args.warmup):
-            cpu_baseline(args.ref_rows)
-        for _ in range(args.steps):
-            base = cpu_baseline(args.ref_rows)
-            vals.append(base["value"])
-            secs.append(base["estimated_s"])
-        value = statistics.median(vals)
-        ms = statistics.median(secs) * 1e3
-        base["value"] = value
+    ms_list, n_tri = ref_cuda_baseline(seeds, args.steps, args.warmup)
+    ms = statistics.median(ms_list)
+    value = W * H / (ms / 1e3) / 1e6
+    base = {"value": value, "unit": "Mpixel/s", "cores": 1, "kind": "reference",
+            "sample": f"full workload every step ({args.steps} steps); " + REF_CUDA_DESC,
+            "ms_per_call": ms_list, "triangles": n_tri}
     line = {
         "metric": METRIC, "value": value, "unit": "Mpixel/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms, "higher_is_better": True,
