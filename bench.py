@@ -77,11 +77,10 @@ def reduce_max(value: float, world: int) -> float:
     return float(t.item())
 
 
-# dram__bytes_read.sum + dram__bytes_write.sum of the dominant stage's kernels
-# for one step of this workload (uniform seeds), from ncu --set full captures:
-# the three cell-list tile rounds (72.6 + 29.1, 72.6 + 33.2, 72.6 + 33.5 MB) and
-# the persistent kernel's tail (113.7 + 30.6 MB)
-TRAFFIC_PER_LAUNCH = {"propagate_ms": 72.6e6 + 29.1e6 + 72.6e6 + 33.2e6 + 72.6e6 + 33.5e6 + 113.7e6 + 30.6e6}
+# DRAM bytes read and written by the propagation's kernels for one step of this
+# workload (uniform seeds) by the direct schedule, from an ncu capture: k_column_off,
+# k_row_win, k_roots, k_suspects, k_resolve
+TRAFFIC_DIRECT = {"propagate_ms": 5.1e6 + 52.2e6 + 70.9e6 + 1.5e6 + 3.9e6}
 
 
 class ClockSampler:
@@ -671,8 +670,9 @@ def run_ours(args, rank, world):
     stage = {k: statistics.mean(p[k] for p in profs) for k in keys}
     p0 = profs[-1]
     hbm, peak_kind = _peaks()
-    # propagation: 8 B per cell update (4-byte label in, label out), counted
-    # by the library over the tiles the schedule actually processed
+    # propagation, counted by the library: 12 B per cell of the direct schedule
+    # (column offsets out and in, labels out and in), or 8 B per cell update of
+    # the passes (label in, label out) over the tiles they processed
     prop_bytes = statistics.mean(p["prop_bytes"] for p in profs)
     prop_gbs = prop_bytes / (stage["propagate_ms"] / 1e3) / 1e9
     canvas = p0["canvas_px"]
@@ -782,7 +782,7 @@ def run_ours(args, rank, world):
                         "tile": [p0["tile_w"], p0["tile_h"]], "steps_per_round": p0["steps_per_round"]},
         "roofline": {"bound": "hbm", "kernel": dom_kernel[:-3], "achieved": achieved, "peak": hbm,
                      "unit": "GB/s", "frac": achieved / hbm, "peak_kind": peak_kind,
-                     "traffic": TRAFFIC_PER_LAUNCH.get(dom_kernel),
+                     "traffic": TRAFFIC_DIRECT.get(dom_kernel) if schedule[0] == _capi.SCHEDULE_DIRECT else None,
                      "per_stage_gbs": {k[:-3]: v for k, v in roof.items()}},
         "clustered": {"value": value_c, "unit": "Mpixel/s", "ms_per_step": ms_c / c_steps,
                       "schedule": schedule_c, "autotune_ms": tuned_c, "passes": profs_c[-1]["passes"],

@@ -180,7 +180,7 @@ IDL_API int idl_context_set_profiling(idl_context* ctx, int enable);
 #define IDL_PROF_CANVAS_PX 12   /* detection canvas pixels */
 #define IDL_PROF_IMAGE_PX 13    /* output pixels */
 #define IDL_PROF_TRIANGLES 14
-#define IDL_PROF_PROP_BYTES 15  /* algorithmic HBM bytes of stage (a): 8 per cell update */
+#define IDL_PROF_PROP_BYTES 15  /* algorithmic HBM bytes of stage (a): 12 per cell, 8 in exact semantics, 8 per cell update of the passes */
 #define IDL_PROF_COUNT 16
 IDL_API int idl_context_last_profile(idl_context* ctx, double* out, int n);
 /* Trace of the persistent propagation kernel in the last profiled run, one

@@ -142,7 +142,7 @@ struct Profile {
     int64_t rounds = 0;           // propagation rounds launched with work
     int64_t tiles = 0;            // tiles processed over all rounds
     int64_t passes = 0;           // propagation passes (reference semantics)
-    double prop_bytes = 0;        // algorithmic HBM bytes of the propagation (8 B per cell update)
+    double prop_bytes = 0;        // algorithmic HBM bytes of the propagation
     int64_t canvas_px = 0;        // detection canvas pixels
     int64_t image_px = 0;         // output pixels
     int64_t n_triangles = 0;

@@ -782,6 +782,7 @@ size_t resolve_reserve(Context& C, const Canvas& cv)
 void resolve_exact(Context& C, const Canvas& cv, const uint32_t* pos, int64_t n, const XImg* images,
                    const int32_t* seed_img, const uint32_t* sorted, const int32_t* label)
 {
+    if (C.prof.enabled) C.prof.prop_bytes += (double)cv.Wd * cv.Hd * 4.0;   // labels in, for the roots
     const int words = ceil_div(cv.Wd, 32);
     const size_t bits = resolve_reserve(C, cv);
     // suspects: 0.02 % of the cells at the usual densities (at most 0.4 % in

@@ -65,6 +65,8 @@ def test_profiled_run(kind):
     assert direct or kind == "circle"
     if direct:   # what the profile describes is the run that was asked for
         assert p["rounds"] == 2 and p["tiles"] == 0
+        # column offsets out and in, labels out, and in again for the roots
+        assert p["prop_bytes"] == 12 * (W + 2 * P) * (H + 2 * P)
     assert all(p[k] > 0 for k in ("seeds_ms", "propagate_ms", "detect_ms", "dedup_ms", "assign_ms"))
     ctx.close()
 
