@@ -10,16 +10,16 @@
 // own (x asc, y asc) order, so within an image the id order -- the Jacobi tie
 // rule, the block rule's lowest-id tie-break and the canonical triangle rank --
 // is the single-image order shifted by a constant.  Then:
-//   * one persistent launch propagates every image (the micro-tile work list
-//     of the sparse kernel is the packed tile queue: images that converge
-//     early drop out of it, images that need many passes keep only their
-//     own active micro-tiles in it);
+//   * the exact diagram's column and row pass run over all images at once, each
+//     image kept within its own canvas, and one resolve over the atlas turns it
+//     into the reference's fixed point (an explicit schedule, or what the resolve
+//     leaves open, runs the passes over the atlas instead);
 //   * one detection + dedup + numbering over the atlas; canonical global
 //     ranks group by image (ids are contiguous per image), so an image's
 //     triangle ids are the global ranks minus the count of earlier images';
-//   * one raster launch over all triangles, each clipped to its own image with
+//   * one set of tile lists over all triangles, each clipped to its own image with
 //     its own image's degenerate-case window (per-image longest side);
-//   * one composition launch writing every image's (H, W, 3) grid.
+//   * one launch draws every tile and writes the images' (H, W, 3) grids.
 // The number of launches and host synchronisations is independent of the
 // number of images.
 #include "raster.cuh"

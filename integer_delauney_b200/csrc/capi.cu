@@ -344,8 +344,8 @@ int64_t run_triangulate(Context& C, int W, int H, int64_t n, const int32_t* vgri
         deliver(cv);
         C.fetch_scalars();
     };
-    // Everything goes out before anything is read back; one wait at the end
-    // tells whether the bounds held and whether the exact diagram decided the
+    // Everything after the seeds' check goes out before anything is read back; one
+    // wait at the end tells whether the bounds held and whether the exact diagram decided the
     // labels.  What failed is run again, each time with room for what is known
     // by then (more triangles than `bound`, as a caller's grid can hold, are not
     // drawn in vain).

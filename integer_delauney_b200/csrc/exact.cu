@@ -15,12 +15,12 @@
 // different columns at equal distance are ordered by column, i.e. by id.
 // Seed ids are (x asc, y asc) ranks, so "higher id" is a comparison of ids.
 //
-// Measured at 4096 x 4096 / 200 000 uniform seeds (B200): column pass 30 us
-// (two bytes per cell written, bound by the walk's loads), row pass 137 us
-// (bound by instruction issue: 84 % of cycles); with a four-byte id and a
+// Measured at 4096 x 4096 / 200 000 uniform seeds (B200): column pass 31 us
+// (two bytes per cell and a table entry per 64 written, 57 % issue), row pass
+// 129 us (bound by instruction issue: 85 % of cycles); with a four-byte id and a
 // four-byte distance plane and a merged hull per row they took 39 + 9 us and
-// 217 us.  With 200 000 clustered seeds 45 and 131 us against 45 + 10 and
-// 249 us; the rows of 512 batch images 0.71 ms against 2.8 ms.
+// 217 us.  With 200 000 clustered seeds 35 and 110 us against 45 + 10 and
+// 249 us; the rows of 512 batch images 0.68 ms against 2.8 ms.
 #include "context.cuh"
 #include "exact_pass.cuh"
 

@@ -9,8 +9,8 @@
 // the mapping of lanes to rows and pixels: 105 to 150 us at 4096 x 4096 /
 // 200 000 seeds, 770 to 890 us for the 59 M pixels of 512 batch images.  With
 // the lists a tile's block also writes the (H, W, 3) output from shared memory,
-// so the ids never make a trip through HBM: lists 28 + 19 us, drawing and
-// output 95 us, where raster and composition took 132 + 74; 180 + 442 us for
+// so the ids never make a trip through HBM: lists 29 + 17 us, drawing and
+// output 93 us, where raster and composition took 132 + 74; 176 + 436 us for
 // the batch.  The drawing is bound by instruction issue (about 70 % of cycles).
 #pragma once
 

@@ -53,15 +53,19 @@
 //      caller runs the pass-by-pass propagation instead; the kernels that
 //      follow, and what is left of the one at work, then end at once.
 //
-// Rules (1) and (2) are checked against the iteration on uniform, clustered,
-// lattice, line and circle seed sets by the tests, on the CPU and the GPU.
+// The kernels' results are checked against the iteration on uniform, clustered,
+// lattice, line and circle seed sets by the GPU tests.
 //
 // Cost at 4096 x 4096, 200 000 uniform seeds: one read of the label plane for
-// the roots (39 us, bound by the latency of its loads), the suspects 12 us, their
-// decisions 30 us (a chain of dependent loads per suspect, 3 034 of them), the
-// writes 4 us.  With the exact diagram's 167 us that is 0.30 ms of
-// propagation; the 51 passes took 1.18 ms.  With 200 000 clustered seeds
-// 0.34 ms, the 1 100 passes 7.8 ms.
+// the roots (37 us, bound by the latency of its loads), the suspects 8 us, their
+// decisions 42 us (a chain of dependent loads per suspect, 3 034 of them; 34 us
+// in the first run on cold caches, the worst suspect's chain decides), the rest
+// 6 us.  With the exact diagram's 160 us that is 0.25 ms of propagation; the 51
+// passes took 1.18 ms.  With 200 000 clustered seeds 0.27 ms, the 1 100 passes
+// 7.8 ms.
+// Where the passes have to run after all, the attempt comes on top of them: 3 to
+// 18 % of a call (seeds on circles, a spiral, a parabola of 2 048 x 2 048), most
+// of it the decisions of the cells that could be decided.
 #include "context.cuh"
 #include "exact_pass.cuh"
 #include "stencil.cuh"
@@ -275,12 +279,17 @@ k_suspects(View V, uint32_t* sus, int32_t* list, int cap, Scalars* sc)
 
 constexpr int RES_WARPS = 4;
 constexpr int MAX_CAND = 16;    // candidates of one suspect, rivals at one cell (2 at most at the sizes above)
-constexpr int MAX_SEARCH = 64;  // cells of a "no" search
+// Cells of a "no" search: 32, 64 and 128 take the same time and leave the same
+// cells open on every set measured.  The first, short one is not sharp either: 8,
+// 16 and 32 cells 72, 76 and 83 us at 200 000 clustered seeds, 855, 882 and 937
+// between lines of seeds.
+constexpr int MAX_SEARCH = 64;
 constexpr int SHORT_SEARCH = 16;
 constexpr int MAX_FRONT = 4;    // line cells per step (2 are reached)
-// Disc columns (in warp strides) a suspect may look at: a few thousand are
-// reached with clustered seeds; beyond it the suspect stays undecided, so that
-// no seed set makes a warp run long.
+// Disc columns (in warp strides) a suspect may look at: 1 600 are reached with
+// clustered seeds, 10 536 between lines of seeds across 4096 x 4096 (all decided;
+// with 2^12 they would run the passes, 2^16 costs the same); beyond it the suspect
+// stays undecided, so that no seed set makes a warp run long: 4 ms.
 constexpr int BUDGET = 1 << 14;
 constexpr int LONG_SPENT = 256;
 
@@ -365,7 +374,7 @@ __device__ __forceinline__ int rivals(const View& V, WarpScratch& S, int x, int 
     if (lane == 0) {
         S.n_rival = 0;
         S.budget -= 1 + (isqrt(d) >> 4);
-        // a long decision (3 % of them with clustered seeds) ends with the others
+        // a long decision (1 % of them with clustered seeds) ends with the others
         if (S.budget < BUDGET - LONG_SPENT && __ldcg(&S.sc->resolve_fail)) S.budget = -1;
     }
     __syncwarp();

@@ -269,8 +269,13 @@ static_assert(RR == 16 && MT == 8 && RK == MT / 2, "lane layout: 16 rows of two 
 constexpr int BK = 12;
 constexpr int BR = MT + 2 * BK;
 static_assert(BR == 32 && SJ_THREADS == BR * BR, "one thread per cell, one warp per region row");
-constexpr int BLOCK_BELOW = 384;    // list length from which a round's next list is one for block rounds
-constexpr int BLOCK_LIMIT = 1536;   // and above which such a list is run in ordinary rounds again
+// List length from which a round's next list is one for block rounds, and above
+// which such a list is run in ordinary rounds again.  Neither is sharp: ten
+// inserts of 1 000 seeds into 2 048 x 2 048 take 1 309, 1 299 and 1 297 us from 192,
+// 384 and 768 on, six of 500 into 1 024 x 1 024 1 023, 1 043 and 1 079; with limits
+// of 768, 1 536 and 3 072 1 299, 1 299 and 1 300 us.
+constexpr int BLOCK_BELOW = 384;
+constexpr int BLOCK_LIMIT = 1536;
 
 // Lists the micro-tile itself and, if any inner cell changed in the round's
 // last pass (columns x0..x1, rows y0..y1 of the micro-tile bound them), the
