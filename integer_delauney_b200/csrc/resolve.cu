@@ -58,10 +58,9 @@
 //
 // Cost at 4096 x 4096, 200 000 uniform seeds: one read of the label plane for
 // the roots (37 us, bound by the latency of its loads), the suspects 8 us, their
-// decisions 42 us (a chain of dependent loads per suspect, 3 034 of them; 34 us
-// in the first run on cold caches, the worst suspect's chain decides), the rest
-// 6 us.  With the exact diagram's 160 us that is 0.25 ms of propagation; the 51
-// passes took 1.18 ms.  With 200 000 clustered seeds 0.27 ms, the 1 100 passes
+// decisions 28 to 42 us (a chain of dependent loads per suspect, 3 034 of them;
+// the worst one's decides), the rest 6 us.  With the exact diagram's 160 us that is 0.25 ms of propagation; the 51
+// passes took 1.18 ms.  With 200 000 clustered seeds 0.28 ms, the 1 100 passes
 // 7.8 ms.
 // Where the passes have to run after all, the attempt comes on top of them: 3 to
 // 18 % of a call (seeds on circles, a spiral, a parabola of 2 048 x 2 048), most
@@ -504,8 +503,8 @@ k_resolve(View V, const int32_t* __restrict__ list, int32_t* __restrict__ res, i
     __shared__ WarpScratch scratch[RES_WARPS];
     WarpScratch& S = scratch[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
-    if (raised(sc, lane)) return;
     const int n = sc->n_roots + sc->n_more;
+    if (__any_sync(FULL, sc->resolve_fail)) return;   // read with the counts
     if (lane == 0) S.sc = sc;
     // More suspects than warps: those without a settled neighbour go first, since
     // too many of them end the run.
