@@ -35,8 +35,8 @@ namespace {
 // Triangles of one image to the lanes of the list kernels: `per` lanes of every
 // warp, eight consecutive triangles at a time, so that the large triangles around
 // one seed, consecutive by their numbers, fall to many warps (a disc of 84 000
-// seeds and five far ones: 72 + 91 us with 32 consecutive ones to a warp, 56 + 53
-// with eight, 47 + 46 with four).  Eight rows, and eight triangles' corners, are
+// seeds and five far ones, an atomic each: 72 + 91 us with 32 consecutive ones to
+// a warp, 56 + 53 with eight, 47 + 46 with four).  Eight rows, and eight triangles' corners, are
 // whole 32-byte sectors; with four, 200 000 uniform seeds took 2 to 10 us more,
 // by the device.
 constexpr int LEAST = 4, CHUNK = 8;

@@ -9,8 +9,8 @@
 // the mapping of lanes to rows and pixels: 105 to 150 us at 4096 x 4096 /
 // 200 000 seeds, 770 to 890 us for the 59 M pixels of 512 batch images.  With
 // the lists a tile's block also writes the (H, W, 3) output from shared memory,
-// so the ids never make a trip through HBM: lists 29 + 17 us, drawing and
-// output 93 us, where raster and composition took 132 + 74; 176 + 436 us for
+// so the ids never make a trip through HBM: lists 26 + 13 us, drawing and
+// output 93 us, where raster and composition took 132 + 74; 124 + 436 us for
 // the batch.  The drawing is bound by instruction issue (about 70 % of cycles).
 #pragma once
 
@@ -130,17 +130,19 @@ __device__ __forceinline__ int warp_prefix(int v)
 }
 
 // The tiles of a W x H image (tiles_x to a row, the first one tile_off) that a
-// proper triangle's pixels can lie in: f(t, tile).  A box of a few tiles is
-// taken whole, by its lane.  In a larger one each tile row takes the columns the
+// proper triangle's pixels can lie in: together(on, t, tile) by all lanes at once
+// for the first tile of the smaller boxes, alone(t, tile) for every other.  A box
+// of a few tiles is taken whole, by its lane.  In a larger one each tile row takes the columns the
 // triangle spans there (its extent in a slab is reached at the slab's ends or at
 // a vertex); a warp works off the tile rows of its larger triangles 32 at a
 // time, then the tiles of those rows 32 at a time: slivers across the image are
-// hundreds of tiles each, and f waits for memory (one triangle after another,
+// hundreds of tiles each, and alone() waits for memory (one triangle after another,
 // 88 seeds 64 pixels apart took 23 + 36 us to list, now 5 + 4; slivers from side
-// to side of 2048 x 2048 106 us to count, now 8).  Every lane of the warp calls it; on: the lane brings triangle u, number t, of a W x H image.
-template <class TILE, class F>
+// to side of 2048 x 2048 106 us to count, now 8).  Every lane of the warp calls
+// it; on: the lane brings triangle u, number t, of a W x H image.
+template <class TILE, class F, class G>
 __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int W, int H, int tile_off, int tiles_x,
-                                          F&& f)
+                                          F&& together, G&& alone)
 {
     const int lane = threadIdx.x & 31;
     const int x0 = max(0, min(u.x[0], min(u.x[1], u.x[2]))), x1 = min(W - 1, max(u.x[0], max(u.x[1], u.x[2])));
@@ -148,9 +150,10 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
     on = on && x0 <= x1 && y0 <= y1;
     const int tx0 = x0 / TILE::W, tx1 = x1 / TILE::W, ty0 = y0 / TILE::H, ty1 = y1 / TILE::H;
     const bool few = on && (tx1 - tx0 + 1) * (ty1 - ty0 + 1) <= TILE_FEW;
+    together(few, t, tile_off + ty0 * tiles_x + tx0);
     if (few)
         for (int ty = ty0; ty <= ty1; ++ty)
-            for (int tx = tx0; tx <= tx1; ++tx) f(t, tile_off + ty * tiles_x + tx);
+            for (int tx = tx0 + (ty == ty0); tx <= tx1; ++tx) alone(t, tile_off + ty * tiles_x + tx);
     __syncwarp();
     const int rows = on && !few ? ty1 - ty0 + 1 : 0;
     if (!__any_sync(0xFFFFFFFFu, rows > 0)) return;
@@ -194,7 +197,7 @@ __device__ __forceinline__ void tri_tiles(bool on, const Tri& u, int32_t t, int 
             const int e = e0 + lane, from = min(lane_of(tiles_incl, e), 31);
             const int32_t of = __shfl_sync(0xFFFFFFFFu, id, from);
             const int tile = e + __shfl_sync(0xFFFFFFFFu, first_tile, from);
-            if (e < all) f(of, tile);
+            if (e < all) alone(of, tile);
         }
     }
 }
@@ -306,6 +309,18 @@ __device__ __forceinline__ Tri unpack_tri(const uint32_t* __restrict__ xy, int32
     return u;
 }
 
+// The lanes of the warp that list a triangle at the same tile as this one (on:
+// this one does).  One atomic serves them all: consecutive triangles mostly start
+// in the same tile, and with a thousand atomics on each counter 2.8 M triangles of
+// 2048 x 2048 took 142 to 269 us to count (by where the counters lay in memory) and
+// 128 to 263 to list, now 96 and 39; a disc of 84 000 seeds and five far ones 54 and
+// 53, now 22 and 20.  For the first tile only: the others are different more often,
+// which is what the match pays for.
+__device__ __forceinline__ unsigned lanes_of_tile(bool on, int tile)
+{
+    return __match_any_sync(0xFFFFFFFFu, on ? tile : -1);   // slower the more different values there are
+}
+
 // Count pass, one triangle per lane (on: there is one): its packed corners, and
 // one for each tile it meets (collinear ones are listed apart).
 template <class TILE>
@@ -317,8 +332,10 @@ __device__ __forceinline__ void raster_count(const RasterWork& w, bool on, int32
         for (int k = 0; k < 3; ++k) w.xy[(size_t)t * 3 + k] = u.line ? 0xFFFFFFFFu : pack_pos(u.x[k], u.y[k]);
         if (u.line) w.lines[atomicAdd(&w.head->n_lines, 1)] = t;
     }
-    tri_tiles<TILE>(on && !u.line, u, t, W, H, tile_off, tiles_x,
-              [&](int32_t, int tile) { atomicAdd(&w.count[tile], 1); });
+    tri_tiles<TILE>(on && !u.line, u, t, W, H, tile_off, tiles_x, [&](bool has, int32_t, int tile) {
+        const unsigned same = lanes_of_tile(has, tile);
+        if (has && (threadIdx.x & 31) == __ffs(same) - 1) atomicAdd(&w.count[tile], __popc(same));
+    }, [&](int32_t, int tile) { atomicAdd(&w.count[tile], 1); });
 }
 
 // The last block of the count pass turns the counts into list offsets.  Every
@@ -388,9 +405,14 @@ __device__ __forceinline__ void raster_fill(const RasterWork& w, bool on, int32_
         on = w.xy[(size_t)t * 3] != 0xFFFFFFFFu;
         if (on) u = unpack_tri(w.xy, t);
     }
-    tri_tiles<TILE>(on, u, t, W, H, tile_off, tiles_x, [&](int32_t id, int tile) {
-        w.list[w.off[tile] + atomicSub(&w.count[tile], 1) - 1] = id;
-    });
+    tri_tiles<TILE>(on, u, t, W, H, tile_off, tiles_x, [&](bool has, int32_t id, int tile) {
+        const unsigned same = lanes_of_tile(has, tile);
+        const int lane = threadIdx.x & 31, first = __ffs(same) - 1;
+        int left = 0;
+        if (has && lane == first) left = w.off[tile] + atomicSub(&w.count[tile], __popc(same));
+        left = __shfl_sync(0xFFFFFFFFu, left, has ? first : lane);
+        if (has) w.list[left - 1 - __popc(same & ((1u << lane) - 1u))] = id;
+    }, [&](int32_t id, int tile) { w.list[w.off[tile] + atomicSub(&w.count[tile], 1) - 1] = id; });
 }
 
 // One tile of a W x H image, by a block: pix[TILE::H * TILE::PITCH] takes the
