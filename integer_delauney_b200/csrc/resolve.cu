@@ -59,11 +59,11 @@
 // Cost at 4096 x 4096, 200 000 uniform seeds: one read of the label plane for
 // the roots (37 us, bound by the latency of its loads), the suspects 8 us, their
 // decisions 28 to 42 us (a chain of dependent loads per suspect, 3 034 of them;
-// the worst one's decides), the rest 6 us.  With the exact diagram's 160 us that is 0.25 ms of propagation; the 51
-// passes took 1.18 ms.  With 200 000 clustered seeds 0.28 ms, the 1 100 passes
-// 7.8 ms.
-// Where the passes have to run after all, the attempt comes on top of them: 3 to
-// 18 % of a call (seeds on circles, a spiral, a parabola of 2 048 x 2 048), most
+// the worst one's decides), the rest 6 us.  With the exact diagram's 160 us that
+// is 0.25 ms of propagation; the 51 passes took 1.18 ms.  With 200 000 clustered
+// seeds 0.28 ms, the 1 100 passes 7.8 ms.
+// Where the passes have to run after all, the attempt comes on top of them: 2 to
+// 14 % of a call (seeds on circles, a spiral, a parabola of 2 048 x 2 048), most
 // of it the decisions of the cells that could be decided.
 #include "context.cuh"
 #include "exact_pass.cuh"
